@@ -35,7 +35,7 @@
 extern "C" {
 #endif
 
-#define FA_B200_ABI_VERSION 4
+#define FA_B200_ABI_VERSION 5
 
 /* argument errors (negative return values) */
 #define FA_B200_OK                 0
@@ -274,6 +274,63 @@ typedef struct fa_b200_linear_small_params {
 } fa_b200_linear_small_params;
 
 int fa_b200_linear_small(const fa_b200_linear_small_params* p);
+
+/* One generation step of a GPT-2 model in one launch: token + position embedding, every transformer
+ * block (LayerNorm, QKV, attention over the K/V caches with the new row appended, output projection,
+ * LayerNorm, MLP with tanh-GELU), final LayerNorm and vocabulary head, for one new token of each of
+ * B <= 8 sequences.  The reference's GPTModel.forward (src/py/model_inference.py:149-190) for a single
+ * position with the earlier keys and values cached.
+ *
+ * Head dimension 64, so the width is C = 64 * H <= 1600; B * H <= 256; at most 64 layers.  All weights are bf16 in
+ * torch.nn.Linear's layout, dense and 16-byte aligned.  `layers` is DEVICE memory holding `n_layers`
+ * records of device pointers (qkv_b may be NULL); the weights of the three projections are one
+ * [3C, C] matrix.  k_cache / v_cache are host arrays of n_layers device pointers to caches of
+ * logical shape [B, cache_rows, H, 64] with the element strides cache_strides = {sequence, row, head}
+ * (multiples of 8), the same for all; row `pos` is written.
+ *
+ * The position is `pos`, or, when pos_device is set, the int64 there, read when the kernel runs (it
+ * is clamped to the cache and to the position table); with `advance` the kernel then stores the next
+ * position there and the next position + 1 in the int32 at length_device (may be NULL).
+ * `logits` [B, vocab] bf16; `next_ids`, when not NULL, receives each row's argmax (lowest index among
+ * equals) as B int64 next_stride apart; it may be the next column of the matrix that `ids` is a
+ * column of.
+ *
+ * `workspace` must be zeroed once before its first use and again after a watchdog code; it belongs to
+ * one launch at a time.  The launch is cooperative.  Asynchronous on p->stream, capturable. */
+typedef struct fa_b200_gpt_layer {
+  const void *ln1_scale, *ln1_shift, *qkv_w, *qkv_b, *proj_w, *proj_b;
+  const void *ln2_scale, *ln2_shift, *fc_w, *fc_b, *out_w, *out_b;
+} fa_b200_gpt_layer;
+
+typedef struct fa_b200_gpt_step_params {
+  const fa_b200_gpt_layer* layers;   /* device memory */
+  const void* tok_emb;               /* [vocab, C] */
+  const void* pos_emb;               /* [n_positions, C] */
+  const void* lnf_scale;
+  const void* lnf_shift;
+  const void* head_w;                /* [vocab, C] */
+  const int64_t* ids;                /* device, B token ids ids_stride apart */
+  int64_t ids_stride;
+  int64_t* pos_device;               /* or NULL */
+  int32_t* length_device;            /* or NULL */
+  void* const* k_cache;              /* host array of n_layers device pointers */
+  void* const* v_cache;
+  int64_t cache_strides[3];
+  void* logits;
+  int64_t* next_ids;                 /* or NULL */
+  int64_t next_stride;
+  void* workspace;
+  int64_t workspace_bytes;
+  int32_t n_layers, B, H, vocab, cache_rows, n_positions;
+  int32_t pos, advance;
+  float eps;
+  int32_t device;
+  void* stream;
+} fa_b200_gpt_step_params;
+
+/* Bytes of workspace for B sequences of a model with H heads (negative: an argument error). */
+int64_t fa_b200_gpt_step_workspace_bytes(int32_t B, int32_t H);
+int fa_b200_gpt_step(const fa_b200_gpt_step_params* p);
 
 /* FA_B200_ABI_VERSION the library was built with. */
 int fa_b200_abi_version(void);

@@ -1,0 +1,116 @@
+"""The one-launch generation step (fa_b200_gpt_step, csrc/gpt_step_sm100.cuh) against the same model
+evaluated in fp32 with the reference's standard-PyTorch attention.
+
+Tolerance: the kernel rounds activations to bf16 about eight times per layer (LayerNorm outputs, q,
+k, v, attention output, hidden row, and the stream where it is normalised) and the logits once.  Each
+rounding adds at most 2^-9 of the value it rounds; treated as independent, the relative error of the
+logits (2-norm) stays below 2^-9 * sqrt(8 L + 4), taken twice."""
+import math
+
+import pytest
+import torch
+
+from tfg_flashattention_b200 import gpt2
+
+pytestmark = pytest.mark.gpu
+
+
+def _model(width, heads, layers, vocab, context, qkv_bias=True, seed=3):
+    cfg = {"vocab_size": vocab, "context_length": context, "emb_dim": width, "n_heads": heads, "n_layers": layers,
+           "drop_rate": 0.0, "qkv_bias": qkv_bias, "impl_type": "cuda"}
+    torch.manual_seed(seed)
+    model = gpt2.GPTModel(cfg, dtype=torch.bfloat16)
+    with torch.no_grad():
+        for name, p in model.named_parameters():
+            if name.endswith(".scale"):
+                p.copy_(1 + 0.2 * torch.randn(p.shape))
+            elif name.endswith("emb.weight"):
+                p.copy_(torch.randn(p.shape))
+            elif p.dim() == 2:
+                p.copy_(torch.randn(p.shape) / math.sqrt(p.shape[1]))
+            else:
+                p.copy_(0.3 * torch.randn(p.shape))
+    exact = gpt2.GPTModel(dict(cfg, impl_type="manual"))
+    exact.load_state_dict(model.state_dict())
+    model = model.cuda().eval().prepare_for_inference()
+    assert model._step_plan is not None
+    return model, exact.cuda().eval()
+
+
+def _check(model, exact, B, pos, seed=0, **kw):
+    """One step at position `pos` behind `pos` cached rows of the exact model (rounded to bf16)."""
+    cfg = model.cfg
+    ids = torch.randint(0, cfg["vocab_size"], (B, pos + 1), generator=torch.Generator().manual_seed(seed)).cuda()
+    caches = model.allocate_kv_cache(B, pos + 2)
+    wide = [tuple(t.float() for t in pair) for pair in caches]
+    with torch.no_grad():
+        if pos:
+            exact(ids[:, :pos], kv_caches=wide, pos=0)
+            for (k, v), (kw_, vw) in zip(caches, wide):
+                k.copy_(kw_)
+                v.copy_(vw)
+                kw_.copy_(k)
+                vw.copy_(v)
+        want = exact(ids[:, pos:], kv_caches=wide, pos=pos)
+        before = [tuple(t.clone() for t in pair) for pair in caches]
+        nxt = torch.full((B, 3), -1, dtype=torch.long, device="cuda")
+        got = model._step(ids[:, pos:], caches, pos, next_ids=nxt[:, 1])
+    from tfg_flashattention_b200 import custom_flash_attn
+    assert custom_flash_attn.last_status() == 0
+    assert got is not None and got.shape == want.shape
+    L = cfg["n_layers"]
+    bound = 2 * 2.0 ** -9 * math.sqrt(8 * L + 4)
+    rel = ((got.float() - want).norm() / want.norm()).item()
+    assert rel <= bound, (rel, bound)
+    # the argmax is that of the logits themselves; the columns beside it are not touched
+    assert torch.equal(nxt[:, 1], got[:, 0].float().argmax(-1)) and (nxt[:, ::2] == -1).all()
+    for (k, v), (kw_, vw), (k0, v0) in zip(caches, wide, before):
+        for new, ref, old in ((k, kw_, k0), (v, vw, v0)):
+            assert ((new[:, pos].float() - ref[:, pos]).norm() / ref[:, pos].norm()).item() <= bound
+            keep = torch.arange(new.shape[1], device="cuda") != pos
+            assert torch.equal(new[:, keep], old[:, keep])               # nothing else is written
+    return caches, ids, got
+
+
+@pytest.mark.parametrize("width,heads,layers,vocab,B,pos,bias", [
+    (64, 1, 2, 97, 1, 0, True),          # no cached rows; fewer rows of W than CTAs
+    (64, 1, 1, 97, 8, 1, True),
+    (320, 5, 2, 503, 3, 15, False),      # 10 columns units: warps without work; no QKV bias
+    (768, 12, 2, 1001, 1, 16, True),     # one chunk per row
+    (768, 12, 1, 1001, 5, 95, True),     # cached rows: one stage less one, ...
+    (1024, 16, 1, 1001, 2, 96, True),    # ... exactly one, ...
+    (1280, 20, 1, 1001, 4, 97, True),    # ... and one row into the second
+    (1600, 25, 2, 50257, 8, 130, True),  # two attention units in some CTAs; the widest model
+])
+def test_step_matches_fp32(fa_lib, width, heads, layers, vocab, B, pos, bias):
+    _check(*_model(width, heads, layers, vocab, 256, bias), B, pos)
+
+
+@pytest.mark.parametrize("B,heads,pos", [(1, 1, 2047), (1, 1, 2048), (2, 2, 5000)])
+def test_step_long_cache_is_split_over_ctas(fa_lib, B, heads, pos):
+    _check(*_model(64 * heads, heads, 1, 211, pos + 8), B, pos)
+
+
+def test_step_advances_a_device_position_and_repeats_bit_for_bit(fa_lib):
+    model, exact = _model(256, 4, 2, 503, 64)
+    caches, ids, first = _check(model, exact, 2, 20)
+    position = gpt2.DevicePosition(torch.device("cuda", torch.cuda.current_device()))
+    position.set(20)
+    for _ in range(3):
+        position.set(20)
+        again = model._step(ids[:, 20:], caches, position, advance=True)
+        assert torch.equal(again, first)
+        assert position.index.item() == 21 and position.length.item() == 22
+    # a replaced parameter is seen: the table is rebuilt
+    model.trf_blocks[0].ff.layers[0].bias = torch.nn.Parameter(model.trf_blocks[0].ff.layers[0].bias + 1)
+    assert not torch.equal(model._step(ids[:, 20:], caches, 20), first)
+
+
+def test_step_declines_what_it_does_not_take(fa_lib):
+    model, _ = _model(256, 4, 1, 503, 64)
+    ids = torch.zeros(2, 1, dtype=torch.long, device="cuda")
+    caches = model.allocate_kv_cache(2, 32)
+    assert model._step(ids, caches, 31) is not None
+    assert model._step(ids, caches, 32) is None                              # past the cache
+    assert model._step(ids, model.allocate_kv_cache(2, 32, dtype=torch.float32), 3) is None
+    assert model._step(torch.zeros(9, 1, dtype=torch.long, device="cuda"), model.allocate_kv_cache(9, 32), 3) is None

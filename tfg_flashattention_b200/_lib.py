@@ -10,7 +10,7 @@ import os
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libfa_b200.so")
 
-ABI_VERSION = 4
+ABI_VERSION = 5
 
 
 class FaParams(ctypes.Structure):
@@ -62,9 +62,26 @@ class FaLinearSmallParams(ctypes.Structure):
     ]
 
 
+class FaGptStepParams(ctypes.Structure):
+    """struct fa_b200_gpt_step_params (include/fa_b200.h)."""
+    _fields_ = [
+        ("layers", ctypes.c_void_p), ("tok_emb", ctypes.c_void_p), ("pos_emb", ctypes.c_void_p),
+        ("lnf_scale", ctypes.c_void_p), ("lnf_shift", ctypes.c_void_p), ("head_w", ctypes.c_void_p),
+        ("ids", ctypes.c_void_p), ("ids_stride", ctypes.c_int64),
+        ("pos_device", ctypes.c_void_p), ("length_device", ctypes.c_void_p),
+        ("k_cache", ctypes.c_void_p), ("v_cache", ctypes.c_void_p), ("cache_strides", ctypes.c_int64 * 3),
+        ("logits", ctypes.c_void_p), ("next_ids", ctypes.c_void_p), ("next_stride", ctypes.c_int64),
+        ("workspace", ctypes.c_void_p), ("workspace_bytes", ctypes.c_int64),
+        ("n_layers", ctypes.c_int32), ("B", ctypes.c_int32), ("H", ctypes.c_int32), ("vocab", ctypes.c_int32),
+        ("cache_rows", ctypes.c_int32), ("n_positions", ctypes.c_int32),
+        ("pos", ctypes.c_int32), ("advance", ctypes.c_int32), ("eps", ctypes.c_float),
+        ("device", ctypes.c_int32), ("stream", ctypes.c_void_p),
+    ]
+
+
 EXPORTS = ("fa_b200_fwd", "fa_b200_fwd_plan", "fa_b200_validate", "fa_b200_strerror", "fa_b200_device_ok",
            "fa_b200_last_status", "fa_b200_abi_version", "fa_b200_decode", "fa_b200_decode_workspace_bytes", "fa_b200_decode_static",
-           "fa_b200_add_layernorm", "fa_b200_linear_small")
+           "fa_b200_add_layernorm", "fa_b200_linear_small", "fa_b200_gpt_step", "fa_b200_gpt_step_workspace_bytes")
 
 SCHEDULES = {-1: "none", 0: "cta_per_tile", 1: "persistent_paired", 2: "persistent_rotated",
              3: "persistent_full"}
@@ -109,6 +126,10 @@ def load() -> ctypes.CDLL:
     lib.fa_b200_add_layernorm.restype = ctypes.c_int
     lib.fa_b200_linear_small.argtypes = [ctypes.POINTER(FaLinearSmallParams)]
     lib.fa_b200_linear_small.restype = ctypes.c_int
+    lib.fa_b200_gpt_step.argtypes = [ctypes.POINTER(FaGptStepParams)]
+    lib.fa_b200_gpt_step.restype = ctypes.c_int
+    lib.fa_b200_gpt_step_workspace_bytes.argtypes = [ctypes.c_int32, ctypes.c_int32]
+    lib.fa_b200_gpt_step_workspace_bytes.restype = ctypes.c_int64
     lib.fa_b200_abi_version.argtypes = []
     lib.fa_b200_abi_version.restype = ctypes.c_int
     if lib.fa_b200_abi_version() != ABI_VERSION:

@@ -14,6 +14,7 @@
 #include "add_layernorm_sm100.cuh"
 #include "fa_decode_sm100.cuh"
 #include "fa_fwd_sm100.cuh"
+#include "gpt_step_sm100.cuh"
 #include "linear_small_sm100.cuh"
 
 namespace {
@@ -715,6 +716,152 @@ int fa_b200_linear_small(const fa_b200_linear_small_params* p) {
   return static_cast<int>(e);
 }
 
+// ------------------------------------------------------------------------- generation step
+namespace {
+
+constexpr int kStepMaxGrid = 160;      // CTAs, one per SM
+std::once_flag g_step_once[kMaxDevices];
+int g_step_error[kMaxDevices];
+
+void step_init(int dev) {   // with `dev` current
+  cudaFuncAttributes attr;
+  cudaError_t e = cudaFuncGetAttributes(&attr, reinterpret_cast<const void*>(&fa::fa_gpt_step_kernel));
+  if (e != cudaSuccess) { g_step_error[dev] = static_cast<int>(e); return; }
+  if (attr.numRegs != fa::kStepLaunchRegs) { g_step_error[dev] = FA_B200_ERR_BUILD; return; }
+  e = cudaFuncSetAttribute(reinterpret_cast<const void*>(&fa::fa_gpt_step_kernel),
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, fa::kStepSmemBytes);
+  g_step_error[dev] = static_cast<int>(e);
+}
+
+// Byte offsets of the workspace's parts, for `B` sequences of `H` heads.
+struct StepWorkspace {
+  int64_t best, arrived, x_att, x_mlp, qkv, ctx, h, part_ml, part_o, bytes;
+  StepWorkspace(int B, int H) {
+    const int64_t words = 8LL * 64 * H * 4, pairs = static_cast<int64_t>(B) * H;   // [8, C] exchange words
+    const int64_t partials = pairs > kStepMaxGrid ? pairs : kStepMaxGrid;          // pairs * splits <= grid where split
+    best = 128;                                                  // in front: generation, done
+    arrived = best + 128;
+    x_att = arrived + fa::kStepMaxPairs * 4;
+    x_mlp = x_att + words;
+    qkv = x_mlp + words;
+    ctx = qkv + 3 * words;
+    h = ctx + words;
+    part_ml = h + 4 * words;
+    part_o = part_ml + (partials * 8 + 127) / 128 * 128;
+    bytes = part_o + partials * 64 * 4;
+  }
+};
+
+bool step_shape_ok(int B, int H) {
+  return B >= 1 && B <= fa::kStepMaxRows && H >= 1 && 64 * H <= fa::kStepMaxWidth && B * H <= 256;
+}
+
+}  // namespace
+
+int64_t fa_b200_gpt_step_workspace_bytes(int32_t B, int32_t H) {
+  if (!step_shape_ok(B, H)) return FA_B200_ERR_SHAPE;
+  return StepWorkspace(B, H).bytes;
+}
+
+int fa_b200_gpt_step(const fa_b200_gpt_step_params* p) {
+  if (p == nullptr || p->layers == nullptr || p->tok_emb == nullptr || p->pos_emb == nullptr ||
+      p->lnf_scale == nullptr || p->lnf_shift == nullptr || p->head_w == nullptr || p->ids == nullptr ||
+      p->k_cache == nullptr || p->v_cache == nullptr || p->logits == nullptr)
+    return FA_B200_ERR_NULL;
+  if (!step_shape_ok(p->B, p->H) || p->n_layers < 1 || p->n_layers > fa::kStepMaxLayers || p->vocab < 1 ||
+      p->cache_rows < 1 || p->n_positions < 1 || p->cache_rows > (1 << 22))
+    return FA_B200_ERR_SHAPE;
+  if (p->pos_device == nullptr && (p->pos < 0 || p->pos >= p->cache_rows || p->pos >= p->n_positions))
+    return FA_B200_ERR_SHAPE;
+  if (!stride_ok(p->cache_strides) || p->cache_strides[1] > 0x7fffffff || p->cache_strides[2] > 0x7fffffff)
+    return FA_B200_ERR_STRIDE;
+  const void* ptrs[7] = {p->tok_emb, p->pos_emb, p->lnf_scale, p->lnf_shift, p->head_w, p->layers, p->workspace};
+  for (const void* q : ptrs)
+    if (reinterpret_cast<uintptr_t>(q) & 15u) return FA_B200_ERR_ALIGN;
+  for (int l = 0; l < p->n_layers; ++l) {
+    if (p->k_cache[l] == nullptr || p->v_cache[l] == nullptr) return FA_B200_ERR_NULL;
+    if ((reinterpret_cast<uintptr_t>(p->k_cache[l]) | reinterpret_cast<uintptr_t>(p->v_cache[l])) & 15u)
+      return FA_B200_ERR_ALIGN;
+  }
+  if ((reinterpret_cast<uintptr_t>(p->ids) | reinterpret_cast<uintptr_t>(p->pos_device) |
+       reinterpret_cast<uintptr_t>(p->next_ids)) & 7u)
+    return FA_B200_ERR_ALIGN;
+  if ((reinterpret_cast<uintptr_t>(p->length_device) & 3u) || (reinterpret_cast<uintptr_t>(p->logits) & 1u))
+    return FA_B200_ERR_ALIGN;
+  if (!(p->eps >= 0.0f)) return FA_B200_ERR_SCALE;
+  if (p->device < 0 || p->device >= kMaxDevices) return FA_B200_ERR_DEVICE;
+  const StepWorkspace ws(p->B, p->H);
+  if (p->workspace == nullptr || p->workspace_bytes < ws.bytes) return FA_B200_ERR_WORKSPACE;
+
+  DeviceGuard guard(p->device);
+  if (guard.error) return guard.error;
+  DeviceState* stp = nullptr;
+  int rc = ready_device(p->device, &stp);
+  if (rc != 0) return rc;
+  std::call_once(g_step_once[p->device], step_init, p->device);
+  if (g_step_error[p->device]) return g_step_error[p->device];
+
+  fa::StepParams kp;
+  static_assert(sizeof(fa::StepLayer) == sizeof(fa_b200_gpt_layer), "layer records are passed through");
+  auto bf = [](const void* q) { return static_cast<const __nv_bfloat16*>(q); };
+  kp.layers = reinterpret_cast<const fa::StepLayer*>(p->layers);
+  kp.tok_emb = bf(p->tok_emb); kp.pos_emb = bf(p->pos_emb);
+  kp.lnf_g = bf(p->lnf_scale); kp.lnf_b = bf(p->lnf_shift);
+  kp.head_w = bf(p->head_w);
+  kp.ids = reinterpret_cast<const long long*>(p->ids);
+  kp.ids_stride = p->ids_stride;
+  kp.pos_ptr = reinterpret_cast<long long*>(p->pos_device);
+  kp.len_ptr = p->length_device;
+  kp.pos = p->pos;
+  kp.advance = p->advance;
+  kp.n_layers = p->n_layers;
+  kp.C = 64 * p->H; kp.H = p->H; kp.V = p->vocab; kp.M = p->B;
+  kp.cache_rows = p->cache_rows;
+  kp.n_positions = p->n_positions;
+  kp.eps = p->eps;
+  kp.scale_log2 = 0.125f * 1.4426950408889634f;                  // 1/sqrt(64) * log2(e)
+  kp.c_sb = p->cache_strides[0];
+  kp.c_sn = static_cast<int>(p->cache_strides[1]);
+  kp.c_sh = static_cast<int>(p->cache_strides[2]);
+  unsigned char* w = static_cast<unsigned char*>(p->workspace);
+  kp.generation = reinterpret_cast<uint32_t*>(w);
+  kp.done = reinterpret_cast<unsigned int*>(w) + 1;
+  kp.best = reinterpret_cast<unsigned long long*>(w + ws.best);
+  kp.arrived = reinterpret_cast<unsigned int*>(w + ws.arrived);
+  kp.x_att = reinterpret_cast<uint32_t*>(w + ws.x_att);
+  kp.x_mlp = reinterpret_cast<uint32_t*>(w + ws.x_mlp);
+  kp.qkv = reinterpret_cast<uint32_t*>(w + ws.qkv);
+  kp.ctx = reinterpret_cast<uint32_t*>(w + ws.ctx);
+  kp.h = reinterpret_cast<uint32_t*>(w + ws.h);
+  kp.part_ml = reinterpret_cast<float2*>(w + ws.part_ml);
+  kp.part_o = reinterpret_cast<float*>(w + ws.part_o);
+  kp.next_ids = reinterpret_cast<long long*>(p->next_ids);
+  kp.next_stride = p->next_stride;
+  kp.logits = static_cast<__nv_bfloat16*>(p->logits);
+  kp.status = stp->status;
+  for (int l = 0; l < p->n_layers; ++l) {
+    kp.k_cache[l] = static_cast<__nv_bfloat16*>(p->k_cache[l]);
+    kp.v_cache[l] = static_cast<__nv_bfloat16*>(p->v_cache[l]);
+  }
+  // at least B * H / 2 CTAs: a CTA then has at most kStepSegs attention units
+  const int grid = stp->sm_count < kStepMaxGrid ? stp->sm_count : kStepMaxGrid;
+  // (and every CTA has rows of the QKV projection and the MLP: the exchange relies on it)
+  if (2 * grid < p->B * p->H || kp.C > fa::kStepTile * grid || 3 * kp.C < grid) return FA_B200_ERR_SHAPE;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(fa::kStepThreads);
+  cfg.dynamicSmemBytes = fa::kStepSmemBytes;
+  cfg.stream = static_cast<cudaStream_t>(p->stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;     // CTAs wait on one another: all must be resident
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, fa::fa_gpt_step_kernel, kp);
+  const cudaError_t last = cudaGetLastError();     // clears the sticky copy of a launch error
+  return static_cast<int>(e != cudaSuccess ? e : last);
+}
+
 #ifdef FA_TRACE
 // Trace builds only: choose the traced CTA / copy the trace buffer to the host (synchronises).
 int fa_b200_trace_select(int block) {
@@ -757,6 +904,9 @@ const char* fa_b200_strerror(int code) {
       case fa::kWaitSFree: return "fa_b200 watchdog: wait for the softmax warps to take S ran out";
       case fa::kWaitOFree: return "fa_b200 watchdog: wait for the epilogue to read O ran out";
       case fa::kWaitQEmpty: return "fa_b200 watchdog: wait for the Q slot to be released ran out";
+      case fa::kWaitStepFull: return "fa_b200 watchdog: generation step, wait for a weight tile ran out";
+      case fa::kWaitStepEmpty: return "fa_b200 watchdog: generation step, wait for a free ring stage ran out";
+      case fa::kWaitStepWords: return "fa_b200 watchdog: generation step, wait for another CTA's values ran out";
       case fa::kWaitOFull: return "fa_b200 watchdog: wait for O += PV ran out";
       default: return "fa_b200 watchdog: a bounded wait ran out";
     }

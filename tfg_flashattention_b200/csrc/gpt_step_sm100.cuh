@@ -1,0 +1,971 @@
+// One generation step of a GPT-2 model (one new token for each of up to 8 sequences) as ONE
+// persistent kernel: embedding, every transformer block over the K/V caches, final LayerNorm and
+// the vocabulary head.
+//
+// The arithmetic is that of the reference's modules (src/py/model_inference.py:39-190: pre-LN
+// blocks, LayerNorm :96-107, tanh GELU :109-117), evaluated for a single position per sequence
+// with the keys and values of earlier positions cached.
+//
+// What bounds it: every weight is read once per step (GPT-2 XL: 3.1 GB, 0.48 ms at the measured
+// copy bandwidth), and a layer is five dependent operations across all SMs, each at least one trip
+// through L2 (about 1000 clocks one way and the wait for it).  As one launch per operation the step
+// is 250 kernels, each of which starts with an idle memory system.
+//
+//   stream       Four warps per CTA run through the CTA's share of ALL weights and of the cached keys
+//                and values in order and copy it into a ring of shared-memory stages; they wait only
+//                for ring slots, never for the other CTAs, and fill the ring while those wait.  (One
+//                warp, or a lane per row, does not issue the copies fast enough: 1000 clocks a stage.)
+//   exchange     No barrier between the operations.  Every value that one CTA hands to others is a
+//                32-bit word, bf16 in the upper half and the generation of its buffer in the lower:
+//                a reader loads the words it needs and loads again until the generation is right.
+//                One trip instead of the four of data, fence, counter and poll.  A buffer is
+//                written again only by CTAs that hold something which depends on everybody's having
+//                read it (its reader's own output, a few operations on).
+//   work split   Output columns of a layer (rows of W) are cut evenly over the CTAs, so a CTA's
+//                share is one contiguous piece of W.  It is taken in tiles of at most 16 rows, K in
+//                passes of d_model columns and chunks of at most 800, one (tile, chunk) per stage.
+//   tensor path  mma.sync m16n8k16 with W as the 16-row operand and the (up to 8) tokens as the
+//                8-column operand: at 8 tokens a scalar product per weight costs more issue slots
+//                than the stream leaves.  tcgen05 needs 64 or 128 rows of one operand per CTA and
+//                gives nothing here, the memory pipe is the limit.  The 16 warps split K: warp w
+//                owns the 32-column units w, w + 16, ...; partial tiles meet in shared memory.
+//   attention    a (sequence, head) pair per CTA, up to two where there are more pairs than CTAs,
+//                split over several CTAs only for caches of thousands of rows.  q.K on the tensor
+//                path with the cached rows as the 16-row operand, P.V on packed fp32.  The cached
+//                rows come through the ring, ahead of the query; the new row comes through the
+//                exchange, so nobody waits for the caches.
+//   precision    bf16 weights, activations rounded to bf16 where the layer-by-layer path rounds
+//                them, fp32 accumulation; the residual stream accumulates in fp32 in the shared
+//                memory of the CTA that owns the column.
+//   what counts  Between two exchanges a warp runs a few hundred instructions at 4 to 8 clocks each
+//                (dependent, few warps): their number, the trips to L2 and the CTA barriers are the
+//                time.  Nothing but an operation's own input is fetched after that input, and
+//                nothing may spill: shared memory leaves so little L1 that a spilled register costs
+//                a trip to L2 (a build with 300 bytes of spills per thread took 2.5 ms per GPT-2 XL
+//                step).  step_tid keeps one operation's addresses out of the other's registers.
+//
+// The grid is launched cooperatively (CTAs wait on one another).  Every wait is bounded: one that
+// runs out leaves its code in the status words and the kernel drains.
+#pragma once
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "add_layernorm_sm100.cuh"   // ln_unpack8
+#include "fa_fwd_sm100.cuh"          // Watch and the watchdog codes
+#include "linear_small_sm100.cuh"    // gelu_tanh
+
+namespace fa {
+
+constexpr int kStepWarps = 16;                        // computing warps
+constexpr int kStepCompute = kStepWarps * 32;
+constexpr int kStepStreamWarps = 4;
+constexpr int kStepThreads = kStepCompute + 32 * kStepStreamWarps;
+// Registers: the computing warpgroups take what the streaming one gives up.  (setmaxnreg.inc waits
+// without a limit for registers of this CTA's launch allocation, hence the check; the host refuses a
+// build whose launch allocation is another.)
+constexpr int kStepLaunchRegs = 96, kStepComputeRegs = 112, kStepStreamRegs = 32;
+static_assert(kStepCompute * kStepComputeRegs + 32 * kStepStreamWarps * kStepStreamRegs <= kStepThreads * kStepLaunchRegs,
+              "setmaxnreg budget exceeds the launch allocation: the kernel would hang");
+constexpr int kStepMaxRows = 8;                       // sequences (the 8-column side of the MMA)
+constexpr int kStepMaxLayers = 64;
+constexpr int kStepMaxPairs = 256;                    // (sequence, head) pairs
+constexpr int kStepTile = 16;                         // rows of W per stage
+constexpr int kStepGroup = 4;                         // tiles reduced together: one output per thread
+constexpr int kStepOutputs = kStepTile * kStepMaxRows;
+static_assert(kStepGroup * kStepOutputs == kStepCompute, "one output per thread");
+constexpr int kStepUnit = 32;                         // columns of W per warp step: 64 bytes
+constexpr int kStepChunkUnits = 25;                   // columns per stage: at most 800
+constexpr int kStepStageBytes = kStepTile * kStepChunkUnits * 64;
+constexpr int kStepStages = 6;
+constexpr int kStepMaxWidth = 1600;                   // d_model: the fragments of 8 rows fill sm.x
+constexpr int kStepMaxUnits = kStepMaxWidth / kStepUnit;
+constexpr int kStepUnits = (kStepMaxUnits + kStepWarps - 1) / kStepWarps;     // 4 per warp and pass
+constexpr int kStepQuads = (kStepMaxWidth / 4 + 63) / 64;                      // 7: columns / 4 of a row per lane of two warps
+constexpr int kStepSegs = 2;                          // attention units of one CTA
+constexpr int kStepBlocks = 6;                        // blocks of 16 cached rows (K, then V) per stage
+static_assert(kStepBlocks * 16 * 256 <= kStepStageBytes, "cached rows fit a stage");
+constexpr int kStepSplitRows = 1024;                  // rows of a unit where pairs are split over CTAs
+constexpr uint32_t kStepBarPolls = 1u << 24;          // bounds of the waits: about 65 clocks a poll of a barrier ...
+constexpr uint32_t kStepWordPolls = 1u << 21;         // ... and a trip to L2 a poll of exchange words: half a second
+
+struct StepLayer {       // one transformer block's parameters (device memory, built once per model)
+  const __nv_bfloat16 *ln1_g, *ln1_b, *qkv_w, *qkv_b, *proj_w, *proj_b;
+  const __nv_bfloat16 *ln2_g, *ln2_b, *fc_w, *fc_b, *out_w, *out_b;
+};
+
+struct StepParams {
+  const StepLayer* layers;
+  const __nv_bfloat16 *tok_emb, *pos_emb, *lnf_g, *lnf_b, *head_w;
+  const long long* ids;            // [M], ids_stride apart
+  long long ids_stride;
+  long long* pos_ptr;              // device position (cache row of the new token), or null: `pos`
+  int* len_ptr;                    // with pos_ptr and advance: set to the new length + 1
+  int pos, advance;
+  int n_layers, C, H, V, M;
+  int cache_rows, n_positions;
+  float eps, scale_log2;
+  long long c_sb;                  // cache strides in elements: sequence, row, head
+  int c_sn, c_sh;
+  // workspace: the exchange buffers (words: bf16 << 16 | generation) ...
+  uint32_t *x_att, *x_mlp;         // [M][C] residual stream after attention and after the MLP (or embedding)
+  uint32_t* qkv;                   // [M][3C]
+  uint32_t* ctx;                   // [C / 32][M][32]: fragment order
+  uint32_t* h;                     // [4C / 32][M][32]
+  uint32_t* generation;            // of the last launch's last layer
+  // ... and what is behind fences
+  float* part_o;                   // [pairs * splits, 64]
+  float2* part_ml;                 // [pairs * splits]
+  unsigned int* arrived;           // per pair: CTAs whose partial is in; zero between launches
+  unsigned long long* best;        // [8] packed argmax keys
+  unsigned int* done;              // CTAs that have delivered their argmax
+  long long* next_ids;             // argmax of the logits, M ids next_stride apart, or null
+  long long next_stride;
+  __nv_bfloat16* logits;           // [M, V]
+  unsigned int* status;
+  __nv_bfloat16* k_cache[kStepMaxLayers];
+  __nv_bfloat16* v_cache[kStepMaxLayers];
+};
+
+// How a [N, K] weight is cut: rows of this CTA, tiles of `tile` rows.
+struct StepCut {
+  int row0, rows, tiles, tile;
+};
+__device__ __forceinline__ StepCut step_cut(int N) {          // N < 2^24, grid <= 160
+  StepCut c;
+  c.row0 = static_cast<int>(blockIdx.x * static_cast<uint32_t>(N) / gridDim.x);
+  c.rows = static_cast<int>((blockIdx.x + 1) * static_cast<uint32_t>(N) / gridDim.x) - c.row0;
+  c.tiles = (c.rows + kStepTile - 1) / kStepTile;
+  c.tile = c.tiles > 0 ? (c.rows + c.tiles - 1) / c.tiles : 0;
+  return c;
+}
+// A pass over d_model columns: `chunks` stages of `units` units (the last may have fewer).
+struct StepPass {
+  int total, units, chunks;
+  uint32_t pitch;
+  __device__ __forceinline__ explicit StepPass(int C) {
+    total = C / kStepUnit;
+    chunks = (total + kStepChunkUnits - 1) / kStepChunkUnits;
+    units = (total + chunks - 1) / chunks;
+    // rows of a stage lie 64 bytes (mod 128) apart: the 8 lanes of a 128-bit load phase read two
+    // rows of 64 bytes each, which then cover all banks (an even `units` is at most 24)
+    pitch = units * 64 + ((units & 1) ? 0 : 64);
+  }
+};
+
+enum StepOp : int { kStepQkv = 0, kStepProj = 1, kStepFc = 2, kStepOut = 3, kStepHead = 4 };
+
+// How the attention over the `rows` earlier positions is cut: `splits` units per (sequence, head)
+// pair, the units evenly over the first CTAs; a CTA has at most kStepSegs.
+struct StepAttnCut {
+  int rows, splits;
+  int first, count;                      // units of this CTA
+  __device__ __forceinline__ StepAttnCut(int pairs, int earlier) {
+    rows = earlier;
+    splits = min(static_cast<int>(gridDim.x) / pairs, (rows + kStepSplitRows - 1) / kStepSplitRows);
+    if (splits < 1 || rows < 2 * kStepSplitRows) splits = 1;
+    const int units = pairs * splits, ctas = min(static_cast<int>(gridDim.x), units);
+    first = count = 0;
+    if (static_cast<int>(blockIdx.x) < ctas) {
+      first = blockIdx.x * units / ctas;
+      count = (blockIdx.x + 1) * units / ctas - first;
+    }
+  }
+};
+// A unit's rows and addresses: the same in every layer, worked out once.
+struct StepUnit {
+  long long head;                        // offset of the head in a cache, elements
+  int pair, slot;                        // which of the pair's units
+  int row0, rows;
+  int query;                             // offset of the pair's q in p.qkv
+  int out;                               // offset of its output in p.ctx
+};
+
+struct __align__(128) StepSmem {
+  uint8_t ring[kStepStages][kStepStageBytes];
+  uint4 x[kStepMaxUnits * 32];                              // LayerNorm's output as MMA fragments
+  union {
+    float red[kStepGroup][kStepWarps][kStepOutputs];        // partial tiles of the warps
+    float seg[kStepSegs][kStepWarps + 1][68];               // attention partials: m, l, -, -, o[64]
+  };
+  uint2 norm[2][kStepMaxWidth / 4];                         // scale and shift of the coming LayerNorm
+  alignas(16) float2 stat[kStepWarps];                      // LayerNorm: sums of a warp's part
+  float shift[kStepMaxRows];                                // ... and the row's mean in the one before
+  float own[kStepOutputs];                                  // this CTA's columns of the residual stream
+  unsigned long long keys[kStepWarps][kStepMaxRows];        // best logit of a warp
+  StepUnit unit[kStepSegs];                                 // this CTA's attention units
+  int units, splits;
+  StepCut cut[5];                                           // by StepOp
+  StepLayer layers[kStepMaxLayers];
+  uint64_t full[kStepStages];
+  uint64_t empty[kStepStages];
+  uint32_t seg_last;                                        // the CTA completes its pair
+  uint32_t abort, abort_who;
+};
+constexpr int kStepSmemBytes = sizeof(StepSmem) + 128;
+static_assert(kStepSmemBytes <= 227 * 1024, "one CTA per SM");
+
+enum StepWaitId : uint32_t { kWaitStepFull = 17, kWaitStepEmpty = 18, kWaitStepWords = 19 };
+
+// The thread index, read anew: what is computed from it stays in the operation that computes it
+// instead of being hoisted out of the loop over the operations.
+__device__ __forceinline__ int step_tid() {
+  int t;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+  return t;
+}
+__device__ __forceinline__ void step_bar() {           // the computing warps only
+  asm volatile("bar.sync 1, %0;" ::"n"(kStepCompute) : "memory");
+}
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t a) {
+  uint4 r;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(a) : "memory");
+  return r;
+}
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                          uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t bf16x2_to_f32x2(uint32_t v) {
+  return pack_f32x2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+}
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(reinterpret_cast<uint64_t>(src)) : "memory");
+}
+// Untiled bulk copy global -> shared (both 16-byte aligned, size a multiple of 16).
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               :: "r"(dst), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<uint64_t>(p)));
+}
+
+struct StepRing {
+  uint32_t stage = 0, parity = 0;
+  __device__ __forceinline__ void next() {
+    if (++stage == kStepStages) { stage = 0; parity ^= 1; }
+  }
+};
+
+struct StepCta {            // what a computing warp carries from operation to operation
+  StepSmem* sm;
+  StepRing ring;
+  bool ok;                  // false: a wait has run out somewhere in the CTA, wait for nothing more
+};
+
+__device__ __forceinline__ void step_give_up(StepSmem& sm, uint32_t id) {
+  volatile uint32_t* abort = &sm.abort;
+  if (*abort == 0) {
+    sm.abort_who = threadIdx.x;
+    *abort = kWatchdogBase | id;
+  }
+}
+// A bounded wait of a converged warp, small because it is inlined in the loops.
+__device__ __forceinline__ bool step_wait(uint32_t bar, uint32_t parity, StepSmem& sm, uint32_t id) {
+  bool ok = false;
+#pragma unroll 1
+  for (uint32_t polls = 0; polls < kStepBarPolls && !ok; ++polls) ok = mbar_try_wait(bar, parity);
+  ok = __all_sync(0xffffffffu, ok);
+  if (!ok) step_give_up(sm, id);
+  return ok;
+}
+
+// ------------------------------------------------------------------------------ exchange words
+__device__ __forceinline__ uint32_t step_word(float v, uint32_t gen) {
+  return (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(v))) << 16) | gen;
+}
+__device__ __forceinline__ void step_put(uint32_t* dst, float v, uint32_t gen) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(dst), "r"(step_word(v, gen)) : "memory");
+}
+__device__ __forceinline__ uint4 step_peek(const uint32_t* src) {       // four words, past L1
+  uint4 r;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(src) : "memory");
+  return r;
+}
+__device__ __forceinline__ uint32_t step_stale(const uint4& w, uint32_t gen) {    // 0: all of this generation
+  return ((w.x ^ gen) | (w.y ^ gen) | (w.z ^ gen) | (w.w ^ gen)) & 0xffffu;
+}
+__device__ __forceinline__ uint32_t step_pair(uint32_t lo, uint32_t hi) {         // two words' values as bf16x2
+  return __byte_perm(lo, hi, 0x7632);
+}
+// Asynchronous copies of this thread so far: the barrier's phase cannot complete before they have.
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+// Loads kN times four words, the i-th from at(i), until all have this generation.
+template <int kN, class At>
+__device__ __forceinline__ void step_take(StepCta& c, uint32_t gen, uint4 (&w)[kN], At at) {
+#pragma unroll 1
+  for (uint32_t polls = 0;; ++polls) {
+    uint32_t bad = 0;
+#pragma unroll
+    for (int i = 0; i < kN; ++i) w[i] = step_peek(at(i));
+#pragma unroll
+    for (int i = 0; i < kN; ++i) bad |= step_stale(w[i], gen);
+    if (!c.ok || !__any_sync(0xffffffffu, bad != 0)) break;
+    if (polls >= kStepWordPolls || *const_cast<volatile uint32_t*>(&c.sm->abort)) {
+      step_give_up(*c.sm, kWaitStepWords);
+      c.ok = false;
+    }
+  }
+}
+
+__device__ __forceinline__ unsigned long long step_key(float v, int n) {
+  // orders by value (NaN above all, as torch.argmax has it), then by the lower index
+  uint32_t b = __float_as_uint(v);
+  b = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+  if (v != v) b = 0xffffffffu;
+  return (static_cast<unsigned long long>(b) << 32) | (0xffffffffu - static_cast<uint32_t>(n));
+}
+
+// ---------------------------------------------------------------------------------- operations
+// y[n, token] for this CTA's rows of W, tile by tile.  Fragments: the 16 bytes of lane 4 token + q
+// hold columns 32 unit + 8 q .. + 7 of the token.  (Which k meets which does not matter to a sum:
+// both operands use the order in which a 16-byte vector comes out of memory.)  The input is in sm.x,
+// or, with `src`, in an exchange buffer.
+__device__ __forceinline__ StepCta step_gemm(StepCta c, const StepParams& p, const uint32_t* src, int op, int layer,
+                                                 int pos, uint32_t gen, const __nv_bfloat16* bias) {
+  const int tid = step_tid(), warp = tid >> 5, lane = tid & 31;
+  const StepPass pass(p.C);
+  unsigned long long key = 0ull;                 // best of this thread's logits (its token: lane % 8)
+  const StepCut cut = c.sm->cut[op];
+  const int passes = op == kStepOut ? 4 : 1;
+  const int M = p.M, g = lane >> 2, q = lane & 3;
+  const uint32_t ring = smem_u32(c.sm->ring) + g * pass.pitch + q * 16;
+  const int mine_units = (pass.total - warp + kStepWarps - 1) / kStepWarps;       // of each pass
+  const bool live = g < M;
+  if (src != nullptr) src += (warp * M + (live ? g : 0)) * 32 + q * 8;            // idle lanes follow token 0
+  // words of the coming pass (of the first tile; operations with `src` have one)
+  uint4 raw[kStepUnits][2];
+  auto peek = [&](const uint32_t* from) {
+#pragma unroll
+    for (int i = 0; i < kStepUnits; ++i) {
+      raw[i][0] = raw[i][1] = make_uint4(gen, gen, gen, gen);
+      if (i < mine_units) {
+        raw[i][0] = step_peek(from + i * kStepWarps * M * 32);
+        raw[i][1] = step_peek(from + i * kStepWarps * M * 32 + 4);
+      }
+    }
+  };
+  if (src != nullptr) peek(src);
+#pragma unroll 1
+  for (int t0 = 0; t0 < cut.tiles; t0 += kStepGroup) {
+    const int tiles = min(kStepGroup, cut.tiles - t0);
+    const int in_tile = (tid >> 3) & (kStepTile - 1), row = (t0 + (tid >> 7)) * cut.tile + in_tile;
+    const int n = cut.row0 + row, tok = tid & 7;
+    const bool mine = (tid >> 7) < tiles && in_tile < cut.tile && row < cut.rows && tok < M;
+    float val = mine && bias != nullptr ? __bfloat162float(bias[n]) : 0.f;
+#pragma unroll 1
+    for (int t = 0; t < tiles; ++t) {
+      float a0[4] = {0.f, 0.f, 0.f, 0.f}, a1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+      for (int ps = 0; ps < passes; ++ps) {
+        uint4 xv[kStepUnits];
+        if (src != nullptr) {
+#pragma unroll 1
+          for (uint32_t polls = 0;; ++polls) {
+            uint32_t bad = 0;
+#pragma unroll
+            for (int i = 0; i < kStepUnits; ++i) bad |= step_stale(raw[i][0], gen) | step_stale(raw[i][1], gen);
+            if (!c.ok || !__any_sync(0xffffffffu, bad != 0)) break;
+            if (polls >= kStepWordPolls || *const_cast<volatile uint32_t*>(&c.sm->abort)) {
+              step_give_up(*c.sm, kWaitStepWords);
+              c.ok = false;
+            }
+            peek(src);
+          }
+#pragma unroll
+          for (int i = 0; i < kStepUnits; ++i)
+            xv[i] = live ? make_uint4(step_pair(raw[i][0].x, raw[i][0].y), step_pair(raw[i][0].z, raw[i][0].w),
+                                      step_pair(raw[i][1].x, raw[i][1].y), step_pair(raw[i][1].z, raw[i][1].w))
+                         : make_uint4(0u, 0u, 0u, 0u);
+          src += pass.total * M * 32;
+          if (ps + 1 < passes) peek(src);        // the next pass's, while this one is multiplied
+        } else {
+#pragma unroll
+          for (int i = 0; i < kStepUnits; ++i) {
+            xv[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (live && i < mine_units) xv[i] = c.sm->x[(warp + kStepWarps * i) * 4 * M + lane];
+          }
+        }
+        // the pass's one or two stages
+        const uint32_t base0 = ring + c.ring.stage * kStepStageBytes;
+        uint32_t base1 = base0, bar0 = smem_u32(&c.sm->empty[c.ring.stage]), bar1 = bar0;
+        if (c.ok) c.ok = step_wait(smem_u32(&c.sm->full[c.ring.stage]), c.ring.parity, *c.sm, kWaitStepFull);
+        c.ring.next();
+        if (pass.chunks > 1) {
+          base1 = ring + c.ring.stage * kStepStageBytes - pass.units * 64;
+          bar1 = smem_u32(&c.sm->empty[c.ring.stage]);
+          if (c.ok) c.ok = step_wait(smem_u32(&c.sm->full[c.ring.stage]), c.ring.parity, *c.sm, kWaitStepFull);
+          c.ring.next();
+        }
+#pragma unroll
+        for (int h = 0; h < kStepUnits; h += 2) {        // two units at a time: their loads overlap
+          uint4 r[2], s[2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int u = min(warp + kStepWarps * (h + i), pass.total - 1);      // past the end: x is zero
+            const uint32_t addr = (u < pass.units ? base0 : base1) + u * 64;
+            r[i] = ld_shared_v4(addr);
+            s[i] = ld_shared_v4(addr + 8 * pass.pitch);
+          }
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            mma_16816(a0, r[i].x, s[i].x, r[i].y, s[i].y, xv[h + i].x, xv[h + i].y);
+            mma_16816(a1, r[i].z, s[i].z, r[i].w, s[i].w, xv[h + i].z, xv[h + i].w);
+          }
+        }
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(bar0);
+          if (pass.chunks > 1) mbar_arrive(bar1);
+        }
+      }
+      float* red = c.sm->red[t][warp] + g * 8 + 2 * q;
+      *reinterpret_cast<float2*>(red) = make_float2(a0[0] + a1[0], a0[1] + a1[1]);
+      *reinterpret_cast<float2*>(red + 64) = make_float2(a0[2] + a1[2], a0[3] + a1[3]);
+    }
+    step_bar();
+    if (mine) {
+      const float* red = c.sm->red[tid >> 7][0] + (tid & (kStepOutputs - 1));
+      float v1 = 0.f;
+#pragma unroll
+      for (int w = 0; w < kStepWarps; w += 2) {
+        val += red[w * kStepOutputs];
+        v1 += red[(w + 1) * kStepOutputs];
+      }
+      val += v1;
+      if (op == kStepQkv) {
+        step_put(p.qkv + tok * 3 * p.C + n, val, gen);
+        if (n >= p.C) {                          // the caches get the row too, for the steps to come
+          const bool is_k = n < 2 * p.C;
+          const int nn = n - (is_k ? p.C : 2 * p.C);
+          (is_k ? p.k_cache[layer] : p.v_cache[layer])[tok * p.c_sb + static_cast<long long>(pos) * p.c_sn + (nn >> 6) * p.c_sh + (nn & 63)] =
+              __float2bfloat16_rn(val);
+        }
+      } else if (op == kStepFc) {
+        step_put(p.h + ((n >> 5) * M + tok) * 32 + (n & 31), gelu_tanh(val), gen);
+      } else if (op == kStepHead) {
+        const __nv_bfloat16 b = __float2bfloat16_rn(val);
+        p.logits[static_cast<long long>(tok) * p.V + n] = b;
+        const unsigned long long kk = step_key(__bfloat162float(b), n);
+        key = kk > key ? kk : key;
+      } else {
+        val += c.sm->own[tid];           // one tile, so the thread is below kStepOutputs
+        c.sm->own[tid] = val;
+        step_put((op == kStepProj ? p.x_att : p.x_mlp) + tok * p.C + n, val, gen);
+      }
+    }
+    if (t0 + kStepGroup < cut.tiles) step_bar();     // before the partial tiles are overwritten
+  }
+  if (op == kStepHead) {
+#pragma unroll
+    for (int o = 8; o <= 16; o <<= 1) {
+      const unsigned long long k = __shfl_xor_sync(0xffffffffu, key, o);
+      key = k > key ? k : key;
+    }
+    if (lane < kStepMaxRows) c.sm->keys[warp][lane] = key;
+  }
+  return c;
+}
+
+// How the warps share the token rows: warp w serves token w / wpt; its lane the groups of four
+// columns (w % wpt) * 32 + lane, + 32 wpt, ...
+struct StepRows {
+  int tok, first, stride, lg;
+  __device__ __forceinline__ StepRows(int M, int warp, int lane) {
+    lg = M <= 1 ? 4 : (M <= 2 ? 3 : (M <= 4 ? 2 : 1));      // log2 of warps per token
+    tok = warp >> lg;
+    first = (warp & ((1 << lg) - 1)) * 32 + lane;
+    stride = 32 << lg;
+  }
+};
+
+// LayerNorm of the residual stream (exchange words at `x`) into the fragments sm.x.  One pass: sums
+// of x - s and (x - s)^2 with s the row's mean in the LayerNorm before (0 in the first), which keeps
+// the difference of squares well conditioned.
+__device__ __forceinline__ StepCta step_layernorm(StepCta c, const StepParams& p, const uint32_t* x, uint32_t gen) {
+  const int tid = step_tid(), warp = tid >> 5, lane = tid & 31;
+  const StepRows rw(p.M, warp, lane);
+  const int quads = p.C >> 2;
+  // rounds of this warp (the same for its lanes: past the end they repeat the last quad, unused)
+  const int n = rw.tok < p.M ? (quads - (rw.first - lane) + rw.stride - 1) / rw.stride : 0;
+  uint4 w[kStepQuads];
+#pragma unroll
+  for (int i = 0; i < kStepQuads; ++i) w[i] = make_uint4(0u, 0u, 0u, 0u);
+  {
+    const uint32_t* src = x + rw.tok * p.C;
+#pragma unroll 1
+    for (uint32_t polls = 0;; ++polls) {
+      uint32_t bad = 0;
+#pragma unroll
+      for (int i = 0; i < kStepQuads; ++i)
+        if (i < n) w[i] = step_peek(src + 4 * min(rw.first + i * rw.stride, quads - 1));
+#pragma unroll
+      for (int i = 0; i < kStepQuads; ++i)
+        if (i < n) bad |= step_stale(w[i], gen);
+      if (!c.ok || !__any_sync(0xffffffffu, bad != 0)) break;
+      if (polls >= kStepWordPolls || *const_cast<volatile uint32_t*>(&c.sm->abort)) {
+        step_give_up(*c.sm, kWaitStepWords);
+        c.ok = false;
+      }
+    }
+  }
+  const float shift = c.sm->shift[rw.tok & (kStepMaxRows - 1)];
+  float sum = 0.f, sq = 0.f;
+#pragma unroll
+  for (int i = 0; i < kStepQuads; ++i) {
+    if (i < n) {
+      w[i].x &= 0xffff0000u; w[i].y &= 0xffff0000u; w[i].z &= 0xffff0000u; w[i].w &= 0xffff0000u;   // now fp32
+      const float f = rw.first + i * rw.stride < quads ? 1.f : 0.f;
+      const float d0 = __uint_as_float(w[i].x) - shift, d1 = __uint_as_float(w[i].y) - shift;
+      const float d2 = __uint_as_float(w[i].z) - shift, d3 = __uint_as_float(w[i].w) - shift;
+      sum = fmaf(f, (d0 + d1) + (d2 + d3), sum);
+      sq = fmaf(f, fmaf(d0, d0, d1 * d1) + fmaf(d2, d2, d3 * d3), sq);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    sq += __shfl_xor_sync(0xffffffffu, sq, o);
+  }
+  if (lane == 0) c.sm->stat[warp] = make_float2(sum, sq);
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  step_bar();                                    // sm.stat and sm.norm are complete, sm.shift is read
+  sum = sq = 0.f;
+  {
+    const float4* st = reinterpret_cast<const float4*>(c.sm->stat + ((rw.tok << rw.lg) & (kStepWarps - 1)));
+#pragma unroll 2
+    for (int i = 0; i < 1 << (rw.lg - 1); ++i) {
+      const float4 two = st[i];
+      sum += two.x + two.z;
+      sq += two.y + two.w;
+    }
+  }
+  const float inv_c = __fdividef(1.f, static_cast<float>(p.C));
+  const float off = sum * inv_c;
+  const float rstd = rsqrtf(fmaxf(sq * inv_c - off * off, 0.f) + p.eps);
+  const float mean = shift + off;
+  if (rw.first == 0 && rw.tok < p.M) c.sm->shift[rw.tok] = mean;
+  uint2* out = reinterpret_cast<uint2*>(c.sm->x) + rw.tok * 8;
+#pragma unroll
+  for (int i = 0; i < kStepQuads; ++i) {
+    const int v = rw.first + i * rw.stride;      // columns 4 v .. 4 v + 3
+    if (i < n && v < quads) {
+      const uint2 gm = c.sm->norm[0][v], bt = c.sm->norm[1][v];
+      const float y0 = fmaf((__uint_as_float(w[i].x) - mean) * rstd, __uint_as_float(gm.x << 16), __uint_as_float(bt.x << 16));
+      const float y1 = fmaf((__uint_as_float(w[i].y) - mean) * rstd, __uint_as_float(gm.x & 0xffff0000u), __uint_as_float(bt.x & 0xffff0000u));
+      const float y2 = fmaf((__uint_as_float(w[i].z) - mean) * rstd, __uint_as_float(gm.y << 16), __uint_as_float(bt.y << 16));
+      const float y3 = fmaf((__uint_as_float(w[i].w) - mean) * rstd, __uint_as_float(gm.y & 0xffff0000u), __uint_as_float(bt.y & 0xffff0000u));
+      out[(v >> 3) * 8 * p.M + (v & 7)] = make_uint2(pack_bf16(y0, y1), pack_bf16(y2, y3));
+    }
+  }
+  step_bar();
+  return c;
+}
+// Scale and shift of the coming LayerNorm on their way to sm.norm; the LayerNorm waits for them.
+__device__ __forceinline__ void step_fetch_norm(StepSmem& sm, const __nv_bfloat16* gamma, const __nv_bfloat16* beta,
+                                                int nvec) {
+  const int tid = step_tid();
+  const int v = tid & 255;               // 200 vectors of 16 bytes at most, one per thread
+  if (v < nvec) cp_async_16(smem_u32(sm.norm[tid >> 8]) + v * 16,
+                            reinterpret_cast<const uint4*>(tid < 256 ? gamma : beta) + v);
+}
+static_assert(kStepMaxWidth / 8 <= 256 && kStepCompute == 512, "one vector per thread");
+
+__device__ __forceinline__ StepCta step_attention(StepCta c, const StepParams& p, int layer, uint32_t gen) {
+  const int tid = step_tid(), warp = tid >> 5, lane = tid & 31, count = c.sm->units, splits = c.sm->splits;
+  const int g = lane >> 2, q = lane & 3, grp = lane >> 3, col = lane & 7;
+#pragma unroll 1
+  for (int i = 0; i < count; ++i) {
+    const StepUnit un = c.sm->unit[i];
+    uint4 q0, q1;
+    {
+      uint4 w[4];                                // columns 8 q .. + 7 and 32 + 8 q .. + 7
+      const uint32_t* src = p.qkv + un.query + q * 8;
+      step_take<4>(c, gen, w, [&](int k) { return src + (k >> 1) * 32 + (k & 1) * 4; });
+      q0 = make_uint4(step_pair(w[0].x, w[0].y), step_pair(w[0].z, w[0].w), step_pair(w[1].x, w[1].y), step_pair(w[1].z, w[1].w));
+      q1 = make_uint4(step_pair(w[2].x, w[2].y), step_pair(w[2].z, w[2].w), step_pair(w[3].x, w[3].y), step_pair(w[3].z, w[3].w));
+    }
+    float m = -1e30f, l = 0.f;
+    uint64_t acc[4] = {0ull, 0ull, 0ull, 0ull};
+    // Stages of kStepBlocks blocks of 16 rows; block b is warp b % 16's.  A row's odd-numbered
+    // neighbour has its 64-byte halves swapped (see step_stream_rows): no bank conflicts.
+    const int blocks = (un.rows + 15) >> 4, swap = (g & 1) << 2, vswap = (grp & 1) << 2;
+#pragma unroll 1
+    for (int b0 = 0; b0 < blocks; b0 += kStepBlocks) {
+      if (c.ok) c.ok = step_wait(smem_u32(&c.sm->full[c.ring.stage]), c.ring.parity, *c.sm, kWaitStepFull);
+      const int j0 = (warp - b0) & (kStepWarps - 1), base = (b0 + j0) * 16;
+      if (j0 < kStepBlocks && base < un.rows) {
+        const uint32_t ks = smem_u32(c.sm->ring) + c.ring.stage * kStepStageBytes + j0 * 16 * 128;
+        const uint32_t vs = ks + kStepBlocks * 16 * 128;
+        const uint4 k0 = ld_shared_v4(ks + g * 128 + (q ^ swap) * 16), k1 = ld_shared_v4(ks + g * 128 + ((q + 4) ^ swap) * 16);
+        const uint4 k2 = ld_shared_v4(ks + (g + 8) * 128 + (q ^ swap) * 16), k3 = ld_shared_v4(ks + (g + 8) * 128 + ((q + 4) ^ swap) * 16);
+        uint4 vr[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) vr[j] = ld_shared_v4(vs + (grp + 4 * j) * 128 + (col ^ vswap) * 16);
+        // scores of rows g (s[0], equal in the lanes of a quad and in s[1]) and g + 8 (s[2], s[3]):
+        // every column of the 8-column operand is the query
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_16816(s, k0.x, k2.x, k0.y, k2.y, q0.x, q0.y);
+        mma_16816(s, k0.z, k2.z, k0.w, k2.w, q0.z, q0.w);
+        mma_16816(s, k1.x, k3.x, k1.y, k3.y, q1.x, q1.y);
+        mma_16816(s, k1.z, k3.z, k1.w, k3.w, q1.z, q1.w);
+        const float sa = base + g < un.rows ? s[0] * p.scale_log2 : -INFINITY;
+        const float sb = base + g + 8 < un.rows ? s[2] * p.scale_log2 : -INFINITY;
+        float m_new = fmaxf(sa, sb);
+#pragma unroll
+        for (int o = 4; o <= 16; o <<= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, o));
+        if (m_new > m) {                         // the same in all lanes
+          const float f = ex2_approx(m - m_new);
+          const uint64_t f2 = pack_f32x2(f, f);
+          l *= f;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[e] = mul_f32x2(acc[e], f2);
+          m = m_new;
+        }
+        const float pa = ex2_approx(sa - m), pb = ex2_approx(sb - m);
+        l += pa + pb;                            // this lane's rows; each row counts in four lanes
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {            // rows grp + 4 j: their p sits in lane 4 (row % 8)
+          const float pr = __shfl_sync(0xffffffffu, j < 2 ? pa : pb, ((grp + 4 * j) & 7) * 4);
+          const uint64_t p2 = pack_f32x2(pr, pr);
+          acc[0] = fma_f32x2(p2, bf16x2_to_f32x2(vr[j].x), acc[0]);
+          acc[1] = fma_f32x2(p2, bf16x2_to_f32x2(vr[j].y), acc[1]);
+          acc[2] = fma_f32x2(p2, bf16x2_to_f32x2(vr[j].z), acc[2]);
+          acc[3] = fma_f32x2(p2, bf16x2_to_f32x2(vr[j].w), acc[3]);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&c.sm->empty[c.ring.stage]));
+      c.ring.next();
+    }
+#pragma unroll
+    for (int o = 4; o <= 16; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    float* dst = c.sm->seg[i][warp];
+    if (lane == 0) { dst[0] = m; dst[1] = l; }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {                // the four row groups
+      float o0, o1;
+      unpack_f32x2(acc[e], o0, o1);
+      o0 += __shfl_xor_sync(0xffffffffu, o0, 8);
+      o1 += __shfl_xor_sync(0xffffffffu, o1, 8);
+      o0 += __shfl_xor_sync(0xffffffffu, o0, 16);
+      o1 += __shfl_xor_sync(0xffffffffu, o1, 16);
+      if (grp == 0) *reinterpret_cast<float2*>(dst + 4 + 8 * col + 2 * e) = make_float2(o0, o1);
+    }
+    if (warp == kStepWarps - 1) {              // the new row, a partial of its own (of one unit)
+      // lanes 0-15: four columns each; the other half of the warp repeats them
+      const uint32_t* src = p.qkv + un.query + (lane & 15) * 4;
+      uint4 w[3];
+      step_take<3>(c, gen, w, [&](int k) { return src + k * p.C; });
+      auto val = [](uint32_t x) { return __uint_as_float(x & 0xffff0000u); };
+      float s = val(w[0].x) * val(w[1].x) + val(w[0].y) * val(w[1].y) + val(w[0].z) * val(w[1].z) + val(w[0].w) * val(w[1].w);
+#pragma unroll
+      for (int o = 1; o <= 8; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      float* fresh = c.sm->seg[i][kStepWarps];
+      const bool counts = un.slot == 0;
+      if (lane == 0) { fresh[0] = counts ? s * p.scale_log2 : -1e30f; fresh[1] = counts ? 1.f : 0.f; }
+      if (lane < 16)
+        *reinterpret_cast<float4*>(fresh + 4 + 4 * lane) = make_float4(val(w[2].x), val(w[2].y), val(w[2].z), val(w[2].w));
+    }
+  }
+  step_bar();
+  const int i = tid >> 6, e = tid & 63;
+  if (i < count) {
+    const StepUnit un = c.sm->unit[i];
+    const float(&seg)[kStepWarps + 1][68] = c.sm->seg[i];
+    float mm = -1e30f, ll = 0.f, oo = 0.f;
+#pragma unroll
+    for (int w = 0; w <= kStepWarps; ++w) mm = fmaxf(mm, seg[w][0]);
+#pragma unroll
+    for (int w = 0; w <= kStepWarps; ++w) {      // (a warp without rows: m = -1e30, l = o = 0)
+      const float f = ex2_approx(seg[w][0] - mm);
+      ll = fmaf(seg[w][1], f, ll);
+      oo = fmaf(seg[w][4 + e], f, oo);
+    }
+    bool write = true;
+    if (splits > 1) {                        // (then the CTA has one unit)
+      float* po = p.part_o + un.pair * splits * 64 + e;
+      float2* pm = p.part_ml + un.pair * splits;
+      __stcg(po + un.slot * 64, oo);
+      if (e == 0) __stcg(pm + un.slot, make_float2(mm, ll));
+      __threadfence();
+      asm volatile("bar.sync 2, 64;" ::: "memory");
+      if (e == 0) c.sm->seg_last = atomicAdd(p.arrived + un.pair, 1u) + 1 == splits;
+      asm volatile("bar.sync 2, 64;" ::: "memory");
+      write = c.sm->seg_last;
+      if (write) {                               // all partials are in: merge them
+        __threadfence();
+        if (e == 0) p.arrived[un.pair] = 0;
+        mm = -1e30f; ll = 0.f; oo = 0.f;
+#pragma unroll 1
+        for (int k = 0; k < splits; ++k) {
+          const float2 ml = __ldcg(pm + k);
+          const float v = __ldcg(po + k * 64);
+          const float m_new = fmaxf(mm, ml.x), f = ex2_approx(mm - m_new), fi = ex2_approx(ml.x - m_new);
+          ll = ll * f + ml.y * fi;
+          oo = oo * f + v * fi;
+          mm = m_new;
+        }
+      }
+    }
+    if (write) step_put(p.ctx + un.out + (e >> 5) * p.M * 32 + (e & 31), __fdividef(oo, ll), gen);
+  }
+  return c;
+}
+
+// Pulls a layer's vectors into L2, spread over the grid: nobody should be the first to touch them
+// between two exchanges.
+__device__ __forceinline__ void step_prefetch(const StepSmem& sm, const StepParams& p, int layer) {
+  const int tid = step_tid();
+  const StepLayer& L = sm.layers[layer];
+  const int at = (blockIdx.x + tid * gridDim.x) * 64;        // 64 elements per 128-byte line
+  if (at < 4 * p.C) {
+    prefetch_l2(L.fc_b + at);
+    if (at < 3 * p.C && L.qkv_b) prefetch_l2(L.qkv_b + at);
+    if (at < p.C) {
+      prefetch_l2(L.ln1_g + at); prefetch_l2(L.ln1_b + at); prefetch_l2(L.ln2_g + at); prefetch_l2(L.ln2_b + at);
+      prefetch_l2(L.proj_b + at); prefetch_l2(L.out_b + at);
+    }
+  }
+}
+
+// Streaming warp `sw`: its quarter of this CTA's rows of one matrix into the ring.
+__device__ __forceinline__ bool step_stream(StepSmem& sm, StepRing& ring, uint32_t& issued, const __nv_bfloat16* w, int op,
+                                            int C, int sw) {
+  const StepCut cut = sm.cut[op];
+  const StepPass pass(C);
+  const int passes = op == kStepOut ? 4 : 1;
+  const long long ldw = static_cast<long long>(passes) * C;
+  w += (cut.row0 + sw) * ldw;
+#pragma unroll 1
+  for (int t = 0; t < cut.tiles; ++t) {
+    // rows sw, sw + 4, ... of the tile
+    const int rows = (min(cut.tile, cut.rows - t * cut.tile) - sw + kStepStreamWarps - 1) / kStepStreamWarps;
+    const __nv_bfloat16* src = w + t * cut.tile * ldw;
+    int in_pass = 0;
+#pragma unroll 1
+    for (int k = 0; k < passes * pass.total;) {
+      const int units = min(pass.units, pass.total - in_pass);       // chunks never cross the end of a pass
+      if (issued >= kStepStages &&
+          !step_wait(smem_u32(&sm.empty[ring.stage]), ring.parity ^ 1, sm, kWaitStepEmpty))
+        return false;
+      if (elect_one()) {
+        fence_proxy_async_smem();                // (the stage may have held cached rows, written by plain copies)
+        const uint32_t bytes = static_cast<uint32_t>(units) * 64;
+        const uint32_t bar = smem_u32(&sm.full[ring.stage]);
+        uint32_t dst = smem_u32(sm.ring[ring.stage]) + sw * pass.pitch;
+        mbar_arrive_expect_tx(bar, bytes * rows);
+#pragma unroll
+        for (int r = 0; r < kStepTile / kStepStreamWarps; ++r)
+          if (r < rows) bulk_load(dst + r * kStepStreamWarps * pass.pitch, src + r * kStepStreamWarps * ldw, bytes, bar);
+      }
+      __syncwarp();
+      ring.next();
+      ++issued;
+      k += units;
+      src += units * kStepUnit;
+      in_pass += units;
+      if (in_pass == pass.total) in_pass = 0;
+    }
+  }
+  return true;
+}
+
+// The cached rows of this CTA's attention units in a layer, kStepBlocks * 16 rows of K and then of V
+// per stage, every fourth group of four rows by streaming warp `sw`.  Odd rows have their 64-byte
+// halves swapped.  Rows past the end are the last row again.
+__device__ __forceinline__ bool step_stream_rows(StepSmem& sm, const StepParams& p, StepRing& ring, uint32_t& issued,
+                                                 int layer, int sw, int lane) {
+  const int chunk = lane & 7, first = sw * 4 + (lane >> 3);    // four rows of eight 16-byte chunks per copy
+  const uint32_t off = first * 128 + ((chunk ^ ((first & 1) << 2)) * 16);
+#pragma unroll 1
+  for (int i = 0; i < sm.units; ++i) {
+    const StepUnit& un = sm.unit[i];
+    const long long at = un.head + static_cast<long long>(un.row0) * p.c_sn + chunk * 8;
+    const __nv_bfloat16 *kb = p.k_cache[layer] + at, *vb = p.v_cache[layer] + at;
+#pragma unroll 1
+    for (int r = 0; r < un.rows; r += kStepBlocks * 16) {
+      if (issued >= kStepStages &&
+          !step_wait(smem_u32(&sm.empty[ring.stage]), ring.parity ^ 1, sm, kWaitStepEmpty))
+        return false;
+      const uint32_t dst = smem_u32(sm.ring[ring.stage]) + off, bar = smem_u32(&sm.full[ring.stage]);
+      const int rows = min(kStepBlocks * 16, (un.rows - r + 15) & ~15);
+#pragma unroll 2
+      for (int j = 0; j < rows; j += 4 * kStepStreamWarps) {
+        const long long row = static_cast<long long>(min(r + j + first, un.rows - 1)) * p.c_sn;
+        cp_async_16(dst + j * 128, kb + row);
+        cp_async_16(dst + (kStepBlocks * 16 + j) * 128, vb + row);
+      }
+      cp_async_arrive(bar);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+      ring.next();
+      ++issued;
+    }
+  }
+  return true;
+}
+
+__global__ void __launch_bounds__(kStepThreads, 1) fa_gpt_step_kernel(const __grid_constant__ StepParams p) {
+  extern __shared__ uint8_t step_raw[];
+  StepSmem& sm = *reinterpret_cast<StepSmem*>(step_raw + ((128u - (smem_u32(step_raw) & 127u)) & 127u));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int C = p.C, M = p.M;
+  const long long pos64 = p.pos_ptr ? *p.pos_ptr : static_cast<long long>(p.pos);
+  const uint32_t generation = *p.generation;
+  const int last = min(p.cache_rows, p.n_positions) - 1;
+  const int pos = pos64 < 0 ? 0 : (pos64 > last ? last : static_cast<int>(pos64));
+  const StepAttnCut cut(M * p.H, pos);
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStepStages; ++i) {
+      mbar_init(smem_u32(&sm.full[i]), kStepStreamWarps);
+      mbar_init(smem_u32(&sm.empty[i]), kStepWarps);
+    }
+    sm.abort = 0;
+    sm.abort_who = 0;
+    fence_mbar_init();
+    if (blockIdx.x == 0) {                       // used at the very end, by CTAs that depend on this one's output
+      *p.done = 0;
+      for (int t = 0; t < kStepMaxRows; ++t) p.best[t] = 0ull;
+      __threadfence();
+    }
+  }
+  {
+    constexpr int kPtrs = sizeof(StepLayer) / sizeof(void*);
+    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(p.layers);
+    unsigned long long* dst = reinterpret_cast<unsigned long long*>(sm.layers);
+    for (int i = threadIdx.x; i < p.n_layers * kPtrs; i += kStepThreads) dst[i] = src[i];
+  }
+  if (threadIdx.x == 0) {
+    sm.units = cut.count;
+    sm.splits = cut.splits;
+  }
+  if (threadIdx.x < kStepMaxRows) sm.shift[threadIdx.x] = 0.f;
+  if (static_cast<int>(threadIdx.x) < cut.count) {
+    const int u = cut.first + threadIdx.x, pair = u / cut.splits, part = u - pair * cut.splits;
+    const int b = pair / p.H, h = pair - b * p.H;
+    StepUnit un;
+    un.pair = pair;
+    un.slot = part;
+    un.row0 = static_cast<int>(static_cast<long long>(part) * cut.rows / cut.splits);
+    un.rows = static_cast<int>(static_cast<long long>(part + 1) * cut.rows / cut.splits) - un.row0;
+    un.head = b * p.c_sb + static_cast<long long>(h) * p.c_sh;
+    un.query = b * 3 * C + h * 64;
+    un.out = (2 * h * M + b) * 32;
+    sm.unit[threadIdx.x] = un;
+  }
+  if (threadIdx.x < 5) {
+    const int op = threadIdx.x;
+    sm.cut[op] = step_cut(op == kStepQkv ? 3 * C : (op == kStepFc ? 4 * C : (op == kStepHead ? p.V : C)));
+  }
+  __syncthreads();
+
+  if (warp >= kStepWarps) {
+    reg_dealloc<kStepStreamRegs>();              // all four warps of the warpgroup
+    // ------------------------------------------------------------------ stream
+    StepRing ring;
+    uint32_t issued = 0;
+    bool ok = true;
+#pragma unroll 1
+    for (int i = 0; i <= 4 * p.n_layers && ok; ++i) {
+      const StepLayer& L = sm.layers[min(i >> 2, p.n_layers - 1)];
+      const int op = i == 4 * p.n_layers ? static_cast<int>(kStepHead) : (i & 3);
+      ok = step_stream(sm, ring, issued,
+                       op == kStepQkv ? L.qkv_w : (op == kStepProj ? L.proj_w : (op == kStepFc ? L.fc_w : (op == kStepOut ? L.out_w : p.head_w))),
+                       op, C, warp - kStepWarps);
+      if (ok && op == kStepQkv) ok = step_stream_rows(sm, p, ring, issued, i >> 2, warp - kStepWarps, lane);
+    }
+    // leave no copy in flight, whatever the computing warps did: the last use of every stage
+#pragma unroll 1
+    for (uint32_t i = 0; i < kStepStages && i < issued; ++i)
+      step_wait(smem_u32(&sm.full[(issued - 1 - i) % kStepStages]), ((issued - 1 - i) / kStepStages) & 1, sm, kWaitDrain);
+  } else {
+    reg_alloc<kStepComputeRegs>();
+    // ------------------------------------------------------------------ computing warps
+    StepCta c;
+    c.sm = &sm;
+    c.ok = true;
+    {  // this CTA's columns of the residual stream: the embeddings' sum (see the outputs in step_gemm)
+      const int tok = threadIdx.x & 7, row = threadIdx.x >> 3, n = sm.cut[kStepProj].row0 + row;
+      if (row < sm.cut[kStepProj].rows && tok < M) {      // one tile, at most 16 rows
+        long long id = p.ids[tok * p.ids_stride];
+        id = id < 0 ? 0 : (id >= p.V ? p.V - 1 : id);
+        const float v = __bfloat162float(__float2bfloat16_rn(
+            __bfloat162float(p.tok_emb[id * C + n]) + __bfloat162float(p.pos_emb[static_cast<long long>(pos) * C + n])));
+        sm.own[threadIdx.x] = v;
+        step_put(p.x_mlp + tok * C + n, v, generation % 65535u + 1u);
+      }
+    }
+    step_prefetch(sm, p, 0);
+#pragma unroll 1
+    for (int i = 0; i <= 4 * p.n_layers; ++i) {
+      const int l = min(i >> 2, p.n_layers - 1);
+      const int op = i == 4 * p.n_layers ? static_cast<int>(kStepHead) : (i & 3);
+      const StepLayer& L = sm.layers[l];
+      const uint32_t before = (generation + l) % 65535u + 1u, gen = (generation + l + 1) % 65535u + 1u;
+      const uint32_t* src = nullptr;
+      const __nv_bfloat16* bias = op == kStepQkv ? L.qkv_b : (op == kStepProj ? L.proj_b : (op == kStepFc ? L.fc_b : (op == kStepOut ? L.out_b : nullptr)));
+      step_bar();                                // the reductions of the operation before are read
+      if (op & 1) {
+        src = op == kStepProj ? p.ctx : p.h;
+      } else {
+        step_fetch_norm(sm, op == kStepQkv ? L.ln1_g : (op == kStepFc ? L.ln2_g : p.lnf_g),
+                        op == kStepQkv ? L.ln1_b : (op == kStepFc ? L.ln2_b : p.lnf_b), C >> 3);
+        c = step_layernorm(c, p, op == kStepFc ? p.x_att : p.x_mlp, op == kStepQkv ? before : gen);
+      }
+      c = step_gemm(c, p, src, op, l, pos, gen, bias);
+      if (op == kStepQkv && sm.units > 0) {
+        step_bar();
+        c = step_attention(c, p, l, gen);
+      }
+      if (op == kStepOut && l + 1 < p.n_layers) step_prefetch(sm, p, l + 1);
+    }
+    if (p.next_ids) {
+      step_bar();
+      if (warp == 0) {
+        if (lane < M) {
+          unsigned long long key = 0ull;
+#pragma unroll
+          for (int w = 0; w < kStepWarps; ++w) key = sm.keys[w][lane] > key ? sm.keys[w][lane] : key;
+          atomicMax(p.best + lane, key);
+        }
+        __threadfence();
+        __syncwarp();
+        if (lane == 0 && atomicAdd(p.done, 1u) + 1 == gridDim.x) {   // the last CTA: all keys are in
+          __threadfence();
+          for (int t = 0; t < M; ++t)
+            p.next_ids[t * p.next_stride] = static_cast<long long>(0xffffffffu - static_cast<uint32_t>(__ldcg(p.best + t)));
+        }
+      }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {   // everyone has read these: their output is in ours
+      *p.generation = generation + p.n_layers + 1;
+      if (p.pos_ptr && p.advance) {
+        *p.pos_ptr = pos64 + 1;
+        if (p.len_ptr) *p.len_ptr = static_cast<int>(pos64) + 2;
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && sm.abort != 0) {
+    if (atomicCAS(p.status, 0u, sm.abort) == 0u) {
+      p.status[1] = blockIdx.x;
+      p.status[2] = sm.abort_who & 0xffffu;
+      p.status[3] = sm.abort_who >> 16;
+    }
+  }
+}
+
+}  // namespace fa

@@ -46,6 +46,8 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from .step import StepPlan
+
 GPT2_SIZES = {   # model_inference.py:392-397
     "gpt2-small": {"emb_dim": 768, "n_layers": 12, "n_heads": 12},
     "gpt2-medium": {"emb_dim": 1024, "n_layers": 24, "n_heads": 16},
@@ -284,6 +286,7 @@ class GPTModel(nn.Module):
         self.out_head = nn.Linear(cfg["emb_dim"], cfg["vocab_size"], bias=False)
         self._head_w = None     # out_head weight padded to a multiple of 64 rows (inference cache)
         self._fused_blocks = False   # residual add + LayerNorm through block_ops.add_layernorm
+        self._step_plan = None       # single-token steps as one kernel launch (step.StepPlan)
         if dtype is not None:
             self.to(dtype)
 
@@ -303,6 +306,7 @@ class GPTModel(nn.Module):
                               and d % 8 == 0 and d <= 2048 and self.cfg["drop_rate"] == 0.0)
         for blk in self.trf_blocks:      # single-token steps: Linear layers as one pass over the weights
             blk.att.small_linear = blk.ff.small_linear = self._fused_blocks
+        self._step_plan = StepPlan.make(self) if self._fused_blocks else None
         return self
 
     def invalidate_inference_cache(self):
@@ -312,7 +316,24 @@ class GPTModel(nn.Module):
             blk.att.small_linear = blk.ff.small_linear = False
         self._head_w = None
         self._fused_blocks = False
+        self._step_plan = None
         return self
+
+    def _apply(self, fn, *args, **kwargs):      # .to(), .cuda(), .half(): the parameters move
+        self._step_plan = None
+        return super()._apply(fn, *args, **kwargs)
+
+    def _step(self, in_idx, kv_caches, pos, **kw):
+        """Logits of a single-token step through the one-launch kernel, or None when this model, batch
+        or cache is not one for it."""
+        plan = self._step_plan
+        if plan is None or self.training or kv_caches is None or not in_idx.is_cuda:
+            return None
+        if not plan.current():                  # a parameter was replaced
+            plan = self._step_plan = StepPlan.make(self)
+            if plan is None:
+                return None
+        return plan.step(in_idx, kv_caches, pos, **kw)
 
     def allocate_kv_cache(self, batch, max_len=None, dtype=None):
         """One (K, V) pair of [B, N_max, H, d] tensors per layer, in the model's device; bf16 when
@@ -417,20 +438,30 @@ class GPTModel(nn.Module):
             for _ in range(warmup):
                 self(static_ids, kv_caches=kv_caches, pos=position)
         torch.cuda.current_stream(dev).wait_stream(side)
+        workspace = None if self._step_plan is None else self._step_plan.new_workspace(batch)
+        torch.cuda.current_stream(dev).synchronize()
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
-            static_logits = self(static_ids, kv_caches=kv_caches, pos=position)
-            position.advance()
+            # the one-launch step moves the position on itself
+            static_logits = self._step(static_ids, kv_caches, position, advance=True, workspace=workspace)
+            if static_logits is None:
+                static_logits = self(static_ids, kv_caches=kv_caches, pos=position)
+                position.advance()
 
         def step(ids):
             static_ids.copy_(ids)
             graph.replay()
             return static_logits
         step.graph = graph
+        step.workspace = workspace
         return step, position
 
     def forward(self, in_idx, last_token_only=False, kv_caches=None, pos=0):
         _, n = in_idx.shape
+        if n == 1 and self._step_plan is not None:
+            logits = self._step(in_idx, kv_caches, pos)
+            if logits is not None:
+                return logits
         if isinstance(pos, DevicePosition):
             x = self.tok_emb(in_idx) + self.pos_emb(pos.index)
         else:
@@ -501,7 +532,23 @@ def generate(model, idx, max_new_tokens, context_size, temperature=1.0, top_k=No
             caches = model.allocate_kv_cache(idx.shape[0], context_size)
             if cuda_graph:
                 step_fn, position = model.capture_decode_step(caches)
+    greedy = None         # [B, prompt + new] ids that the one-launch step extends by itself
+    if use_cache and temperature <= 0.0 and max_new_tokens > 1 and isinstance(model, GPTModel) and model._step_plan is not None:
+        greedy = torch.empty(idx.shape[0], idx.shape[1] + max_new_tokens, dtype=torch.long, device=idx.device)
     for step in range(max_new_tokens):
+        if greedy is not None and step > 0:
+            # the step kernel reads its token from, and leaves the argmax of its logits in, a column
+            n = idx.shape[1]
+            if (pos + 1 <= context_size
+                    and model._step(greedy[:, n - 1:n], caches, pos, next_ids=greedy[:, n]) is not None):
+                pos += 1
+                if eos_id is not None and idx.shape[0] == 1 and int(greedy[0, n]) == eos_id:
+                    break
+                idx = greedy[:, :n + 1]
+                continue
+            greedy = None
+            if position is not None:
+                position.set(pos)
         if use_cache and step > 0 and pos + 1 > context_size:
             use_cache = False              # the cache is full: recompute over the sliding window from here on
         if use_cache and step > 0 and step_fn is not None:
@@ -527,7 +574,9 @@ def generate(model, idx, max_new_tokens, context_size, temperature=1.0, top_k=No
         if eos_id is not None and idx.shape[0] == 1 and int(idx_next) == eos_id:   # as the reference, :224
             break
         idx = torch.cat((idx, idx_next), dim=1)
-    return idx
+        if greedy is not None:
+            greedy[:, :idx.shape[1]] = idx
+    return idx.contiguous()
 
 
 def init_random(model: GPTModel, seed: int, std: float = 0.02) -> GPTModel:

@@ -1,0 +1,173 @@
+"""The single-token step of a GPT-2 model as one kernel launch (fa_b200_gpt_step).
+
+A `StepPlan` is what the launch needs of a model: the table of its parameters' addresses on the GPU
+and, per stream, a workspace.  gpt2.GPTModel makes one in prepare_for_inference() and uses it for
+every forward of one token per sequence against K/V caches that the kernel can take; other shapes
+go layer by layer.
+"""
+from __future__ import annotations
+
+import ctypes
+from collections import OrderedDict
+
+import torch
+
+from . import _lib
+
+MAX_BATCH = 8
+MAX_PAIRS = 256            # sequences x heads
+MAX_LAYERS = 64
+MAX_WIDTH = 1600
+MAX_WORKSPACES = 8         # streams that keep a workspace (about 1 MB each)
+
+
+class StepPlan:
+    """Parameter table of one prepared bf16 model.  `make` returns None for a model the kernel does
+    not take."""
+
+    @classmethod
+    def make(cls, model):
+        cfg = model.cfg
+        width, heads, layers = cfg["emb_dim"], cfg["n_heads"], cfg["n_layers"]
+        if width != 64 * heads or width > MAX_WIDTH or not 1 <= layers <= MAX_LAYERS or heads > MAX_PAIRS:
+            return None
+        plan = cls()
+        owned = []           # (module's parameter dict, name, tensor): what the table was built from
+        rows = []
+
+        def take(module, name, shape, optional=False):
+            t = module._parameters[name]
+            owned.append((module._parameters, name, t))
+            if t is None:
+                if not optional:
+                    raise TypeError(name)
+                return 0
+            return plan._address(t, shape)
+
+        try:
+            for blk in model.trf_blocks:
+                att, fc, out = blk.att, blk.ff.layers[0], blk.ff.layers[2]
+                row = [take(blk.norm1, "scale", (width,)), take(blk.norm1, "shift", (width,)),
+                       plan._address(att._qkv_w, (3 * width, width)),
+                       0 if att._qkv_b is None else plan._address(att._qkv_b, (3 * width,)),
+                       take(att.out_proj, "weight", (width, width)), take(att.out_proj, "bias", (width,)),
+                       take(blk.norm2, "scale", (width,)), take(blk.norm2, "shift", (width,)),
+                       take(fc, "weight", (4 * width, width)), take(fc, "bias", (4 * width,)),
+                       take(out, "weight", (width, 4 * width)), take(out, "bias", (width,))]
+                if blk.norm1.eps != model.final_norm.eps or blk.norm2.eps != model.final_norm.eps:
+                    return None
+                rows.append(row)
+            plan.vocab = model.out_head.weight.shape[0]
+            plan.positions = model.pos_emb.weight.shape[0]
+            ends = [take(model.tok_emb, "weight", (plan.vocab, width)),
+                    take(model.pos_emb, "weight", (plan.positions, width)),
+                    take(model.final_norm, "scale", (width,)), take(model.final_norm, "shift", (width,)),
+                    take(model.out_head, "weight", (plan.vocab, width))]
+        except TypeError:
+            return None
+        plan.owned = owned
+        plan.qkv = [(blk.att, blk.att._qkv_w) for blk in model.trf_blocks]
+        plan.heads, plan.layers, plan.eps = heads, layers, model.final_norm.eps
+        plan.device = model.tok_emb.weight.device
+        plan.table = torch.tensor(rows, dtype=torch.int64).to(plan.device)
+        plan.ends = ends
+        plan.workspaces = OrderedDict()
+        return plan
+
+    @staticmethod
+    def _address(t, shape):
+        if (not t.is_cuda or t.dtype != torch.bfloat16 or tuple(t.shape) != shape or not t.is_contiguous()
+                or t.data_ptr() % 16):
+            raise TypeError("not a dense bf16 CUDA parameter of the expected shape")
+        return t.data_ptr()
+
+    def current(self):
+        """False when a parameter object has been replaced since the table was built."""
+        for params, name, t in self.owned:
+            if params[name] is not t:
+                return False
+        for att, w in self.qkv:
+            if att._qkv_w is not w:
+                return False
+        return True
+
+    def _caches(self, kv_caches, batch):
+        """The caches' addresses and common shape, or None when the kernel cannot take them."""
+        if len(kv_caches) != self.layers:
+            return None
+        k0 = kv_caches[0][0]
+        shape, stride = k0.shape, k0.stride()
+        if (k0.dim() != 4 or shape[0] != batch or shape[2] != self.heads or shape[3] != 64 or stride[3] != 1
+                or k0.device != self.device):
+            return None
+        table = (ctypes.c_void_p * (2 * self.layers))()
+        for i, pair in enumerate(kv_caches):
+            for j in (0, 1):
+                t = pair[j]
+                if t.dtype != torch.bfloat16 or t.shape != shape or t.stride() != stride or not t.is_cuda:
+                    return None
+                table[j * self.layers + i] = t.data_ptr()
+        if any(s % 8 for s in stride[:3]) or any(s <= 0 for s in stride[:3]):
+            return None
+        return table, shape[1], stride
+
+    def new_workspace(self, batch):
+        need = _lib.load().fa_b200_gpt_step_workspace_bytes(batch, self.heads)
+        return torch.zeros(need, dtype=torch.uint8, device=self.device)
+
+    def _workspace(self, batch, stream):
+        """A zeroed workspace that only this stream uses (a launch leaves its counters at zero)."""
+        if torch.cuda.is_current_stream_capturing():
+            return self.new_workspace(batch)     # belongs to the graph
+        key = (stream, batch)
+        ws = self.workspaces.get(key)
+        if ws is None:
+            ws = self.workspaces[key] = self.new_workspace(batch)
+            while len(self.workspaces) > MAX_WORKSPACES:
+                self.workspaces.popitem(last=False)
+        return ws
+
+    def step(self, ids, kv_caches, pos, advance=False, next_ids=None, workspace=None):
+        """Logits [B, 1, vocab] of one new token per sequence, or None when this call is not one for
+        the kernel.  `ids` int64 [B, 1]; `pos` an int or a gpt2.DevicePosition (which `advance`
+        moves on); `next_ids` int64 [B] (any stride) receives the argmax of each row."""
+        batch = ids.shape[0]
+        if not 1 <= batch <= MAX_BATCH or batch * self.heads > MAX_PAIRS or ids.device != self.device:
+            return None
+        found = self._caches(kv_caches, batch)
+        if found is None:
+            return None
+        table, rows, stride = found
+        on_device = not isinstance(pos, int)
+        if not on_device and not 0 <= pos < min(rows, self.positions):
+            return None
+        if ids.dtype != torch.int64:
+            ids = ids.long()
+        stream = torch.cuda.current_stream(self.device).cuda_stream
+        ws = self._workspace(batch, stream) if workspace is None else workspace
+        logits = torch.empty(batch, 1, self.vocab, dtype=torch.bfloat16, device=self.device)
+        p = _lib.FaGptStepParams()
+        p.layers = self.table.data_ptr()
+        p.tok_emb, p.pos_emb, p.lnf_scale, p.lnf_shift, p.head_w = self.ends
+        p.ids, p.ids_stride = ids.data_ptr(), ids.stride(0)
+        if on_device:
+            p.pos_device, p.length_device = pos.index.data_ptr(), pos.length.data_ptr()
+        else:
+            p.pos = pos
+        p.advance = 1 if advance else 0
+        p.k_cache = ctypes.addressof(table)
+        p.v_cache = ctypes.addressof(table) + 8 * self.layers
+        p.cache_strides[0], p.cache_strides[1], p.cache_strides[2] = stride[0], stride[1], stride[2]
+        if batch == 1:
+            p.cache_strides[0] = 64              # never used to address anything
+        p.logits = logits.data_ptr()
+        if next_ids is not None:
+            p.next_ids, p.next_stride = next_ids.data_ptr(), next_ids.stride(0)
+        p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
+        p.n_layers, p.B, p.H, p.vocab = self.layers, batch, self.heads, self.vocab
+        p.cache_rows, p.n_positions, p.eps = rows, self.positions, self.eps
+        p.device, p.stream = self.device.index, stream
+        rc = _lib.load().fa_b200_gpt_step(ctypes.byref(p))
+        if rc != 0:
+            raise RuntimeError(f"generation step failed ({rc}): {_lib.strerror(rc)}")
+        return logits
