@@ -11,7 +11,7 @@ import ctypes
 
 import torch
 
-from . import _lib
+from . import _lib, custom_flash_attn
 
 __all__ = ["add_layernorm", "linear_small", "LINEAR_SMALL_MAX_ROWS"]
 
@@ -31,6 +31,9 @@ def add_layernorm(a, resid, scale, shift, eps: float = 1e-5, return_sum: bool = 
     """`s = a + resid` (resid may be None), `y = LayerNorm(s) * scale + shift` over the last
     dimension, one pass.  Returns `(s, y)` when `return_sum` and a residual is given, else `y`.
     The normalised row is the bf16-rounded sum (what a later reader of `s` sees)."""
+    ext = custom_flash_attn.extension()
+    if ext is not None:
+        return ext.add_layernorm(a, resid, scale, shift, eps, return_sum, sum_out, norm_out)
     cols = a.shape[-1]
     _dense2d(a, "a", cols)
     if resid is not None:

@@ -1,8 +1,12 @@
-// pybind11 / torch-extension binding of the attention forward: the compiled counterpart of the
-// reference's src/cpp/torch_bind.cpp:21-49 (`PYBIND11_MODULE ... m.def("forward", ...)`), in front
-// of this library's C ABI (include/fa_b200.h) instead of the reference's launcher template.
+// Python binding of the library's entry points that a program calls per layer or per token: the
+// compiled counterpart of the reference's src/cpp/torch_bind.cpp:21-49 (`PYBIND11_MODULE ...
+// m.def("forward", ...)`), in front of this library's C ABI (include/fa_b200.h) instead of the
+// reference's launcher template.
 //
 //   forward(Q, K_mat, V, causal=True, return_lse=False, softmax_scale=None, out=None)
+//   decode(Q, K_cache, V_cache, kv_len, return_lse=False, softmax_scale=None, out=None,
+//          k_new=None, v_new=None)
+//   add_layernorm(a, resid, scale, shift, eps=1e-5, return_sum=True, sum_out=None, norm_out=None)
 //
 // Three positional tensors behave as the reference's binding: CUDA + bfloat16 checked the same way
 // (CHECK_CUDA / the dtype branch, torch_bind.cpp:13-19, 33-42), O = empty_like(Q) (:31), causal,
@@ -11,22 +15,98 @@
 // launch goes to the current stream of Q's device, the GIL is released around the library call,
 // and the library's error code becomes a RuntimeError (the reference drops its cudaError_t).
 // PyTorch is used for what it owns: tensors, the current device and stream.
+//
+// The functions are plain CPython vector calls: for the smallest problems the call IS the time, and
+// pybind11's argument casters cost about as much as the launch (a decode call through ctypes: 31-38
+// us of host time for 4-9 us of GPU work).
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
 #include <torch/extension.h>
 
 #include "../../include/fa_b200.h"
 
 namespace {
 
-// Argument and library errors leave as std::runtime_error, which pybind11 turns into the same
+// Argument and library errors leave as std::runtime_error, which `guarded` turns into the same
 // Python RuntimeError that TORCH_CHECK produces in the reference binding.
 #define FA_CHECK(cond, ...)                                        \
   do {                                                             \
     if (!(cond)) throw std::runtime_error(c10::str(__VA_ARGS__)); \
   } while (0)
 
-void check_input(const torch::Tensor& t, const char* name) {
+struct TypeError : std::runtime_error {
+  using std::runtime_error::runtime_error;
+};
+struct PythonError {};      // the Python error is set already
+
+template <class F>
+PyObject* guarded(F f) {
+  try {
+    return f();
+  } catch (const PythonError&) {
+    return nullptr;
+  } catch (const TypeError& e) {
+    PyErr_SetString(PyExc_TypeError, e.what());
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  }
+  return nullptr;
+}
+
+// Positional and keyword arguments into `out` by the order of `names`; missing ones stay null.
+template <size_t kN>
+void take_args(const char* fn, const char* const (&names)[kN], size_t required, PyObject* const* args, Py_ssize_t nargs,
+               PyObject* kwnames, PyObject* (&out)[kN]) {
+  if (nargs > static_cast<Py_ssize_t>(kN)) throw TypeError(c10::str(fn, "() takes at most ", kN, " arguments"));
+  for (size_t i = 0; i < kN; ++i) out[i] = i < static_cast<size_t>(nargs) ? args[i] : nullptr;
+  const Py_ssize_t nkw = kwnames ? PyTuple_GET_SIZE(kwnames) : 0;
+  for (Py_ssize_t k = 0; k < nkw; ++k) {
+    PyObject* name = PyTuple_GET_ITEM(kwnames, k);
+    size_t i = 0;
+    while (i < kN && PyUnicode_CompareWithASCIIString(name, names[i]) != 0) ++i;
+    if (i == kN) throw TypeError(c10::str(fn, "() got an unexpected keyword argument"));
+    if (out[i] != nullptr) throw TypeError(c10::str(fn, "() got multiple values for argument '", names[i], "'"));
+    out[i] = args[nargs + k];
+  }
+  for (size_t i = 0; i < required; ++i)
+    if (out[i] == nullptr) throw TypeError(c10::str(fn, "() missing required argument '", names[i], "'"));
+}
+const at::Tensor& tensor_arg(PyObject* o, const char* name) {
+  if (!THPVariable_Check(o)) throw TypeError(c10::str(name, " must be a torch.Tensor"));
+  return THPVariable_Unpack(o);
+}
+bool given(PyObject* o) { return o != nullptr && o != Py_None; }
+bool flag_arg(PyObject* o, bool absent) {
+  if (o == nullptr) return absent;
+  const int v = PyObject_IsTrue(o);
+  if (v < 0) throw PythonError();
+  return v != 0;
+}
+double number_arg(PyObject* o, double absent) {
+  if (!given(o)) return absent;
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) throw PythonError();
+  return v;
+}
+PyObject* pair(const at::Tensor& a, const at::Tensor& b) {
+  PyObject* t = PyTuple_New(2);
+  if (t == nullptr) throw PythonError();
+  PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(a));
+  PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(b));
+  return t;
+}
+template <class Call>
+void launch(const char* what, Call call) {
+  int rc;
+  {
+    py::gil_scoped_release release;
+    rc = call();
+  }
+  FA_CHECK(rc == 0, what, " failed (", rc, "): ", fa_b200_strerror(rc));
+}
+
+void check_input(const at::Tensor& t, const char* name) {
   FA_CHECK(t.device().is_cuda(), name, " must be a CUDA tensor");
   FA_CHECK(t.scalar_type() == torch::kBFloat16, "Unsupported tensor dtype. Use bfloat16.");
   FA_CHECK(t.dim() == 4, name, " must have shape [B, H, N, d]");
@@ -34,7 +114,7 @@ void check_input(const torch::Tensor& t, const char* name) {
 
 // Element strides {batch, head, row}; strides of size-1 dimensions are never dereferenced, so they
 // are replaced by a canonical value that always passes the library's checks.
-void strides3(const torch::Tensor& t, const char* name, int64_t out[3]) {
+void strides3(const at::Tensor& t, const char* name, int64_t out[3]) {
   const int64_t H = t.size(1), N = t.size(2), d = t.size(3);
   FA_CHECK(d <= 1 || t.stride(3) == 1, name, ": the last dimension must be dense (stride 1)");
   int64_t sb = t.stride(0), sh = t.stride(1), sn = t.stride(2);
@@ -44,63 +124,222 @@ void strides3(const torch::Tensor& t, const char* name, int64_t out[3]) {
   out[0] = sb; out[1] = sh; out[2] = sn;
 }
 
-py::object forward(const torch::Tensor& Q, const torch::Tensor& K_mat, const torch::Tensor& V, bool causal,
-                   bool return_lse, const c10::optional<double>& softmax_scale,
-                   const c10::optional<torch::Tensor>& out) {
-  check_input(Q, "Q");
-  check_input(K_mat, "K_mat");
-  check_input(V, "V");
-  FA_CHECK(K_mat.sizes() == Q.sizes() && V.sizes() == Q.sizes(),
-              "Q, K_mat and V must have the same shape [B, H, N, d]");
-  FA_CHECK(K_mat.device() == Q.device() && V.device() == Q.device(),
-              "Q, K_mat and V must be on the same device");
-  torch::Tensor O;
-  if (out.has_value()) {
-    check_input(*out, "out");
-    FA_CHECK(out->sizes() == Q.sizes() && out->device() == Q.device(), "out must match Q in shape and device");
-    O = *out;
-  } else {
-    O = torch::empty_like(Q);   // same allocation rule as the reference (torch_bind.cpp:31)
-  }
-  const c10::cuda::CUDAGuard guard(Q.device());
-  torch::Tensor lse;
-  if (return_lse) lse = torch::empty({Q.size(0), Q.size(1), Q.size(2)}, Q.options().dtype(torch::kFloat32));
+PyObject* forward(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+  return guarded([&]() -> PyObject* {
+    static const char* const names[] = {"Q", "K_mat", "V", "causal", "return_lse", "softmax_scale", "out"};
+    PyObject* a[7];
+    take_args("forward", names, 3, args, nargs, kwnames, a);
+    const at::Tensor &Q = tensor_arg(a[0], "Q"), &K_mat = tensor_arg(a[1], "K_mat"), &V = tensor_arg(a[2], "V");
+    const bool return_lse = flag_arg(a[4], false);
+    check_input(Q, "Q");
+    check_input(K_mat, "K_mat");
+    check_input(V, "V");
+    FA_CHECK(K_mat.sizes() == Q.sizes() && V.sizes() == Q.sizes(),
+             "Q, K_mat and V must have the same shape [B, H, N, d]");
+    FA_CHECK(K_mat.device() == Q.device() && V.device() == Q.device(),
+             "Q, K_mat and V must be on the same device");
+    at::Tensor O;
+    if (given(a[6])) {
+      O = tensor_arg(a[6], "out");
+      check_input(O, "out");
+      FA_CHECK(O.sizes() == Q.sizes() && O.device() == Q.device(), "out must match Q in shape and device");
+    } else {
+      O = at::empty_like(Q);   // same allocation rule as the reference (torch_bind.cpp:31)
+    }
+    at::Tensor lse;
+    if (return_lse) lse = at::empty({Q.size(0), Q.size(1), Q.size(2)}, Q.options().dtype(torch::kFloat32));
 
-  fa_b200_params p{};
-  p.B = static_cast<int32_t>(Q.size(0));
-  p.H = static_cast<int32_t>(Q.size(1));
-  p.N = static_cast<int32_t>(Q.size(2));
-  p.d = static_cast<int32_t>(Q.size(3));
-  if (Q.numel() > 0) {
-    p.q = Q.data_ptr(); p.k = K_mat.data_ptr(); p.v = V.data_ptr(); p.o = O.data_ptr();
-    strides3(Q, "Q", p.q_strides);
-    strides3(K_mat, "K_mat", p.k_strides);
-    strides3(V, "V", p.v_strides);
-    strides3(O, "out", p.o_strides);
-  } else {            // empty problem: nothing is read, any valid pointers and strides do
-    p.q = p.k = p.v = p.o = reinterpret_cast<void*>(16);
-    for (int i = 0; i < 3; ++i) p.q_strides[i] = p.k_strides[i] = p.v_strides[i] = p.o_strides[i] = 8;
-  }
-  p.lse = return_lse && Q.numel() > 0 ? lse.data_ptr<float>() : nullptr;
-  p.softmax_scale = softmax_scale.has_value() ? static_cast<float>(*softmax_scale) : 0.0f;
-  p.causal = causal ? 1 : 0;
-  p.device = Q.device().index();
-  p.stream = c10::cuda::getCurrentCUDAStream(Q.device().index()).stream();
-  int rc;
-  {
-    py::gil_scoped_release release;
-    rc = fa_b200_fwd(&p);
-  }
-  FA_CHECK(rc == 0, "custom_flash_attn.forward failed (", rc, "): ", fa_b200_strerror(rc));
-  if (return_lse) return py::make_tuple(O, lse);
-  return py::cast(O);
+    fa_b200_params p{};
+    p.B = static_cast<int32_t>(Q.size(0));
+    p.H = static_cast<int32_t>(Q.size(1));
+    p.N = static_cast<int32_t>(Q.size(2));
+    p.d = static_cast<int32_t>(Q.size(3));
+    if (Q.numel() > 0) {
+      p.q = Q.data_ptr(); p.k = K_mat.data_ptr(); p.v = V.data_ptr(); p.o = O.data_ptr();
+      strides3(Q, "Q", p.q_strides);
+      strides3(K_mat, "K_mat", p.k_strides);
+      strides3(V, "V", p.v_strides);
+      strides3(O, "out", p.o_strides);
+    } else {            // empty problem: nothing is read, any valid pointers and strides do
+      p.q = p.k = p.v = p.o = reinterpret_cast<void*>(16);
+      for (int i = 0; i < 3; ++i) p.q_strides[i] = p.k_strides[i] = p.v_strides[i] = p.o_strides[i] = 8;
+    }
+    p.lse = return_lse && Q.numel() > 0 ? lse.data_ptr<float>() : nullptr;
+    p.softmax_scale = static_cast<float>(number_arg(a[5], 0.0));
+    p.causal = flag_arg(a[3], true) ? 1 : 0;
+    p.device = Q.device().index();
+    p.stream = c10::cuda::getCurrentCUDAStream(Q.device().index()).stream();
+    launch("custom_flash_attn.forward", [&] { return fa_b200_fwd(&p); });
+    return return_lse ? pair(O, lse) : THPVariable_Wrap(O);
+  });
 }
+
+// [B, H, 1, 64] as [B, H, 64]
+at::Tensor one_row(const at::Tensor& t) { return t.dim() == 4 ? t.select(2, 0) : t; }
+
+// {batch, head} strides of [B, H, 64]; size-1 dimensions get a canonical stride
+void strides2(const at::Tensor& t, int64_t out[2]) {
+  out[1] = t.size(1) == 1 ? 64 : t.stride(1);
+  out[0] = t.size(0) == 1 ? std::max<int64_t>(t.size(1) * out[1], 64) : t.stride(0);
+}
+void cache_strides(const at::Tensor& t, int64_t out[3]) {
+  out[2] = t.size(2) == 1 ? 64 : t.stride(2);
+  out[1] = t.size(1) == 1 ? std::max<int64_t>(t.size(2) * out[2], 64) : t.stride(1);
+  out[0] = t.size(0) == 1 ? std::max<int64_t>(t.size(1) * out[1], 64) : t.stride(0);
+}
+
+PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+  return guarded([&]() -> PyObject* {
+    static const char* const names[] = {"Q", "K_cache", "V_cache", "kv_len", "return_lse", "softmax_scale", "out",
+                                        "k_new", "v_new"};
+    PyObject* a[9];
+    take_args("decode", names, 4, args, nargs, kwnames, a);
+    const at::Tensor &Q = tensor_arg(a[0], "Q"), &K = tensor_arg(a[1], "K_cache"), &V = tensor_arg(a[2], "V_cache");
+    const bool squeeze = Q.dim() == 4;
+    for (const auto& [t, name] : {std::pair<const at::Tensor&, const char*>{Q, "Q"}, {K, "K_cache"}, {V, "V_cache"}}) {
+      FA_CHECK(t.device().is_cuda(), name, " must be a CUDA tensor");
+      FA_CHECK(t.scalar_type() == torch::kBFloat16, "Unsupported tensor dtype. Use bfloat16.");
+    }
+    FA_CHECK(!squeeze || Q.size(2) == 1, "Q must hold one query row per head: [B, H, 64] or [B, H, 1, 64]");
+    FA_CHECK((squeeze || Q.dim() == 3) && K.dim() == 4 && V.dim() == 4, "expected Q [B, H, d] and caches [B, H, N, d]");
+    const at::Tensor q = squeeze ? Q.select(2, 0) : Q;
+    const int64_t B = q.size(0), H = q.size(1), d = q.size(2), rows = K.size(2);
+    FA_CHECK(K.size(0) == B && K.size(1) == H && V.sizes() == K.sizes() && K.size(3) == d,
+             "Q, K_cache and V_cache disagree on B, H or d");
+    fa_b200_decode_params p{};
+    int64_t kv_len = rows;
+    if (THPVariable_Check(a[3])) {
+      // the length lives on the device (an int32 scalar that the caller advances between steps): the
+      // launch is sized for the whole cache and the kernel reads the length when it runs, which is
+      // what lets one recorded CUDA-graph launch serve every step of a generation loop
+      const at::Tensor& n = THPVariable_Unpack(a[3]);
+      FA_CHECK(n.is_cuda() && n.scalar_type() == torch::kInt32 && n.numel() == 1,
+               "a tensor kv_len must be one int32 on the GPU");
+      p.kv_len_device = n.data_ptr<int32_t>();
+    } else {
+      kv_len = PyLong_Check(a[3]) ? PyLong_AsLongLong(a[3]) : static_cast<int64_t>(number_arg(a[3], 0.0));
+      if (kv_len == -1 && PyErr_Occurred()) throw PythonError();
+    }
+    FA_CHECK(kv_len >= 1 && kv_len <= rows, "kv_len must be between 1 and the cache length");
+    FA_CHECK(q.stride(2) == 1, "Q: the last dimension must be dense (stride 1)");
+    FA_CHECK(K.stride(3) == 1, "K_cache: the last dimension must be dense (stride 1)");
+    FA_CHECK(V.stride(3) == 1, "V_cache: the last dimension must be dense (stride 1)");
+    at::Tensor O;
+    if (given(a[6])) {
+      O = one_row(tensor_arg(a[6], "out"));
+      FA_CHECK(O.sizes() == q.sizes() && O.scalar_type() == torch::kBFloat16 && O.device() == Q.device() && O.stride(2) == 1,
+               "out must match Q in shape, dtype and device");
+    } else {
+      O = at::empty({B, H, d}, Q.options());
+    }
+    const bool return_lse = flag_arg(a[4], false);
+    at::Tensor lse, workspace;
+    if (return_lse) lse = at::empty({B, H}, Q.options().dtype(torch::kFloat32));
+    p.B = static_cast<int32_t>(B); p.H = static_cast<int32_t>(H);
+    p.kv_len = static_cast<int32_t>(kv_len); p.d = static_cast<int32_t>(d);
+    const int64_t need = fa_b200_decode_workspace_bytes(p.B, p.H, p.kv_len);
+    FA_CHECK(need >= 0, "custom_flash_attn.decode failed (", need, "): ", fa_b200_strerror(static_cast<int>(need)));
+    if (need > 0) {     // from torch's allocator on every call: safe with several streams and threads
+      workspace = at::empty({need}, Q.options().dtype(torch::kUInt8));
+      p.workspace = workspace.data_ptr();
+      p.workspace_bytes = need;
+    }
+    if (B * H > 0) {
+      p.q = q.data_ptr(); p.k_cache = K.data_ptr(); p.v_cache = V.data_ptr(); p.o = O.data_ptr();
+      strides2(q, p.q_strides);
+      strides2(O, p.o_strides);
+      cache_strides(K, p.k_strides);
+      cache_strides(V, p.v_strides);
+    } else {
+      p.q = p.k_cache = p.v_cache = p.o = reinterpret_cast<void*>(16);
+      for (int i = 0; i < 2; ++i) p.q_strides[i] = p.o_strides[i] = 64;
+      for (int i = 0; i < 3; ++i) p.k_strides[i] = p.v_strides[i] = 64;
+    }
+    p.lse = return_lse ? lse.data_ptr<float>() : nullptr;
+    p.softmax_scale = static_cast<float>(number_arg(a[5], 0.0));
+    FA_CHECK(given(a[7]) == given(a[8]), "k_new and v_new go together");
+    if (given(a[7])) {
+      const at::Tensor kn = one_row(tensor_arg(a[7], "k_new")), vn = one_row(tensor_arg(a[8], "v_new"));
+      for (const auto& [t, name] : {std::pair<const at::Tensor&, const char*>{kn, "k_new"}, {vn, "v_new"}})
+        FA_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.sizes() == q.sizes() && t.stride(2) == 1,
+                 name, " must be a CUDA bfloat16 tensor [B, H, 64] with a dense last dimension");
+      int64_t vs[2];
+      strides2(kn, p.new_strides);
+      strides2(vn, vs);
+      FA_CHECK(vs[0] == p.new_strides[0] && vs[1] == p.new_strides[1], "k_new and v_new must have the same strides");
+      p.k_new = kn.data_ptr();
+      p.v_new = vn.data_ptr();
+    }
+    p.device = Q.device().index();
+    p.stream = c10::cuda::getCurrentCUDAStream(Q.device().index()).stream();
+    launch("custom_flash_attn.decode", [&] { return fa_b200_decode(&p); });
+    const at::Tensor result = given(a[6]) ? THPVariable_Unpack(a[6]) : (squeeze ? O.unsqueeze(2) : O);
+    return return_lse ? pair(result, lse) : THPVariable_Wrap(result);
+  });
+}
+
+const at::Tensor& dense2d(PyObject* o, const char* name, int64_t cols) {
+  FA_CHECK(THPVariable_Check(o), name, " must be a CUDA bfloat16 tensor");
+  const at::Tensor& t = THPVariable_Unpack(o);
+  FA_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16, name, " must be a CUDA bfloat16 tensor");
+  FA_CHECK(t.dim() > 0 && t.size(-1) == cols && t.is_contiguous(), name, " must be contiguous with ", cols, " columns");
+  return t;
+}
+
+PyObject* add_layernorm(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+  return guarded([&]() -> PyObject* {
+    static const char* const names[] = {"a", "resid", "scale", "shift", "eps", "return_sum", "sum_out", "norm_out"};
+    PyObject* v[8];
+    take_args("add_layernorm", names, 4, args, nargs, kwnames, v);
+    const at::Tensor& a = tensor_arg(v[0], "a");
+    FA_CHECK(a.dim() > 0, "a must have at least one dimension");
+    const int64_t cols = a.size(-1);
+    dense2d(v[0], "a", cols);
+    fa_b200_add_layernorm_params p{};
+    p.a = a.data_ptr();
+    if (given(v[1])) {
+      const at::Tensor& resid = dense2d(v[1], "resid", cols);
+      FA_CHECK(resid.sizes() == a.sizes(), "a and resid must have the same shape");
+      p.resid = resid.data_ptr();
+    }
+    const at::Tensor &scale = dense2d(v[2], "scale", cols), &shift = dense2d(v[3], "shift", cols);
+    FA_CHECK(scale.numel() == cols, "scale must have ", cols, " elements");
+    FA_CHECK(shift.numel() == cols, "shift must have ", cols, " elements");
+    const bool keep = flag_arg(v[5], true) && given(v[1]);
+    at::Tensor sum, norm;
+    if (keep) sum = given(v[6]) ? tensor_arg(v[6], "sum_out") : at::empty_like(a);
+    norm = given(v[7]) ? tensor_arg(v[7], "norm_out") : at::empty_like(a);
+    p.scale = scale.data_ptr();
+    p.shift = shift.data_ptr();
+    p.sum_out = keep ? sum.data_ptr() : nullptr;
+    p.norm_out = norm.data_ptr();
+    p.rows = cols ? a.numel() / cols : 0;
+    p.cols = static_cast<int32_t>(cols);
+    p.eps = static_cast<float>(number_arg(v[4], 1e-5));
+    p.device = a.device().index();
+    p.stream = c10::cuda::getCurrentCUDAStream(a.device().index()).stream();
+    int rc;
+    {
+      py::gil_scoped_release release;
+      rc = fa_b200_add_layernorm(&p);
+    }
+    FA_CHECK(rc == 0, fa_b200_strerror(rc));
+    return keep ? pair(sum, norm) : THPVariable_Wrap(norm);
+  });
+}
+
+PyMethodDef methods[] = {
+    {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&forward)), METH_FASTCALL | METH_KEYWORDS,
+     "FlashAttention forward on B200 (libfa_b200.so)"},
+    {"decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&decode)), METH_FASTCALL | METH_KEYWORDS,
+     "Single-query attention against a K/V cache"},
+    {"add_layernorm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&add_layernorm)),
+     METH_FASTCALL | METH_KEYWORDS, "Shortcut addition and LayerNorm in one pass"},
+    {nullptr, nullptr, 0, nullptr}};
 
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
-  m.def("forward", &forward, "FlashAttention forward on B200 (libfa_b200.so)", py::arg("Q"), py::arg("K_mat"),
-        py::arg("V"), py::arg("causal") = true, py::arg("return_lse") = false,
-        py::arg("softmax_scale") = py::none(), py::arg("out") = py::none());
+  if (PyModule_AddFunctions(m.ptr(), methods) != 0) throw py::error_already_set();
   m.attr("abi_version") = FA_B200_ABI_VERSION;   // the header this module was compiled against
 }

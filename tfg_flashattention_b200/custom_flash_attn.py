@@ -32,8 +32,8 @@ from . import _lib
 
 __all__ = ["forward", "forward_host", "decode", "last_status", "plan", "binding", "set_binding"]
 
-# Two bindings of `forward` over the same C ABI:
-#   "ext"     the compiled pybind11 / torch extension (csrc/torch_binding.cpp, built by
+# Two bindings of `forward` and `decode` over the same C ABI:
+#   "ext"     the compiled torch extension (csrc/torch_binding.cpp, built by
 #             build.build_torch_binding()): the counterpart of the reference's torch_bind.cpp, a few
 #             microseconds of host time per call, GIL released around the launch;
 #   "ctypes"  pure Python over ctypes: needs no compiler beyond the one that built the library.
@@ -78,6 +78,11 @@ def binding() -> str:
     if _binding is None:
         set_binding(os.environ.get("FA_B200_BINDING", "auto"))
     return _binding
+
+
+def extension():
+    """The compiled binding when it is the one in use, else None."""
+    return _ext if (_binding or binding()) == "ext" else None
 
 
 def _check_input(t: torch.Tensor, name: str) -> None:
@@ -175,9 +180,6 @@ def plan(Q, K, V, causal=True):
     return _lib.SCHEDULES[schedule.value], grid.value
 
 
-_decode_workspaces = {}
-
-
 def decode(Q, K_cache, V_cache, kv_len, return_lse=False, softmax_scale=None, out=None,
            k_new=None, v_new=None):
     """Single-query attention against a K/V cache (one generation step; the reference has no
@@ -189,9 +191,10 @@ def decode(Q, K_cache, V_cache, kv_len, return_lse=False, softmax_scale=None, ou
     k_new, v_new [B, H, 64] (optional, both): the key / value of the token being generated; the
     kernel uses them as row kv_len-1 and writes them into that row of the caches (the cache
     append of the step without a separate copy kernel).
-    Returns O shaped like Q (and LSE [B, H] fp32 when asked).  The split-KV workspace is a cached
-    torch buffer per device; calls on one stream may share it, calls that overlap on different
-    streams of one device must not (pass through separate processes or serialise them)."""
+    Returns O shaped like Q (and LSE [B, H] fp32 when asked).  The split-KV workspace comes from
+    torch's allocator on every call: calls on different streams do not share anything."""
+    if binding() == "ext":
+        return _ext.decode(Q, K_cache, V_cache, kv_len, return_lse, softmax_scale, out, k_new, v_new)
     squeeze = Q.dim() == 4
     q3 = Q[:, :, 0, :] if squeeze else Q
     for t, name in ((q3, "Q"), (K_cache, "K_cache"), (V_cache, "V_cache")):
@@ -232,12 +235,7 @@ def decode(Q, K_cache, V_cache, kv_len, return_lse=False, softmax_scale=None, ou
     need = lib.fa_b200_decode_workspace_bytes(B, H, kv_len)
     if need < 0:
         raise RuntimeError(f"custom_flash_attn.decode failed ({need}): {_lib.strerror(int(need))}")
-    ws = None
-    if need > 0:
-        ws = _decode_workspaces.get(Q.device)
-        if ws is None or ws.numel() < need:
-            ws = _decode_workspaces[Q.device] = torch.empty(max(need, 1 << 20), dtype=torch.uint8,
-                                                            device=Q.device)
+    ws = torch.empty(need, dtype=torch.uint8, device=Q.device) if need > 0 else None
 
     def two(t):      # {batch, head} strides; size-1 dimensions get a canonical stride
         sb, sh = t.stride(0), t.stride(1)
