@@ -182,6 +182,30 @@ int encode_map(CUtensorMap* map, const void* base, const fa_b200_params* p, cons
   return 0;
 }
 
+// Launch with programmatic dependent launch (the kernels wait for the previous one before their first
+// access to global memory, see pdl_wait): back-to-back launches overlap the start-up of one with the
+// end of the other.  `cluster` > 1: clusters of that many CTAs along x.
+template <class... Params, class... Args>
+cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, unsigned block, size_t smem, cudaStream_t stream,
+                          unsigned cluster, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  const cudaError_t last = cudaGetLastError();     // (clears the sticky copy)
+  return e != cudaSuccess ? e : last;
+}
+
 // How one forward call is scheduled (the rule behind fa_b200_fwd and fa_b200_fwd_plan).
 struct FwdPlan {
   bool persistent;     // grid of resident CTAs striding through the work list
@@ -293,16 +317,11 @@ int fa_b200_fwd(const fa_b200_params* p) {
   kp.div_half = fa::make_fast_div(static_cast<uint32_t>(kp.n_qtiles > 1 ? kp.n_qtiles / 2 : 1));
   const cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   const bool ragged = (p->N % fa::kBlockN) != 0;   // non-causal only: the causal mask covers the columns past N
-  if (pl.persistent) {
-    if (kp.causal) fa::fa_fwd_kernel<true, true><<<pl.grid, fa::kNumThreads, fa::kSmemBytes, stream>>>(mq, mk, mv, mo, kp);
-    else if (ragged) fa::fa_fwd_kernel<true, false, true><<<pl.grid, fa::kNumThreads, fa::kSmemBytes, stream>>>(mq, mk, mv, mo, kp);
-    else fa::fa_fwd_kernel<true, false><<<pl.grid, fa::kNumThreads, fa::kSmemBytes, stream>>>(mq, mk, mv, mo, kp);
-  } else {
-    if (kp.causal) fa::fa_fwd_kernel<false, true><<<pl.grid, fa::kNumThreads, fa::kSmemBytes, stream>>>(mq, mk, mv, mo, kp);
-    else if (ragged) fa::fa_fwd_kernel<false, false, true><<<pl.grid, fa::kNumThreads, fa::kSmemBytes, stream>>>(mq, mk, mv, mo, kp);
-    else fa::fa_fwd_kernel<false, false><<<pl.grid, fa::kNumThreads, fa::kSmemBytes, stream>>>(mq, mk, mv, mo, kp);
-  }
-  return static_cast<int>(cudaGetLastError());
+  auto* kernel = pl.persistent ? (kp.causal ? &fa::fa_fwd_kernel<true, true>
+                                            : (ragged ? &fa::fa_fwd_kernel<true, false, true> : &fa::fa_fwd_kernel<true, false>))
+                               : (kp.causal ? &fa::fa_fwd_kernel<false, true>
+                                            : (ragged ? &fa::fa_fwd_kernel<false, false, true> : &fa::fa_fwd_kernel<false, false>));
+  return static_cast<int>(launch_kernel(kernel, dim3(pl.grid), fa::kNumThreads, fa::kSmemBytes, stream, 1, mq, mk, mv, mo, kp));
 }
 
 int fa_b200_fwd_plan(const fa_b200_params* p, int32_t* schedule, int32_t* grid) {
@@ -442,15 +461,19 @@ int decode_launch(const fa_b200_decode_params* p, float* scratch, int splits, in
   kp.scale_log2 = scale * 1.4426950408889634f;
 
   const cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
-  const dim3 grid(static_cast<unsigned>(p->B * p->H), static_cast<unsigned>(splits));
-  if (wide) fa::fa_decode_partial_kernel<fa::kDecodeWideThreads><<<grid, fa::kDecodeWideThreads, 0, stream>>>(kp);
-  else fa::fa_decode_partial_kernel<fa::kDecodeThreads><<<grid, fa::kDecodeThreads, 0, stream>>>(kp);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return static_cast<int>(e);
-  if (splits > 1) {
-    fa::fa_decode_combine_kernel<<<static_cast<unsigned>(p->B * p->H), 64, 0, stream>>>(kp);
-    e = cudaGetLastError();
+  const unsigned heads = static_cast<unsigned>(p->B * p->H);
+  const dim3 grid(heads, static_cast<unsigned>(splits));
+  if (wide) {
+    // a cluster per head while that makes more CTAs than SMs hardly at all (8 x 37 = 4 x 74 = 2 x 148
+    // = 296 CTAs of 512 threads: two per SM of a 148-SM part), beyond it one wide CTA per head
+    const unsigned cluster = heads <= 37 ? 8 : (heads <= 74 ? 4 : (heads <= 148 ? 2 : 1));
+    if (cluster > 1)
+      return static_cast<int>(launch_kernel(&fa::fa_decode_cluster_kernel, dim3(cluster, heads), fa::kDecodeClusterThreads, 0, stream, cluster, kp));
+    return static_cast<int>(launch_kernel(&fa::fa_decode_partial_kernel<fa::kDecodeWideThreads>, grid, fa::kDecodeWideThreads, 0, stream, 1, kp));
   }
+  cudaError_t e = launch_kernel(&fa::fa_decode_partial_kernel<fa::kDecodeThreads>, grid, fa::kDecodeThreads, 0, stream, 1, kp);
+  if (e == cudaSuccess && splits > 1)
+    e = launch_kernel(&fa::fa_decode_combine_kernel, dim3(heads), 64, 0, stream, 1, kp);
   return static_cast<int>(e);
 }
 

@@ -18,6 +18,8 @@
 #include <math_constants.h>
 #include <stdint.h>
 
+#include "ptx_sm100.cuh"
+
 namespace fa {
 
 constexpr int kDecodeThreads = 128;          // a warp's 32 lanes = 4 groups of 8 lanes
@@ -25,6 +27,8 @@ constexpr int kDecodeGroups = kDecodeThreads / 8;   // 16 lane groups, each owns
 constexpr int kDecodeWideThreads = 1024;            // the one-CTA-per-head form for few heads
 constexpr int kDecodeUnroll = 4;             // rows in flight per lane group (8: 3.3-4.0 TB/s against 4.3-5.2)
 constexpr int kDecodePartial = 66;           // floats per partial: m, l, o[64]
+constexpr int kDecodeClusterThreads = 512;          // the one-cluster-per-head form for very few heads
+constexpr int kDecodeClusterMax = 8;                // CTAs per cluster (the portable limit)
 
 struct DecodeParams {
   const __nv_bfloat16* q;      // [B, H, 64]
@@ -81,6 +85,8 @@ __global__ void __launch_bounds__(kThreads) fa_decode_partial_kernel(const Decod
   const int g = tid >> 3;
   const int c = tid & 7;
 
+  pdl_trigger();
+  pdl_wait();
   float qf[8];
   {
     const uint4 raw = *reinterpret_cast<const uint4*>(p.q + b * p.q_sb + h * p.q_sh + 8 * c);
@@ -198,12 +204,146 @@ __global__ void __launch_bounds__(kThreads) fa_decode_partial_kernel(const Decod
   }
 }
 
+// grid (ctas, B*H) in clusters of (ctas, 1, 1), block 512: very few heads (a single sequence's step).
+// One CTA per head leaves most of the chip idle and pulls the head's keys through one SM (25 heads x
+// 900 rows: 8.6 us a launch); two launches cost more than the work.  Here a head is a cluster of 2,
+// 4 or 8 CTAs, each with an equal share of the rows that are there when the kernel runs, and the
+// partials meet in the first CTA's shared memory (distributed shared memory, one cluster barrier).
+// A CTA's share is at most a few hundred rows: all its loads are in flight at once.
+__global__ void __launch_bounds__(kDecodeClusterThreads) fa_decode_cluster_kernel(const DecodeParams p) {
+  constexpr int kWarps = kDecodeClusterThreads / 32, kGroups = kDecodeClusterThreads / 8, kUnroll = 4;
+  __shared__ float sm_w[kWarps][kDecodePartial];            // this CTA's warps
+  __shared__ float sm_c[kDecodeClusterMax][kDecodePartial]; // rank 0: the cluster's CTAs
+  const int rank = blockIdx.x, ctas = gridDim.x, bh = blockIdx.y;
+  const int b = bh / p.H, h = bh - b * p.H;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = tid >> 3, c = tid & 7;
+  // every CTA of the cluster has started before anyone writes to rank 0's shared memory
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  pdl_trigger();
+  pdl_wait();
+  const int kv_len = p.kv_len_ptr ? max(1, min(__ldg(p.kv_len_ptr), p.kv_len)) : p.kv_len;
+  const int r0 = static_cast<int>(static_cast<long long>(rank) * kv_len / ctas);
+  const int r1 = static_cast<int>(static_cast<long long>(rank + 1) * kv_len / ctas);
+  __nv_bfloat16* kbase = const_cast<__nv_bfloat16*>(p.k) + b * p.k_sb + h * p.k_sh + 8 * c;
+  __nv_bfloat16* vbase = const_cast<__nv_bfloat16*>(p.v) + b * p.v_sb + h * p.v_sh + 8 * c;
+  const long long new_off = b * p.new_sb + h * p.new_sh + 8 * c;
+  float qf[8], acc[8];
+  bf16x8_to_float(*reinterpret_cast<const uint4*>(p.q + b * p.q_sb + h * p.q_sh + 8 * c), qf);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) { qf[i] *= p.scale_log2; acc[i] = 0.f; }
+  float m = -1e30f, l = 0.f;                       // finite: a group without rows weighs nothing
+  for (int base = r0; base < r1; base += kGroups * kUnroll) {
+    uint4 kraw[kUnroll], vraw[kUnroll];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const int r = base + g + u * kGroups;
+      kraw[u] = vraw[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (r < r1) {
+        uint4* kp = reinterpret_cast<uint4*>(kbase + r * p.k_sn);
+        uint4* vp = reinterpret_cast<uint4*>(vbase + r * p.v_sn);
+        if (p.k_new != nullptr && r == kv_len - 1) {        // the row being appended
+          kraw[u] = *reinterpret_cast<const uint4*>(p.k_new + new_off);
+          vraw[u] = *reinterpret_cast<const uint4*>(p.v_new + new_off);
+          *kp = kraw[u];
+          *vp = vraw[u];
+        } else {
+          kraw[u] = __ldcs(kp);
+          vraw[u] = __ldcs(vp);
+        }
+      }
+    }
+    float s[kUnroll], m_new = m;
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      float kf[8];
+      bf16x8_to_float(kraw[u], kf);
+      s[u] = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s[u] = fmaf(qf[i], kf[i], s[u]);
+    }
+#pragma unroll
+    for (int o = 1; o <= 4; o <<= 1) {
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+    }
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      if (base + g + u * kGroups >= r1) s[u] = -CUDART_INF_F;
+      m_new = fmaxf(m_new, s[u]);
+    }
+    const float f = exp2f(m - m_new);
+    l *= f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] *= f;
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const float pr = exp2f(s[u] - m_new);
+      float vf[8];
+      bf16x8_to_float(vraw[u], vf);
+      l += pr;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = fmaf(pr, vf[i], acc[i]);
+    }
+    m = m_new;
+  }
+#pragma unroll
+  for (int o = 8; o <= 16; o <<= 1) {              // the warp's four lane groups
+    const float m_o = __shfl_xor_sync(0xffffffffu, m, o), l_o = __shfl_xor_sync(0xffffffffu, l, o);
+    const float m_n = fmaxf(m, m_o), fa = exp2f(m - m_n), fb = exp2f(m_o - m_n);
+    l = l * fa + l_o * fb;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = acc[i] * fa + __shfl_xor_sync(0xffffffffu, acc[i], o) * fb;
+    m = m_n;
+  }
+  if (lane < 8) {
+    if (c == 0) { sm_w[warp][0] = m; sm_w[warp][1] = l; }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sm_w[warp][2 + 8 * c + i] = acc[i];
+  }
+  __syncthreads();
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  if (tid < 64) {
+    float mm = -1e30f, ll = 0.f, oo = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) mm = fmaxf(mm, sm_w[w][0]);
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const float f = exp2f(sm_w[w][0] - mm);
+      ll = fmaf(sm_w[w][1], f, ll);
+      oo = fmaf(sm_w[w][2 + tid], f, oo);
+    }
+    uint32_t dst;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(dst) : "r"(smem_u32(sm_c[rank])));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + 4 * (2 + tid)), "f"(oo) : "memory");
+    if (tid == 0) {
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(mm) : "memory");
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + 4), "f"(ll) : "memory");
+    }
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (rank == 0 && tid < 64) {
+    float mm = -1e30f, ll = 0.f, oo = 0.f;
+    for (int k = 0; k < ctas; ++k) mm = fmaxf(mm, sm_c[k][0]);
+    for (int k = 0; k < ctas; ++k) {
+      const float f = exp2f(sm_c[k][0] - mm);
+      ll = fmaf(sm_c[k][1], f, ll);
+      oo = fmaf(sm_c[k][2 + tid], f, oo);
+    }
+    p.o[b * p.o_sb + h * p.o_sh + tid] = __float2bfloat16_rn(oo / ll);
+    if (tid == 0 && p.lse != nullptr) p.lse[bh] = 0.6931471805599453f * (mm + log2f(ll));
+  }
+}
+
 // grid B*H, block 64: merge the `splits` partials of one head.
 __global__ void __launch_bounds__(64) fa_decode_combine_kernel(const DecodeParams p) {
   const int bh = blockIdx.x;
   const int b = bh / p.H;
   const int h = bh - b * p.H;
   const int tid = threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
   const float* part = p.scratch + (long long)bh * p.splits * kDecodePartial;
   float mm = -CUDART_INF_F;
   for (int s = 0; s < p.splits; ++s) mm = fmaxf(mm, part[s * kDecodePartial]);

@@ -328,6 +328,9 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     const bool has = decode_item(threadIdx.x, t);
     sm.items[threadIdx.x] = has ? make_int4(t.q_row, t.ns, t.h, t.b) : make_int4(0, 0, 0, 0);
   }
+  // everything above touches no global memory and may run beside the previous kernel's last CTAs
+  pdl_trigger();
+  pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

@@ -40,6 +40,14 @@ __device__ __forceinline__ void reg_dealloc() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs));
 }
 
+// Programmatic dependent launch: a kernel launched with that attribute may start while the one in
+// front of it in the stream still runs; pdl_wait returns when that one has completed and its writes
+// are visible, and must come before the first access to global memory.  pdl_trigger lets the next
+// kernel of the stream start (once every CTA of this one has said so); it then holds nothing but an
+// idle slot until this kernel is through.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ----------------------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
