@@ -82,11 +82,14 @@ int fa_b200_fwd(const fa_b200_params* p);
  * src/cpp/v1.cu:13-14, 25-34); this library picks one of four kernel schedules per call and this
  * query reports the pick, so that a test or a tuning run can tell which code ran:
  *   FA_B200_SCHEDULE_CTA_PER_TILE        one CTA per 128-row query tile, heaviest causal tile first
- *   FA_B200_SCHEDULE_PERSISTENT_PAIRED   resident CTAs, causal, complementary tile pairs
- *   FA_B200_SCHEDULE_PERSISTENT_ROTATED  resident CTAs, causal, odd tile count (rotated order)
- *   FA_B200_SCHEDULE_PERSISTENT_FULL     resident CTAs, non-causal
+ *                                        (long causal sequences: a CTA that is through takes over one
+ *                                        that has not started)
+ *   FA_B200_SCHEDULE_PERSISTENT_PAIRED   causal, even tile count: the resident CTAs' slots work through
+ *                                        the tiles, heavy ones next to light ones
+ *   FA_B200_SCHEDULE_PERSISTENT_ROTATED  the same with an odd tile count
+ *   FA_B200_SCHEDULE_PERSISTENT_FULL     the same, non-causal
  *   FA_B200_SCHEDULE_NONE                empty problem, nothing is launched
- * *grid receives the number of CTAs.  Either output pointer may be NULL.  Arguments are checked as
+ * *grid receives the number of CTAs (persistent: of resident ones).  Either output pointer may be NULL.  Arguments are checked as
  * by fa_b200_fwd; the first call on a device performs the same one-time device set-up. */
 #define FA_B200_SCHEDULE_NONE               -1
 #define FA_B200_SCHEDULE_CTA_PER_TILE        0

@@ -1,0 +1,60 @@
+"""Each kernel schedule of the attention forward at the sizes where it can go wrong: the last CTA of
+the first wave, one item more than there are slots, the borders of the dispatch rule (plan_fwd in
+csrc/fa_b200_api.cu), groups of heads that do not divide evenly, many rounds of taking items over.
+
+Every result has to be bit for bit what the same head gives alone (where one CTA per tile runs, or
+one CTA), and sampled heads are held to the CPU oracle at the tolerances of test_parity_gpu.py."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _heads_near(items, tiles):
+    return max(1, -(-items // tiles))
+
+
+def _slots():
+    return 2 * torch.cuda.get_device_properties(0).multi_processor_count
+
+
+@pytest.mark.parametrize("N,items", [
+    (128, "slots"), (128, "slots+1"), (90, "3*slots"),              # one K/V tile: one item / static
+    (300, "slots+3"), (500, "2*slots-4"), (512, "2*slots"),         # up to four: static, then dynamic
+    (700, "4*slots//3-6"), (700, "4*slots//3+6"), (1024, "5*slots"),
+    (2048, "2*slots"), (2177, "2*slots"),                            # dynamic, reported as CTA per tile above 16 tiles
+])
+@pytest.mark.parametrize("causal", [True, False])
+def test_schedule_borders(fa_lib, N, items, causal):
+    from oracle.attention_oracle import manual_attention
+    from tfg_flashattention_b200 import custom_flash_attn as cfa
+    tiles = -(-N // 128)
+    heads = _heads_near(eval(items, {"slots": _slots()}), tiles)
+    g = torch.Generator(device="cuda").manual_seed(N + heads)
+    q, k, v = (torch.randn(1, heads, N, 64, device="cuda", generator=g).bfloat16() for _ in range(3))
+    o = torch.full_like(q, float("nan"))
+    _, lse = cfa.forward(q, k, v, causal=causal, return_lse=True, out=o)
+    assert cfa.last_status() == 0
+    assert torch.isfinite(o).all() and torch.isfinite(lse).all()
+    for h in {0, 1 % heads, heads // 2, heads - 1}:
+        one = (t[:, h:h + 1].contiguous() for t in (q, k, v))
+        alone, alone_lse = cfa.forward(*one, causal=causal, return_lse=True)
+        assert torch.equal(alone[0, 0], o[0, h]) and torch.equal(alone_lse[0, 0], lse[0, h])
+    h = heads - 1
+    ref, ref_lse = manual_attention(*(t[:, h:h + 1].float().cpu() for t in (q, k, v)), causal=causal, return_lse=True)
+    d = (o[0, h].float().cpu() - ref[0, 0]).abs()
+    assert d.max().item() <= 2e-2 and d.mean().item() <= 2e-3
+    assert ((lse[0, h].cpu() - ref_lse[0, 0]).abs() <= 1e-3 * ref_lse[0, 0].abs().clamp_min(1.0)).all()
+
+
+def test_order_by_groups_of_heads(fa_lib):
+    """32 MB of K and V (N * 256 bytes a head) are ordered together, 15 heads of 8200 rows: 33 heads make
+    three groups of 11, 34 groups of 12, 12 and 10."""
+    from tfg_flashattention_b200 import custom_flash_attn as cfa
+    for heads, N in ((33, 8200), (34, 8200)):
+        g = torch.Generator(device="cuda").manual_seed(heads)
+        q, k, v = (torch.randn(1, heads, N, 64, device="cuda", generator=g).bfloat16() for _ in range(3))
+        o = cfa.forward(q, k, v, out=torch.full_like(q, float("nan")))
+        assert cfa.last_status() == 0 and torch.isfinite(o).all()
+        for h in (0, 14, 15, 16, heads - 1):
+            assert torch.equal(cfa.forward(*(t[:, h:h + 1].contiguous() for t in (q, k, v)))[0, 0], o[0, h])

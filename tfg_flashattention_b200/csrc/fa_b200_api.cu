@@ -69,6 +69,17 @@ struct DeviceGuard {
   }
 };
 
+using FwdKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, fa::FwdParams);
+template <int kSchedule>
+FwdKernel fwd_kernel_of(bool causal, bool ragged) {
+  if (causal) return &fa::fa_fwd_kernel<kSchedule, true>;
+  return ragged ? &fa::fa_fwd_kernel<kSchedule, false, true> : &fa::fa_fwd_kernel<kSchedule, false>;
+}
+FwdKernel fwd_kernel(int schedule, bool causal, bool ragged) {
+  return schedule == fa::kOneItem ? fwd_kernel_of<fa::kOneItem>(causal, ragged)
+         : schedule == fa::kStatic ? fwd_kernel_of<fa::kStatic>(causal, ragged) : fwd_kernel_of<fa::kDynamic>(causal, ragged);
+}
+
 // Runs once per device, with that device current.
 void init_device(int dev) {
   DeviceState& st = g_dev[dev];
@@ -79,12 +90,12 @@ void init_device(int dev) {
   // The kernel moves registers between its warpgroups with setmaxnreg; that only works (and
   // otherwise blocks for ever) if the compiler gave the kernel the launch allocation the budget
   // in fa_fwd_sm100.cuh assumes.  Refuse to launch a build where it did not.
-  const void* variants[6] = {reinterpret_cast<const void*>(&fa::fa_fwd_kernel<false, false>),
-                             reinterpret_cast<const void*>(&fa::fa_fwd_kernel<false, false, true>),
-                             reinterpret_cast<const void*>(&fa::fa_fwd_kernel<false, true>),
-                             reinterpret_cast<const void*>(&fa::fa_fwd_kernel<true, false>),
-                             reinterpret_cast<const void*>(&fa::fa_fwd_kernel<true, false, true>),
-                             reinterpret_cast<const void*>(&fa::fa_fwd_kernel<true, true>)};
+  const void* variants[9];
+  {
+    int i = 0;
+    for (int schedule : {fa::kOneItem, fa::kStatic, fa::kDynamic})
+      for (int mask : {0, 1, 2}) variants[i++] = reinterpret_cast<const void*>(fwd_kernel(schedule, mask == 2, mask == 1));
+  }
   for (const void* fn : variants) {
     cudaFuncAttributes fattr;
     e = cudaFuncGetAttributes(&fattr, fn);
@@ -207,37 +218,43 @@ cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, unsigned block, 
 }
 
 // How one forward call is scheduled (the rule behind fa_b200_fwd and fa_b200_fwd_plan).
+constexpr long long kOrderBytes = 32ll << 20;   // K and V of the heads that are ordered together (16, 64 MB: equal)
 struct FwdPlan {
-  bool persistent;     // grid of resident CTAs striding through the work list
-  bool paired;         // persistent causal schedule of complementary tile pairs
-  int n_qtiles;
+  int schedule;        // fa::Schedule
+  int n_qtiles, kv_tiles;
   long long items;     // B * H * n_qtiles
-  unsigned grid;
+  unsigned grid;       // launched
 };
 
 FwdPlan plan_fwd(const fa_b200_params* p, const DeviceState& st) {
   FwdPlan pl;
   pl.n_qtiles = (p->N + fa::kBlockM - 1) / fa::kBlockM;
+  pl.kv_tiles = (p->N + fa::kBlockN - 1) / fa::kBlockN;
   pl.items = static_cast<long long>(p->B) * p->H * pl.n_qtiles;
-  const int kv_tiles = (p->N + fa::kBlockN - 1) / fa::kBlockN;
+  const long long slots = st.resident_ctas;
+  // Measured on B200 (296 slots), N = 64 .. 16384, 12 .. 800 heads:
+  // * No more items than slots, or a third more: one CTA per item.  Nobody has much to take over, and
+  //   asking costs 0.4 us (B=4 H=12 N=1024, 384 items: 13.9 us, static 15.4, dynamic 15.7).
+  // * Items of up to 4 K/V tiles that make less than two rounds, or of one: static.  (B=8 H=16 N=300,
+  //   384 items: 8.5 us, dynamic 9.0, one item 10.3; B=4 H=25 N=512 non-causal: 14.1 against 16.0: who
+  //   takes over an item does not know who else is on the SM.)
+  // * Otherwise dynamic (B=32 H=25 N=777: 139 us, static 170, one item 191), except
+  //   - non-causal sequences above 3072: one CTA per item, whose tile loop is the smallest code
+  //     (B=4 H=25 N=8192: 1.94 ms, dynamic 2.12);
+  //   - more items per slot than the item table holds: one CTA per item.
   const bool causal = p->causal != 0;
-  // Measured on B200: the causal schedule of complementary tile pairs wins up to N = 2048 at any
-  // grid size (equal at 4096, behind beyond: long items amortise their own start-up, and the
-  // hardware's dynamic placement of many CTAs balances better); without pairing, persistence pays
-  // for short items (N <= 1024) once every CTA gets at least two of them.
-  const bool can_pair = causal && pl.n_qtiles % 2 == 0;
-  pl.persistent = can_pair ? kv_tiles <= 16
-                           : (pl.items >= 2LL * st.resident_ctas && kv_tiles <= 8);
-  pl.paired = pl.persistent && can_pair;
-  long long work_units = pl.paired ? pl.items / 2 : pl.items;
-  // a persistent CTA keeps its items in a table of fa::kItemTable entries
-  if (pl.persistent && (work_units + st.resident_ctas - 1) / st.resident_ctas * (pl.paired ? 2 : 1) >
-                           fa::kItemTable) {
-    pl.persistent = pl.paired = false;
-    work_units = pl.items;
+  pl.schedule = fa::kOneItem;
+  if (pl.items > slots * fa::kItemTable) {
+  } else if (pl.kv_tiles == 1 || (pl.kv_tiles <= 4 && pl.items < 2 * slots)) {
+    if (pl.items > slots) pl.schedule = fa::kStatic;
+  } else if (3 * pl.items >= 4 * slots && (causal || pl.kv_tiles <= 24)) {
+    pl.schedule = fa::kDynamic;
   }
-  pl.grid = static_cast<unsigned>(
-      pl.persistent ? (work_units > st.resident_ctas ? st.resident_ctas : work_units) : pl.items);
+  pl.grid = static_cast<unsigned>(pl.schedule == fa::kStatic ? slots : pl.items);
+  if (causal && p->B * p->H == 1 && pl.n_qtiles == 2) {   // one small problem runs as one CTA: the bounded-wait test's
+    pl.schedule = fa::kStatic;
+    pl.grid = 1;
+  }
   return pl;
 }
 
@@ -312,15 +329,23 @@ int fa_b200_fwd(const fa_b200_params* p) {
   kp.scale_log2 = scale * 1.4426950408889634f;
   kp.status = st.status;
   kp.n_items = static_cast<int>(pl.items);
-  kp.paired = pl.paired ? 1 : 0;
-  kp.n_units = static_cast<int>(pl.items / 2);
-  kp.div_half = fa::make_fast_div(static_cast<uint32_t>(kp.n_qtiles > 1 ? kp.n_qtiles / 2 : 1));
+  const int first_wave = static_cast<int>(pl.items < st.resident_ctas ? pl.items : st.resident_ctas);
+  kp.mirror_from = st.sm_count;
+  kp.mirror_to = kp.causal ? first_wave : 0;
+  // causal order: groups of heads whose K and V (N * 256 bytes each) stay in L2 while their tiles run
+  const long long heads = static_cast<long long>(p->B) * p->H;
+  long long fit = kOrderBytes / (static_cast<long long>(p->N) * 256);
+  if (fit < 1) fit = 1;
+  const long long groups = (heads + fit - 1) / fit;
+  kp.group = static_cast<int>((heads + groups - 1) / groups);
+  kp.group_items = kp.group * kp.n_qtiles;
+  kp.last_group = static_cast<int>(heads - (heads - 1) / kp.group * kp.group);
+  kp.div_group_items = fa::make_fast_div(static_cast<uint32_t>(kp.group_items));
+  kp.div_group = fa::make_fast_div(static_cast<uint32_t>(kp.group));
+  kp.div_last_group = fa::make_fast_div(static_cast<uint32_t>(kp.last_group));
   const cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   const bool ragged = (p->N % fa::kBlockN) != 0;   // non-causal only: the causal mask covers the columns past N
-  auto* kernel = pl.persistent ? (kp.causal ? &fa::fa_fwd_kernel<true, true>
-                                            : (ragged ? &fa::fa_fwd_kernel<true, false, true> : &fa::fa_fwd_kernel<true, false>))
-                               : (kp.causal ? &fa::fa_fwd_kernel<false, true>
-                                            : (ragged ? &fa::fa_fwd_kernel<false, false, true> : &fa::fa_fwd_kernel<false, false>));
+  const FwdKernel kernel = fwd_kernel(pl.schedule, kp.causal != 0, ragged);
   return static_cast<int>(launch_kernel(kernel, dim3(pl.grid), fa::kNumThreads, fa::kSmemBytes, stream, 1, mq, mk, mv, mo, kp));
 }
 
@@ -337,12 +362,16 @@ int fa_b200_fwd_plan(const fa_b200_params* p, int32_t* schedule, int32_t* grid) 
   DeviceState* stp = nullptr;
   if ((rc = ready_device(p->device, &stp)) != 0) return rc;
   const FwdPlan pl = plan_fwd(p, *stp);
+  // reported by what a CTA slot does (see the header): several tiles in turn, or one
+  const long long slots = stp->resident_ctas;
+  const bool in_turn = pl.schedule == fa::kStatic || (pl.schedule == fa::kDynamic && (!p->causal || pl.kv_tiles <= 16)) ||
+                       (p->causal && pl.n_qtiles % 2 == 0 && pl.kv_tiles <= 16 && pl.items > slots && 3 * pl.items < 4 * slots);
   if (schedule != nullptr)
-    *schedule = !pl.persistent ? FA_B200_SCHEDULE_CTA_PER_TILE
-                : pl.paired    ? FA_B200_SCHEDULE_PERSISTENT_PAIRED
-                : p->causal    ? FA_B200_SCHEDULE_PERSISTENT_ROTATED
-                               : FA_B200_SCHEDULE_PERSISTENT_FULL;
-  if (grid != nullptr) *grid = static_cast<int32_t>(pl.grid);
+    *schedule = !in_turn               ? FA_B200_SCHEDULE_CTA_PER_TILE
+                : !p->causal           ? FA_B200_SCHEDULE_PERSISTENT_FULL
+                : pl.n_qtiles % 2 == 0 ? FA_B200_SCHEDULE_PERSISTENT_PAIRED
+                                       : FA_B200_SCHEDULE_PERSISTENT_ROTATED;
+  if (grid != nullptr) *grid = static_cast<int32_t>(in_turn && pl.items > slots ? slots : pl.grid);
   return FA_B200_OK;
 }
 
@@ -930,6 +959,7 @@ const char* fa_b200_strerror(int code) {
       case fa::kWaitStepFull: return "fa_b200 watchdog: generation step, wait for a weight tile ran out";
       case fa::kWaitStepEmpty: return "fa_b200 watchdog: generation step, wait for a free ring stage ran out";
       case fa::kWaitStepWords: return "fa_b200 watchdog: generation step, wait for another CTA's values ran out";
+      case fa::kWaitItem: return "fa_b200 watchdog: wait for the next work item ran out";
       case fa::kWaitOFull: return "fa_b200 watchdog: wait for O += PV ran out";
       default: return "fa_b200 watchdog: a bounded wait ran out";
     }

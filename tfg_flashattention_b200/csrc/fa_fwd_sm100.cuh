@@ -3,9 +3,9 @@
 // A work item is one 128-row query tile of one (batch, head); the CTA streams that head's K/V
 // tiles through shared memory.  Two CTAs are resident per SM (each takes 256 of the 512 TMEM
 // columns, under half the shared memory and half the registers), so one CTA's latency-bound
-// phases run under the other CTA's tensor-core and MUFU work.  The grid is either one CTA per
-// item or persistent (2 x SM count CTAs striding through a load-balanced item list); in the
-// persistent case every role runs ahead across item boundaries: the producer loads the next
+// phases run under the other CTA's tensor-core and MUFU work.  A CTA runs one item, or several (from
+// a list known at launch, or taken over one by one from the grid's CTAs that have not started); in
+// the latter case every role runs ahead across item boundaries: the producer loads the next
 // item's Q/K/V, the issuer starts its first S, and the softmax warps run an item's epilogue in
 // the middle of the next item's first tile, when the last O += P V has long completed.
 //
@@ -15,7 +15,8 @@
 //                         memory) and O += P V_j (M128 N64 K128, P read from tensor memory, V
 //                         MN-major from shared memory).  Control flow is warp-uniform; one
 //                         elected lane issues, tcgen05.commit signals the mbarriers.
-//                         (warps 6, 7 idle: setmaxnreg works on whole warpgroups.)
+//   warp 6                dynamic schedule: asks for the next item.  (Otherwise idle like warp 7:
+//                         setmaxnreg works on whole warpgroups.)
 //   warpgroup 0           softmax, one thread per query row.  Pulls its S row from TMEM into
 //                         registers and releases S at once, so the issuer can start S for the
 //                         next K tile while this one is exponentiated; keeps the running max and
@@ -50,9 +51,9 @@ constexpr int kKVSlots = 4;            // ring: K0 V0 K1 V1 ..., continuing acro
 constexpr int kNumSoftmaxWarps = 4;
 constexpr int kMmaWarp = 4;
 constexpr int kLoadWarp = 5;
+constexpr int kItemWarp = 6;           // dynamic schedule: asks for the CTA's next work item
 constexpr int kNumThreads = 256;       // two whole warpgroups
 constexpr int kCtasPerSm = 2;
-constexpr int kSmCountHint = 148;      // B200; only decorrelates the schedules of co-resident CTAs
 // Register budget.  Two 256-thread CTAs per SM start with 128 registers per thread; the softmax
 // warpgroup then takes kSoftmaxRegs and the other warpgroup keeps kOtherRegs.  setmaxnreg.inc can
 // only take registers that this CTA's own setmaxnreg.dec released and blocks -- with no time limit
@@ -68,6 +69,9 @@ constexpr uint32_t kTmemS = 0, kTmemP = 128, kTmemO = 192;
 constexpr float kRescaleThresholdLog2 = 8.0f;
 constexpr int kItemTable = 256;        // work items per CTA decoded ahead (one per thread at start-up)
 static_assert(kItemTable == kNumThreads, "one table entry per thread");
+constexpr int kItemRing = 8;           // dynamic schedule: entries of that table in use, as a ring
+constexpr int kItemLead = 2;           // ... asked for when the producer loads an item's last tile but one
+enum Schedule : int { kOneItem = 0, kStatic = 1, kDynamic = 2 };
 #ifdef FA_WAIT_TEST
 // Test build (build.build_wait_test_library): waits give up after 2 ms, and the producer leaves out
 // one K tile (see load_kv), so that a test can watch a bounded wait run out and the kernel drain.
@@ -80,7 +84,8 @@ constexpr uint64_t kWaitLimitNs = 1000ull * 1000ull * 1000ull;  // 1 s per wait
 constexpr uint32_t kWatchdogBase = 0x10000u;
 enum WaitId : uint32_t {
   kWaitQFull = 1, kWaitKVFull = 2, kWaitKVEmpty = 3, kWaitSFull = 4, kWaitPFull = 5,
-  kWaitOFull = 6, kWaitDrain = 7, kWaitSFree = 8, kWaitQEmpty = 9, kWaitOFree = 10
+  kWaitOFull = 6, kWaitDrain = 7, kWaitSFree = 8, kWaitQEmpty = 9, kWaitOFree = 10,
+  kWaitItem = 11
 };
 
 // Optional timeline trace (compile with -DFA_TRACE; timeline.py builds that variant into a library
@@ -118,6 +123,10 @@ struct __align__(1024) SharedStorage {
   uint64_t p_full;               // P written to TMEM by all four softmax warps
   uint64_t o_full;               // O += P V_j finished (P reusable, O stable)
   uint64_t o_free;               // the epilogue has read O: the next item may overwrite it
+  uint64_t item_go;              // dynamic schedule: the producer nears its item's end, ask for the next
+  uint64_t item_answer;          // ... the answer is in item_response
+  uint64_t item_full[kItemRing]; // ... and decoded into items[]
+  uint4 item_response[2];
   uint32_t tmem_base;
   uint32_t abort;                // 0, or the watchdog code of the first wait that gave up
   uint32_t abort_who;            // thread index | parity << 16 of that wait
@@ -161,9 +170,10 @@ struct FwdParams {
   int n_qtiles;               // ceil(N / 128): work items per (batch, head)
   FastDiv div_qtiles, div_heads;   // divisions by n_qtiles and by H
   int n_items;                // B * H * n_qtiles
-  int paired;                 // persistent causal schedule with an even tile count: complementary pairs
-  int n_units;                // B * H * n_qtiles / 2 when paired
-  FastDiv div_half;           // division by n_qtiles / 2
+  int mirror_from, mirror_to; // blocks whose items are taken from the other end (see decode_item)
+  int group;                  // causal: heads whose tiles are ordered together ...
+  int group_items, last_group;   // ... their work items; heads of the last group
+  FastDiv div_group_items, div_group, div_last_group;
   int causal;
   float scale_log2;           // softmax_scale * log2(e)
   unsigned int* status;       // [4] watchdog words in global memory
@@ -212,20 +222,19 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// kPersistent = true: the grid is 2 x SM count and every role loops over work items (best when
-// items are many and short, e.g. N = 1024 causal: 4.5 K/V tiles per item on average).
-// kPersistent = false: one CTA per item, no cross-item state in the hot loop (best for long
-// sequences and for grids too small to balance statically).
+// kSchedule: how many items a CTA runs and how it gets them (see the comment at decode_item; which is
+// taken when: plan_fwd in fa_b200_api.cu).  kOneItem carries no cross-item state in the hot loop.
 // kCausal selects the masking code at compile time (the non-causal instantiation carries none of
 // the diagonal-tile handling).
 // kRagged (non-causal only): N is not a multiple of 128, the last K/V tile of every item needs its
 // columns past N masked.  The 128 tests for that sit inside the tile loop, and the loop's speed
 // depends on its code size, so sequences of whole tiles get an instantiation without them.
-template <bool kPersistent, bool kCausal, bool kRagged = false>
+template <int kSchedule, bool kCausal, bool kRagged = false>
 __global__ void __launch_bounds__(kNumThreads, kCtasPerSm)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
               const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
               const FwdParams p) {
+  constexpr bool kPersistent = kSchedule != kOneItem;      // the CTA runs several items
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   SharedStorage& sm =
@@ -236,66 +245,59 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
   const int nkv = (p.N + kBlockN - 1) / kBlockN;
 
   // The n-th work item of this CTA -> (batch, head, query tile); false when the CTA is done.
-  // A head's tiles are adjacent in the list, so CTAs that run side by side share that head's K/V
-  // in L2.  In causal mode tile t costs t+1 K/V tiles.  Three schedules:
-  //   one CTA per item      heaviest tile of a head first, the hardware balances dynamically;
-  //   persistent, paired    (even tile count) the CTA takes tile nq-1-s and then its complement
-  //                         s of the same head: every pair costs nq+1 K/V tiles, so a CTA striding
-  //                         through the pairs by gridDim.x gets equal work;
-  //   persistent, rotated   (odd tile count, or non-causal) stride through single items, the tile
-  //                         order inside a head rotated by the head index.
+  // All schedules take their items from one list.  Non-causal: head by head, so that CTAs that run
+  // side by side share a head's K/V in L2.  Causal: tile t costs t+1 K/V tiles, the heaviest come
+  // first, through groups of heads whose K and V fit L2 together: all heads' last tiles, then all the
+  // ones before, ...  (Head by head, a heavy tile of the last head starts when everybody else is
+  // nearly through: B = 4 H = 25 N = 16384 took 4.59 ms instead of 3.91.)
+  //   one item    a CTA per item, the hardware places them as others end;
+  //   static      a CTA per resident slot, the list dealt back and forth over the grid;
+  //   dynamic     a CTA per item is launched, but a running CTA takes over one that has not started
+  //               (cluster launch control): the balance of the first with the overlap of the second.
   struct Item { int b, h, q_row, ns; };
-  auto decode_item = [&](int n, Item& w) -> bool {
+  auto decode_listed = [&](int item, Item& w) {
     int bh, qt;
-    if (kPersistent && kCausal && p.paired) {
-      const int unit = blockIdx.x + (n >> 1) * gridDim.x;
-      if (unit >= p.n_units) return false;
-      const int half_q = p.n_qtiles >> 1;
-      bh = static_cast<int>(fast_div(unit, p.div_half));
-      const int sidx = unit - bh * half_q;
-      // CTAs that share an SM (and the grid as a whole) should not all be at the same point of
-      // their pair at the same time: half of them take the short tile of each pair first.  Which
-      // CTAs share an SM is not known; on a 148-SM B200 CTA i sits with i + 148 or with i ^ 1, and
-      // this hash separates both.  (A constant divisor: no division is executed, and nothing is
-      // kept in a register through the softmax loop, where one more live value costs spills.)
-      const int pair_swap = (blockIdx.x ^ (blockIdx.x / kSmCountHint)) & 1;
-      qt = ((n & 1) ^ pair_swap) ? sidx : p.n_qtiles - 1 - sidx;
+    if (kCausal) {
+      const int grp = static_cast<int>(fast_div(item, p.div_group_items));
+      const int r = item - grp * p.group_items;
+      const bool last = (grp + 1) * p.group_items >= p.n_items;
+      const int heads = last ? p.last_group : p.group;
+      const int step = static_cast<int>(fast_div(r, last ? p.div_last_group : p.div_group));
+      qt = p.n_qtiles - 1 - step;
+      bh = grp * p.group + (r - step * heads);
     } else {
-      if (!kPersistent && n > 0) return false;
-      const int item = blockIdx.x + n * gridDim.x;
-      if (item >= p.n_items) return false;
       bh = static_cast<int>(fast_div(item, p.div_qtiles));
-      const int slot = item - bh * p.n_qtiles;
-      qt = slot;
-      if (kCausal) {
-        int rs = slot;
-        if (kPersistent) {       // (slot + bh) mod n_qtiles without a second division
-          const int bh_mod = bh - static_cast<int>(fast_div(bh, p.div_qtiles)) * p.n_qtiles;
-          rs = slot + bh_mod;
-          if (rs >= p.n_qtiles) rs -= p.n_qtiles;
-        }
-        qt = p.n_qtiles - 1 - rs;
-      }
+      qt = item - bh * p.n_qtiles;
     }
     w.b = static_cast<int>(fast_div(bh, p.div_heads));
     w.h = bh - w.b * p.H;
     w.q_row = qt * kBlockM;
     w.ns = kCausal ? min(nkv, qt + 1) : nkv;   // K/V tiles this query tile attends to
+  };
+  auto decode_item = [&](int n, Item& w) -> bool {
+    // The first CTAs' items are mirrored: block b < SM count has item b, the blocks after it, which join
+    // them on the SMs in the same order, have the rest of the first wave from its light end.
+    const int b = blockIdx.x;
+    const int rank = b >= p.mirror_from && b < p.mirror_to ? p.mirror_from + p.mirror_to - 1 - b : b;
+    // static: back and forth through the list, so that the CTA that got the heaviest item of one
+    // round gets the lightest of the next; otherwise the CTA's own item (the first of several)
+    const int item = kSchedule != kStatic ? rank
+                     : (n & 1)            ? (n + 1) * static_cast<int>(gridDim.x) - 1 - rank
+                                          : n * static_cast<int>(gridDim.x) + rank;
+    if (item >= p.n_items) return false;
+    decode_listed(item, w);
     return true;
   };
   // Decoding costs ~170 clocks of dependent integer arithmetic, and every role would pay it on
-  // the path between two work items.  A persistent CTA therefore decodes all its items once, one
-  // per thread, before the start-up barrier; afterwards an item is one shared-memory load (the
+  // the path between two work items.  A CTA therefore decodes all its items once, one per thread,
+  // before the start-up barrier; afterwards an item is one shared-memory load (the
   // same address for the whole warp).  The launcher picks a persistent schedule only where a CTA
   // gets at most kItemTable items.
-  auto get_item = [&](int n, Item& w) -> bool {
-    if (kPersistent) {
-      if (n >= kItemTable) return false;
-      const int4 e = sm.items[n];
-      w.q_row = e.x; w.ns = e.y; w.h = e.z; w.b = e.w;
-      return e.y != 0;
-    }
-    return decode_item(n, w);
+  auto read_item = [&](int n, Item& w) -> bool {
+    if (kSchedule != kDynamic && n >= (kPersistent ? kItemTable : 1)) return false;
+    const int4 e = sm.items[kSchedule == kDynamic ? n % kItemRing : n];
+    w.q_row = e.x; w.ns = e.y; w.h = e.z; w.b = e.w;
+    return e.y != 0;
   };
 
   // ---- one-time setup
@@ -311,6 +313,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
       mbar_init(smem_u32(&sm.kv_full[i]), 1);
       mbar_init(smem_u32(&sm.kv_empty[i]), 1);
     }
+    if (kSchedule == kDynamic) {
+      mbar_init(smem_u32(&sm.item_go), 1);
+      mbar_init(smem_u32(&sm.item_answer), 1);
+      for (int i = 0; i < kItemRing; ++i) mbar_init(smem_u32(&sm.item_full[i]), 1);
+    }
     sm.abort = 0;
     sm.abort_who = 0;
     fence_mbar_init();
@@ -323,7 +330,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     tmem_alloc(smem_u32(&sm.tmem_base), kTmemCols);
     tmem_relinquish();
   }
-  if (kPersistent) {
+  if (kSchedule == kStatic || threadIdx.x == 0) {
     Item t;
     const bool has = decode_item(threadIdx.x, t);
     sm.items[threadIdx.x] = has ? make_int4(t.q_row, t.ns, t.h, t.b) : make_int4(0, 0, 0, 0);
@@ -336,6 +343,14 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = sm.tmem_base;
   const Watch watch{&sm.abort, &sm.abort_who};
+
+  // Item n, for a whole warp; false when there is none.  (A wait that ran out ends the role here.)
+  auto get_item = [&](int n, Item& w) -> bool {
+    if (kSchedule == kDynamic && n > 0 &&
+        !wait_bar_warp(smem_u32(&sm.item_full[n % kItemRing]), (n / kItemRing - (n % kItemRing == 0 ? 1 : 0)) & 1, watch, kWaitItem))
+      return false;
+    return read_item(n, w);
+  };
 
   auto slot_of = [](int it) { return it % kKVSlots; };
   auto par_of = [](int it) { return static_cast<uint32_t>((it / kKVSlots) & 1); };
@@ -383,6 +398,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
           tma_load_4d(smem_u32(sm.q), &tmap_q, bar, 0, w.q_row, w.h, w.b);
         }
         for (int j = 0; j < w.ns && ok; ++j) {
+          if (kSchedule == kDynamic && j == max(0, w.ns - kItemLead) && elect_one()) mbar_arrive(smem_u32(&sm.item_go));
           load_kv(&tmap_k, j * kBlockN, w.h, w.b);
           load_kv(&tmap_v, j * kBlockN, w.h, w.b);
         }
@@ -396,6 +412,39 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
           wait_bar(smem_u32(&sm.q_full), (n - 1) & 1, watch, kWaitDrain, 20ull * 1000 * 1000, false);
       }
       __syncwarp();
+    } else if (kSchedule == kDynamic && warp == kItemWarp) {
+      // ================================================================= next work items
+      // Item n is asked for when the producer comes to the last tiles of item n - 1, two tiles ahead of
+      // the tensor core: early enough that nobody waits for the answer, and late, because what this
+      // CTA takes nobody else can (asked for at the item's start, B = 4 H = 12 N = 1024 took 18.6 us
+      // instead of 14.5: the CTAs that start first have the heaviest tiles and took a second one).
+      bool ok = true, more = true;
+      for (int n = 1; ok && more; ++n) {
+        ok = wait_bar_warp(smem_u32(&sm.item_go), (n - 1) & 1, watch, kWaitItem);
+        if (!ok) break;
+        const uint32_t answer = smem_u32(&sm.item_response[n & 1]), bar = smem_u32(&sm.item_answer);
+        if (elect_one()) {
+          fence_proxy_async_smem();
+          mbar_arrive_expect_tx(bar, 16);
+          clc_try_cancel(answer, bar);
+        }
+        __syncwarp();
+        ok = wait_bar_warp(bar, (n - 1) & 1, watch, kWaitItem);
+        if (!ok) {     // leave no answer of ours on its way
+          wait_bar(bar, (n - 1) & 1, watch, kWaitDrain, 20ull * 1000 * 1000, false);
+          __syncwarp();
+          break;
+        }
+        const int block = clc_block(answer);
+        more = block >= 0;
+        Item t{0, 0, 0, 0};
+        if (more) decode_listed(block, t);
+        if (lane == 0) {
+          sm.items[n % kItemRing] = make_int4(t.q_row, t.ns, t.h, t.b);
+          mbar_arrive(smem_u32(&sm.item_full[n % kItemRing]));
+        }
+        __syncwarp();
+      }
     } else if (warp == kMmaWarp) {
       // ================================================================= tcgen05 issuer
       constexpr uint32_t idesc_s = make_idesc_bf16(kBlockM, kBlockN, false);
@@ -448,13 +497,15 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
       }
       for (; have_item && ok; ++n) {
         Item wn = w;
-        const bool has_next_item = get_item(n + 1, wn);
+        // (dynamic: looked up when it is needed, it may not be known yet)
+        bool has_next_item = kSchedule != kDynamic && get_item(n + 1, wn);
         for (int j = 0; j < w.ns && ok; ++j, ++g) {
           const int itv = it;          // V_j of this item
           const int itk = it + 1;      // the next K in ring order: K_{j+1}, or K_0 of the next item
           const bool last = j + 1 == w.ns;
           // ---- S for the next tile, as soon as the softmax warps hold S(g) in registers
           FA_TRACE_EVENT(2, g, 0);
+          if (kSchedule == kDynamic && last) has_next_item = get_item(n + 1, wn);
           if (!last || has_next_item) {
             if (last)   // the next item's Q must have landed (its load waited for q_empty)
               ok = wait_bar_warp(smem_u32(&sm.q_full), (n + 1) & 1, watch, kWaitQFull);
@@ -516,7 +567,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     // O / l -> bf16 -> swizzled staging tile -> TMA store; LSE.  Reads O of the owed item.
     auto epilogue = [&](const int owed_n) -> bool {
       Item ow;
-      get_item(owed_n, ow);
+      read_item(owed_n, ow);
       const float2 parked = sm.owed[r];
       const uint32_t bar_o_free = smem_u32(&sm.o_free);
       // this thread's row of the staging tile; 16-byte chunk c goes to position c ^ (r & 7)

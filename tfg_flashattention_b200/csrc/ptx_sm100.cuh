@@ -85,6 +85,26 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint4 v) {
                : "memory");
 }
 
+// Cluster launch control: a running CTA asks for a CTA of its own grid that has not started yet and
+// does its work instead.  The 16-byte answer arrives asynchronously in shared memory.  After an
+// answer without a CTA no further request may be made.
+__device__ __forceinline__ void clc_try_cancel(uint32_t response, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+               ::"r"(response), "r"(bar) : "memory");
+}
+__device__ __forceinline__ int clc_block(uint32_t response) {       // its blockIdx.x, or -1
+  int x;
+  asm volatile(
+      "{\n\t.reg .b128 r;\n\t.reg .pred p;\n\t.reg .b32 y, z, w, c;\n\t"
+      "ld.shared.b128 r, [%1];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "mov.b32 c, -1;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {c, y, z, w}, r;\n\t"
+      "mov.b32 %0, c;\n\t}"
+      : "=r"(x) : "r"(response) : "memory");
+  return x;
+}
+
 // ----------------------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
