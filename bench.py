@@ -781,7 +781,7 @@ def main():
                            "gbs_per_gpu": round(nbytes / (dms * 1e-3) / 1e9, 1),
                            "frac_of_hbm_peak": round(nbytes / (dms * 1e-3) / 1e9 / peaks["hbm_gbs"], 3),
                            "cache_sets_rotated": n_sets,
-                           "kernels": "fa::fa_decode_partial_kernel (+ fa::fa_decode_combine_kernel when keys are split)"})
+                           "kernels": "fa::fa_decode_kernel"})
             del caches, dq, do
             torch.cuda.empty_cache()
         if cfa.last_status() != 0:

@@ -131,11 +131,10 @@ int fa_b200_last_status(int device, void* stream);
  *
  * q and o are bf16 [B, H, 64] (strides {batch, head} in elements, multiples of 8); the caches are
  * bf16 [B, H, >= kv_len, 64] with strides {batch, head, row}; lse (optional) is fp32 [B, H].
- * With few (batch, head) pairs and a long cache the keys of a head are processed in several chunks
- * whose partial results pass through `workspace` (few pairs with at most 4096 rows run as one
- * wide CTA per head and need none): device memory of at least
- * fa_b200_decode_workspace_bytes(B, H, kv_len) bytes, 16-byte aligned, owned by the caller and not
- * shared by calls that may overlap on the GPU (it may be NULL when that function returns 0).
+ * `workspace` is device memory of at least fa_b200_decode_workspace_bytes(B, H, kv_len) bytes,
+ * 16-byte aligned, owned by the caller (it may be NULL when that function returns 0).  The present
+ * kernel merges the parts of a head inside a thread-block cluster and does not touch it;
+ * fa_b200_decode_direct does not ask for it.
  */
 typedef struct fa_b200_decode_params {
   const void* q;
@@ -178,35 +177,23 @@ int64_t fa_b200_decode_workspace_bytes(int32_t B, int32_t H, int32_t kv_len);
  * FA_B200_ERR_WORKSPACE when the workspace is missing, too small or misaligned. */
 int fa_b200_decode(const fa_b200_decode_params* p);
 
-/* Largest split-KV scratch fa_b200_decode_static can serve, in bytes (the size of the buffer that
- * is compiled into the library; it occupies this much memory on every GPU that loads the library,
- * until the process exits). */
+/* The same without a workspace, for every size: p->workspace and p->workspace_bytes are ignored. */
+int fa_b200_decode_direct(const fa_b200_decode_params* p);
+
+/* The size limit of fa_b200_decode_static, in bytes of partial results (see there). */
 #define FA_B200_STATIC_SCRATCH_BYTES (256 * 1024)
 
-/* fa_b200_decode for callers that must not allocate device memory and have none to lend: the
- * split-KV partial results go to a fixed buffer that lives inside the library image instead of
- * p->workspace (p->workspace and p->workspace_bytes are ignored).  Typical callers: a serving
- * process whose framework has already claimed all device memory for its own pool, so that a
- * cudaMalloc from a plug-in fails or is forbidden; a request path on which cudaMalloc / cudaFree
- * are banned because they can synchronise the whole device and stall every other stream; a small
- * C host with a fixed memory map and no allocator to call.  This function itself calls no
- * cudaMalloc, cudaFree or other allocating routine.
+/* fa_b200_decode for callers that must not allocate device memory and have none to lend (p->workspace
+ * and p->workspace_bytes are ignored): a serving process whose framework has claimed all device memory
+ * for its own pool; a request path on which cudaMalloc / cudaFree are banned because they can
+ * synchronise the whole device; a small C host with a fixed memory map.  It calls no allocating routine.
  *
- *   - The keys of a head are cut into 592 / (B * H) chunks of at least 64 rows (fa_b200_decode
- *     cuts caches of 2048 rows and more finer than that, which this entry point does not follow,
- *     so that what fits the buffer does not move with that tuning).  Problems whose partial
- *     results -- 264 bytes per (batch, head) pair and chunk -- exceed FA_B200_STATIC_SCRATCH_BYTES
- *     are refused with FA_B200_ERR_STATIC_SCRATCH; nothing is launched.  (Up to 496 (batch, head)
- *     pairs always fit; from 592 pairs on no scratch is used.)
- *   - The first call on each device looks up the buffer's device address; make that first call
- *     outside of any stream capture.
- *   - All calls on a device share the one buffer, and it keeps whatever the previous call left in
- *     it.  Nothing in it needs clearing -- every partial result is written before it is read --
- *     but two calls that may run on the GPU at the same time (different streams, different host
- *     threads) race on it: serialise them, or use fa_b200_decode with separate workspaces.
- *
- * Results are identical to fa_b200_decode wherever both cut the keys into the same chunks, and
- * equal within rounding otherwise.  This entry point has no counterpart in the reference. */
+ * It refuses what its original form refused, which kept partial results in a fixed buffer: with the
+ * keys of a head cut into 592 / (B * H) chunks of at least 64 rows, problems whose partial results --
+ * 264 bytes per (batch, head) pair and chunk -- exceed FA_B200_STATIC_SCRATCH_BYTES get
+ * FA_B200_ERR_STATIC_SCRATCH and nothing is launched.  (Up to 496 (batch, head) pairs always fit; from
+ * 592 pairs on nothing is cut.)  fa_b200_decode_direct has no such limit.  Results are those of
+ * fa_b200_decode.  This entry point has no counterpart in the reference. */
 int fa_b200_decode_static(const fa_b200_decode_params* p);
 
 /* Residual add + LayerNorm in one pass (bf16 in / out, fp32 arithmetic), for the transformer block

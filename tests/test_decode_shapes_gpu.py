@@ -1,0 +1,58 @@
+"""Every launch shape of the decode kernel (decode_shape in csrc/fa_b200_api.cu): clusters of 1 to 16
+CTAs, 128 to 512 threads, at the borders of the rule and of a CTA's rows (four rows per lane group and
+step), against attention of the same bf16 numbers in fp64.
+
+The kernel rounds once, to bf16: 8 significant bits, so at most 2^-8 of the value.  Its fp32 sums over
+n <= 4100 rows of values up to about 5 and the exponentials (2^-22) add well under 1e-3 of their scale;
+the part that is left where terms cancel is covered by 1e-4 absolute."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _close(o, want):
+    return ((o.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
+
+
+@pytest.mark.parametrize("B,H,kv", [
+    (1, 1, 1), (1, 3, 31), (1, 12, 95), (1, 12, 96), (2, 12, 191), (1, 25, 193), (4, 25, 383),   # clusters 1, 2, 4
+    (1, 25, 767), (1, 25, 769), (2, 25, 1025),                                                    # 8, 16
+    (1, 12, 1024), (1, 12, 1025), (1, 25, 2049), (1, 25, 4096), (1, 12, 2049), (1, 12, 4100),     # 256, 512 threads
+    (41, 25, 64), (41, 25, 300), (42, 25, 300), (20, 25, 130), (21, 25, 777),                     # around 1036 heads, 518
+])
+@pytest.mark.parametrize("append", [False, True])
+def test_decode_shapes(fa_lib, B, H, kv, append):
+    from tfg_flashattention_b200 import custom_flash_attn as cfa
+    g = torch.Generator(device="cuda").manual_seed(B * 100003 + H * 1009 + kv)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    rows = kv + 5
+    q, k, v = rnd(B, H, 64), rnd(B, rows, H, 64).transpose(1, 2), rnd(B, H, rows, 64)
+    kn, vn = rnd(B, H, 64), rnd(B, H, 64)
+    k_ref, v_ref = k.clone(), v.clone()
+    if append:
+        k_ref[:, :, kv - 1], v_ref[:, :, kv - 1] = kn, vn
+    new = dict(k_new=kn, v_new=vn) if append else {}
+    o, lse = cfa.decode(q, k, v, kv, return_lse=True, **new)
+    assert torch.equal(k, k_ref) and torch.equal(v, v_ref)
+    s = torch.einsum("bhd,bhnd->bhn", q.double(), k_ref[:, :, :kv].double()) / 8.0
+    want = torch.einsum("bhn,bhnd->bhd", torch.softmax(s, -1), v_ref[:, :, :kv].double())
+    assert _close(o, want)
+    assert (lse.double() - torch.logsumexp(s, -1)).abs().max().item() <= 1e-4
+    # a device length inside a launch sized for the whole cache: some CTAs then have few rows or none
+    for n in {1, max(1, kv // 3), kv}:
+        o2 = cfa.decode(q, k, v, torch.full((1,), n, dtype=torch.int32, device="cuda"))
+        s = torch.einsum("bhd,bhnd->bhn", q.double(), k[:, :, :n].double()) / 8.0
+        want = torch.einsum("bhn,bhnd->bhd", torch.softmax(s, -1), v[:, :, :n].double())
+        assert _close(o2, want)
+
+
+def test_more_heads_than_a_grid_dimension_of_65535(fa_lib):
+    from tfg_flashattention_b200 import custom_flash_attn as cfa
+    B, H = 70000, 1
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q, k, v = (torch.randn(*s, device="cuda", generator=g).bfloat16() for s in ((B, H, 64), (B, H, 2, 64), (B, H, 2, 64)))
+    o = cfa.decode(q, k, v, 2)
+    s = torch.einsum("bhd,bhnd->bhn", q.double(), k.double()) / 8.0
+    want = torch.einsum("bhn,bhnd->bhd", torch.softmax(s, -1), v.double())
+    assert _close(o, want)

@@ -80,7 +80,7 @@ class FaGptStepParams(ctypes.Structure):
 
 
 EXPORTS = ("fa_b200_fwd", "fa_b200_fwd_plan", "fa_b200_validate", "fa_b200_strerror", "fa_b200_device_ok",
-           "fa_b200_last_status", "fa_b200_abi_version", "fa_b200_decode", "fa_b200_decode_workspace_bytes", "fa_b200_decode_static",
+           "fa_b200_last_status", "fa_b200_abi_version", "fa_b200_decode", "fa_b200_decode_workspace_bytes", "fa_b200_decode_static", "fa_b200_decode_direct",
            "fa_b200_add_layernorm", "fa_b200_linear_small", "fa_b200_gpt_step", "fa_b200_gpt_step_workspace_bytes")
 
 SCHEDULES = {-1: "none", 0: "cta_per_tile", 1: "persistent_paired", 2: "persistent_rotated",
@@ -118,6 +118,8 @@ def load() -> ctypes.CDLL:
     lib.fa_b200_last_status.restype = ctypes.c_int
     lib.fa_b200_decode.argtypes = [ctypes.POINTER(FaDecodeParams)]
     lib.fa_b200_decode.restype = ctypes.c_int
+    lib.fa_b200_decode_direct.argtypes = [ctypes.POINTER(FaDecodeParams)]
+    lib.fa_b200_decode_direct.restype = ctypes.c_int
     lib.fa_b200_decode_static.argtypes = [ctypes.POINTER(FaDecodeParams)]
     lib.fa_b200_decode_static.restype = ctypes.c_int
     lib.fa_b200_decode_workspace_bytes.argtypes = [ctypes.c_int32, ctypes.c_int32, ctypes.c_int32]

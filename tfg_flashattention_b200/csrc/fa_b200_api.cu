@@ -120,6 +120,12 @@ void init_device(int dev) {
   // a slot only starts later -- work items are partitioned by grid stride, no CTA waits on another.
   st.resident_ctas = fa::kCtasPerSm * prop.multiProcessorCount;
   st.sm_count = prop.multiProcessorCount;
+  for (const void* fn : {reinterpret_cast<const void*>(&fa::fa_decode_kernel<128, 7, true>),
+                         reinterpret_cast<const void*>(&fa::fa_decode_kernel<256, 4, true>),
+                         reinterpret_cast<const void*>(&fa::fa_decode_kernel<512, 2, true>)}) {
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) { st.init_error = static_cast<int>(e); return; }
+  }
   void* addr = nullptr;
   e = cudaGetSymbolAddress(&addr, g_fa_status);
   if (e != cudaSuccess) { st.init_error = static_cast<int>(e); return; }
@@ -378,45 +384,42 @@ int fa_b200_fwd_plan(const fa_b200_params* p, int32_t* schedule, int32_t* grid) 
 // ------------------------------------------------------------------------------------ decode
 namespace {
 
-// CTAs the split aims for.  Every CTA keeps a fixed 16 KB of loads in flight, so bandwidth grows
-// with the number of resident CTAs: measured on B200 at B=8, H=25, kv_len=8192, 600 / 1800 / 2400
-// CTAs give 4.3 / 4.6 / 5.2 TB/s.  Short caches are latency-bound and pay for the second launch
-// and the partials instead (B=32, kv_len=1024: 4.8 TB/s unsplit, 4.4 split in two), so the high
-// target and its coarser chunks apply from 2048 rows on.
-constexpr int kDecodeTargetCtas = 592;        // 4 CTAs per SM on a 148-SM part
-constexpr int kDecodeTargetCtasLong = 2368;   // 16 CTAs per SM: every thread slot of the part
+// Bytes of workspace that callers of fa_b200_decode lend, by the rule of the kernels that needed one:
+// chunks of a head's keys, 66 floats each.  Today's kernel merges inside a cluster and touches none of
+// it; the sizes stay what callers have been told.
+constexpr int kDecodeTargetCtas = 592, kDecodeTargetCtasLong = 2368;
 constexpr int kDecodeLongLen = 2048;
-constexpr int kDecodeMinRows = 64, kDecodeMinRowsLong = 512;   // rows per chunk, at least
-
-constexpr int kDecodeWideMaxHeads = 296;   // two 1024-thread CTAs per SM on a 148-SM part
-constexpr int kDecodeWideMaxLen = 4096;    // up to 1 MB of K/V per head through one SM
-
-// How the keys of one head are cut: `splits` chunks of `rows` rows (a multiple of the 16 lane
-// groups of a CTA).  The same rule sizes the workspace and launches the kernel.  Few heads with
-// short caches take the one-launch form instead (`wide`: one 1024-thread CTA per head, no split).
-// `fine_for_long` = false keeps the short-cache rule at every length: the allocation-free entry
-// point cuts that way, so that what fits its fixed scratch buffer does not depend on this tuning.
-void decode_split(int B, int H, int kv_len, int* splits, int* rows, bool* wide = nullptr,
-                  bool fine_for_long = true) {
+constexpr int kDecodeChunkRows = 64, kDecodeChunkRowsLong = 512;   // rows per chunk, at least
+int64_t decode_workspace(int B, int H, int kv_len, bool fine_for_long) {
   const long long heads = static_cast<long long>(B) * H;
-  const bool w = heads <= kDecodeWideMaxHeads && kv_len <= kDecodeWideMaxLen;
-  if (wide != nullptr) *wide = w;
-  if (w) {
-    *splits = 1;
-    *rows = (kv_len + 127) / 128 * 128;
-    return;
-  }
+  if (heads == 0 || (heads <= 296 && kv_len <= 4096)) return 0;
   const bool long_cache = fine_for_long && kv_len >= kDecodeLongLen;
-  const long long target = long_cache ? kDecodeTargetCtasLong : kDecodeTargetCtas;
-  const long long min_rows = long_cache ? kDecodeMinRowsLong : kDecodeMinRows;
-  long long want = (target + heads - 1) / heads;
-  const long long max_splits = (kv_len + min_rows - 1) / min_rows;
-  if (want > max_splits) want = max_splits;
-  if (want < 1) want = 1;
-  long long r = (kv_len + want - 1) / want;
-  r = (r + fa::kDecodeGroups - 1) / fa::kDecodeGroups * fa::kDecodeGroups;
-  *rows = static_cast<int>(r);
-  *splits = static_cast<int>((kv_len + r - 1) / r);
+  const long long min_rows = long_cache ? kDecodeChunkRowsLong : kDecodeChunkRows;
+  long long want = ((long_cache ? kDecodeTargetCtasLong : kDecodeTargetCtas) + heads - 1) / heads;
+  const long long most = (kv_len + min_rows - 1) / min_rows;
+  want = want > most ? most : (want < 1 ? 1 : want);
+  const long long rows = ((kv_len + want - 1) / want + 15) / 16 * 16;
+  const long long chunks = (kv_len + rows - 1) / rows;
+  return chunks == 1 ? 0 : heads * chunks * fa::kDecodePartial * static_cast<int64_t>(sizeof(float));
+}
+
+// How a problem is launched: CTAs per head (a cluster) and their threads.  As many CTAs as are resident
+// at seven per SM, the cluster a power of two, no CTA with less than kDecodeMinRows rows; where clusters
+// of 16 still leave the chip half empty and a CTA has more rows than it loads at once (threads / 2),
+// larger CTAs.  (H = 12, B=1 kv 8192: 12.1 us with 128 threads, 7.5 with 512; H = 25: 14.8, 11.8 with
+// 256; from 48 heads on nothing.)
+struct DecodeShape {
+  int cluster, threads;
+};
+DecodeShape decode_shape(long long heads, int kv_len, int sm_count) {
+  DecodeShape s{1, 128};
+  const long long slots = 7LL * sm_count;
+  while (s.cluster < fa::kDecodeClusterMax && heads * s.cluster * 2 <= slots && kv_len >= s.cluster * 2 * fa::kDecodeMinRows)
+    s.cluster *= 2;
+  if (s.cluster == fa::kDecodeClusterMax)
+    while (s.threads < 512 && heads * s.cluster * s.threads * 2 <= slots * 128 && kv_len > s.cluster * s.threads / 2)
+      s.threads *= 2;
+  return s;
 }
 
 bool stride_ok_n(const int64_t* s, int n) {
@@ -457,24 +460,32 @@ int decode_validate(const fa_b200_decode_params* p) {
 int64_t fa_b200_decode_workspace_bytes(int32_t B, int32_t H, int32_t kv_len) {
   if (B < 0 || H < 0 || kv_len < 1) return FA_B200_ERR_SHAPE;
   if (B == 0 || H == 0) return 0;
-  int splits = 1, rows = 0;
-  decode_split(B, H, kv_len, &splits, &rows);
-  if (splits == 1) return 0;
-  return static_cast<int64_t>(B) * H * splits * fa::kDecodePartial * static_cast<int64_t>(sizeof(float));
+  return decode_workspace(B, H, kv_len, /*fine_for_long=*/true);
 }
 
+extern "C++" {
 namespace {
 
-// The launch shared by fa_b200_decode and fa_b200_decode_static; they differ only in where the
-// split-KV scratch lives.  `p` has been validated, the device is current and set up.
-int decode_launch(const fa_b200_decode_params* p, float* scratch, int splits, int rows, bool wide) {
+template <int kThreads, int kCtasPerSm>
+cudaError_t decode_launch_cluster(const fa::DecodeParams& kp, unsigned heads, int cluster, cudaStream_t stream) {
+  return launch_kernel(&fa::fa_decode_kernel<kThreads, kCtasPerSm, true>, dim3(heads * static_cast<unsigned>(cluster)),
+                       kThreads, 0, stream, static_cast<unsigned>(cluster), kp);
+}
+
+// The launch shared by the decode entry points.  `p` has been validated.
+int decode_launch(const fa_b200_decode_params* p) {
+  if (p->B == 0 || p->H == 0) return FA_B200_OK;
+  DeviceGuard guard(p->device);
+  if (guard.error) return guard.error;
+  DeviceState* stp = nullptr;
+  const int rc = ready_device(p->device, &stp);
+  if (rc != 0) return rc;
   fa::DecodeParams kp;
   kp.q = static_cast<const __nv_bfloat16*>(p->q);
   kp.k = static_cast<const __nv_bfloat16*>(p->k_cache);
   kp.v = static_cast<const __nv_bfloat16*>(p->v_cache);
   kp.o = static_cast<__nv_bfloat16*>(p->o);
   kp.lse = p->lse;
-  kp.scratch = scratch;
   kp.q_sb = p->q_strides[0]; kp.q_sh = p->q_strides[1];
   kp.o_sb = p->o_strides[0]; kp.o_sh = p->o_strides[1];
   kp.k_sb = p->k_strides[0]; kp.k_sh = p->k_strides[1]; kp.k_sn = p->k_strides[2];
@@ -484,95 +495,45 @@ int decode_launch(const fa_b200_decode_params* p, float* scratch, int splits, in
   kp.k_new = static_cast<const __nv_bfloat16*>(p->k_new);
   kp.v_new = static_cast<const __nv_bfloat16*>(p->v_new);
   kp.new_sb = p->new_strides[0]; kp.new_sh = p->new_strides[1];
-  kp.splits = splits;
-  kp.rows_per_split = rows;
   const float scale = p->softmax_scale > 0.0f ? p->softmax_scale : 1.0f / std::sqrt(static_cast<float>(p->d));
   kp.scale_log2 = scale * 1.4426950408889634f;
 
   const cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   const unsigned heads = static_cast<unsigned>(p->B * p->H);
-  const dim3 grid(heads, static_cast<unsigned>(splits));
-  if (wide) {
-    // a cluster per head while that makes more CTAs than SMs hardly at all (8 x 37 = 4 x 74 = 2 x 148
-    // = 296 CTAs of 512 threads: two per SM of a 148-SM part), beyond it one wide CTA per head
-    const unsigned cluster = heads <= 37 ? 8 : (heads <= 74 ? 4 : (heads <= 148 ? 2 : 1));
-    if (cluster > 1)
-      return static_cast<int>(launch_kernel(&fa::fa_decode_cluster_kernel, dim3(cluster, heads), fa::kDecodeClusterThreads, 0, stream, cluster, kp));
-    return static_cast<int>(launch_kernel(&fa::fa_decode_partial_kernel<fa::kDecodeWideThreads>, grid, fa::kDecodeWideThreads, 0, stream, 1, kp));
-  }
-  cudaError_t e = launch_kernel(&fa::fa_decode_partial_kernel<fa::kDecodeThreads>, grid, fa::kDecodeThreads, 0, stream, 1, kp);
-  if (e == cudaSuccess && splits > 1)
-    e = launch_kernel(&fa::fa_decode_combine_kernel, dim3(heads), 64, 0, stream, 1, kp);
-  return static_cast<int>(e);
+  const DecodeShape shape = decode_shape(heads, p->kv_len, stp->sm_count);
+  kp.cluster_log2 = 0;
+  while ((1 << kp.cluster_log2) < shape.cluster) ++kp.cluster_log2;
+  if (shape.cluster == 1)
+    return static_cast<int>(launch_kernel(&fa::fa_decode_kernel<128, 7, false>, dim3(heads), 128, 0, stream, 1, kp));
+  return static_cast<int>(shape.threads == 128   ? decode_launch_cluster<128, 7>(kp, heads, shape.cluster, stream)
+                          : shape.threads == 256 ? decode_launch_cluster<256, 4>(kp, heads, shape.cluster, stream)
+                                                 : decode_launch_cluster<512, 2>(kp, heads, shape.cluster, stream));
 }
 
 }  // namespace
+}  // extern "C++"
 
 int fa_b200_decode(const fa_b200_decode_params* p) {
-  int rc = decode_validate(p);
+  const int rc = decode_validate(p);
   if (rc != FA_B200_OK) return rc;
-  if (p->B == 0 || p->H == 0) return FA_B200_OK;
-  int splits = 1, rows = 0;
-  bool wide = false;
-  decode_split(p->B, p->H, p->kv_len, &splits, &rows, &wide);
-  if (splits > 1) {
-    const int64_t need = fa_b200_decode_workspace_bytes(p->B, p->H, p->kv_len);
-    if (p->workspace == nullptr || p->workspace_bytes < need ||
-        (reinterpret_cast<uintptr_t>(p->workspace) & 15u))
-      return FA_B200_ERR_WORKSPACE;
-  }
-  DeviceGuard guard(p->device);
-  if (guard.error) return guard.error;
-  DeviceState* stp = nullptr;
-  if ((rc = ready_device(p->device, &stp)) != 0) return rc;
-  return decode_launch(p, static_cast<float*>(p->workspace), splits, rows, wide);
+  const int64_t need = decode_workspace(p->B, p->H, p->kv_len, /*fine_for_long=*/true);
+  if (need > 0 && (p->workspace == nullptr || p->workspace_bytes < need ||
+                   (reinterpret_cast<uintptr_t>(p->workspace) & 15u)))
+    return FA_B200_ERR_WORKSPACE;
+  return decode_launch(p);
 }
 
-// ----------------------------------------------------------- decode without any allocation
-namespace {
-
-// Split-KV scratch compiled into the library image: one copy per GPU that loads the module.
-// In host code this name is only a handle for the runtime's symbol functions, never a device
-// address; kernels get the address that cudaGetSymbolAddress returns for the current device.
-static __device__ __align__(256) unsigned char g_fa_decode_static_scratch[FA_B200_STATIC_SCRATCH_BYTES];
-
-struct StaticScratchState {
-  std::once_flag once;
-  int error = 0;          // cudaError_t of the address look-up, if it failed
-  float* ptr = nullptr;   // device address of the buffer on this device
-};
-StaticScratchState g_static_scratch[kMaxDevices];
-
-// Runs once per device, with that device current.
-void init_static_scratch(int dev) {
-  StaticScratchState& ss = g_static_scratch[dev];
-  void* addr = nullptr;
-  const cudaError_t e = cudaGetSymbolAddress(&addr, g_fa_decode_static_scratch);
-  if (e != cudaSuccess) { ss.error = static_cast<int>(e); return; }
-  ss.ptr = static_cast<float*>(addr);
+int fa_b200_decode_direct(const fa_b200_decode_params* p) {
+  const int rc = decode_validate(p);
+  return rc != FA_B200_OK ? rc : decode_launch(p);
 }
-
-}  // namespace
 
 int fa_b200_decode_static(const fa_b200_decode_params* p) {
-  int rc = decode_validate(p);
+  const int rc = decode_validate(p);
   if (rc != FA_B200_OK) return rc;
-  if (p->B == 0 || p->H == 0) return FA_B200_OK;
-  int splits = 1, rows = 0;
-  bool wide = false;
-  decode_split(p->B, p->H, p->kv_len, &splits, &rows, &wide, /*fine_for_long=*/false);
-  if (splits > 1 && static_cast<int64_t>(p->B) * p->H * splits * fa::kDecodePartial *
-                            static_cast<int64_t>(sizeof(float)) > static_cast<int64_t>(FA_B200_STATIC_SCRATCH_BYTES))
+  if (decode_workspace(p->B, p->H, p->kv_len, /*fine_for_long=*/false) > static_cast<int64_t>(FA_B200_STATIC_SCRATCH_BYTES))
     return FA_B200_ERR_STATIC_SCRATCH;
-
-  DeviceGuard guard(p->device);
-  if (guard.error) return guard.error;
-  DeviceState* stp = nullptr;
-  if ((rc = ready_device(p->device, &stp)) != 0) return rc;   // architecture check, no allocation
-  StaticScratchState& ss = g_static_scratch[p->device];
-  std::call_once(ss.once, init_static_scratch, p->device);  // first call on this device only
-  if (ss.error) return ss.error;
-  return decode_launch(p, ss.ptr, splits, rows, wide);
+  return decode_launch(p);
 }
 
 int fa_b200_device_ok(int device) {

@@ -261,6 +261,14 @@ __device__ __forceinline__ uint64_t sub_f32x2(uint64_t a, uint64_t b) {
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t bf16x2_to_f32x2(uint32_t v) {
+  return pack_f32x2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+}
 // 2^x for two values on the FMA pipe (no MUFU): x is clamped to >= -126, split into
 // round(x) + f with f in [-0.5, 0.5] by the 1.5 * 2^23 shift, 2^f is a cubic (relative error
 // below 1e-4, far under the bf16 rounding of P that follows) and round(x) goes into the exponent.

@@ -233,17 +233,10 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* k
       O = at::empty({B, H, d}, Q.options());
     }
     const bool return_lse = flag_arg(a[4], false);
-    at::Tensor lse, workspace;
+    at::Tensor lse;
     if (return_lse) lse = at::empty({B, H}, Q.options().dtype(torch::kFloat32));
     p.B = static_cast<int32_t>(B); p.H = static_cast<int32_t>(H);
     p.kv_len = static_cast<int32_t>(kv_len); p.d = static_cast<int32_t>(d);
-    const int64_t need = fa_b200_decode_workspace_bytes(p.B, p.H, p.kv_len);
-    FA_CHECK(need >= 0, "custom_flash_attn.decode failed (", need, "): ", fa_b200_strerror(static_cast<int>(need)));
-    if (need > 0) {     // from torch's allocator on every call: safe with several streams and threads
-      workspace = at::empty({need}, Q.options().dtype(torch::kUInt8));
-      p.workspace = workspace.data_ptr();
-      p.workspace_bytes = need;
-    }
     if (B * H > 0) {
       p.q = q.data_ptr(); p.k_cache = K.data_ptr(); p.v_cache = V.data_ptr(); p.o = O.data_ptr();
       strides2(q, p.q_strides);
@@ -272,7 +265,7 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* k
     }
     p.device = Q.device().index();
     p.stream = c10::cuda::getCurrentCUDAStream(Q.device().index()).stream();
-    launch("custom_flash_attn.decode", [&] { return fa_b200_decode(&p); });
+    launch("custom_flash_attn.decode", [&] { return fa_b200_decode_direct(&p); });
     const at::Tensor result = given(a[6]) ? THPVariable_Unpack(a[6]) : (squeeze ? O.unsqueeze(2) : O);
     return return_lse ? pair(result, lse) : THPVariable_Wrap(result);
   });

@@ -191,8 +191,8 @@ def decode(Q, K_cache, V_cache, kv_len, return_lse=False, softmax_scale=None, ou
     k_new, v_new [B, H, 64] (optional, both): the key / value of the token being generated; the
     kernel uses them as row kv_len-1 and writes them into that row of the caches (the cache
     append of the step without a separate copy kernel).
-    Returns O shaped like Q (and LSE [B, H] fp32 when asked).  The split-KV workspace comes from
-    torch's allocator on every call: calls on different streams do not share anything."""
+    Returns O shaped like Q (and LSE [B, H] fp32 when asked).  Calls on
+    different streams share nothing."""
     if binding() == "ext":
         return _ext.decode(Q, K_cache, V_cache, kv_len, return_lse, softmax_scale, out, k_new, v_new)
     squeeze = Q.dim() == 4
@@ -232,10 +232,6 @@ def decode(Q, K_cache, V_cache, kv_len, return_lse=False, softmax_scale=None, ou
     lse = torch.empty((B, H), dtype=torch.float32, device=Q.device) if return_lse else None
 
     lib = _lib.load()
-    need = lib.fa_b200_decode_workspace_bytes(B, H, kv_len)
-    if need < 0:
-        raise RuntimeError(f"custom_flash_attn.decode failed ({need}): {_lib.strerror(int(need))}")
-    ws = torch.empty(need, dtype=torch.uint8, device=Q.device) if need > 0 else None
 
     def two(t):      # {batch, head} strides; size-1 dimensions get a canonical stride
         sb, sh = t.stride(0), t.stride(1)
@@ -258,8 +254,6 @@ def decode(Q, K_cache, V_cache, kv_len, return_lse=False, softmax_scale=None, ou
     p = _lib.FaDecodeParams()
     p.q, p.k_cache, p.v_cache, p.o = q3.data_ptr(), K_cache.data_ptr(), V_cache.data_ptr(), O.data_ptr()
     p.lse = lse.data_ptr() if lse is not None else None
-    p.workspace = ws.data_ptr() if ws is not None else None
-    p.workspace_bytes = ws.numel() if ws is not None else 0
     p.B, p.H, p.kv_len, p.d = B, H, kv_len, d
     if B * H > 0:
         p.q_strides, p.o_strides = two(q3), two(O)
@@ -284,7 +278,7 @@ def decode(Q, K_cache, V_cache, kv_len, return_lse=False, softmax_scale=None, ou
         if two(kn)[:] != two(vn)[:]:
             raise RuntimeError("k_new and v_new must have the same strides")
         p.k_new, p.v_new, p.new_strides = kn.data_ptr(), vn.data_ptr(), two(kn)
-    rc = lib.fa_b200_decode(ctypes.byref(p))
+    rc = lib.fa_b200_decode_direct(ctypes.byref(p))
     if rc != 0:
         raise RuntimeError(f"custom_flash_attn.decode failed ({rc}): {_lib.strerror(rc)}")
     result = out if out is not None else (O.unsqueeze(2) if squeeze else O)
