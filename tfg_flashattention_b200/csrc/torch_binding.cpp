@@ -19,6 +19,7 @@
 // The functions are plain CPython vector calls: for the smallest problems the call IS the time, and
 // pybind11's argument casters cost about as much as the launch (a decode call through ctypes: 31-38
 // us of host time for 4-9 us of GPU work).
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -96,6 +97,16 @@ PyObject* pair(const at::Tensor& a, const at::Tensor& b) {
   PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(b));
   return t;
 }
+// Outputs come from the allocator directly: the dispatcher's way to it (autograd, device guards, the
+// factory function's own dispatch) costs as much as the allocation, and nothing here is differentiated.
+at::Tensor empty_cuda(at::IntArrayRef sizes, at::ScalarType type, const at::Device& device) {
+  return at::detail::empty_cuda(sizes, type, device, std::nullopt);
+}
+at::Tensor empty_like_cuda(const at::Tensor& t) {
+  if (!t.is_non_overlapping_and_dense()) return at::empty_like(t);      // chooses the strides itself
+  return at::detail::empty_strided_cuda(t.sizes(), t.strides(), t.scalar_type(), t.device());
+}
+
 template <class Call>
 void launch(const char* what, Call call) {
   int rc;
@@ -144,10 +155,10 @@ PyObject* forward(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* 
       check_input(O, "out");
       FA_CHECK(O.sizes() == Q.sizes() && O.device() == Q.device(), "out must match Q in shape and device");
     } else {
-      O = at::empty_like(Q);   // same allocation rule as the reference (torch_bind.cpp:31)
+      O = empty_like_cuda(Q);   // same allocation rule as the reference (torch_bind.cpp:31)
     }
     at::Tensor lse;
-    if (return_lse) lse = at::empty({Q.size(0), Q.size(1), Q.size(2)}, Q.options().dtype(torch::kFloat32));
+    if (return_lse) lse = empty_cuda({Q.size(0), Q.size(1), Q.size(2)}, torch::kFloat32, Q.device());
 
     fa_b200_params p{};
     p.B = static_cast<int32_t>(Q.size(0));
@@ -174,10 +185,13 @@ PyObject* forward(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* 
   });
 }
 
-// [B, H, 1, 64] as [B, H, 64]
-at::Tensor one_row(const at::Tensor& t) { return t.dim() == 4 ? t.select(2, 0) : t; }
-
-// {batch, head} strides of [B, H, 64]; size-1 dimensions get a canonical stride
+// Whether t is [B, H, 64] or [B, H, 1, 64], dense in the last dimension.  (No view is made of it: three
+// of them cost more host time than the launch's arguments.)
+bool is_row(const at::Tensor& t, int64_t B, int64_t H, int64_t d) {
+  const int64_t n = t.dim();
+  return (n == 3 || (n == 4 && t.size(2) == 1)) && t.size(0) == B && t.size(1) == H && t.size(n - 1) == d && t.stride(n - 1) == 1;
+}
+// {batch, head} strides of it; size-1 dimensions get a canonical stride
 void strides2(const at::Tensor& t, int64_t out[2]) {
   out[1] = t.size(1) == 1 ? 64 : t.stride(1);
   out[0] = t.size(0) == 1 ? std::max<int64_t>(t.size(1) * out[1], 64) : t.stride(0);
@@ -202,8 +216,7 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* k
     }
     FA_CHECK(!squeeze || Q.size(2) == 1, "Q must hold one query row per head: [B, H, 64] or [B, H, 1, 64]");
     FA_CHECK((squeeze || Q.dim() == 3) && K.dim() == 4 && V.dim() == 4, "expected Q [B, H, d] and caches [B, H, N, d]");
-    const at::Tensor q = squeeze ? Q.select(2, 0) : Q;
-    const int64_t B = q.size(0), H = q.size(1), d = q.size(2), rows = K.size(2);
+    const int64_t B = Q.size(0), H = Q.size(1), d = Q.size(Q.dim() - 1), rows = K.size(2);
     FA_CHECK(K.size(0) == B && K.size(1) == H && V.sizes() == K.sizes() && K.size(3) == d,
              "Q, K_cache and V_cache disagree on B, H or d");
     fa_b200_decode_params p{};
@@ -221,25 +234,26 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* k
       if (kv_len == -1 && PyErr_Occurred()) throw PythonError();
     }
     FA_CHECK(kv_len >= 1 && kv_len <= rows, "kv_len must be between 1 and the cache length");
-    FA_CHECK(q.stride(2) == 1, "Q: the last dimension must be dense (stride 1)");
+    FA_CHECK(Q.stride(Q.dim() - 1) == 1, "Q: the last dimension must be dense (stride 1)");
     FA_CHECK(K.stride(3) == 1, "K_cache: the last dimension must be dense (stride 1)");
     FA_CHECK(V.stride(3) == 1, "V_cache: the last dimension must be dense (stride 1)");
     at::Tensor O;
     if (given(a[6])) {
-      O = one_row(tensor_arg(a[6], "out"));
-      FA_CHECK(O.sizes() == q.sizes() && O.scalar_type() == torch::kBFloat16 && O.device() == Q.device() && O.stride(2) == 1,
+      O = tensor_arg(a[6], "out");
+      FA_CHECK(O.scalar_type() == torch::kBFloat16 && O.device() == Q.device() && is_row(O, B, H, d),
                "out must match Q in shape, dtype and device");
     } else {
-      O = at::empty({B, H, d}, Q.options());
+      const int64_t sizes[4] = {B, H, 1, d}, flat[3] = {B, H, d};
+      O = squeeze ? empty_cuda(sizes, torch::kBFloat16, Q.device()) : empty_cuda(flat, torch::kBFloat16, Q.device());
     }
     const bool return_lse = flag_arg(a[4], false);
     at::Tensor lse;
-    if (return_lse) lse = at::empty({B, H}, Q.options().dtype(torch::kFloat32));
+    if (return_lse) lse = empty_cuda({B, H}, torch::kFloat32, Q.device());
     p.B = static_cast<int32_t>(B); p.H = static_cast<int32_t>(H);
     p.kv_len = static_cast<int32_t>(kv_len); p.d = static_cast<int32_t>(d);
     if (B * H > 0) {
-      p.q = q.data_ptr(); p.k_cache = K.data_ptr(); p.v_cache = V.data_ptr(); p.o = O.data_ptr();
-      strides2(q, p.q_strides);
+      p.q = Q.data_ptr(); p.k_cache = K.data_ptr(); p.v_cache = V.data_ptr(); p.o = O.data_ptr();
+      strides2(Q, p.q_strides);
       strides2(O, p.o_strides);
       cache_strides(K, p.k_strides);
       cache_strides(V, p.v_strides);
@@ -252,9 +266,9 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* k
     p.softmax_scale = static_cast<float>(number_arg(a[5], 0.0));
     FA_CHECK(given(a[7]) == given(a[8]), "k_new and v_new go together");
     if (given(a[7])) {
-      const at::Tensor kn = one_row(tensor_arg(a[7], "k_new")), vn = one_row(tensor_arg(a[8], "v_new"));
+      const at::Tensor &kn = tensor_arg(a[7], "k_new"), &vn = tensor_arg(a[8], "v_new");
       for (const auto& [t, name] : {std::pair<const at::Tensor&, const char*>{kn, "k_new"}, {vn, "v_new"}})
-        FA_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && t.sizes() == q.sizes() && t.stride(2) == 1,
+        FA_CHECK(t.is_cuda() && t.scalar_type() == torch::kBFloat16 && is_row(t, B, H, d),
                  name, " must be a CUDA bfloat16 tensor [B, H, 64] with a dense last dimension");
       int64_t vs[2];
       strides2(kn, p.new_strides);
@@ -266,8 +280,7 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* k
     p.device = Q.device().index();
     p.stream = c10::cuda::getCurrentCUDAStream(Q.device().index()).stream();
     launch("custom_flash_attn.decode", [&] { return fa_b200_decode_direct(&p); });
-    const at::Tensor result = given(a[6]) ? THPVariable_Unpack(a[6]) : (squeeze ? O.unsqueeze(2) : O);
-    return return_lse ? pair(result, lse) : THPVariable_Wrap(result);
+    return return_lse ? pair(O, lse) : THPVariable_Wrap(O);
   });
 }
 
@@ -300,8 +313,8 @@ PyObject* add_layernorm(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyOb
     FA_CHECK(shift.numel() == cols, "shift must have ", cols, " elements");
     const bool keep = flag_arg(v[5], true) && given(v[1]);
     at::Tensor sum, norm;
-    if (keep) sum = given(v[6]) ? tensor_arg(v[6], "sum_out") : at::empty_like(a);
-    norm = given(v[7]) ? tensor_arg(v[7], "norm_out") : at::empty_like(a);
+    if (keep) sum = given(v[6]) ? tensor_arg(v[6], "sum_out") : empty_like_cuda(a);
+    norm = given(v[7]) ? tensor_arg(v[7], "norm_out") : empty_like_cuda(a);
     p.scale = scale.data_ptr();
     p.shift = shift.data_ptr();
     p.sum_out = keep ? sum.data_ptr() : nullptr;
