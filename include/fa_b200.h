@@ -227,6 +227,22 @@ typedef struct fa_b200_add_layernorm_params {
 
 int fa_b200_add_layernorm(const fa_b200_add_layernorm_params* p);
 
+/* Copies the new keys and values of a prompt into the K/V caches, both in one launch: k, v are bf16
+ * [B, N, H, 64] with element strides {sequence, row, head}, written to rows 0 .. N-1 of k_cache / v_cache
+ * (strides cache_strides in the same order; to start at a later row pass that row's address).  All
+ * strides are positive multiples of 8, all pointers 16-byte aligned.  Asynchronous on p->stream. */
+typedef struct fa_b200_cache_write_params {
+  const void *k, *v;
+  void *k_cache, *v_cache;
+  int64_t strides[3];
+  int64_t cache_strides[3];
+  int32_t B, N, H;
+  int32_t device;
+  void* stream;
+} fa_b200_cache_write_params;
+
+int fa_b200_cache_write(const fa_b200_cache_write_params* p);
+
 /* y = act(x W^T + bias) for at most 8 rows of x (the Linear layers of a generation step):
  * x [M, K], W [N, K] with row stride ldw (elements; the layout of torch.nn.Linear.weight), bias
  * [N] or NULL, y [M, N]; all bf16, fp32 accumulation; act 0 = none, 1 = tanh-GELU.

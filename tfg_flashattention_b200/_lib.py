@@ -62,6 +62,16 @@ class FaLinearSmallParams(ctypes.Structure):
     ]
 
 
+class FaCacheWriteParams(ctypes.Structure):
+    """struct fa_b200_cache_write_params (include/fa_b200.h)."""
+    _fields_ = [
+        ("k", ctypes.c_void_p), ("v", ctypes.c_void_p), ("k_cache", ctypes.c_void_p), ("v_cache", ctypes.c_void_p),
+        ("strides", ctypes.c_int64 * 3), ("cache_strides", ctypes.c_int64 * 3),
+        ("B", ctypes.c_int32), ("N", ctypes.c_int32), ("H", ctypes.c_int32),
+        ("device", ctypes.c_int32), ("stream", ctypes.c_void_p),
+    ]
+
+
 class FaGptStepParams(ctypes.Structure):
     """struct fa_b200_gpt_step_params (include/fa_b200.h)."""
     _fields_ = [
@@ -81,7 +91,7 @@ class FaGptStepParams(ctypes.Structure):
 
 EXPORTS = ("fa_b200_fwd", "fa_b200_fwd_plan", "fa_b200_validate", "fa_b200_strerror", "fa_b200_device_ok",
            "fa_b200_last_status", "fa_b200_abi_version", "fa_b200_decode", "fa_b200_decode_workspace_bytes", "fa_b200_decode_static", "fa_b200_decode_direct",
-           "fa_b200_add_layernorm", "fa_b200_linear_small", "fa_b200_gpt_step", "fa_b200_gpt_step_workspace_bytes")
+           "fa_b200_add_layernorm", "fa_b200_linear_small", "fa_b200_gpt_step", "fa_b200_gpt_step_workspace_bytes", "fa_b200_cache_write")
 
 SCHEDULES = {-1: "none", 0: "cta_per_tile", 1: "persistent_paired", 2: "persistent_rotated",
              3: "persistent_full"}
@@ -128,6 +138,8 @@ def load() -> ctypes.CDLL:
     lib.fa_b200_add_layernorm.restype = ctypes.c_int
     lib.fa_b200_linear_small.argtypes = [ctypes.POINTER(FaLinearSmallParams)]
     lib.fa_b200_linear_small.restype = ctypes.c_int
+    lib.fa_b200_cache_write.argtypes = [ctypes.POINTER(FaCacheWriteParams)]
+    lib.fa_b200_cache_write.restype = ctypes.c_int
     lib.fa_b200_gpt_step.argtypes = [ctypes.POINTER(FaGptStepParams)]
     lib.fa_b200_gpt_step.restype = ctypes.c_int
     lib.fa_b200_gpt_step_workspace_bytes.argtypes = [ctypes.c_int32, ctypes.c_int32]

@@ -19,6 +19,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ptx_sm100.cuh"
+
 namespace fa {
 
 constexpr int kLnWarpsPerCta = 8;
@@ -63,6 +65,8 @@ __global__ void __launch_bounds__(kLnWarpsPerCta * 32) fa_add_layernorm_kernel(c
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * kLnWarpsPerCta + (threadIdx.x >> 5);
   if (row >= p.rows) return;                       // whole warps leave together
+  pdl_trigger();
+  pdl_wait();
   const int nvec = p.cols >> 3;                    // 16-byte vectors per row
   const uint4* a = reinterpret_cast<const uint4*>(p.a + row * p.cols);
   const uint4* rs = p.resid ? reinterpret_cast<const uint4*>(p.resid + row * p.cols) : nullptr;

@@ -12,6 +12,7 @@
 
 #include "../../include/fa_b200.h"
 #include "add_layernorm_sm100.cuh"
+#include "cache_write_sm100.cuh"
 #include "fa_decode_sm100.cuh"
 #include "fa_fwd_sm100.cuh"
 #include "gpt_step_sm100.cuh"
@@ -575,8 +576,8 @@ namespace {
 template <int kVec>
 cudaError_t launch_add_ln(const fa::AddLnParams& kp, cudaStream_t stream) {
   const long long ctas = (kp.rows + fa::kLnWarpsPerCta - 1) / fa::kLnWarpsPerCta;
-  fa::fa_add_layernorm_kernel<kVec><<<static_cast<unsigned>(ctas), fa::kLnWarpsPerCta * 32, 0, stream>>>(kp);
-  return cudaGetLastError();
+  return launch_kernel(&fa::fa_add_layernorm_kernel<kVec>, dim3(static_cast<unsigned>(ctas)), fa::kLnWarpsPerCta * 32, 0,
+                       stream, 1, kp);
 }
 
 }  // namespace
@@ -626,6 +627,38 @@ int fa_b200_add_layernorm(const fa_b200_add_layernorm_params* p) {
     default: e = launch_add_ln<8>(kp, stream); break;
   }
   return static_cast<int>(e);
+}
+
+// ------------------------------------------------------------------------------ cache write
+int fa_b200_cache_write(const fa_b200_cache_write_params* p) {
+  if (p == nullptr || p->k == nullptr || p->v == nullptr || p->k_cache == nullptr || p->v_cache == nullptr)
+    return FA_B200_ERR_NULL;
+  if (p->B < 0 || p->N < 0 || p->H < 0) return FA_B200_ERR_SHAPE;
+  if (!stride_ok(p->strides) || !stride_ok(p->cache_strides)) return FA_B200_ERR_STRIDE;
+  if ((reinterpret_cast<uintptr_t>(p->k) | reinterpret_cast<uintptr_t>(p->v) | reinterpret_cast<uintptr_t>(p->k_cache) |
+       reinterpret_cast<uintptr_t>(p->v_cache)) & 15u)
+    return FA_B200_ERR_ALIGN;
+  if (p->device < 0 || p->device >= kMaxDevices) return FA_B200_ERR_DEVICE;
+  fa::CacheWriteParams kp;
+  kp.total = 8LL * p->B * p->N * p->H;
+  if (kp.total == 0) return FA_B200_OK;
+  const long long ctas = (kp.total + fa::kCacheWriteThreads - 1) / fa::kCacheWriteThreads;
+  if (ctas > 0x7fffffffLL) return FA_B200_ERR_SHAPE;
+  DeviceGuard guard(p->device);
+  if (guard.error) return guard.error;
+  DeviceState* stp = nullptr;
+  const int rc = ready_device(p->device, &stp);
+  if (rc != 0) return rc;
+  kp.k = static_cast<const __nv_bfloat16*>(p->k);
+  kp.v = static_cast<const __nv_bfloat16*>(p->v);
+  kp.k_cache = static_cast<__nv_bfloat16*>(p->k_cache);
+  kp.v_cache = static_cast<__nv_bfloat16*>(p->v_cache);
+  kp.s_b = p->strides[0]; kp.s_n = p->strides[1]; kp.s_h = p->strides[2];
+  kp.c_b = p->cache_strides[0]; kp.c_n = p->cache_strides[1]; kp.c_h = p->cache_strides[2];
+  kp.N = p->N;
+  kp.H = p->H;
+  return static_cast<int>(launch_kernel(&fa::fa_cache_write_kernel, dim3(static_cast<unsigned>(ctas)),
+                                        fa::kCacheWriteThreads, 0, static_cast<cudaStream_t>(p->stream), 1, kp));
 }
 
 // ------------------------------------------------------------------- Linear for a few rows

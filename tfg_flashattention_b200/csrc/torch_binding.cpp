@@ -19,9 +19,12 @@
 // The functions are plain CPython vector calls: for the smallest problems the call IS the time, and
 // pybind11's argument casters cost about as much as the launch (a decode call through ctypes: 31-38
 // us of host time for 4-9 us of GPU work).
+#include <ATen/cuda/CUDAContextLight.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <cublasLt.h>
+#include <dlfcn.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/extension.h>
 
@@ -334,6 +337,233 @@ PyObject* add_layernorm(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyOb
   });
 }
 
+// ---- GEMMs of the block loop: cuBLASLt, which torch's linear calls too, but asked for an algorithm once
+// per shape.  Torch asks on every call: 17 us of host time per GEMM, four per layer, more than the
+// kernels themselves take for a few hundred tokens; with the plan kept it is a launch.
+// The library is the one torch has loaded; where it cannot be found the loop uses at::linear.
+struct LtApi {
+  decltype(&cublasLtMatmulDescCreate) desc_create = nullptr;
+  decltype(&cublasLtMatmulDescDestroy) desc_destroy = nullptr;
+  decltype(&cublasLtMatmulDescSetAttribute) desc_set = nullptr;
+  decltype(&cublasLtMatrixLayoutCreate) layout_create = nullptr;
+  decltype(&cublasLtMatrixLayoutDestroy) layout_destroy = nullptr;
+  decltype(&cublasLtMatmulPreferenceCreate) pref_create = nullptr;
+  decltype(&cublasLtMatmulPreferenceSetAttribute) pref_set = nullptr;
+  decltype(&cublasLtMatmulPreferenceDestroy) pref_destroy = nullptr;
+  decltype(&cublasLtMatmulAlgoGetHeuristic) heuristic = nullptr;
+  decltype(&cublasLtMatmul) matmul = nullptr;
+  bool ok = false;
+  LtApi() {
+    void* lib = dlopen("libcublasLt.so.12", RTLD_NOW | RTLD_NOLOAD);
+    if (lib == nullptr) return;
+    auto get = [&](auto& fn, const char* name) { fn = reinterpret_cast<std::decay_t<decltype(fn)>>(dlsym(lib, name)); return fn != nullptr; };
+    ok = get(desc_create, "cublasLtMatmulDescCreate") && get(desc_destroy, "cublasLtMatmulDescDestroy") &&
+         get(desc_set, "cublasLtMatmulDescSetAttribute") && get(layout_destroy, "cublasLtMatrixLayoutDestroy") &&
+         get(layout_create, "cublasLtMatrixLayoutCreate") && get(pref_create, "cublasLtMatmulPreferenceCreate") &&
+         get(pref_set, "cublasLtMatmulPreferenceSetAttribute") && get(pref_destroy, "cublasLtMatmulPreferenceDestroy") &&
+         get(heuristic, "cublasLtMatmulAlgoGetHeuristic") && get(matmul, "cublasLtMatmul");
+  }
+};
+const LtApi& lt() {
+  static const LtApi api;
+  return api;
+}
+constexpr size_t kLtWorkspace = 32u << 20;       // (0, 1, 4 and 8 MB: within 2 % at 8 to 1200 rows)
+struct LtKey {
+  int device;
+  int64_t m, n, k;
+  int epilogue;
+  bool operator==(const LtKey& o) const { return device == o.device && m == o.m && n == o.n && k == o.k && epilogue == o.epilogue; }
+};
+struct LtPlan {
+  LtKey key;
+  bool usable = false;
+  cublasLtMatmulDesc_t desc = nullptr;
+  cublasLtMatrixLayout_t w = nullptr, x = nullptr, y = nullptr;
+  cublasLtMatmulAlgo_t algo;
+  void clear() {
+    for (cublasLtMatrixLayout_t* l : {&w, &x, &y})
+      if (*l != nullptr) { lt().layout_destroy(*l); *l = nullptr; }
+    if (desc != nullptr) { lt().desc_destroy(desc); desc = nullptr; }
+  }
+  ~LtPlan() { clear(); }
+};
+// y [m, n] = x [m, k] w [n, k]^T + bias, tanh-GELU with `gelu`.  Plans are per host thread (a descriptor
+// is written on every call: the bias address), the last 64 of them.
+bool lt_linear(const at::Tensor& x, const at::Tensor& w, const at::Tensor* bias, bool gelu, at::Tensor& y, void* workspace,
+               void* stream) {
+  const LtApi& api = lt();
+  if (!api.ok || !w.is_contiguous() || !x.is_contiguous() || (gelu && bias == nullptr)) return false;
+  if ((reinterpret_cast<uintptr_t>(w.data_ptr()) | reinterpret_cast<uintptr_t>(x.data_ptr()) |
+       (bias ? reinterpret_cast<uintptr_t>(bias->data_ptr()) : 0)) & 15u)
+    return false;
+  constexpr int kPlans = 64;
+  static thread_local LtPlan plans[kPlans];
+  static thread_local int next = 0;
+  const int64_t k = w.size(1), n = w.size(0), m = x.numel() / k;
+  const int epilogue = gelu ? CUBLASLT_EPILOGUE_GELU_BIAS : (bias ? CUBLASLT_EPILOGUE_BIAS : CUBLASLT_EPILOGUE_DEFAULT);
+  const LtKey key{x.device().index(), m, n, k, epilogue};
+  LtPlan* plan = nullptr;
+  for (LtPlan& p : plans)
+    if (p.desc != nullptr && p.key == key) { plan = &p; break; }
+  const cublasLtHandle_t handle = at::cuda::getCurrentCUDABlasLtHandle();
+  if (plan == nullptr) {
+    plan = &plans[next];
+    next = (next + 1) % kPlans;
+    plan->clear();
+    plan->key = key;
+    plan->usable = false;
+    // (row-major operands are column-major transposes: y^T [n, m] = w [n, k] x^T [k, m])
+    auto ok = [](cublasStatus_t s) { return s == CUBLAS_STATUS_SUCCESS; };
+    const cublasOperation_t trans = CUBLAS_OP_T;
+    const cublasLtEpilogue_t ep = static_cast<cublasLtEpilogue_t>(epilogue);
+    const cudaDataType_t type = CUDA_R_16BF;
+    cublasLtMatmulPreference_t pref = nullptr;
+    cublasLtMatmulHeuristicResult_t found[1];
+    int count = 0;
+    const uint64_t limit = kLtWorkspace;
+    const void* any = reinterpret_cast<const void*>(256);
+    plan->usable = ok(api.desc_create(&plan->desc, CUBLAS_COMPUTE_32F, CUDA_R_32F)) &&
+                   ok(api.desc_set(plan->desc, CUBLASLT_MATMUL_DESC_TRANSA, &trans, sizeof(trans))) &&
+                   ok(api.desc_set(plan->desc, CUBLASLT_MATMUL_DESC_EPILOGUE, &ep, sizeof(ep))) &&
+                   (bias == nullptr || (ok(api.desc_set(plan->desc, CUBLASLT_MATMUL_DESC_BIAS_DATA_TYPE, &type, sizeof(type))) &&
+                                        ok(api.desc_set(plan->desc, CUBLASLT_MATMUL_DESC_BIAS_POINTER, &any, sizeof(any))))) &&
+                   ok(api.layout_create(&plan->w, type, k, n, k)) && ok(api.layout_create(&plan->x, type, k, m, k)) &&
+                   ok(api.layout_create(&plan->y, type, n, m, n)) && ok(api.pref_create(&pref)) &&
+                   ok(api.pref_set(pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &limit, sizeof(limit))) &&
+                   ok(api.heuristic(handle, plan->desc, plan->w, plan->x, plan->y, plan->y, pref, 1, found, &count)) && count > 0;
+    if (pref != nullptr) api.pref_destroy(pref);
+    if (plan->usable) plan->algo = found[0].algo;
+  }
+  if (!plan->usable) return false;
+  if (bias != nullptr) {
+    const void* at = bias->data_ptr();
+    if (api.desc_set(plan->desc, CUBLASLT_MATMUL_DESC_BIAS_POINTER, &at, sizeof(at)) != CUBLAS_STATUS_SUCCESS) return false;
+  }
+  const float one = 1.f, zero = 0.f;
+  return api.matmul(handle, plan->desc, &one, w.data_ptr(), plan->w, x.data_ptr(), plan->x, &zero, y.data_ptr(), plan->y,
+                    y.data_ptr(), plan->y, &plan->algo, workspace, kLtWorkspace, static_cast<cudaStream_t>(stream)) ==
+         CUBLAS_STATUS_SUCCESS;
+}
+
+// The block stack of a prompt, one native loop instead of a dozen Python calls per layer (those cost
+// more than their kernels for a few hundred tokens: GPT-2 small, 72 tokens: 0.9 ms of host time for
+// 0.57 ms of kernels).  The same operations in the same order as GPTModel._blocks_fused.
+void add_ln(const at::Tensor& a, const at::Tensor* resid, const at::Tensor& g, const at::Tensor& b, double eps,
+            void* sum_out, at::Tensor& norm, void* stream) {
+  fa_b200_add_layernorm_params p{};
+  const int64_t cols = a.size(-1);
+  p.a = a.data_ptr();
+  p.resid = resid ? resid->data_ptr() : nullptr;
+  p.scale = g.data_ptr();
+  p.shift = b.data_ptr();
+  p.sum_out = sum_out;
+  p.norm_out = norm.data_ptr();
+  p.rows = a.numel() / cols;
+  p.cols = static_cast<int32_t>(cols);
+  p.eps = static_cast<float>(eps);
+  p.device = a.device().index();
+  p.stream = stream;
+  const int rc = fa_b200_add_layernorm(&p);
+  FA_CHECK(rc == 0, fa_b200_strerror(rc));
+}
+
+// blocks(x, layers, caches, heads, eps, lnf_scale, lnf_shift, last_token_only): x [B, n, C] is the
+// residual stream (overwritten); layers a list of tuples (ln1 scale, shift, qkv weight, bias or None, proj
+// weight, bias, ln2 scale, shift, fc weight, bias, out weight, bias); caches a list of (K, V) pairs
+// [B, N_max, H, 64] whose rows 0 .. n-1 are written, or None.  Returns the final LayerNorm's output.
+PyObject* blocks(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+  return guarded([&]() -> PyObject* {
+    static const char* const names[] = {"x", "layers", "caches", "heads", "eps", "lnf_scale", "lnf_shift", "last_token_only"};
+    PyObject* a[8];
+    take_args("blocks", names, 8, args, nargs, kwnames, a);
+    at::Tensor x = tensor_arg(a[0], "x");
+    FA_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.dim() == 3 && x.is_contiguous(), "x must be a contiguous bfloat16 CUDA tensor [B, n, C]");
+    FA_CHECK(PyList_Check(a[1]) && (a[2] == Py_None || PyList_Check(a[2])), "layers and caches are lists");
+    const int64_t B = x.size(0), n = x.size(1), C = x.size(2), H = PyLong_AsLongLong(a[3]);
+    FA_CHECK(H > 0 && C == 64 * H, "the width must be 64 * heads");
+    const double eps = number_arg(a[4], 1e-5);
+    const at::Tensor lnf_g = tensor_arg(a[5], "lnf_scale"), lnf_b = tensor_arg(a[6], "lnf_shift");
+    const bool last_only = flag_arg(a[7], false), cached = a[2] != Py_None;
+    struct Layer { at::Tensor t[12], k, v; };
+    std::vector<Layer> layers(static_cast<size_t>(PyList_GET_SIZE(a[1])));
+    FA_CHECK(!cached || PyList_GET_SIZE(a[2]) == static_cast<Py_ssize_t>(layers.size()), "one cache per layer");
+    for (size_t l = 0; l < layers.size(); ++l) {
+      PyObject* t = PyList_GET_ITEM(a[1], l);
+      FA_CHECK(PyTuple_Check(t) && PyTuple_GET_SIZE(t) == 12, "a layer has twelve tensors");
+      for (int i = 0; i < 12; ++i)
+        if (PyTuple_GET_ITEM(t, i) != Py_None) layers[l].t[i] = tensor_arg(PyTuple_GET_ITEM(t, i), "a layer's parameter");
+      if (cached) {
+        PyObject* kv = PyList_GET_ITEM(a[2], l);
+        FA_CHECK(PyTuple_Check(kv) && PyTuple_GET_SIZE(kv) == 2, "a cache is a pair");
+        for (int i = 0; i < 2; ++i) {
+          const at::Tensor& c = tensor_arg(PyTuple_GET_ITEM(kv, i), "a cache");
+          FA_CHECK(c.is_cuda() && c.scalar_type() == torch::kBFloat16 && c.dim() == 4 && c.size(0) == B && c.size(1) >= n &&
+                       c.size(2) == H && c.size(3) == 64 && c.stride(3) == 1 &&
+                       (i == 0 || c.strides() == layers[l].k.strides()),
+                   "the caches must be bfloat16 [B, >= n, H, 64] with the same strides");
+          (i ? layers[l].v : layers[l].k) = c;
+        }
+      }
+    }
+    at::Tensor result;
+    {
+      py::gil_scoped_release release;
+      const at::AutoDispatchBelowADInplaceOrView below_autograd;
+      const c10::cuda::CUDAGuard guard(x.device());
+      void* stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+      at::Tensor branch, h = empty_like_cuda(x);
+      const at::Tensor workspace = empty_cuda({static_cast<int64_t>(kLtWorkspace)}, torch::kUInt8, x.device());
+      auto linear = [&](const at::Tensor& in, const at::Tensor& w, const at::Tensor& bias) {
+        at::Tensor y = empty_cuda({B, n, w.size(0)}, torch::kBFloat16, x.device());
+        if (lt_linear(in, w, bias.defined() ? &bias : nullptr, false, y, workspace.data_ptr(), stream)) return y;
+        return at::linear(in, w, bias.defined() ? std::optional<at::Tensor>(bias) : std::nullopt);
+      };
+      for (const Layer& L : layers) {
+        if (branch.defined()) add_ln(branch, &x, L.t[0], L.t[1], eps, x.data_ptr(), h, stream);
+        else add_ln(x, nullptr, L.t[0], L.t[1], eps, nullptr, h, stream);
+        const at::Tensor qkv = linear(h, L.t[2], L.t[3]);
+        const at::Tensor ctx = empty_like_cuda(x);
+        auto* base = static_cast<at::BFloat16*>(qkv.data_ptr());
+        fa_b200_params p{};
+        p.B = static_cast<int32_t>(B); p.H = static_cast<int32_t>(H); p.N = static_cast<int32_t>(n); p.d = 64;
+        p.q = base; p.k = base + C; p.v = base + 2 * C; p.o = ctx.data_ptr();
+        for (int64_t* s : {p.q_strides, p.k_strides, p.v_strides}) { s[0] = 3 * C * n; s[1] = 64; s[2] = 3 * C; }
+        p.o_strides[0] = C * n; p.o_strides[1] = 64; p.o_strides[2] = C;
+        p.causal = 1;
+        p.device = x.device().index();
+        p.stream = stream;
+        int rc = 0;
+        if (cached) {
+          fa_b200_cache_write_params c{};
+          c.k = p.k; c.v = p.v; c.k_cache = L.k.data_ptr(); c.v_cache = L.v.data_ptr();
+          c.strides[0] = 3 * C * n; c.strides[1] = 3 * C; c.strides[2] = 64;
+          for (int i = 0; i < 3; ++i) c.cache_strides[i] = L.k.size(i) == 1 ? 64 : L.k.stride(i);   // (size 1: never used)
+          c.B = p.B; c.N = p.N; c.H = p.H; c.device = p.device; c.stream = stream;
+          rc = fa_b200_cache_write(&c);
+          FA_CHECK(rc == 0, "cache write failed (", rc, "): ", fa_b200_strerror(rc));
+        }
+        rc = fa_b200_fwd(&p);
+        FA_CHECK(rc == 0, "custom_flash_attn.forward failed (", rc, "): ", fa_b200_strerror(rc));
+        branch = linear(ctx, L.t[4], L.t[5]);
+        add_ln(branch, &x, L.t[6], L.t[7], eps, x.data_ptr(), h, stream);
+        at::Tensor mid = empty_cuda({B, n, L.t[8].size(0)}, torch::kBFloat16, x.device());
+        if (!lt_linear(h, L.t[8], &L.t[9], true, mid, workspace.data_ptr(), stream))
+          mid = at::_addmm_activation(L.t[9], h.view({B * n, C}), L.t[8].t(), 1, 1, /*use_gelu=*/true).view({B, n, L.t[8].size(0)});
+        branch = linear(mid, L.t[10], L.t[11]);
+      }
+      if (last_only) {                 // what generate() consumes
+        x = x.slice(1, n - 1, n).contiguous();
+        if (branch.defined()) branch = branch.slice(1, n - 1, n).contiguous();
+      }
+      result = empty_like_cuda(x);
+      if (branch.defined()) add_ln(branch, &x, lnf_g, lnf_b, eps, nullptr, result, stream);
+      else add_ln(x, nullptr, lnf_g, lnf_b, eps, nullptr, result, stream);
+    }
+    return THPVariable_Wrap(result);
+  });
+}
+
 PyMethodDef methods[] = {
     {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&forward)), METH_FASTCALL | METH_KEYWORDS,
      "FlashAttention forward on B200 (libfa_b200.so)"},
@@ -341,6 +571,8 @@ PyMethodDef methods[] = {
      "Single-query attention against a K/V cache"},
     {"add_layernorm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&add_layernorm)),
      METH_FASTCALL | METH_KEYWORDS, "Shortcut addition and LayerNorm in one pass"},
+    {"blocks", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&blocks)), METH_FASTCALL | METH_KEYWORDS,
+     "The transformer blocks of a prompt"},
     {nullptr, nullptr, 0, nullptr}};
 
 }  // namespace

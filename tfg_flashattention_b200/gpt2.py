@@ -287,6 +287,7 @@ class GPTModel(nn.Module):
         self._head_w = None     # out_head weight padded to a multiple of 64 rows (inference cache)
         self._fused_blocks = False   # residual add + LayerNorm through block_ops.add_layernorm
         self._step_plan = None       # single-token steps as one kernel launch (step.StepPlan)
+        self._block_params, self._block_owned = None, []    # for the binding's loop over the blocks
         if dtype is not None:
             self.to(dtype)
 
@@ -307,6 +308,9 @@ class GPTModel(nn.Module):
         for blk in self.trf_blocks:      # single-token steps: Linear layers as one pass over the weights
             blk.att.small_linear = blk.ff.small_linear = self._fused_blocks
         self._step_plan = StepPlan.make(self) if self._fused_blocks else None
+        self._block_params, self._block_owned = None, []
+        if self._fused_blocks:
+            self._list_block_params()
         return self
 
     def invalidate_inference_cache(self):
@@ -317,10 +321,12 @@ class GPTModel(nn.Module):
         self._head_w = None
         self._fused_blocks = False
         self._step_plan = None
+        self._block_params, self._block_owned = None, []
         return self
 
     def _apply(self, fn, *args, **kwargs):      # .to(), .cuda(), .half(): the parameters move
         self._step_plan = None
+        self._block_params, self._block_owned = None, []
         return super()._apply(fn, *args, **kwargs)
 
     def _step(self, in_idx, kv_caches, pos, **kw):
@@ -344,9 +350,64 @@ class GPTModel(nn.Module):
         n_max = self.cfg["context_length"] if max_len is None else max_len
         if dtype is None:
             dtype = torch.bfloat16 if self.cfg["impl_type"] == "cuda" else self.tok_emb.weight.dtype
-        return [(torch.zeros(batch, n_max, h, d, dtype=dtype, device=dev),
-                 torch.zeros(batch, n_max, h, d, dtype=dtype, device=dev))
-                for _ in range(self.cfg["n_layers"])]
+        layers = self.cfg["n_layers"]       # one allocation and one fill instead of two per layer
+        kv = torch.zeros(2 * layers, batch, n_max, h, d, dtype=dtype, device=dev).unbind(0)
+        return list(zip(kv[::2], kv[1::2]))
+
+    def _native_blocks(self, x, kv_caches, pos):
+        """The binding's loop over the blocks when this call is one for it (a prompt or whole sequences,
+        no gradients, no hooks, every parameter the bf16 one it expects), else None."""
+        from . import custom_flash_attn
+        ext = custom_flash_attn.extension()
+        if (ext is None or torch.is_grad_enabled() or torch.is_autocast_enabled() or not isinstance(pos, int) or pos != 0
+                or (kv_caches is not None and x.shape[1] == 1) or x.numel() == 0):
+            return None
+        width, heads = self.cfg["emb_dim"], self.cfg["n_heads"]
+        if width != 64 * heads:
+            return None
+        for params, name, t in self._block_owned:
+            if params[name] is not t:                       # replaced since the list was made
+                self._list_block_params()
+                break
+        if self._block_params is None:
+            return None
+        for blk, row in zip(self.trf_blocks, self._block_params):
+            att, ff = blk.att, blk.ff
+            if (att._forward_hooks or att._forward_pre_hooks or ff._forward_hooks or ff._forward_pre_hooks
+                    or att.impl_type != "cuda" or att._qkv_w is not row[2]):
+                return None
+        if kv_caches is not None:
+            if not isinstance(kv_caches, list) or len(kv_caches) != len(self._block_params):
+                return None
+            for pair in kv_caches:
+                k, v = pair
+                if (type(pair) is not tuple or k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16
+                        or k.shape != v.shape or k.stride() != v.stride() or not k.is_cuda):
+                    return None
+        return ext.blocks
+
+    def _list_block_params(self):
+        """The blocks' parameters in the order the native loop takes them, and where they came from."""
+        self._block_owned, self._block_params = [], []
+        for blk in self.trf_blocks:
+            row = []
+            for module, name in ((blk.norm1, "scale"), (blk.norm1, "shift"), (None, None), (None, None),
+                                 (blk.att.out_proj, "weight"), (blk.att.out_proj, "bias"),
+                                 (blk.norm2, "scale"), (blk.norm2, "shift"),
+                                 (blk.ff.layers[0], "weight"), (blk.ff.layers[0], "bias"),
+                                 (blk.ff.layers[2], "weight"), (blk.ff.layers[2], "bias")):
+                if module is None:
+                    row.append((blk.att._qkv_w, blk.att._qkv_b)[len(row) - 2])
+                    continue
+                t = module._parameters[name]
+                self._block_owned.append((module._parameters, name, t))
+                row.append(t)
+            if (any(t is None or t.dtype != torch.bfloat16 or not t.is_cuda for i, t in enumerate(row) if i != 3)
+                    or any(not row[i].is_contiguous() for i in (0, 1, 6, 7))
+                    or any(m.eps != self.final_norm.eps for m in (blk.norm1, blk.norm2))):
+                self._block_params = None
+                return
+            self._block_params.append(tuple(row))
 
     def _blocks_fused(self, x, kv_caches, pos, last_token_only):
         """The block stack and the final norm with every shortcut addition folded into the
@@ -354,6 +415,10 @@ class GPTModel(nn.Module):
         norm1(x)), then x + ff(norm2(x))).  `x` is the residual stream, updated in place; `branch`
         is the output of the previous sub-layer that has not been added to it yet."""
         from .block_ops import add_layernorm
+        native = self._native_blocks(x, kv_caches, pos)
+        if native is not None:
+            return native(x, self._block_params, kv_caches, self.cfg["n_heads"], self.final_norm.eps,
+                          self.final_norm.scale, self.final_norm.shift, last_token_only)
         branch = None
         for i, blk in enumerate(self.trf_blocks):
             cache = None if kv_caches is None else kv_caches[i]

@@ -32,12 +32,12 @@ class StepPlan:
         if width != 64 * heads or width > MAX_WIDTH or not 1 <= layers <= MAX_LAYERS or heads > MAX_PAIRS:
             return None
         plan = cls()
-        owned = []           # (module's parameter dict, name, tensor): what the table was built from
+        owned = []           # (module's parameter dict, name, tensor, address): what the table was built from
         rows = []
 
         def take(module, name, shape, optional=False):
             t = module._parameters[name]
-            owned.append((module._parameters, name, t))
+            owned.append((module._parameters, name, t, 0 if t is None else t.data_ptr()))
             if t is None:
                 if not optional:
                     raise TypeError(name)
@@ -82,9 +82,9 @@ class StepPlan:
         return t.data_ptr()
 
     def current(self):
-        """False when a parameter object has been replaced since the table was built."""
-        for params, name, t in self.owned:
-            if params[name] is not t:
+        """False when a parameter, or its storage, has been replaced since the table was built."""
+        for params, name, t, address in self.owned:
+            if params[name] is not t or (t is not None and t.data_ptr() != address):
                 return False
         for att, w in self.qkv:
             if att._qkv_w is not w:
