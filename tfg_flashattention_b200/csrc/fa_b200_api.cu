@@ -862,6 +862,12 @@ int fa_b200_gpt_step(const fa_b200_gpt_step_params* p) {
   kp.advance = p->advance;
   kp.n_layers = p->n_layers;
   kp.C = 64 * p->H; kp.H = p->H; kp.V = p->vocab; kp.M = p->B;
+  const int columns = kp.C / fa::kStepUnit;                      // units; even
+  kp.lg_chunks = columns > fa::kStepChunkUnits ? 1 : 0;
+  kp.stage_units = columns >> kp.lg_chunks;
+  kp.stage_pitch = fa::step_pitch(kp.stage_units);
+  kp.batch_units = 4 * fa::kStepTake / kp.M;
+  kp.inv_c = 1.0f / static_cast<float>(kp.C);
   kp.cache_rows = p->cache_rows;
   kp.n_positions = p->n_positions;
   kp.eps = p->eps;

@@ -22,13 +22,24 @@
 //                written again only by CTAs that hold something which depends on everybody's having
 //                read it (its reader's own output, a few operations on).
 //   work split   Output columns of a layer (rows of W) are cut evenly over the CTAs, so a CTA's
-//                share is one contiguous piece of W.  It is taken in tiles of at most 16 rows, K in
-//                passes of d_model columns and chunks of at most 800, one (tile, chunk) per stage.
+//                share is one contiguous piece of W.  It is taken in tiles of at most 12 rows, K in
+//                pieces of d_model columns or half of that where they are more than 800: a ring stage.
+//   ahead        Before an operation's weights go into the ring, the next one's are sent for as far as
+//                L2: the ring is too short (154 KB of the 415 KB a CTA reads per XL layer) to keep the
+//                memory busy while the operations wait for one another.  One operation ahead: XL 785
+//                us per step against 832 without and 790 with two (before the ring and the split were
+//                as they are now: 985, 1085, 1014, and 1152 and 1255 with three and four); with the
+//                cached rows sent for in the same way it was slower, 2030 against 1860 at 8 sequences.
 //   tensor path  mma.sync m16n8k16 with W as the 16-row operand and the (up to 8) tokens as the
 //                8-column operand: at 8 tokens a scalar product per weight costs more issue slots
 //                than the stream leaves.  tcgen05 needs 64 or 128 rows of one operand per CTA and
-//                gives nothing here, the memory pipe is the limit.  The 16 warps split K: warp w
-//                owns the 32-column units w, w + 16, ...; partial tiles meet in shared memory.
+//                gives nothing here, the memory pipe is the limit.  The 8 warps split K: a warp has the
+//                same part of every row, which lies in one ring stage, so it waits for one barrier
+//                per tile, holds its input in registers over all tiles, and the partial tiles meet in
+//                shared memory.  Per step of GPT-2 small / XL, 1 sequence, 100 rows, us: 242 / 1138
+//                with 16 warps that all go over all stages, 228 / 1083 with 8, 178 / 1078 with a
+//                warp to a whole stage (shared memory is the limit for XL: the input is read again
+//                for every tile), 153 / 770 like this.
 //   attention    a (sequence, head) pair per CTA, up to two where there are more pairs than CTAs,
 //                split over several CTAs only for caches of thousands of rows.  q.K on the tensor
 //                path with the cached rows as the 16-row operand, P.V on packed fp32.  The cached
@@ -57,37 +68,49 @@
 
 namespace fa {
 
-constexpr int kStepWarps = 16;                        // computing warps
+constexpr int kStepWarps = 8;                         // computing warps
+constexpr int kStepLgWarps = 3;
+static_assert(kStepWarps == 1 << kStepLgWarps, "warps are divided by shifts");
 constexpr int kStepCompute = kStepWarps * 32;
 constexpr int kStepStreamWarps = 4;
 constexpr int kStepThreads = kStepCompute + 32 * kStepStreamWarps;
 // Registers: the computing warpgroups take what the streaming one gives up.  (setmaxnreg.inc waits
 // without a limit for registers of this CTA's launch allocation, hence the check; the host refuses a
 // build whose launch allocation is another.)
-constexpr int kStepLaunchRegs = 96, kStepComputeRegs = 112, kStepStreamRegs = 32;
+constexpr int kStepLaunchRegs = 168, kStepComputeRegs = 216, kStepStreamRegs = 40;
 static_assert(kStepCompute * kStepComputeRegs + 32 * kStepStreamWarps * kStepStreamRegs <= kStepThreads * kStepLaunchRegs,
               "setmaxnreg budget exceeds the launch allocation: the kernel would hang");
 constexpr int kStepMaxRows = 8;                       // sequences (the 8-column side of the MMA)
 constexpr int kStepMaxLayers = 64;
 constexpr int kStepMaxPairs = 256;                    // (sequence, head) pairs
-constexpr int kStepTile = 16;                         // rows of W per stage
-constexpr int kStepGroup = 4;                         // tiles reduced together: one output per thread
-constexpr int kStepOutputs = kStepTile * kStepMaxRows;
-static_assert(kStepGroup * kStepOutputs == kStepCompute, "one output per thread");
+constexpr int kStepTile = 12;                         // rows of W per stage (of the MMA's 16)
+constexpr int kStepMmaRows = 16;
+constexpr int kStepGroup = 4;                         // tiles whose partial sums are added up together
+constexpr int kStepRedPitch = 20;                     // partial tiles: [token][row], conflict-free for the MMA's layout
+constexpr int kStepRed = kStepRedPitch * kStepMaxRows;
+constexpr int kStepOutputs = kStepMmaRows * kStepMaxRows;
 constexpr int kStepUnit = 32;                         // columns of W per warp step: 64 bytes
 constexpr int kStepChunkUnits = 25;                   // columns per stage: at most 800
 constexpr int kStepStageBytes = kStepTile * kStepChunkUnits * 64;
-constexpr int kStepStages = 6;
+constexpr int kStepStages = 8;                        // one per warp: a group of tiles has at most as many
+static_assert(kStepStages >= kStepWarps, "a wait by parity is for the slot's next stage only while the one before is not given back");
+constexpr int kStepAhead = 1;
+constexpr bool kStepAheadKv = false;
+constexpr uint32_t kStepAheadBytes = 192 * 1024, kStepAheadPiece = 2048;
 constexpr int kStepMaxWidth = 1600;                   // d_model: the fragments of 8 rows fill sm.x
 constexpr int kStepMaxUnits = kStepMaxWidth / kStepUnit;
-constexpr int kStepUnits = (kStepMaxUnits + kStepWarps - 1) / kStepWarps;     // 4 per warp and pass
-constexpr int kStepQuads = (kStepMaxWidth / 4 + 63) / 64;                      // 7: columns / 4 of a row per lane of two warps
+constexpr int kStepQuads = (kStepMaxWidth / 4 + 31) / 32;     // 13: columns / 4 of a row per lane of a warp
+constexpr int kStepTake = 8;                          // words of a batch: 32 lanes x kStepTake x 4
 constexpr int kStepSegs = 2;                          // attention units of one CTA
-constexpr int kStepBlocks = 6;                        // blocks of 16 cached rows (K, then V) per stage
+constexpr int kStepBlocks = 4;                        // blocks of 16 cached rows (K, then V) per stage
 static_assert(kStepBlocks * 16 * 256 <= kStepStageBytes, "cached rows fit a stage");
 constexpr int kStepSplitRows = 1024;                  // rows of a unit where pairs are split over CTAs
 constexpr uint32_t kStepBarPolls = 1u << 24;          // bounds of the waits: about 65 clocks a poll of a barrier ...
 constexpr uint32_t kStepWordPolls = 1u << 21;         // ... and a trip to L2 a poll of exchange words: half a second
+
+// Rows of a stage lie 64 bytes (mod 128) apart: the 8 lanes of a 128-bit load phase read two rows of
+// 64 bytes each, which then cover all banks (an even `units` is at most 24).
+constexpr int step_pitch(int units) { return units * 64 + ((units & 1) ? 0 : 64); }
 
 struct StepLayer {       // one transformer block's parameters (device memory, built once per model)
   const __nv_bfloat16 *ln1_g, *ln1_b, *qkv_w, *qkv_b, *proj_w, *proj_b;
@@ -103,6 +126,10 @@ struct StepParams {
   int* len_ptr;                    // with pos_ptr and advance: set to the new length + 1
   int pos, advance;
   int n_layers, C, H, V, M;
+  int stage_units, lg_chunks;      // units of 32 columns per ring stage, stages per d_model columns: 1 or 2
+  int stage_pitch;                 // bytes between a stage's rows, see step_pitch
+  int batch_units;                 // units whose exchange words a warp takes at once
+  float inv_c;                     // 1 / C
   int cache_rows, n_positions;
   float eps, scale_log2;
   long long c_sb;                  // cache strides in elements: sequence, row, head
@@ -127,29 +154,34 @@ struct StepParams {
   __nv_bfloat16* v_cache[kStepMaxLayers];
 };
 
-// How a [N, K] weight is cut: rows of this CTA, tiles of `tile` rows.
-struct StepCut {
-  int row0, rows, tiles, tile;
+// How a [N, K] weight is cut: rows of this CTA, tiles of `tile` rows, taken in groups of 1 << lg_group.
+struct __align__(16) StepCut {
+  int row0, rows;
+  short tiles, tile;
+  int lg_group;
 };
-__device__ __forceinline__ StepCut step_cut(int N) {          // N < 2^24, grid <= 160
+__device__ __forceinline__ StepCut step_cut(int N, bool head) {          // N < 2^24, grid <= 160
   StepCut c;
   c.row0 = static_cast<int>(blockIdx.x * static_cast<uint32_t>(N) / gridDim.x);
   c.rows = static_cast<int>((blockIdx.x + 1) * static_cast<uint32_t>(N) / gridDim.x) - c.row0;
-  c.tiles = (c.rows + kStepTile - 1) / kStepTile;
-  c.tile = c.tiles > 0 ? (c.rows + c.tiles - 1) / c.tiles : 0;
+  const int tiles = (c.rows + kStepTile - 1) / kStepTile;
+  c.tiles = static_cast<short>(tiles);
+  c.tile = static_cast<short>(tiles > 0 ? (c.rows + tiles - 1) / tiles : 0);
+  c.lg_group = 0;
+  while ((1 << c.lg_group) < (head ? kStepGroup : min(tiles, kStepGroup))) ++c.lg_group;
   return c;
 }
-// A pass over d_model columns: `chunks` stages of `units` units (the last may have fewer).
-struct StepPass {
-  int total, units, chunks;
-  uint32_t pitch;
-  __device__ __forceinline__ explicit StepPass(int C) {
-    total = C / kStepUnit;
-    chunks = (total + kStepChunkUnits - 1) / kStepChunkUnits;
-    units = (total + chunks - 1) / chunks;
-    // rows of a stage lie 64 bytes (mod 128) apart: the 8 lanes of a 128-bit load phase read two
-    // rows of 64 bytes each, which then cover all banks (an even `units` is at most 24)
-    pitch = units * 64 + ((units & 1) ? 0 : 64);
+// Which columns of a row are a warp's: `units` units from unit `first`, in ring stage `stage` of the
+// 1 << lg_stages that hold a tile, from unit `at` of that stage.
+struct StepPart {
+  int stage, lg_stages, first, units, at;
+  __device__ __forceinline__ StepPart(int warp, int lg, int stage_units) {
+    lg_stages = lg;
+    stage = warp >> (kStepLgWarps - lg);
+    const int parts = kStepWarps >> lg, per = (stage_units + parts - 1) / parts;
+    at = (warp & (parts - 1)) * per;
+    units = max(min(per, stage_units - at), 0);
+    first = stage * stage_units + at;
   }
 };
 
@@ -184,15 +216,14 @@ struct StepUnit {
 struct __align__(128) StepSmem {
   uint8_t ring[kStepStages][kStepStageBytes];
   uint4 x[kStepMaxUnits * 32];                              // LayerNorm's output as MMA fragments
-  union {
-    float red[kStepGroup][kStepWarps][kStepOutputs];        // partial tiles of the warps
-    float seg[kStepSegs][kStepWarps + 1][68];               // attention partials: m, l, -, -, o[64]
-  };
+  float red[kStepGroup][kStepWarps][kStepRed];              // partial tiles of the warps
+  float red_one[kStepWarps][kStepRed];                      // ... where the input comes through the exchange
+  float seg[kStepSegs][kStepWarps + 1][68];                 // attention partials: m, l, -, -, o[64]
   uint2 norm[2][kStepMaxWidth / 4];                         // scale and shift of the coming LayerNorm
   alignas(16) float2 stat[kStepWarps];                      // LayerNorm: sums of a warp's part
   float shift[kStepMaxRows];                                // ... and the row's mean in the one before
   float own[kStepOutputs];                                  // this CTA's columns of the residual stream
-  unsigned long long keys[kStepWarps][kStepMaxRows];        // best logit of a warp
+  unsigned long long keys[kStepMaxRows][2];                 // best logits: a token's of two warps
   StepUnit unit[kStepSegs];                                 // this CTA's attention units
   int units, splits;
   StepCut cut[5];                                           // by StepOp
@@ -237,6 +268,10 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                :: "r"(dst), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar) : "memory");
 }
+// (16-byte aligned, a multiple of 16 bytes)
+__device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<uint64_t>(src)), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<uint64_t>(p)));
 }
@@ -245,6 +280,10 @@ struct StepRing {
   uint32_t stage = 0, parity = 0;
   __device__ __forceinline__ void next() {
     if (++stage == kStepStages) { stage = 0; parity ^= 1; }
+  }
+  __device__ __forceinline__ void skip(uint32_t n) {      // n <= kStepWarps
+    stage += n;
+    if (stage >= kStepStages) { stage -= kStepStages; parity ^= 1; }
   }
 };
 
@@ -293,6 +332,14 @@ __device__ __forceinline__ uint32_t step_pair(uint32_t lo, uint32_t hi) {       
 __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
+// (Only by warps whose waits have been met: others would arrive out of turn, more often than a phase has
+// arrivals left.  Where one has run out the stream's waits run out too.)
+__device__ __forceinline__ void mbar_arrive_many(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void st_shared_v2(uint32_t a, uint32_t x, uint32_t y) {
+  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory");
+}
 // Loads kN times four words, the i-th from at(i), until all have this generation.
 template <int kN, class At>
 __device__ __forceinline__ void step_take(StepCta& c, uint32_t gen, uint4 (&w)[kN], At at) {
@@ -320,152 +367,223 @@ __device__ __forceinline__ unsigned long long step_key(float v, int n) {
 }
 
 // ---------------------------------------------------------------------------------- operations
-// y[n, token] for this CTA's rows of W, tile by tile.  Fragments: the 16 bytes of lane 4 token + q
-// hold columns 32 unit + 8 q .. + 7 of the token.  (Which k meets which does not matter to a sum:
-// both operands use the order in which a 16-byte vector comes out of memory.)  The input is in sm.x,
-// or, with `src`, in an exchange buffer.
-__device__ __forceinline__ StepCta step_gemm(StepCta c, const StepParams& p, const uint32_t* src, int op, int layer,
-                                                 int pos, uint32_t gen, const __nv_bfloat16* bias) {
-  const int tid = step_tid(), warp = tid >> 5, lane = tid & 31;
-  const StepPass pass(p.C);
-  unsigned long long key = 0ull;                 // best of this thread's logits (its token: lane % 8)
-  const StepCut cut = c.sm->cut[op];
-  const int passes = op == kStepOut ? 4 : 1;
-  const int M = p.M, g = lane >> 2, q = lane & 3;
-  const uint32_t ring = smem_u32(c.sm->ring) + g * pass.pitch + q * 16;
-  const int mine_units = (pass.total - warp + kStepWarps - 1) / kStepWarps;       // of each pass
-  const bool live = g < M;
-  if (src != nullptr) src += (warp * M + (live ? g : 0)) * 32 + q * 8;            // idle lanes follow token 0
-  // words of the coming pass (of the first tile; operations with `src` have one)
-  uint4 raw[kStepUnits][2];
-  auto peek = [&](const uint32_t* from) {
+// y[n, token] for this CTA's rows of W.  Every warp takes its columns (StepPart) of every tile, so it waits
+// for one barrier per tile; the partial tiles meet in shared memory, a group of tiles at a time.
+// Fragments: the 16 bytes of lane 4 token + q hold columns 32 unit + 8 q .. + 7 of the token.  (Which k
+// meets which does not matter to a sum: both operands use the order in which a 16-byte vector comes out
+// of memory.)
+
+// Adds kN (<= 4) units: `w` and `x(i)` are this lane's 16 bytes of row g and of token g.  Past unit `last`
+// that unit again: x is zero there, and what lies behind it in shared memory may not be a number.
+template <int kN, class X>
+__device__ __forceinline__ void step_mma(float (&a)[4][4], uint32_t w, int last, uint32_t pitch, X x) {
+  uint4 r[kN], s[kN];
 #pragma unroll
-    for (int i = 0; i < kStepUnits; ++i) {
-      raw[i][0] = raw[i][1] = make_uint4(gen, gen, gen, gen);
-      if (i < mine_units) {
-        raw[i][0] = step_peek(from + i * kStepWarps * M * 32);
-        raw[i][1] = step_peek(from + i * kStepWarps * M * 32 + 4);
-      }
-    }
-  };
-  if (src != nullptr) peek(src);
+  for (int i = 0; i < kN; ++i) {
+    const uint32_t at = w + min(i, last) * 64;
+    r[i] = ld_shared_v4(at);
+    s[i] = ld_shared_v4(at + 8 * pitch);         // (rows past the tile's: their products are used by nobody)
+  }
+#pragma unroll
+  for (int i = 0; i < kN; ++i) mma_16816(a[i], r[i].x, s[i].x, r[i].y, s[i].y, x(i).x, x(i).y);
+#pragma unroll
+  for (int i = 0; i < kN; ++i) mma_16816(a[i], r[i].z, s[i].z, r[i].w, s[i].w, x(i).z, x(i).w);
+}
+__device__ __forceinline__ void step_red_store(float* red, const float (&a)[4][4], int g, int q) {
+  float* at = red + 2 * q * kStepRedPitch + g;
+  at[0] = (a[0][0] + a[1][0]) + (a[2][0] + a[3][0]);
+  at[kStepRedPitch] = (a[0][1] + a[1][1]) + (a[2][1] + a[3][1]);
+  at[8] = (a[0][2] + a[1][2]) + (a[2][2] + a[3][2]);
+  at[kStepRedPitch + 8] = (a[0][3] + a[1][3]) + (a[2][3] + a[3][3]);
+}
+// Output o of a group: token o >> (4 + lg), row (o & 15) of tile (o >> 4) of the group: neighbouring
+// lanes have neighbouring rows, which lie next to each other wherever outputs go.
+struct StepOutput {
+  int row, n, tok, tile;
+  bool mine;
+  __device__ __forceinline__ StepOutput(const StepCut& cut, int t0, int o, int M) {
+    const int in_tile = o & (kStepMmaRows - 1);
+    tile = (o >> 4) & ((1 << cut.lg_group) - 1);
+    tok = o >> (4 + cut.lg_group);
+    row = (t0 + tile) * cut.tile + in_tile;
+    n = cut.row0 + row;
+    mine = in_tile < cut.tile && row < cut.rows && tok < M;
+  }
+};
+__device__ __forceinline__ uint32_t step_bias(const __nv_bfloat16* bias, int n) {
+  return __ldg(reinterpret_cast<const unsigned short*>(bias) + n);
+}
+__device__ __forceinline__ float step_red_sum(const float* red) {
+  float v[kStepWarps];
+#pragma unroll
+  for (int w = 0; w < kStepWarps; ++w) v[w] = red[w * kStepRed];
+  return ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+}
+
+constexpr int kStepPart = (kStepChunkUnits + kStepWarps / 2 - 1) / (kStepWarps / 2);     // 7 units of a warp
+static_assert(kStepChunkUnits <= kStepPart * kStepWarps && kStepMaxUnits <= kStepPart * kStepWarps, "columns fit the warps");
+
+// ... of the LayerNorm's output in sm.x: QKV projection, first MLP layer, head.
+__device__ __forceinline__ StepCta step_linear(StepCta c, const StepParams& p, const StepPart& part, int op, int layer,
+                                               int pos, uint32_t gen, const __nv_bfloat16* bias) {
+  const int tid = step_tid(), warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3, M = p.M;
+  unsigned long long key[2] = {0ull, 0ull};      // best of this thread's logits, of its two tokens
+  const StepCut cut = c.sm->cut[op];
+  uint32_t raw_bias = 0;                         // of the first output: comes while the tiles are multiplied
+  {
+    const StepOutput out(cut, 0, tid, M);
+    if (bias != nullptr && out.mine) raw_bias = step_bias(bias, out.n);
+  }
+  uint4 xv[kStepPart];
+#pragma unroll
+  for (int i = 0; i < kStepPart; ++i) {
+    xv[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (i < part.units && g < M) xv[i] = c.sm->x[(part.first + i) * 4 * M + lane];
+  }
+  const uint32_t pitch = p.stage_pitch, base = smem_u32(c.sm->ring[0]) + part.at * 64 + g * pitch + q * 16;
 #pragma unroll 1
   for (int t0 = 0; t0 < cut.tiles; t0 += kStepGroup) {
     const int tiles = min(kStepGroup, cut.tiles - t0);
-    const int in_tile = (tid >> 3) & (kStepTile - 1), row = (t0 + (tid >> 7)) * cut.tile + in_tile;
-    const int n = cut.row0 + row, tok = tid & 7;
-    const bool mine = (tid >> 7) < tiles && in_tile < cut.tile && row < cut.rows && tok < M;
-    float val = mine && bias != nullptr ? __bfloat162float(bias[n]) : 0.f;
 #pragma unroll 1
     for (int t = 0; t < tiles; ++t) {
-      float a0[4] = {0.f, 0.f, 0.f, 0.f}, a1[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 1
-      for (int ps = 0; ps < passes; ++ps) {
-        uint4 xv[kStepUnits];
-        if (src != nullptr) {
-#pragma unroll 1
-          for (uint32_t polls = 0;; ++polls) {
-            uint32_t bad = 0;
+      StepRing at = c.ring;
+      at.skip(part.stage);
+      c.ring.skip(1 << part.lg_stages);
+      if (c.ok) c.ok = step_wait(smem_u32(&c.sm->full[at.stage]), at.parity, *c.sm, kWaitStepFull);
+      const uint32_t w = base + at.stage * kStepStageBytes;
+      float a[4][4];
 #pragma unroll
-            for (int i = 0; i < kStepUnits; ++i) bad |= step_stale(raw[i][0], gen) | step_stale(raw[i][1], gen);
-            if (!c.ok || !__any_sync(0xffffffffu, bad != 0)) break;
-            if (polls >= kStepWordPolls || *const_cast<volatile uint32_t*>(&c.sm->abort)) {
-              step_give_up(*c.sm, kWaitStepWords);
-              c.ok = false;
-            }
-            peek(src);
-          }
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int i = 0; i < kStepUnits; ++i)
-            xv[i] = live ? make_uint4(step_pair(raw[i][0].x, raw[i][0].y), step_pair(raw[i][0].z, raw[i][0].w),
-                                      step_pair(raw[i][1].x, raw[i][1].y), step_pair(raw[i][1].z, raw[i][1].w))
-                         : make_uint4(0u, 0u, 0u, 0u);
-          src += pass.total * M * 32;
-          if (ps + 1 < passes) peek(src);        // the next pass's, while this one is multiplied
-        } else {
-#pragma unroll
-          for (int i = 0; i < kStepUnits; ++i) {
-            xv[i] = make_uint4(0u, 0u, 0u, 0u);
-            if (live && i < mine_units) xv[i] = c.sm->x[(warp + kStepWarps * i) * 4 * M + lane];
-          }
-        }
-        // the pass's one or two stages
-        const uint32_t base0 = ring + c.ring.stage * kStepStageBytes;
-        uint32_t base1 = base0, bar0 = smem_u32(&c.sm->empty[c.ring.stage]), bar1 = bar0;
-        if (c.ok) c.ok = step_wait(smem_u32(&c.sm->full[c.ring.stage]), c.ring.parity, *c.sm, kWaitStepFull);
-        c.ring.next();
-        if (pass.chunks > 1) {
-          base1 = ring + c.ring.stage * kStepStageBytes - pass.units * 64;
-          bar1 = smem_u32(&c.sm->empty[c.ring.stage]);
-          if (c.ok) c.ok = step_wait(smem_u32(&c.sm->full[c.ring.stage]), c.ring.parity, *c.sm, kWaitStepFull);
-          c.ring.next();
-        }
-#pragma unroll
-        for (int h = 0; h < kStepUnits; h += 2) {        // two units at a time: their loads overlap
-          uint4 r[2], s[2];
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const int u = min(warp + kStepWarps * (h + i), pass.total - 1);      // past the end: x is zero
-            const uint32_t addr = (u < pass.units ? base0 : base1) + u * 64;
-            r[i] = ld_shared_v4(addr);
-            s[i] = ld_shared_v4(addr + 8 * pass.pitch);
-          }
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            mma_16816(a0, r[i].x, s[i].x, r[i].y, s[i].y, xv[h + i].x, xv[h + i].y);
-            mma_16816(a1, r[i].z, s[i].z, r[i].w, s[i].w, xv[h + i].z, xv[h + i].w);
-          }
-        }
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(bar0);
-          if (pass.chunks > 1) mbar_arrive(bar1);
-        }
-      }
-      float* red = c.sm->red[t][warp] + g * 8 + 2 * q;
-      *reinterpret_cast<float2*>(red) = make_float2(a0[0] + a1[0], a0[1] + a1[1]);
-      *reinterpret_cast<float2*>(red + 64) = make_float2(a0[2] + a1[2], a0[3] + a1[3]);
+        for (int j = 0; j < 4; ++j) a[i][j] = 0.f;
+      if (part.units > 0) step_mma<4>(a, w, part.units - 1, pitch, [&](int i) -> const uint4& { return xv[i]; });
+      if (part.units > 4) step_mma<kStepPart - 4>(a, w + 256, part.units - 5, pitch, [&](int i) -> const uint4& { return xv[4 + i]; });
+      __syncwarp();
+      if (lane == 0 && c.ok) mbar_arrive_many(smem_u32(&c.sm->empty[at.stage]), 1u << part.lg_stages);
+      step_red_store(c.sm->red[t][warp], a, g, q);
     }
     step_bar();
-    if (mine) {
-      const float* red = c.sm->red[tid >> 7][0] + (tid & (kStepOutputs - 1));
-      float v1 = 0.f;
 #pragma unroll
-      for (int w = 0; w < kStepWarps; w += 2) {
-        val += red[w * kStepOutputs];
-        v1 += red[(w + 1) * kStepOutputs];
-      }
-      val += v1;
-      if (op == kStepQkv) {
-        step_put(p.qkv + tok * 3 * p.C + n, val, gen);
-        if (n >= p.C) {                          // the caches get the row too, for the steps to come
-          const bool is_k = n < 2 * p.C;
-          const int nn = n - (is_k ? p.C : 2 * p.C);
-          (is_k ? p.k_cache[layer] : p.v_cache[layer])[tok * p.c_sb + static_cast<long long>(pos) * p.c_sn + (nn >> 6) * p.c_sh + (nn & 63)] =
-              __float2bfloat16_rn(val);
+    for (int k = 0; k < 2; ++k) {                // at most 512 outputs
+      const int o = tid + k * kStepCompute;
+      const StepOutput out(cut, t0, o, M);
+      if (out.mine) {
+        if (bias != nullptr && (k > 0 || t0 > 0)) raw_bias = step_bias(bias, out.n);
+        const float val = __uint_as_float(raw_bias << 16) + step_red_sum(&c.sm->red[out.tile][0][out.tok * kStepRedPitch + (o & (kStepMmaRows - 1))]);
+        const int n = out.n, tok = out.tok;
+        if (op == kStepQkv) {
+          step_put(p.qkv + tok * 3 * p.C + n, val, gen);
+          if (n >= p.C) {                          // the caches get the row too, for the steps to come
+            const bool is_k = n < 2 * p.C;
+            const int nn = n - (is_k ? p.C : 2 * p.C);
+            (is_k ? p.k_cache[layer] : p.v_cache[layer])[tok * p.c_sb + static_cast<long long>(pos) * p.c_sn + (nn >> 6) * p.c_sh + (nn & 63)] =
+                __float2bfloat16_rn(val);
+          }
+        } else if (op == kStepFc) {
+          step_put(p.h + ((n >> 5) * M + tok) * 32 + (n & 31), gelu_tanh(val), gen);
+        } else {
+          const __nv_bfloat16 b = __float2bfloat16_rn(val);
+          p.logits[static_cast<long long>(tok) * p.V + n] = b;
+          const unsigned long long kk = step_key(__bfloat162float(b), n);
+          key[k] = kk > key[k] ? kk : key[k];
         }
-      } else if (op == kStepFc) {
-        step_put(p.h + ((n >> 5) * M + tok) * 32 + (n & 31), gelu_tanh(val), gen);
-      } else if (op == kStepHead) {
-        const __nv_bfloat16 b = __float2bfloat16_rn(val);
-        p.logits[static_cast<long long>(tok) * p.V + n] = b;
-        const unsigned long long kk = step_key(__bfloat162float(b), n);
-        key = kk > key ? kk : key;
-      } else {
-        val += c.sm->own[tid];           // one tile, so the thread is below kStepOutputs
-        c.sm->own[tid] = val;
-        step_put((op == kStepProj ? p.x_att : p.x_mlp) + tok * p.C + n, val, gen);
       }
     }
     if (t0 + kStepGroup < cut.tiles) step_bar();     // before the partial tiles are overwritten
   }
-  if (op == kStepHead) {
+  if (op == kStepHead) {                         // groups of 4 tiles: 64 rows, so two warps per token
 #pragma unroll
-    for (int o = 8; o <= 16; o <<= 1) {
-      const unsigned long long k = __shfl_xor_sync(0xffffffffu, key, o);
-      key = k > key ? k : key;
+    for (int k = 0; k < 2; ++k) {
+#pragma unroll
+      for (int o = 1; o <= 16; o <<= 1) {
+        const unsigned long long other = __shfl_xor_sync(0xffffffffu, key[k], o);
+        key[k] = other > key[k] ? other : key[k];
+      }
+      if (lane == 0) c.sm->keys[(warp >> 1) + 4 * k][warp & 1] = key[k];
     }
-    if (lane < kStepMaxRows) c.sm->keys[warp][lane] = key;
+  }
+  return c;
+}
+static_assert(kStepGroup == 4 && kStepWarps == 8 && kStepMaxRows == 8, "512 outputs of a group, two per thread; a token's are two warps'");
+
+// ... of an exchange buffer, for the few rows (one tile) of the attention's projection and the second MLP
+// layer: a warp takes the words of its own columns, 32 unit rows at a time, and packs them into its piece
+// of sm.x.
+__device__ __forceinline__ StepCta step_linear_words(StepCta c, const StepParams& p, const StepPart& part, const uint32_t* src,
+                                                     uint32_t* dst, int op, uint32_t gen, const __nv_bfloat16* bias) {
+  const int tid = step_tid(), warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3, M = p.M;
+  const uint32_t* words = src + (part.first * M * 8 + lane) * 4;
+  uint4 raw[kStepTake];
+  auto peek = [&](int b0, int nb) {                            // the words of units b0 .. + nb
+#pragma unroll
+    for (int i = 0; i < kStepTake; ++i) {
+      raw[i] = make_uint4(gen, gen, gen, gen);
+      if (i * 32 + lane < nb * M * 8) raw[i] = step_peek(words + b0 * M * 32 + i * 128);
+    }
+  };
+  const int batch = p.batch_units, units = part.units;
+  peek(0, min(batch, units));
+  const StepCut cut = c.sm->cut[op];
+  const StepOutput out(cut, 0, tid, M);
+  uint32_t raw_bias = 0;
+  if (bias != nullptr && out.mine) raw_bias = step_bias(bias, out.n);
+  if (cut.tiles > 0) {
+    StepRing at = c.ring;
+    at.skip(part.stage);
+    c.ring.skip(1 << part.lg_stages);
+    if (c.ok) c.ok = step_wait(smem_u32(&c.sm->full[at.stage]), at.parity, *c.sm, kWaitStepFull);
+    const uint32_t pitch = p.stage_pitch;
+    uint32_t w = smem_u32(c.sm->ring[0]) + at.stage * kStepStageBytes + part.at * 64 + g * pitch + q * 16;
+    const uint32_t pack = smem_u32(c.sm->x) + warp * (kStepTake * 256), x0 = pack + lane * 16, x_step = M * 64;
+    float a[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) a[i][j] = 0.f;
+#pragma unroll 1
+    for (int b0 = 0; b0 < units; b0 += batch) {
+      const int nb = min(batch, units - b0);
+#pragma unroll 1
+      for (uint32_t polls = 0;; ++polls) {
+        uint32_t bad = 0;
+#pragma unroll
+        for (int i = 0; i < kStepTake; ++i) bad |= step_stale(raw[i], gen);
+        if (!c.ok || !__any_sync(0xffffffffu, bad != 0)) break;
+        if (polls >= kStepWordPolls || *const_cast<volatile uint32_t*>(&c.sm->abort)) {
+          step_give_up(*c.sm, kWaitStepWords);
+          c.ok = false;
+        }
+        peek(b0, nb);
+      }
+#pragma unroll
+      for (int i = 0; i < kStepTake; ++i)
+        if (i * 32 < nb * M * 8)                 // (what lies past the end of the units is not read)
+          st_shared_v2(pack + (i * 32 + lane) * 8, step_pair(raw[i].x, raw[i].y), step_pair(raw[i].z, raw[i].w));
+      __syncwarp();
+      if (b0 + batch < units) peek(b0 + batch, min(batch, units - b0 - batch));
+      uint32_t x = x0;
+#pragma unroll 1
+      for (int u = 0; u < nb; u += 4) {          // four units at a time: their loads overlap
+        uint4 xv[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          xv[i] = make_uint4(0u, 0u, 0u, 0u);
+          if (u + i < nb && g < M) xv[i] = ld_shared_v4(x + i * x_step);
+        }
+        step_mma<4>(a, w + u * 64, nb - 1 - u, pitch, [&](int i) -> const uint4& { return xv[i]; });
+        x += 4 * x_step;
+      }
+      w += nb * 64;
+      __syncwarp();                              // before the words are overwritten, the stage given back
+    }
+    if (lane == 0 && c.ok) mbar_arrive_many(smem_u32(&c.sm->empty[at.stage]), 1u << part.lg_stages);
+    step_red_store(c.sm->red_one[warp], a, g, q);
+  }
+  step_bar();
+  if (out.mine) {
+    const float val = __uint_as_float(raw_bias << 16) + step_red_sum(&c.sm->red_one[0][out.tok * kStepRedPitch + out.row]) + c.sm->own[tid];
+    c.sm->own[tid] = val;
+    step_put(dst + out.tok * p.C + out.n, val, gen);
   }
   return c;
 }
@@ -475,7 +593,7 @@ __device__ __forceinline__ StepCta step_gemm(StepCta c, const StepParams& p, con
 struct StepRows {
   int tok, first, stride, lg;
   __device__ __forceinline__ StepRows(int M, int warp, int lane) {
-    lg = M <= 1 ? 4 : (M <= 2 ? 3 : (M <= 4 ? 2 : 1));      // log2 of warps per token
+    lg = M <= 1 ? 3 : (M <= 2 ? 2 : (M <= 4 ? 1 : 0));      // log2 of warps per token
     tok = warp >> lg;
     first = (warp & ((1 << lg) - 1)) * 32 + lane;
     stride = 32 << lg;
@@ -485,26 +603,24 @@ struct StepRows {
 // LayerNorm of the residual stream (exchange words at `x`) into the fragments sm.x.  One pass: sums
 // of x - s and (x - s)^2 with s the row's mean in the LayerNorm before (0 in the first), which keeps
 // the difference of squares well conditioned.
-__device__ __forceinline__ StepCta step_layernorm(StepCta c, const StepParams& p, const uint32_t* x, uint32_t gen) {
-  const int tid = step_tid(), warp = tid >> 5, lane = tid & 31;
-  const StepRows rw(p.M, warp, lane);
+// kN: rounds of the warps over a row's groups of four columns, at least as many as there are.  (One kN for
+// the widest row of a warp, with the rounds that are not there branched around, took 2300 clocks where
+// there was one round.)
+template <int kN>
+__device__ __forceinline__ StepCta step_layernorm(StepCta c, const StepParams& p, const uint32_t* x, uint32_t gen,
+                                                  const StepRows& rw) {
+  const int lane = step_tid() & 31, warp = step_tid() >> 5;
   const int quads = p.C >> 2;
-  // rounds of this warp (the same for its lanes: past the end they repeat the last quad, unused)
-  const int n = rw.tok < p.M ? (quads - (rw.first - lane) + rw.stride - 1) / rw.stride : 0;
-  uint4 w[kStepQuads];
-#pragma unroll
-  for (int i = 0; i < kStepQuads; ++i) w[i] = make_uint4(0u, 0u, 0u, 0u);
-  {
-    const uint32_t* src = x + rw.tok * p.C;
+  uint4 w[kN];
+  {                                              // (past the end the last quad again, unused)
+    const uint32_t* src = x + min(rw.tok, p.M - 1) * p.C;
 #pragma unroll 1
     for (uint32_t polls = 0;; ++polls) {
       uint32_t bad = 0;
 #pragma unroll
-      for (int i = 0; i < kStepQuads; ++i)
-        if (i < n) w[i] = step_peek(src + 4 * min(rw.first + i * rw.stride, quads - 1));
+      for (int i = 0; i < kN; ++i) w[i] = step_peek(src + 4 * min(rw.first + i * rw.stride, quads - 1));
 #pragma unroll
-      for (int i = 0; i < kStepQuads; ++i)
-        if (i < n) bad |= step_stale(w[i], gen);
+      for (int i = 0; i < kN; ++i) bad |= step_stale(w[i], gen);
       if (!c.ok || !__any_sync(0xffffffffu, bad != 0)) break;
       if (polls >= kStepWordPolls || *const_cast<volatile uint32_t*>(&c.sm->abort)) {
         step_give_up(*c.sm, kWaitStepWords);
@@ -515,15 +631,13 @@ __device__ __forceinline__ StepCta step_layernorm(StepCta c, const StepParams& p
   const float shift = c.sm->shift[rw.tok & (kStepMaxRows - 1)];
   float sum = 0.f, sq = 0.f;
 #pragma unroll
-  for (int i = 0; i < kStepQuads; ++i) {
-    if (i < n) {
-      w[i].x &= 0xffff0000u; w[i].y &= 0xffff0000u; w[i].z &= 0xffff0000u; w[i].w &= 0xffff0000u;   // now fp32
-      const float f = rw.first + i * rw.stride < quads ? 1.f : 0.f;
-      const float d0 = __uint_as_float(w[i].x) - shift, d1 = __uint_as_float(w[i].y) - shift;
-      const float d2 = __uint_as_float(w[i].z) - shift, d3 = __uint_as_float(w[i].w) - shift;
-      sum = fmaf(f, (d0 + d1) + (d2 + d3), sum);
-      sq = fmaf(f, fmaf(d0, d0, d1 * d1) + fmaf(d2, d2, d3 * d3), sq);
-    }
+  for (int i = 0; i < kN; ++i) {
+    w[i].x &= 0xffff0000u; w[i].y &= 0xffff0000u; w[i].z &= 0xffff0000u; w[i].w &= 0xffff0000u;   // now fp32
+    const float f = rw.first + i * rw.stride < quads ? 1.f : 0.f;
+    const float d0 = __uint_as_float(w[i].x) - shift, d1 = __uint_as_float(w[i].y) - shift;
+    const float d2 = __uint_as_float(w[i].z) - shift, d3 = __uint_as_float(w[i].w) - shift;
+    sum = fmaf(f, (d0 + d1) + (d2 + d3), sum);
+    sq = fmaf(f, fmaf(d0, d0, d1 * d1) + fmaf(d2, d2, d3 * d3), sq);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -533,26 +647,23 @@ __device__ __forceinline__ StepCta step_layernorm(StepCta c, const StepParams& p
   if (lane == 0) c.sm->stat[warp] = make_float2(sum, sq);
   asm volatile("cp.async.wait_all;" ::: "memory");
   step_bar();                                    // sm.stat and sm.norm are complete, sm.shift is read
-  sum = sq = 0.f;
-  {
+  if (rw.lg > 0) {                               // 1, 2 or 4 pairs of warps
     const float4* st = reinterpret_cast<const float4*>(c.sm->stat + ((rw.tok << rw.lg) & (kStepWarps - 1)));
-#pragma unroll 2
-    for (int i = 0; i < 1 << (rw.lg - 1); ++i) {
-      const float4 two = st[i];
-      sum += two.x + two.z;
-      sq += two.y + two.w;
-    }
+    float4 two[kStepWarps / 2];
+#pragma unroll
+    for (int i = 0; i < kStepWarps / 2; ++i) two[i] = i < 1 << (rw.lg - 1) ? st[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    sum = ((two[0].x + two[0].z) + (two[1].x + two[1].z)) + ((two[2].x + two[2].z) + (two[3].x + two[3].z));
+    sq = ((two[0].y + two[0].w) + (two[1].y + two[1].w)) + ((two[2].y + two[2].w) + (two[3].y + two[3].w));
   }
-  const float inv_c = __fdividef(1.f, static_cast<float>(p.C));
-  const float off = sum * inv_c;
-  const float rstd = rsqrtf(fmaxf(sq * inv_c - off * off, 0.f) + p.eps);
+  const float off = sum * p.inv_c;
+  const float rstd = rsqrtf(fmaxf(sq * p.inv_c - off * off, 0.f) + p.eps);
   const float mean = shift + off;
   if (rw.first == 0 && rw.tok < p.M) c.sm->shift[rw.tok] = mean;
   uint2* out = reinterpret_cast<uint2*>(c.sm->x) + rw.tok * 8;
 #pragma unroll
-  for (int i = 0; i < kStepQuads; ++i) {
+  for (int i = 0; i < kN; ++i) {
     const int v = rw.first + i * rw.stride;      // columns 4 v .. 4 v + 3
-    if (i < n && v < quads) {
+    if (rw.tok < p.M && v < quads) {
       const uint2 gm = c.sm->norm[0][v], bt = c.sm->norm[1][v];
       const float y0 = fmaf((__uint_as_float(w[i].x) - mean) * rstd, __uint_as_float(gm.x << 16), __uint_as_float(bt.x << 16));
       const float y1 = fmaf((__uint_as_float(w[i].y) - mean) * rstd, __uint_as_float(gm.x & 0xffff0000u), __uint_as_float(bt.x & 0xffff0000u));
@@ -568,11 +679,12 @@ __device__ __forceinline__ StepCta step_layernorm(StepCta c, const StepParams& p
 __device__ __forceinline__ void step_fetch_norm(StepSmem& sm, const __nv_bfloat16* gamma, const __nv_bfloat16* beta,
                                                 int nvec) {
   const int tid = step_tid();
-  const int v = tid & 255;               // 200 vectors of 16 bytes at most, one per thread
-  if (v < nvec) cp_async_16(smem_u32(sm.norm[tid >> 8]) + v * 16,
-                            reinterpret_cast<const uint4*>(tid < 256 ? gamma : beta) + v);
+  const bool second = tid >= kStepCompute / 2;
+  const uint32_t dst = smem_u32(sm.norm[second ? 1 : 0]);
+  const uint4* src = reinterpret_cast<const uint4*>(second ? beta : gamma);
+#pragma unroll 1
+  for (int v = second ? tid - kStepCompute / 2 : tid; v < nvec; v += kStepCompute / 2) cp_async_16(dst + v * 16, src + v);
 }
-static_assert(kStepMaxWidth / 8 <= 256 && kStepCompute == 512, "one vector per thread");
 
 __device__ __forceinline__ StepCta step_attention(StepCta c, const StepParams& p, int layer, uint32_t gen) {
   const int tid = step_tid(), warp = tid >> 5, lane = tid & 31, count = c.sm->units, splits = c.sm->splits;
@@ -590,7 +702,7 @@ __device__ __forceinline__ StepCta step_attention(StepCta c, const StepParams& p
     }
     float m = -1e30f, l = 0.f;
     uint64_t acc[4] = {0ull, 0ull, 0ull, 0ull};
-    // Stages of kStepBlocks blocks of 16 rows; block b is warp b % 16's.  A row's odd-numbered
+    // Stages of kStepBlocks blocks of 16 rows; block b is warp b % 8's.  A row's odd-numbered
     // neighbour has its 64-byte halves swapped (see step_stream_rows): no bank conflicts.
     const int blocks = (un.rows + 15) >> 4, swap = (g & 1) << 2, vswap = (grp & 1) << 2;
 #pragma unroll 1
@@ -638,7 +750,7 @@ __device__ __forceinline__ StepCta step_attention(StepCta c, const StepParams& p
         }
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&c.sm->empty[c.ring.stage]));
+      if (lane == 0 && c.ok) mbar_arrive(smem_u32(&c.sm->empty[c.ring.stage]));
       c.ring.next();
     }
 #pragma unroll
@@ -732,43 +844,68 @@ __device__ __forceinline__ void step_prefetch(const StepSmem& sm, const StepPara
   }
 }
 
+// The streaming warps' ops in order: 4 per layer, then the head.
+__device__ __forceinline__ const __nv_bfloat16* step_weight(const StepSmem& sm, const StepParams& p, int i, int& op) {
+  if (i >= 4 * p.n_layers) { op = kStepHead; return p.head_w; }
+  op = i & 3;
+  const StepLayer& L = sm.layers[i >> 2];
+  return op == kStepQkv ? L.qkv_w : (op == kStepProj ? L.proj_w : (op == kStepFc ? L.fc_w : L.out_w));
+}
+__device__ __forceinline__ void step_ahead(const StepSmem& sm, const StepParams& p, int i, int sw, int lane) {
+  if (i > 4 * p.n_layers) return;
+  int op;
+  const __nv_bfloat16* w = step_weight(sm, p, i, op);
+  const StepCut& cut = sm.cut[op];
+  const uint32_t row = (op == kStepOut ? 4 * p.C : p.C) * 2u, bytes = min(cut.rows * row, kStepAheadBytes);
+  const char* at = reinterpret_cast<const char*>(w) + static_cast<long long>(cut.row0) * row;
+#pragma unroll 1
+  for (uint32_t b = (sw * 32 + lane) * kStepAheadPiece; b < bytes; b += 32 * kStepStreamWarps * kStepAheadPiece)
+    bulk_prefetch_l2(at + b, min(kStepAheadPiece, bytes - b));
+}
+__device__ __forceinline__ void step_ahead_rows(const StepSmem& sm, const StepParams& p, int layer, int sw, int lane) {
+#pragma unroll 1
+  for (int i = 0; i < sm.units; ++i) {
+    const StepUnit& un = sm.unit[i];
+    const long long at = un.head + static_cast<long long>(un.row0) * p.c_sn;
+#pragma unroll 1
+    for (int r = sw * 32 + lane; r < un.rows; r += 32 * kStepStreamWarps) {
+      prefetch_l2(p.k_cache[layer] + at + static_cast<long long>(r) * p.c_sn);
+      prefetch_l2(p.v_cache[layer] + at + static_cast<long long>(r) * p.c_sn);
+    }
+  }
+}
+
 // Streaming warp `sw`: its quarter of this CTA's rows of one matrix into the ring.
-__device__ __forceinline__ bool step_stream(StepSmem& sm, StepRing& ring, uint32_t& issued, const __nv_bfloat16* w, int op,
-                                            int C, int sw) {
+__device__ __forceinline__ bool step_stream(StepSmem& sm, const StepParams& p, StepRing& ring, uint32_t& issued,
+                                            const __nv_bfloat16* w, int op, int sw) {
   const StepCut cut = sm.cut[op];
-  const StepPass pass(C);
-  const int passes = op == kStepOut ? 4 : 1;
-  const long long ldw = static_cast<long long>(passes) * C;
+  const long long ldw = op == kStepOut ? 4 * p.C : p.C;
+  const int stages = 1 << (p.lg_chunks + (op == kStepOut ? 2 : 0));
+  const uint32_t bytes = static_cast<uint32_t>(p.stage_units) * 64;
   w += (cut.row0 + sw) * ldw;
 #pragma unroll 1
   for (int t = 0; t < cut.tiles; ++t) {
     // rows sw, sw + 4, ... of the tile
     const int rows = (min(cut.tile, cut.rows - t * cut.tile) - sw + kStepStreamWarps - 1) / kStepStreamWarps;
     const __nv_bfloat16* src = w + t * cut.tile * ldw;
-    int in_pass = 0;
 #pragma unroll 1
-    for (int k = 0; k < passes * pass.total;) {
-      const int units = min(pass.units, pass.total - in_pass);       // chunks never cross the end of a pass
+    for (int st = 0; st < stages; ++st) {
       if (issued >= kStepStages &&
           !step_wait(smem_u32(&sm.empty[ring.stage]), ring.parity ^ 1, sm, kWaitStepEmpty))
         return false;
       if (elect_one()) {
         fence_proxy_async_smem();                // (the stage may have held cached rows, written by plain copies)
-        const uint32_t bytes = static_cast<uint32_t>(units) * 64;
         const uint32_t bar = smem_u32(&sm.full[ring.stage]);
-        uint32_t dst = smem_u32(sm.ring[ring.stage]) + sw * pass.pitch;
+        uint32_t dst = smem_u32(sm.ring[ring.stage]) + sw * p.stage_pitch;
         mbar_arrive_expect_tx(bar, bytes * rows);
 #pragma unroll
         for (int r = 0; r < kStepTile / kStepStreamWarps; ++r)
-          if (r < rows) bulk_load(dst + r * kStepStreamWarps * pass.pitch, src + r * kStepStreamWarps * ldw, bytes, bar);
+          if (r < rows) bulk_load(dst + r * kStepStreamWarps * p.stage_pitch, src + r * kStepStreamWarps * ldw, bytes, bar);
       }
       __syncwarp();
       ring.next();
       ++issued;
-      k += units;
-      src += units * kStepUnit;
-      in_pass += units;
-      if (in_pass == pass.total) in_pass = 0;
+      src += p.stage_units * kStepUnit;
     }
   }
   return true;
@@ -860,24 +997,28 @@ __global__ void __launch_bounds__(kStepThreads, 1) fa_gpt_step_kernel(const __gr
   }
   if (threadIdx.x < 5) {
     const int op = threadIdx.x;
-    sm.cut[op] = step_cut(op == kStepQkv ? 3 * C : (op == kStepFc ? 4 * C : (op == kStepHead ? p.V : C)));
+    sm.cut[op] = step_cut(op == kStepQkv ? 3 * C : (op == kStepFc ? 4 * C : (op == kStepHead ? p.V : C)),
+                          op == kStepHead);
   }
   __syncthreads();
 
   if (warp >= kStepWarps) {
     reg_dealloc<kStepStreamRegs>();              // all four warps of the warpgroup
     // ------------------------------------------------------------------ stream
+    const int sw = warp - kStepWarps;
     StepRing ring;
     uint32_t issued = 0;
     bool ok = true;
+    for (int i = 1; i < kStepAhead; ++i) step_ahead(sm, p, i, sw, lane);
+    if (kStepAheadKv) step_ahead_rows(sm, p, 0, sw, lane);
 #pragma unroll 1
     for (int i = 0; i <= 4 * p.n_layers && ok; ++i) {
-      const StepLayer& L = sm.layers[min(i >> 2, p.n_layers - 1)];
-      const int op = i == 4 * p.n_layers ? static_cast<int>(kStepHead) : (i & 3);
-      ok = step_stream(sm, ring, issued,
-                       op == kStepQkv ? L.qkv_w : (op == kStepProj ? L.proj_w : (op == kStepFc ? L.fc_w : (op == kStepOut ? L.out_w : p.head_w))),
-                       op, C, warp - kStepWarps);
-      if (ok && op == kStepQkv) ok = step_stream_rows(sm, p, ring, issued, i >> 2, warp - kStepWarps, lane);
+      int op;
+      const __nv_bfloat16* w = step_weight(sm, p, i, op);
+      step_ahead(sm, p, i + kStepAhead, sw, lane);
+      if (kStepAheadKv && (i & 3) == kStepFc && (i >> 2) + 1 < p.n_layers) step_ahead_rows(sm, p, (i >> 2) + 1, sw, lane);
+      ok = step_stream(sm, p, ring, issued, w, op, sw);
+      if (ok && op == kStepQkv) ok = step_stream_rows(sm, p, ring, issued, i >> 2, sw, lane);
     }
     // leave no copy in flight, whatever the computing warps did: the last use of every stage
 #pragma unroll 1
@@ -889,9 +1030,10 @@ __global__ void __launch_bounds__(kStepThreads, 1) fa_gpt_step_kernel(const __gr
     StepCta c;
     c.sm = &sm;
     c.ok = true;
-    {  // this CTA's columns of the residual stream: the embeddings' sum (see the outputs in step_gemm)
-      const int tok = threadIdx.x & 7, row = threadIdx.x >> 3, n = sm.cut[kStepProj].row0 + row;
-      if (row < sm.cut[kStepProj].rows && tok < M) {      // one tile, at most 16 rows
+    {  // this CTA's columns of the residual stream: the embeddings' sum
+      const StepOutput out(sm.cut[kStepProj], 0, threadIdx.x, M);
+      const int tok = out.tok, n = out.n;
+      if (out.mine) {
         long long id = p.ids[tok * p.ids_stride];
         id = id < 0 ? 0 : (id >= p.V ? p.V - 1 : id);
         const float v = __bfloat162float(__float2bfloat16_rn(
@@ -901,25 +1043,30 @@ __global__ void __launch_bounds__(kStepThreads, 1) fa_gpt_step_kernel(const __gr
       }
     }
     step_prefetch(sm, p, 0);
+    const StepPart narrow(warp, p.lg_chunks, p.stage_units), wide(warp, p.lg_chunks + 2, p.stage_units);
 #pragma unroll 1
     for (int i = 0; i <= 4 * p.n_layers; ++i) {
       const int l = min(i >> 2, p.n_layers - 1);
       const int op = i == 4 * p.n_layers ? static_cast<int>(kStepHead) : (i & 3);
       const StepLayer& L = sm.layers[l];
       const uint32_t before = (generation + l) % 65535u + 1u, gen = (generation + l + 1) % 65535u + 1u;
-      const uint32_t* src = nullptr;
       const __nv_bfloat16* bias = op == kStepQkv ? L.qkv_b : (op == kStepProj ? L.proj_b : (op == kStepFc ? L.fc_b : (op == kStepOut ? L.out_b : nullptr)));
-      step_bar();                                // the reductions of the operation before are read
       if (op & 1) {
-        src = op == kStepProj ? p.ctx : p.h;
+        const bool proj = op == kStepProj;
+        c = step_linear_words(c, p, proj ? narrow : wide, proj ? p.ctx : p.h, proj ? p.x_att : p.x_mlp, op, gen, bias);
       } else {
         step_fetch_norm(sm, op == kStepQkv ? L.ln1_g : (op == kStepFc ? L.ln2_g : p.lnf_g),
                         op == kStepQkv ? L.ln1_b : (op == kStepFc ? L.ln2_b : p.lnf_b), C >> 3);
-        c = step_layernorm(c, p, op == kStepFc ? p.x_att : p.x_mlp, op == kStepQkv ? before : gen);
+        const uint32_t* x = op == kStepFc ? p.x_att : p.x_mlp;
+        const uint32_t want = op == kStepQkv ? before : gen;
+        const StepRows rw(M, step_tid() >> 5, step_tid() & 31);
+        if (C <= 8 * rw.stride) c = step_layernorm<2>(c, p, x, want, rw);
+        else if (C <= 16 * rw.stride) c = step_layernorm<4>(c, p, x, want, rw);
+        else if (C <= 28 * rw.stride) c = step_layernorm<7>(c, p, x, want, rw);
+        else c = step_layernorm<kStepQuads>(c, p, x, want, rw);
+        c = step_linear(c, p, narrow, op, l, pos, gen, bias);
       }
-      c = step_gemm(c, p, src, op, l, pos, gen, bias);
       if (op == kStepQkv && sm.units > 0) {
-        step_bar();
         c = step_attention(c, p, l, gen);
       }
       if (op == kStepOut && l + 1 < p.n_layers) step_prefetch(sm, p, l + 1);
@@ -930,7 +1077,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) fa_gpt_step_kernel(const __gr
         if (lane < M) {
           unsigned long long key = 0ull;
 #pragma unroll
-          for (int w = 0; w < kStepWarps; ++w) key = sm.keys[w][lane] > key ? sm.keys[w][lane] : key;
+          for (int w = 0; w < 2; ++w) key = sm.keys[lane][w] > key ? sm.keys[lane][w] : key;
           atomicMax(p.best + lane, key);
         }
         __threadfence();
