@@ -103,8 +103,9 @@ constexpr int kStepQuads = (kStepMaxWidth / 4 + 31) / 32;     // 13: columns / 4
 constexpr int kStepTake = 8;                          // words of a batch: 32 lanes x kStepTake x 4
 constexpr int kStepSegs = 2;                          // attention units of one CTA
 constexpr int kStepBlocks = 4;                        // blocks of 16 cached rows (K, then V) per stage
+static_assert(kStepBlocks == kStepWarps / 2 && kStepStages % 2 == 0, "half the warps to a stage, by the slot's parity");
 static_assert(kStepBlocks * 16 * 256 <= kStepStageBytes, "cached rows fit a stage");
-constexpr int kStepSplitRows = 1024;                  // rows of a unit where pairs are split over CTAs
+constexpr int kStepSplitRows = 384;                   // rows of a unit where pairs are split over CTAs
 constexpr uint32_t kStepBarPolls = 1u << 24;          // bounds of the waits: about 65 clocks a poll of a barrier ...
 constexpr uint32_t kStepWordPolls = 1u << 21;         // ... and a trip to L2 a poll of exchange words: half a second
 
@@ -702,59 +703,72 @@ __device__ __forceinline__ StepCta step_attention(StepCta c, const StepParams& p
     }
     float m = -1e30f, l = 0.f;
     uint64_t acc[4] = {0ull, 0ull, 0ull, 0ull};
-    // Stages of kStepBlocks blocks of 16 rows; block b is warp b % 8's.  A row's odd-numbered
-    // neighbour has its 64-byte halves swapped (see step_stream_rows): no bank conflicts.
-    const int blocks = (un.rows + 15) >> 4, swap = (g & 1) << 2, vswap = (grp & 1) << 2;
+    // Stages of kStepBlocks blocks of 16 rows, one warp to a block: warps 0 to 3 take the even ring slots, 4
+    // to 7 the odd ones (so a warp that waits for a slot has also waited for the slot's stage before).  A
+    // row's odd-numbered neighbour has its 64-byte halves swapped (see step_stream_rows): no bank conflicts.
+    // Lane group grp (of 8 lanes) sums rows grp, grp + 4, + 8, + 12 of the blocks with a maximum of its own.
+    // A GPT-2 XL unit of 900 rows, clocks: 8900 with one maximum per warp and waits for all stages, XX so.
+    const int swap = (g & 1) << 2, vswap = (grp & 1) << 2;
 #pragma unroll 1
-    for (int b0 = 0; b0 < blocks; b0 += kStepBlocks) {
-      if (c.ok) c.ok = step_wait(smem_u32(&c.sm->full[c.ring.stage]), c.ring.parity, *c.sm, kWaitStepFull);
-      const int j0 = (warp - b0) & (kStepWarps - 1), base = (b0 + j0) * 16;
-      if (j0 < kStepBlocks && base < un.rows) {
-        const uint32_t ks = smem_u32(c.sm->ring) + c.ring.stage * kStepStageBytes + j0 * 16 * 128;
-        const uint32_t vs = ks + kStepBlocks * 16 * 128;
-        const uint4 k0 = ld_shared_v4(ks + g * 128 + (q ^ swap) * 16), k1 = ld_shared_v4(ks + g * 128 + ((q + 4) ^ swap) * 16);
-        const uint4 k2 = ld_shared_v4(ks + (g + 8) * 128 + (q ^ swap) * 16), k3 = ld_shared_v4(ks + (g + 8) * 128 + ((q + 4) ^ swap) * 16);
-        uint4 vr[4];
+    for (int r0 = 0; r0 < un.rows; r0 += kStepBlocks * 16) {
+      if ((c.ring.stage & 1) == warp / kStepBlocks) {
+        if (c.ok) c.ok = step_wait(smem_u32(&c.sm->full[c.ring.stage]), c.ring.parity, *c.sm, kWaitStepFull);
+        const int j0 = warp & (kStepBlocks - 1), left = un.rows - r0 - j0 * 16;        // rows of the block and after
+        if (left > 0) {
+          const uint32_t ks = smem_u32(c.sm->ring) + c.ring.stage * kStepStageBytes + j0 * 16 * 128;
+          const uint32_t vs = ks + kStepBlocks * 16 * 128;
+          const uint4 k0 = ld_shared_v4(ks + g * 128 + (q ^ swap) * 16), k1 = ld_shared_v4(ks + g * 128 + ((q + 4) ^ swap) * 16);
+          const uint4 k2 = ld_shared_v4(ks + (g + 8) * 128 + (q ^ swap) * 16), k3 = ld_shared_v4(ks + (g + 8) * 128 + ((q + 4) ^ swap) * 16);
+          uint4 vr[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) vr[j] = ld_shared_v4(vs + (grp + 4 * j) * 128 + (col ^ vswap) * 16);
-        // scores of rows g (s[0], equal in the lanes of a quad and in s[1]) and g + 8 (s[2], s[3]):
-        // every column of the 8-column operand is the query
-        float s[4] = {0.f, 0.f, 0.f, 0.f};
-        mma_16816(s, k0.x, k2.x, k0.y, k2.y, q0.x, q0.y);
-        mma_16816(s, k0.z, k2.z, k0.w, k2.w, q0.z, q0.w);
-        mma_16816(s, k1.x, k3.x, k1.y, k3.y, q1.x, q1.y);
-        mma_16816(s, k1.z, k3.z, k1.w, k3.w, q1.z, q1.w);
-        const float sa = base + g < un.rows ? s[0] * p.scale_log2 : -INFINITY;
-        const float sb = base + g + 8 < un.rows ? s[2] * p.scale_log2 : -INFINITY;
-        float m_new = fmaxf(sa, sb);
+          for (int j = 0; j < 4; ++j) vr[j] = ld_shared_v4(vs + (grp + 4 * j) * 128 + (col ^ vswap) * 16);
+          // scores of rows g ([0], equal in the lanes of a quad and in [1]) and g + 8 ([2], [3]): every
+          // column of the 8-column operand is the query
+          float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+          mma_16816(s0, k0.x, k2.x, k0.y, k2.y, q0.x, q0.y);
+          mma_16816(s1, k0.z, k2.z, k0.w, k2.w, q0.z, q0.w);
+          mma_16816(s0, k1.x, k3.x, k1.y, k3.y, q1.x, q1.y);
+          mma_16816(s1, k1.z, k3.z, k1.w, k3.w, q1.z, q1.w);
+          const float sa = g < left ? (s0[0] + s1[0]) * p.scale_log2 : -INFINITY;
+          const float sb = g + 8 < left ? (s0[2] + s1[2]) * p.scale_log2 : -INFINITY;
+          float sc[4];                             // rows grp + 4 j: lane 4 (row % 8) has them
 #pragma unroll
-        for (int o = 4; o <= 16; o <<= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, o));
-        if (m_new > m) {                         // the same in all lanes
+          for (int j = 0; j < 4; ++j) sc[j] = __shfl_sync(0xffffffffu, j < 2 ? sa : sb, ((grp + 4 * j) & 7) * 4);
+          const float m_new = fmaxf(fmaxf(m, fmaxf(sc[0], sc[1])), fmaxf(sc[2], sc[3]));
           const float f = ex2_approx(m - m_new);
           const uint64_t f2 = pack_f32x2(f, f);
+          m = m_new;
           l *= f;
 #pragma unroll
           for (int e = 0; e < 4; ++e) acc[e] = mul_f32x2(acc[e], f2);
-          m = m_new;
-        }
-        const float pa = ex2_approx(sa - m), pb = ex2_approx(sb - m);
-        l += pa + pb;                            // this lane's rows; each row counts in four lanes
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {            // rows grp + 4 j: their p sits in lane 4 (row % 8)
-          const float pr = __shfl_sync(0xffffffffu, j < 2 ? pa : pb, ((grp + 4 * j) & 7) * 4);
-          const uint64_t p2 = pack_f32x2(pr, pr);
-          acc[0] = fma_f32x2(p2, bf16x2_to_f32x2(vr[j].x), acc[0]);
-          acc[1] = fma_f32x2(p2, bf16x2_to_f32x2(vr[j].y), acc[1]);
-          acc[2] = fma_f32x2(p2, bf16x2_to_f32x2(vr[j].z), acc[2]);
-          acc[3] = fma_f32x2(p2, bf16x2_to_f32x2(vr[j].w), acc[3]);
+          for (int j = 0; j < 4; ++j) {
+            const float pr = ex2_approx(sc[j] - m);
+            l += pr;
+            const uint64_t p2 = pack_f32x2(pr, pr);
+            acc[0] = fma_f32x2(p2, bf16x2_to_f32x2(vr[j].x), acc[0]);
+            acc[1] = fma_f32x2(p2, bf16x2_to_f32x2(vr[j].y), acc[1]);
+            acc[2] = fma_f32x2(p2, bf16x2_to_f32x2(vr[j].z), acc[2]);
+            acc[3] = fma_f32x2(p2, bf16x2_to_f32x2(vr[j].w), acc[3]);
+          }
         }
+        __syncwarp();
+        if (lane == 0 && c.ok) mbar_arrive_many(smem_u32(&c.sm->empty[c.ring.stage]), kStepWarps / kStepBlocks);
       }
-      __syncwarp();
-      if (lane == 0 && c.ok) mbar_arrive(smem_u32(&c.sm->empty[c.ring.stage]));
       c.ring.next();
     }
+    {                                            // the four groups' maxima, and their sums
+      float m_all = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+      m_all = fmaxf(m_all, __shfl_xor_sync(0xffffffffu, m_all, 16));
+      const float f = ex2_approx(m - m_all);
+      const uint64_t f2 = pack_f32x2(f, f);
+      m = m_all;
+      l *= f;
 #pragma unroll
-    for (int o = 4; o <= 16; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+      for (int e = 0; e < 4; ++e) acc[e] = mul_f32x2(acc[e], f2);
+      l += __shfl_xor_sync(0xffffffffu, l, 8);
+      l += __shfl_xor_sync(0xffffffffu, l, 16);
+    }
     float* dst = c.sm->seg[i][warp];
     if (lane == 0) { dst[0] = m; dst[1] = l; }
 #pragma unroll
