@@ -937,18 +937,30 @@ __device__ __forceinline__ bool step_stream_rows(StepSmem& sm, const StepParams&
     const StepUnit& un = sm.unit[i];
     const long long at = un.head + static_cast<long long>(un.row0) * p.c_sn + chunk * 8;
     const __nv_bfloat16 *kb = p.k_cache[layer] + at, *vb = p.v_cache[layer] + at;
+    const long long step = 4ll * kStepStreamWarps * p.c_sn, ahead = static_cast<long long>(first) * p.c_sn;
+    const __nv_bfloat16 *kr = kb + ahead, *vr = vb + ahead;      // this lane's first row of the stage
 #pragma unroll 1
     for (int r = 0; r < un.rows; r += kStepBlocks * 16) {
       if (issued >= kStepStages &&
           !step_wait(smem_u32(&sm.empty[ring.stage]), ring.parity ^ 1, sm, kWaitStepEmpty))
         return false;
       const uint32_t dst = smem_u32(sm.ring[ring.stage]) + off, bar = smem_u32(&sm.full[ring.stage]);
-      const int rows = min(kStepBlocks * 16, (un.rows - r + 15) & ~15);
-#pragma unroll 2
-      for (int j = 0; j < rows; j += 4 * kStepStreamWarps) {
-        const long long row = static_cast<long long>(min(r + j + first, un.rows - 1)) * p.c_sn;
-        cp_async_16(dst + j * 128, kb + row);
-        cp_async_16(dst + (kStepBlocks * 16 + j) * 128, vb + row);
+      if (un.rows - r >= kStepBlocks * 16) {
+#pragma unroll
+        for (int j = 0; j < kStepBlocks * 16; j += 4 * kStepStreamWarps) {
+          cp_async_16(dst + j * 128, kr);
+          cp_async_16(dst + (kStepBlocks * 16 + j) * 128, vr);
+          kr += step;
+          vr += step;
+        }
+      } else {
+        const int rows = (un.rows - r + 15) & ~15;
+#pragma unroll 1
+        for (int j = 0; j < rows; j += 4 * kStepStreamWarps) {
+          const long long row = static_cast<long long>(min(r + j + first, un.rows - 1)) * p.c_sn;
+          cp_async_16(dst + j * 128, kb + row);
+          cp_async_16(dst + (kStepBlocks * 16 + j) * 128, vb + row);
+        }
       }
       cp_async_arrive(bar);
       __syncwarp();
