@@ -41,7 +41,7 @@
 //                warp to a whole stage (shared memory is the limit for XL: the input is read again
 //                for every tile), 153 / 770 like this.
 //   attention    a (sequence, head) pair per CTA, up to two where there are more pairs than CTAs,
-//                split over several CTAs only for caches of thousands of rows.  q.K on the tensor
+//                split over several CTAs from 768 rows on.  q.K on the tensor
 //                path with the cached rows as the 16-row operand, P.V on packed fp32.  The cached
 //                rows come through the ring, ahead of the query; the new row comes through the
 //                exchange, so nobody waits for the caches.
@@ -94,8 +94,7 @@ constexpr int kStepChunkUnits = 25;                   // columns per stage: at m
 constexpr int kStepStageBytes = kStepTile * kStepChunkUnits * 64;
 constexpr int kStepStages = 8;                        // one per warp: a group of tiles has at most as many
 static_assert(kStepStages >= kStepWarps, "a wait by parity is for the slot's next stage only while the one before is not given back");
-constexpr int kStepAhead = 1;
-constexpr bool kStepAheadKv = false;
+constexpr int kStepAhead = 1;                         // operations: weights sent for to L2 in advance
 constexpr uint32_t kStepAheadBytes = 192 * 1024, kStepAheadPiece = 2048;
 constexpr int kStepMaxWidth = 1600;                   // d_model: the fragments of 8 rows fill sm.x
 constexpr int kStepMaxUnits = kStepMaxWidth / kStepUnit;
@@ -105,7 +104,10 @@ constexpr int kStepSegs = 2;                          // attention units of one 
 constexpr int kStepBlocks = 4;                        // blocks of 16 cached rows (K, then V) per stage
 static_assert(kStepBlocks == kStepWarps / 2 && kStepStages % 2 == 0, "half the warps to a stage, by the slot's parity");
 static_assert(kStepBlocks * 16 * 256 <= kStepStageBytes, "cached rows fit a stage");
-constexpr int kStepSplitRows = 384;                   // rows of a unit where pairs are split over CTAs
+// Rows of a unit where pairs are split over CTAs, from twice as many on.  Merging costs a fence and an
+// atomic per part: 1 x 900 rows, small / XL, us per step: unsplit 204 / 997, parts of 384 191 / 927, of
+// 192 191 / 956.
+constexpr int kStepSplitRows = 384;
 constexpr uint32_t kStepBarPolls = 1u << 24;          // bounds of the waits: about 65 clocks a poll of a barrier ...
 constexpr uint32_t kStepWordPolls = 1u << 21;         // ... and a trip to L2 a poll of exchange words: half a second
 
@@ -707,7 +709,7 @@ __device__ __forceinline__ StepCta step_attention(StepCta c, const StepParams& p
     // to 7 the odd ones (so a warp that waits for a slot has also waited for the slot's stage before).  A
     // row's odd-numbered neighbour has its 64-byte halves swapped (see step_stream_rows): no bank conflicts.
     // Lane group grp (of 8 lanes) sums rows grp, grp + 4, + 8, + 12 of the blocks with a maximum of its own.
-    // A GPT-2 XL unit of 900 rows, clocks: 8900 with one maximum per warp and waits for all stages, XX so.
+    // A GPT-2 XL unit of 900 rows, clocks: 8900 with one maximum per warp and waits for all stages, 7500 so.
     const int swap = (g & 1) << 2, vswap = (grp & 1) << 2;
 #pragma unroll 1
     for (int r0 = 0; r0 < un.rows; r0 += kStepBlocks * 16) {
@@ -876,19 +878,6 @@ __device__ __forceinline__ void step_ahead(const StepSmem& sm, const StepParams&
   for (uint32_t b = (sw * 32 + lane) * kStepAheadPiece; b < bytes; b += 32 * kStepStreamWarps * kStepAheadPiece)
     bulk_prefetch_l2(at + b, min(kStepAheadPiece, bytes - b));
 }
-__device__ __forceinline__ void step_ahead_rows(const StepSmem& sm, const StepParams& p, int layer, int sw, int lane) {
-#pragma unroll 1
-  for (int i = 0; i < sm.units; ++i) {
-    const StepUnit& un = sm.unit[i];
-    const long long at = un.head + static_cast<long long>(un.row0) * p.c_sn;
-#pragma unroll 1
-    for (int r = sw * 32 + lane; r < un.rows; r += 32 * kStepStreamWarps) {
-      prefetch_l2(p.k_cache[layer] + at + static_cast<long long>(r) * p.c_sn);
-      prefetch_l2(p.v_cache[layer] + at + static_cast<long long>(r) * p.c_sn);
-    }
-  }
-}
-
 // Streaming warp `sw`: its quarter of this CTA's rows of one matrix into the ring.
 __device__ __forceinline__ bool step_stream(StepSmem& sm, const StepParams& p, StepRing& ring, uint32_t& issued,
                                             const __nv_bfloat16* w, int op, int sw) {
@@ -1036,13 +1025,11 @@ __global__ void __launch_bounds__(kStepThreads, 1) fa_gpt_step_kernel(const __gr
     uint32_t issued = 0;
     bool ok = true;
     for (int i = 1; i < kStepAhead; ++i) step_ahead(sm, p, i, sw, lane);
-    if (kStepAheadKv) step_ahead_rows(sm, p, 0, sw, lane);
 #pragma unroll 1
     for (int i = 0; i <= 4 * p.n_layers && ok; ++i) {
       int op;
       const __nv_bfloat16* w = step_weight(sm, p, i, op);
       step_ahead(sm, p, i + kStepAhead, sw, lane);
-      if (kStepAheadKv && (i & 3) == kStepFc && (i >> 2) + 1 < p.n_layers) step_ahead_rows(sm, p, (i >> 2) + 1, sw, lane);
       ok = step_stream(sm, p, ring, issued, w, op, sw);
       if (ok && op == kStepQkv) ok = step_stream_rows(sm, p, ring, issued, i >> 2, sw, lane);
     }
