@@ -19,6 +19,7 @@
 // The functions are plain CPython vector calls: for the smallest problems the call IS the time, and
 // pybind11's argument casters cost about as much as the launch (a decode call through ctypes: 31-38
 // us of host time for 4-9 us of GPU work).
+#include <algorithm>
 #include <ATen/cuda/CUDAContextLight.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -514,18 +515,24 @@ PyObject* blocks(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* k
       const at::AutoDispatchBelowADInplaceOrView below_autograd;
       const c10::cuda::CUDAGuard guard(x.device());
       void* stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
-      at::Tensor branch, h = empty_like_cuda(x);
+      // Buffers for all layers.  The hidden layer lies where the projection and the attention's output lay,
+      // which are dead by then: 7 instead of 11 widths per row, so that more of a prompt stays in L2.
+      const int64_t rows = B * n;
+      int64_t wide = 4 * C;
+      for (const Layer& L : layers) wide = std::max(wide, L.t[8].size(0));
+      const at::Tensor arena = empty_cuda({rows * wide}, torch::kBFloat16, x.device());
+      at::Tensor qkv = arena.narrow(0, 0, rows * 3 * C).view({B, n, 3 * C});
+      at::Tensor ctx = arena.narrow(0, rows * 3 * C, rows * C).view({B, n, C}), mid;
+      at::Tensor branch, added = empty_like_cuda(x), h = empty_like_cuda(x);
       const at::Tensor workspace = empty_cuda({static_cast<int64_t>(kLtWorkspace)}, torch::kUInt8, x.device());
-      auto linear = [&](const at::Tensor& in, const at::Tensor& w, const at::Tensor& bias) {
-        at::Tensor y = empty_cuda({B, n, w.size(0)}, torch::kBFloat16, x.device());
-        if (lt_linear(in, w, bias.defined() ? &bias : nullptr, false, y, workspace.data_ptr(), stream)) return y;
-        return at::linear(in, w, bias.defined() ? std::optional<at::Tensor>(bias) : std::nullopt);
+      auto linear = [&](const at::Tensor& in, const at::Tensor& w, const at::Tensor& bias, at::Tensor& y) {
+        if (!lt_linear(in, w, bias.defined() ? &bias : nullptr, false, y, workspace.data_ptr(), stream))
+          y.copy_(at::linear(in, w, bias.defined() ? std::optional<at::Tensor>(bias) : std::nullopt));
       };
       for (const Layer& L : layers) {
         if (branch.defined()) add_ln(branch, &x, L.t[0], L.t[1], eps, x.data_ptr(), h, stream);
         else add_ln(x, nullptr, L.t[0], L.t[1], eps, nullptr, h, stream);
-        const at::Tensor qkv = linear(h, L.t[2], L.t[3]);
-        const at::Tensor ctx = empty_like_cuda(x);
+        linear(h, L.t[2], L.t[3], qkv);
         auto* base = static_cast<at::BFloat16*>(qkv.data_ptr());
         fa_b200_params p{};
         p.B = static_cast<int32_t>(B); p.H = static_cast<int32_t>(H); p.N = static_cast<int32_t>(n); p.d = 64;
@@ -547,12 +554,14 @@ PyObject* blocks(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* k
         }
         rc = fa_b200_fwd(&p);
         FA_CHECK(rc == 0, "custom_flash_attn.forward failed (", rc, "): ", fa_b200_strerror(rc));
-        branch = linear(ctx, L.t[4], L.t[5]);
+        branch = added;
+        linear(ctx, L.t[4], L.t[5], branch);
         add_ln(branch, &x, L.t[6], L.t[7], eps, x.data_ptr(), h, stream);
-        at::Tensor mid = empty_cuda({B, n, L.t[8].size(0)}, torch::kBFloat16, x.device());
+        const int64_t hidden = L.t[8].size(0);
+        if (!mid.defined() || mid.size(2) != hidden) mid = arena.narrow(0, 0, rows * hidden).view({B, n, hidden});
         if (!lt_linear(h, L.t[8], &L.t[9], true, mid, workspace.data_ptr(), stream))
-          mid = at::_addmm_activation(L.t[9], h.view({B * n, C}), L.t[8].t(), 1, 1, /*use_gelu=*/true).view({B, n, L.t[8].size(0)});
-        branch = linear(mid, L.t[10], L.t[11]);
+          mid.copy_(at::_addmm_activation(L.t[9], h.view({rows, C}), L.t[8].t(), 1, 1, /*use_gelu=*/true).view({B, n, hidden}));
+        linear(mid, L.t[10], L.t[11], branch);
       }
       if (last_only) {                 // what generate() consumes
         x = x.slice(1, n - 1, n).contiguous();
