@@ -58,3 +58,26 @@ def test_order_by_groups_of_heads(fa_lib):
         assert cfa.last_status() == 0 and torch.isfinite(o).all()
         for h in (0, 14, 15, 16, heads - 1):
             assert torch.equal(cfa.forward(*(t[:, h:h + 1].contiguous() for t in (q, k, v)))[0, 0], o[0, h])
+
+
+@pytest.mark.parametrize("B,N", [(32, 1024), (12, 1100)])
+def test_taking_over_while_the_first_wave_waits(fa_lib, B, N):
+    """Part of the resident slots are held by another stream's kernel, so that running CTAs take over CTAs
+    of the first wave, whose items are not those of their block index (the mirror in fa_fwd_sm100.cuh).
+    The other kernel: 128 tiles of one head, 16384 rows, one per SM, about 150 us."""
+    from tfg_flashattention_b200 import custom_flash_attn as cfa
+    g = torch.Generator(device="cuda").manual_seed(N)
+    q, k, v = (torch.randn(B, 25, N, 64, device="cuda", generator=g).bfloat16() for _ in range(3))
+    long = torch.randn(1, 1, 16384, 64, device="cuda", generator=g).bfloat16()
+    want, want_lse = cfa.forward(q, k, v, return_lse=True)
+    held, side = torch.empty_like(long), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(4):
+        o = torch.full_like(q, float("nan"))
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            cfa.forward(long, long, long, causal=False, out=held)
+        _, lse = cfa.forward(q, k, v, return_lse=True, out=o)
+        torch.cuda.synchronize()
+        assert cfa.last_status() == 0
+        assert torch.equal(o, want) and torch.equal(lse, want_lse)

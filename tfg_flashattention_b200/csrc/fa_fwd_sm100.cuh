@@ -274,11 +274,13 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     w.q_row = qt * kBlockM;
     w.ns = kCausal ? min(nkv, qt + 1) : nkv;   // K/V tiles this query tile attends to
   };
+  // The first CTAs' items are mirrored: block b < SM count has item b, the blocks after it, which join
+  // them on the SMs in the same order, have the rest of the first wave from its light end.  A block has
+  // the same item whether it starts or is taken over: where other kernels hold slots, blocks of the first
+  // wave are taken over as well.
+  auto rank_of = [&](int b) { return b >= p.mirror_from && b < p.mirror_to ? p.mirror_from + p.mirror_to - 1 - b : b; };
   auto decode_item = [&](int n, Item& w) -> bool {
-    // The first CTAs' items are mirrored: block b < SM count has item b, the blocks after it, which join
-    // them on the SMs in the same order, have the rest of the first wave from its light end.
-    const int b = blockIdx.x;
-    const int rank = b >= p.mirror_from && b < p.mirror_to ? p.mirror_from + p.mirror_to - 1 - b : b;
+    const int rank = rank_of(blockIdx.x);
     // static: back and forth through the list, so that the CTA that got the heaviest item of one
     // round gets the lightest of the next; otherwise the CTA's own item (the first of several)
     const int item = kSchedule != kStatic ? rank
@@ -438,7 +440,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         const int block = clc_block(answer);
         more = block >= 0;
         Item t{0, 0, 0, 0};
-        if (more) decode_listed(block, t);
+        if (more) decode_listed(rank_of(block), t);
         if (lane == 0) {
           sm.items[n % kItemRing] = make_int4(t.q_row, t.ns, t.h, t.b);
           mbar_arrive(smem_u32(&sm.item_full[n % kItemRing]));
