@@ -117,3 +117,46 @@ def test_step_declines_what_it_does_not_take(fa_lib):
     assert model._step(ids, caches, 32) is None                              # past the cache
     assert model._step(ids, model.allocate_kv_cache(2, 32, dtype=torch.float32), 3) is None
     assert model._step(torch.zeros(9, 1, dtype=torch.long, device="cuda"), model.allocate_kv_cache(9, 32), 3) is None
+
+
+@pytest.mark.parametrize("lose", ["to", "invalidate", "prepare"])
+def test_recorded_step_keeps_what_it_reads(fa_lib, lose):
+    """The graph holds the address of the parameter table, the table those of the weights.  (Whether they
+    are still owned is looked at before anything is replayed.)"""
+    import gc
+    model, exact = _model(256, 4, 2, 503, 64)
+    session = gpt2.GenerationSession(model, 2, 64)
+    read = [model._step_plan.table] + [w for _, w, *_ in model._step_plan.qkv]
+    addresses = [t.untyped_storage().data_ptr() for t in read]
+    del read
+    ids = torch.randint(0, 503, (2, 1), device="cuda")
+    session.position.set(0)
+    before = session.step_fn(ids).clone()
+    {"to": lambda: model.to("cuda"), "invalidate": model.invalidate_inference_cache, "prepare": model.prepare_for_inference}[lose]()
+    gc.collect()
+    torch.cuda.synchronize()
+    taken = [torch.full((n,), 7, dtype=torch.uint8, device="cuda") for n in (512, 1024, 2048, 400000) for _ in range(8)]
+    kept = {t.untyped_storage().data_ptr() for t in getattr(session.step_fn, "reads", []) if isinstance(t, torch.Tensor)}
+    assert kept.issuperset(addresses) and len(taken) == 32
+    session.position.set(0)
+    assert torch.equal(session.step_fn(ids), before)
+
+
+def test_graph_of_the_caller_keeps_the_table(fa_lib):
+    """The same for a graph that a program records around the model itself; the weights stay in place."""
+    import gc
+    model, exact = _model(256, 4, 2, 503, 64)
+    caches = model.allocate_kv_cache(2, 64)
+    ids = torch.randint(0, 503, (2, 1), device="cuda")
+    with torch.no_grad():
+        before = model(ids, kv_caches=caches, pos=5)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = model(ids, kv_caches=caches, pos=5)
+    weights, table = [w for _, w, *_ in model._step_plan.qkv], model._step_plan.table.data_ptr()
+    model.invalidate_inference_cache()
+    gc.collect()
+    assert [t.data_ptr() for t in getattr(model, "_recorded_tables", [])] == [table] and len(weights) == 2
+    out.zero_()
+    graph.replay()
+    assert torch.equal(out, before)

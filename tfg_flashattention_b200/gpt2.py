@@ -287,6 +287,7 @@ class GPTModel(nn.Module):
         self._head_w = None     # out_head weight padded to a multiple of 64 rows (inference cache)
         self._fused_blocks = False   # residual add + LayerNorm through block_ops.add_layernorm
         self._step_plan = None       # single-token steps as one kernel launch (step.StepPlan)
+        self._recorded_tables = []   # parameter tables that graphs recorded by a caller read
         self._block_params, self._block_owned = None, []    # for the binding's loop over the blocks
         if dtype is not None:
             self.to(dtype)
@@ -492,7 +493,9 @@ class GPTModel(nn.Module):
         call `position.set(prompt_len)` after the prefill has filled the caches, then `step` once
         per token.  A step is then one graph launch instead of ~15 kernel launches per layer, which
         is what bounds small-batch generation.  The warm-up steps write cache row 0 and are
-        overwritten by the prefill, so capture BEFORE running the prompt."""
+        overwritten by the prefill, so capture BEFORE running the prompt.  The recorded step keeps the
+        weights it was recorded with: values written into them are seen, a parameter that is replaced
+        or moved is not (record again)."""
         dev = self.tok_emb.weight.device
         batch = kv_caches[0][0].shape[0]
         position = DevicePosition(dev)
@@ -510,6 +513,7 @@ class GPTModel(nn.Module):
             # the one-launch step moves the position on itself
             static_logits = self._step(static_ids, kv_caches, position, advance=True, workspace=workspace)
             if static_logits is None:
+                workspace = None
                 static_logits = self(static_ids, kv_caches=kv_caches, pos=position)
                 position.advance()
 
@@ -519,6 +523,8 @@ class GPTModel(nn.Module):
             return static_logits
         step.graph = graph
         step.workspace = workspace
+        # a replay reads addresses, whatever becomes of the model: what lies there stays for as long as it can run
+        step.reads = [position, kv_caches] + ([] if workspace is None else self._step_plan.memory())
         return step, position
 
     def forward(self, in_idx, last_token_only=False, kv_caches=None, pos=0):

@@ -66,10 +66,11 @@ class StepPlan:
         except TypeError:
             return None
         plan.owned = owned
-        plan.qkv = [(blk.att, blk.att._qkv_w) for blk in model.trf_blocks]
+        plan.qkv = [(blk.att, blk.att._qkv_w, blk.att._qkv_b) for blk in model.trf_blocks]
         plan.heads, plan.layers, plan.eps = heads, layers, model.final_norm.eps
         plan.device = model.tok_emb.weight.device
         plan.table = torch.tensor(rows, dtype=torch.int64).to(plan.device)
+        plan.recorded = model._recorded_tables
         plan.ends = ends
         plan.workspaces = OrderedDict()
         return plan
@@ -86,10 +87,17 @@ class StepPlan:
         for params, name, t, address in self.owned:
             if params[name] is not t or (t is not None and t.data_ptr() != address):
                 return False
-        for att, w in self.qkv:
-            if att._qkv_w is not w:
+        for att, w, b in self.qkv:
+            if att._qkv_w is not w or att._qkv_b is not b:
                 return False
         return True
+
+    def memory(self):
+        """Everything a launch reads through this plan: the table and the tensors whose addresses are in
+        it, under names of their own (a parameter that is moved or replaced takes its storage along).  For
+        a recorded launch, which reads them for as long as it is replayed."""
+        kept = [self.table] + [t for _, _, t, _ in self.owned] + [t for _, w, b in self.qkv for t in (w, b)]
+        return [t.detach() for t in kept if t is not None]
 
     def _caches(self, kv_caches, batch):
         """The caches' addresses and common shape, or None when the kernel cannot take them."""
@@ -118,6 +126,11 @@ class StepPlan:
     def _workspace(self, batch, stream):
         """A zeroed workspace that only this stream uses (a launch leaves its counters at zero)."""
         if torch.cuda.is_current_stream_capturing():
+            # The graph is the caller's: it reads the table for as long as it is replayed, so the model keeps
+            # it (a few KB).  Weights that are replaced meanwhile are the caller's business as ever, but no
+            # address that the kernel follows becomes something else.
+            if not any(t is self.table for t in self.recorded):
+                self.recorded.append(self.table)
             return self.new_workspace(batch)     # belongs to the graph
         key = (stream, batch)
         ws = self.workspaces.get(key)
