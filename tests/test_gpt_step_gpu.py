@@ -160,3 +160,27 @@ def test_graph_of_the_caller_keeps_the_table(fa_lib):
     out.zero_()
     graph.replay()
     assert torch.equal(out, before)
+
+
+@pytest.mark.parametrize("B", [8, 9, 11])
+def test_session_of_more_sequences_than_the_kernel_takes(fa_lib, B):
+    """... is recorded layer by layer, and generates what the same sequences give in two sessions."""
+    model, _ = _model(256, 4, 2, 503, 64)
+    ids = torch.randint(0, 503, (B, 5), generator=torch.Generator().manual_seed(B)).cuda()
+    session = gpt2.GenerationSession(model, B, 64)
+    assert (session.step_fn.workspace is not None) == (B <= 8)
+    step, position, caches = session.step_fn, session.position, session.caches
+    with torch.no_grad():
+        model(ids[:, :4], kv_caches=caches, pos=0)
+        position.set(4)
+        got = step(ids[:, 4:]).float()
+        parts = []
+        for half in ids.split(4):
+            part = model.allocate_kv_cache(half.shape[0], 64)
+            model(half[:, :4], kv_caches=part, pos=0)
+            parts.append(model(half[:, 4:], kv_caches=part, pos=4).float())
+    want = torch.cat(parts)
+    # two layers at the tolerance of the file's head, each side with its own roundings
+    assert ((got - want).norm() / want.norm()).item() <= 2 * 2.0 ** -8 * math.sqrt(8 * 2 + 4)
+    out = gpt2.generate(model, ids, 4, 64, temperature=0.0, session=session)
+    assert out.shape == (B, 9) and torch.equal(out[:, :5], ids)

@@ -120,8 +120,9 @@ class StepPlan:
         return table, shape[1], stride
 
     def new_workspace(self, batch):
+        """A zeroed workspace, or None for a batch that the kernel does not take."""
         need = _lib.load().fa_b200_gpt_step_workspace_bytes(batch, self.heads)
-        return torch.zeros(need, dtype=torch.uint8, device=self.device)
+        return torch.zeros(need, dtype=torch.uint8, device=self.device) if need > 0 else None
 
     def _workspace(self, batch, stream):
         """A zeroed workspace that only this stream uses (a launch leaves its counters at zero)."""
