@@ -58,3 +58,71 @@ def test_native_loop_steps_aside(fa_lib, torch_binding):
         changed = model(ids)
         model._native_blocks = lambda *a: None
         assert not torch.equal(changed, before) and torch.equal(model(ids), changed)
+
+
+@pytest.mark.parametrize("change", ["out_proj", "second mlp layer", "adapter", "head", "final norm", "fewer blocks",
+                                    "other order", "impl_type", "moved"])
+def test_replaced_modules_are_used(fa_lib, torch_binding, change):
+    """Prompts and single-token steps of a model whose modules were replaced after it was prepared, against a
+    model of the same modules that is prepared then."""
+    import copy
+    import torch.nn as nn
+    bf = dict(dtype=torch.bfloat16, device="cuda")
+
+    class Adapter(nn.Linear):
+        def forward(self, x):
+            return super().forward(x) + 0.25 * x
+
+    def apply(m):
+        torch.manual_seed(11)
+        blk = m.trf_blocks[1]
+        if change == "out_proj":
+            blk.att.out_proj = nn.Linear(256, 256, **bf)
+        elif change == "second mlp layer":
+            blk.ff.layers[2] = nn.Linear(1024, 256, **bf)
+        elif change == "adapter":
+            new = Adapter(256, 256, **bf)
+            new.load_state_dict(blk.att.out_proj.state_dict())
+            blk.att.out_proj = new
+        elif change == "head":
+            m.out_head = nn.Linear(256, 503, bias=False, **bf)
+        elif change == "final norm":
+            m.final_norm = gpt2.LayerNorm(m.cfg).cuda().bfloat16()
+            with torch.no_grad():
+                m.final_norm.shift.fill_(0.5)
+        elif change == "fewer blocks":
+            m.trf_blocks = m.trf_blocks[:2]
+        elif change == "other order":
+            m.trf_blocks = nn.Sequential(*reversed(m.trf_blocks))
+        elif change == "impl_type":
+            blk.att.impl_type = "manual"
+        else:
+            m.to("cuda")
+
+    model, fresh = _model(), _model()
+    caches = model.allocate_kv_cache(2, 32)
+    ids = torch.randint(0, 503, (2, 20), device="cuda")
+    with torch.no_grad():
+        model(ids[:, :19], kv_caches=caches, pos=0)
+        old = model(ids[:, 19:], kv_caches=caches, pos=19)
+    apply(model)
+    apply(fresh)
+    fresh.prepare_for_inference()
+    model._head_w = fresh._head_w                        # the padded copy for long prompts is prepare's own
+    # as the modules themselves have it: no path past them
+    fresh._native_blocks = lambda *a: None
+    fresh._step = lambda *a, **k: None
+    with torch.no_grad():
+        got_caches, want_caches = model.allocate_kv_cache(2, 32), model.allocate_kv_cache(2, 32)
+        got = model(ids[:, :19], kv_caches=got_caches, pos=0)
+        want = fresh(ids[:, :19], kv_caches=want_caches, pos=0)
+        assert torch.equal(got, want)
+        got = model(ids[:, 19:], kv_caches=got_caches, pos=19).float()
+        want = fresh(ids[:, 19:], kv_caches=want_caches, pos=19).float()
+    # three layers of the one-launch step's and the modules' own roundings, see test_gpt_step_gpu.py
+    assert ((got - want).norm() / want.norm()).item() <= 2 * 2.0 ** -8 * (8 * 3 + 4) ** 0.5
+    if change == "moved":
+        assert torch.equal(got, old.float()) and model._step_plan is not None and model._native_blocks(
+            torch.zeros(2, 3, 256, **bf), None, 0) is None    # (gradients on)
+    elif change != "impl_type":
+        assert not torch.equal(got, old.float())

@@ -46,7 +46,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .step import StepPlan
+from .step import PLAIN_TENSORS, ModelWatch, StepPlan, plain_modules
 
 GPT2_SIZES = {   # model_inference.py:392-397
     "gpt2-small": {"emb_dim": 768, "n_layers": 12, "n_heads": 12},
@@ -286,9 +286,8 @@ class GPTModel(nn.Module):
         self.out_head = nn.Linear(cfg["emb_dim"], cfg["vocab_size"], bias=False)
         self._head_w = None     # out_head weight padded to a multiple of 64 rows (inference cache)
         self._fused_blocks = False   # residual add + LayerNorm through block_ops.add_layernorm
-        self._step_plan = None       # single-token steps as one kernel launch (step.StepPlan)
+        self._made = {}              # what the paths past the modules are made from, see _from_modules
         self._recorded_tables = []   # parameter tables that graphs recorded by a caller read
-        self._block_params, self._block_owned = None, []    # for the binding's loop over the blocks
         if dtype is not None:
             self.to(dtype)
 
@@ -308,10 +307,9 @@ class GPTModel(nn.Module):
                               and d % 8 == 0 and d <= 2048 and self.cfg["drop_rate"] == 0.0)
         for blk in self.trf_blocks:      # single-token steps: Linear layers as one pass over the weights
             blk.att.small_linear = blk.ff.small_linear = self._fused_blocks
-        self._step_plan = StepPlan.make(self) if self._fused_blocks else None
-        self._block_params, self._block_owned = None, []
+        self._made = {}
         if self._fused_blocks:
-            self._list_block_params()
+            self._step_plan, self._block_rows
         return self
 
     def invalidate_inference_cache(self):
@@ -321,26 +319,43 @@ class GPTModel(nn.Module):
             blk.att.small_linear = blk.ff.small_linear = False
         self._head_w = None
         self._fused_blocks = False
-        self._step_plan = None
-        self._block_params, self._block_owned = None, []
+        self._made = {}
         return self
 
     def _apply(self, fn, *args, **kwargs):      # .to(), .cuda(), .half(): the parameters move
-        self._step_plan = None
-        self._block_params, self._block_owned = None, []
+        self._made = {}
         return super()._apply(fn, *args, **kwargs)
+
+    def _from_modules(self, name, make):
+        """`make(self)`, kept for as long as the model consists of the modules, parameters and settings that it
+        was made from (None, too: a model with an adapter in it goes through its modules until that is
+        taken out again)."""
+        made = self.__dict__.setdefault("_made", {})
+        kept = made.get(name)
+        if kept is None or not kept[0].holds():
+            if torch.cuda.is_available() and torch.cuda.is_current_stream_capturing():
+                return None                     # making copies to the GPU: not while a graph is recorded
+            watch = ModelWatch(self)            # first: what changes meanwhile is seen at the next call
+            kept = made[name] = (watch, make(self))
+        return kept[1]
+
+    @property
+    def _step_plan(self):
+        """Single-token steps as one kernel launch (step.StepPlan), or None."""
+        return self._from_modules("step", StepPlan.make) if self._fused_blocks else None
+
+    @property
+    def _block_rows(self):
+        """The blocks' parameters for the binding's loop over the blocks, or None."""
+        return self._from_modules("blocks", GPTModel._list_block_rows) if self._fused_blocks else None
 
     def _step(self, in_idx, kv_caches, pos, **kw):
         """Logits of a single-token step through the one-launch kernel, or None when this model, batch
         or cache is not one for it."""
-        plan = self._step_plan
-        if plan is None or self.training or kv_caches is None or not in_idx.is_cuda:
+        if self.training or kv_caches is None or not in_idx.is_cuda:
             return None
-        if not plan.current():                  # a parameter was replaced
-            plan = self._step_plan = StepPlan.make(self)
-            if plan is None:
-                return None
-        return plan.step(in_idx, kv_caches, pos, **kw)
+        plan = self._step_plan
+        return None if plan is None else plan.step(in_idx, kv_caches, pos, **kw)
 
     def allocate_kv_cache(self, batch, max_len=None, dtype=None):
         """One (K, V) pair of [B, N_max, H, d] tensors per layer, in the model's device; bf16 when
@@ -356,8 +371,8 @@ class GPTModel(nn.Module):
         return list(zip(kv[::2], kv[1::2]))
 
     def _native_blocks(self, x, kv_caches, pos):
-        """The binding's loop over the blocks when this call is one for it (a prompt or whole sequences,
-        no gradients, no hooks, every parameter the bf16 one it expects), else None."""
+        """The binding's loop over the blocks and its parameters when this call is one for it (a prompt or whole
+        sequences, no gradients, no hooks, every parameter the bf16 one it expects), else None."""
         from . import custom_flash_attn
         ext = custom_flash_attn.extension()
         if (ext is None or torch.is_grad_enabled() or torch.is_autocast_enabled() or not isinstance(pos, int) or pos != 0
@@ -366,49 +381,46 @@ class GPTModel(nn.Module):
         width, heads = self.cfg["emb_dim"], self.cfg["n_heads"]
         if width != 64 * heads:
             return None
-        for params, name, t in self._block_owned:
-            if params[name] is not t:                       # replaced since the list was made
-                self._list_block_params()
-                break
-        if self._block_params is None:
+        rows = self._block_rows
+        if rows is None:
             return None
-        for blk, row in zip(self.trf_blocks, self._block_params):
+        for blk in self.trf_blocks:
             att, ff = blk.att, blk.ff
-            if (att._forward_hooks or att._forward_pre_hooks or ff._forward_hooks or ff._forward_pre_hooks
-                    or att.impl_type != "cuda" or att._qkv_w is not row[2]):
+            if att._forward_hooks or att._forward_pre_hooks or ff._forward_hooks or ff._forward_pre_hooks:
                 return None
         if kv_caches is not None:
-            if not isinstance(kv_caches, list) or len(kv_caches) != len(self._block_params):
+            if not isinstance(kv_caches, list) or len(kv_caches) != len(rows):
                 return None
             for pair in kv_caches:
                 k, v = pair
                 if (type(pair) is not tuple or k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16
                         or k.shape != v.shape or k.stride() != v.stride() or not k.is_cuda):
                     return None
-        return ext.blocks
+        return ext.blocks, rows
 
-    def _list_block_params(self):
-        """The blocks' parameters in the order the native loop takes them, and where they came from."""
-        self._block_owned, self._block_params = [], []
+    def _list_block_rows(self):
+        """The blocks' parameters in the order the native loop takes them, or None for a model it does not take."""
+        if not plain_modules(self):
+            return None
+        width, rows = self.cfg["emb_dim"], []
         for blk in self.trf_blocks:
-            row = []
-            for module, name in ((blk.norm1, "scale"), (blk.norm1, "shift"), (None, None), (None, None),
-                                 (blk.att.out_proj, "weight"), (blk.att.out_proj, "bias"),
-                                 (blk.norm2, "scale"), (blk.norm2, "shift"),
-                                 (blk.ff.layers[0], "weight"), (blk.ff.layers[0], "bias"),
-                                 (blk.ff.layers[2], "weight"), (blk.ff.layers[2], "bias")):
-                if module is None:
-                    row.append((blk.att._qkv_w, blk.att._qkv_b)[len(row) - 2])
+            att = blk.att
+            n1, n2, proj, fc, out = (m._parameters.get for m in (blk.norm1, blk.norm2, att.out_proj, blk.ff.layers[0], blk.ff.layers[2]))
+            row = (n1("scale"), n1("shift"), att._qkv_w, att._qkv_b, proj("weight"), proj("bias"),
+                   n2("scale"), n2("shift"), fc("weight"), fc("bias"), out("weight"), out("bias"))
+            hidden = 0 if row[8] is None else row[8].shape[0]
+            shapes = ((width,), (width,), (3 * width, width), (3 * width,), (width, width), (width,),
+                      (width,), (width,), (hidden, width), (hidden,), (width, hidden), (width,))
+            for i, (t, shape) in enumerate(zip(row, shapes)):
+                if t is None and i == 3:
                     continue
-                t = module._parameters[name]
-                self._block_owned.append((module._parameters, name, t))
-                row.append(t)
-            if (any(t is None or t.dtype != torch.bfloat16 or not t.is_cuda for i, t in enumerate(row) if i != 3)
-                    or any(not row[i].is_contiguous() for i in (0, 1, 6, 7))
-                    or any(m.eps != self.final_norm.eps for m in (blk.norm1, blk.norm2))):
-                self._block_params = None
-                return
-            self._block_params.append(tuple(row))
+                if (type(t) not in PLAIN_TENSORS or t.dtype != torch.bfloat16 or t.device != self.tok_emb.weight.device
+                        or tuple(t.shape) != shape):
+                    return None
+            if any(not row[i].is_contiguous() for i in (0, 1, 6, 7)):
+                return None
+            rows.append(row)
+        return rows
 
     def _blocks_fused(self, x, kv_caches, pos, last_token_only):
         """The block stack and the final norm with every shortcut addition folded into the
@@ -418,8 +430,9 @@ class GPTModel(nn.Module):
         from .block_ops import add_layernorm
         native = self._native_blocks(x, kv_caches, pos)
         if native is not None:
-            return native(x, self._block_params, kv_caches, self.cfg["n_heads"], self.final_norm.eps,
-                          self.final_norm.scale, self.final_norm.shift, last_token_only)
+            loop, rows = native
+            return loop(x, rows, kv_caches, self.cfg["n_heads"], self.final_norm.eps,
+                        self.final_norm.scale, self.final_norm.shift, last_token_only)
         branch = None
         for i, blk in enumerate(self.trf_blocks):
             cache = None if kv_caches is None else kv_caches[i]
@@ -506,7 +519,8 @@ class GPTModel(nn.Module):
             for _ in range(warmup):
                 self(static_ids, kv_caches=kv_caches, pos=position)
         torch.cuda.current_stream(dev).wait_stream(side)
-        workspace = None if self._step_plan is None else self._step_plan.new_workspace(batch)
+        plan = self._step_plan
+        workspace = None if plan is None else plan.new_workspace(batch)
         torch.cuda.current_stream(dev).synchronize()
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
@@ -524,12 +538,12 @@ class GPTModel(nn.Module):
         step.graph = graph
         step.workspace = workspace
         # a replay reads addresses, whatever becomes of the model: what lies there stays for as long as it can run
-        step.reads = [position, kv_caches] + ([] if workspace is None else self._step_plan.memory())
+        step.reads = [position, kv_caches] + ([] if workspace is None else plan.memory())
         return step, position
 
     def forward(self, in_idx, last_token_only=False, kv_caches=None, pos=0):
         _, n = in_idx.shape
-        if n == 1 and self._step_plan is not None:
+        if n == 1 and self._fused_blocks:
             logits = self._step(in_idx, kv_caches, pos)
             if logits is not None:
                 return logits

@@ -8,9 +8,11 @@ go layer by layer.
 from __future__ import annotations
 
 import ctypes
+import operator
 from collections import OrderedDict
 
 import torch
+import torch.nn as nn
 
 from . import _lib
 
@@ -18,7 +20,68 @@ MAX_BATCH = 8
 MAX_PAIRS = 256            # sequences x heads
 MAX_LAYERS = 64
 MAX_WIDTH = 1600
+PLAIN_TENSORS = (torch.Tensor, nn.Parameter)     # a subclass may keep its numbers in another form
 MAX_WORKSPACES = 8         # streams that keep a workspace (about 1 MB each)
+
+
+class ModelWatch:
+    """The modules, parameters and settings of a GPTModel that the paths past its modules stand in for (the
+    one-launch step here, the binding's loop over the blocks of a prompt), as they are when this is made.
+    `holds()` says whether the model still consists of the same ones; it runs on every call, so it is
+    a comparison of identities without a loop in Python (37 entries a block: 17 us for GPT-2 small)."""
+
+    UNREAD = ("W_query", "W_key", "W_value", "dropout", "drop_shortcut")    # replaced by _qkv_w / identities
+
+    def __init__(self, model):
+        entries = []                   # (dict, key, value): parameters, submodules, plain attributes
+        tensors = []
+        todo = [model]
+        while todo:
+            m = todo.pop()
+            d = m.__dict__
+            for name, t in m._parameters.items():
+                entries.append((m._parameters, name, t))
+                if t is not None:
+                    tensors.append(t)
+            for name, child in m._modules.items():
+                if name not in self.UNREAD:
+                    entries.append((m._modules, name, child))
+                    if child is not None:
+                        todo.append(child)
+            entries += [(d, name, d[name]) for name in ("impl_type", "num_heads", "d_out", "eps", "_qkv_w", "_qkv_b") if name in d]
+        self.dicts, self.keys, self.values = (list(part) for part in zip(*entries))
+        self.tensors, self.addresses = tensors, [t.data_ptr() for t in tensors]
+        self.blocks = model.trf_blocks._modules
+        self.n_blocks = len(self.blocks)
+
+    def holds(self):
+        return (all(map(operator.is_, map(dict.get, self.dicts, self.keys), self.values))
+                and len(self.blocks) == self.n_blocks
+                and list(map(torch.Tensor.data_ptr, self.tensors)) == self.addresses)
+
+
+def plain_modules(model):
+    """Whether the model is built of the modules that those paths know, one head size and width throughout."""
+    from . import gpt2
+    cfg = model.cfg
+    width, heads = cfg["emb_dim"], cfg["n_heads"]
+    if type(model.final_norm) is not gpt2.LayerNorm or type(model.out_head) is not nn.Linear:
+        return False
+    if type(model.tok_emb) is not nn.Embedding or type(model.pos_emb) is not nn.Embedding:
+        return False
+    for blk in model.trf_blocks:
+        if type(blk) is not gpt2.TransformerBlock or type(blk.att) is not gpt2.MultiHeadAttention or type(blk.ff) is not gpt2.FeedForward:
+            return False
+        att, layers = blk.att, blk.ff.layers
+        if type(blk.norm1) is not gpt2.LayerNorm or type(blk.norm2) is not gpt2.LayerNorm or type(layers) is not nn.Sequential:
+            return False
+        if type(att.out_proj) is not nn.Linear or type(layers[0]) is not nn.Linear or type(layers[2]) is not nn.Linear:
+            return False
+        if att.num_heads != heads or att.d_out != width or att.impl_type != "cuda" or att._qkv_w is None:
+            return False
+        if blk.norm1.eps != model.final_norm.eps or blk.norm2.eps != model.final_norm.eps:
+            return False
+    return True
 
 
 class StepPlan:
@@ -28,76 +91,58 @@ class StepPlan:
     @classmethod
     def make(cls, model):
         cfg = model.cfg
-        width, heads, layers = cfg["emb_dim"], cfg["n_heads"], cfg["n_layers"]
+        width, heads, layers = cfg["emb_dim"], cfg["n_heads"], len(model.trf_blocks)
         if width != 64 * heads or width > MAX_WIDTH or not 1 <= layers <= MAX_LAYERS or heads > MAX_PAIRS:
             return None
+        if not plain_modules(model):
+            return None
         plan = cls()
-        owned = []           # (module's parameter dict, name, tensor, address): what the table was built from
+        plan.device = model.tok_emb.weight.device
+        plan.weights = []    # what the table points at
         rows = []
 
         def take(module, name, shape, optional=False):
-            t = module._parameters[name]
-            owned.append((module._parameters, name, t, 0 if t is None else t.data_ptr()))
-            if t is None:
-                if not optional:
-                    raise TypeError(name)
-                return 0
-            return plan._address(t, shape)
+            return plan._take(module._parameters.get(name), shape, optional)
 
         try:
             for blk in model.trf_blocks:
                 att, fc, out = blk.att, blk.ff.layers[0], blk.ff.layers[2]
-                row = [take(blk.norm1, "scale", (width,)), take(blk.norm1, "shift", (width,)),
-                       plan._address(att._qkv_w, (3 * width, width)),
-                       0 if att._qkv_b is None else plan._address(att._qkv_b, (3 * width,)),
-                       take(att.out_proj, "weight", (width, width)), take(att.out_proj, "bias", (width,)),
-                       take(blk.norm2, "scale", (width,)), take(blk.norm2, "shift", (width,)),
-                       take(fc, "weight", (4 * width, width)), take(fc, "bias", (4 * width,)),
-                       take(out, "weight", (width, 4 * width)), take(out, "bias", (width,))]
-                if blk.norm1.eps != model.final_norm.eps or blk.norm2.eps != model.final_norm.eps:
-                    return None
-                rows.append(row)
+                rows.append([take(blk.norm1, "scale", (width,)), take(blk.norm1, "shift", (width,)),
+                             plan._take(att._qkv_w, (3 * width, width)), plan._take(att._qkv_b, (3 * width,), optional=True),
+                             take(att.out_proj, "weight", (width, width)), take(att.out_proj, "bias", (width,)),
+                             take(blk.norm2, "scale", (width,)), take(blk.norm2, "shift", (width,)),
+                             take(fc, "weight", (4 * width, width)), take(fc, "bias", (4 * width,)),
+                             take(out, "weight", (width, 4 * width)), take(out, "bias", (width,))])
             plan.vocab = model.out_head.weight.shape[0]
             plan.positions = model.pos_emb.weight.shape[0]
-            ends = [take(model.tok_emb, "weight", (plan.vocab, width)),
-                    take(model.pos_emb, "weight", (plan.positions, width)),
-                    take(model.final_norm, "scale", (width,)), take(model.final_norm, "shift", (width,)),
-                    take(model.out_head, "weight", (plan.vocab, width))]
+            plan.ends = [take(model.tok_emb, "weight", (plan.vocab, width)),
+                         take(model.pos_emb, "weight", (plan.positions, width)),
+                         take(model.final_norm, "scale", (width,)), take(model.final_norm, "shift", (width,)),
+                         take(model.out_head, "weight", (plan.vocab, width))]
         except TypeError:
             return None
-        plan.owned = owned
         plan.qkv = [(blk.att, blk.att._qkv_w, blk.att._qkv_b) for blk in model.trf_blocks]
         plan.heads, plan.layers, plan.eps = heads, layers, model.final_norm.eps
-        plan.device = model.tok_emb.weight.device
         plan.table = torch.tensor(rows, dtype=torch.int64).to(plan.device)
-        plan.recorded = model._recorded_tables
-        plan.ends = ends
+        plan.recorded = model.__dict__.setdefault("_recorded_tables", [])
         plan.workspaces = OrderedDict()
         return plan
 
-    @staticmethod
-    def _address(t, shape):
-        if (not t.is_cuda or t.dtype != torch.bfloat16 or tuple(t.shape) != shape or not t.is_contiguous()
-                or t.data_ptr() % 16):
+    def _take(self, t, shape, optional=False):
+        """The address of a parameter of this shape (0 for one that is not there and need not be)."""
+        if t is None and optional:
+            return 0
+        if (type(t) not in PLAIN_TENSORS or not t.is_cuda or t.device != self.device or t.dtype != torch.bfloat16 or tuple(t.shape) != shape
+                or not t.is_contiguous() or t.data_ptr() % 16):
             raise TypeError("not a dense bf16 CUDA parameter of the expected shape")
+        self.weights.append(t)
         return t.data_ptr()
-
-    def current(self):
-        """False when a parameter, or its storage, has been replaced since the table was built."""
-        for params, name, t, address in self.owned:
-            if params[name] is not t or (t is not None and t.data_ptr() != address):
-                return False
-        for att, w, b in self.qkv:
-            if att._qkv_w is not w or att._qkv_b is not b:
-                return False
-        return True
 
     def memory(self):
         """Everything a launch reads through this plan: the table and the tensors whose addresses are in
         it, under names of their own (a parameter that is moved or replaced takes its storage along).  For
         a recorded launch, which reads them for as long as it is replayed."""
-        kept = [self.table] + [t for _, _, t, _ in self.owned] + [t for _, w, b in self.qkv for t in (w, b)]
-        return [t.detach() for t in kept if t is not None]
+        return [t.detach() for t in [self.table] + self.weights]
 
     def _caches(self, kv_caches, batch):
         """The caches' addresses and common shape, or None when the kernel cannot take them."""
