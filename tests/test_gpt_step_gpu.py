@@ -184,3 +184,42 @@ def test_session_of_more_sequences_than_the_kernel_takes(fa_lib, B):
     assert ((got - want).norm() / want.norm()).item() <= 2 * 2.0 ** -8 * math.sqrt(8 * 2 + 4)
     out = gpt2.generate(model, ids, 4, 64, temperature=0.0, session=session)
     assert out.shape == (B, 9) and torch.equal(out[:, :5], ids)
+
+
+@pytest.mark.parametrize("B", [1, 2])
+@pytest.mark.parametrize("where", ["tok_emb", "att", "ff", "out_proj", "layers.2", "forward", "autocast"])
+def test_step_leaves_calls_to_the_modules(fa_lib, where, B):
+    """Hooks and a module's own forward are called as often as the layer-by-layer loop calls them, in steps and
+    in prompts; under autocast nothing goes past the modules."""
+    model, _ = _model(256, 4, 2, 503, 64)
+    blk = model.trf_blocks[1]
+    module = {"tok_emb": model.tok_emb, "att": blk.att, "ff": blk.ff, "out_proj": blk.att.out_proj,
+              "layers.2": blk.ff.layers[2], "forward": blk.att, "autocast": blk.att}[where]
+    ids = torch.randint(0, 503, (B, 6), device="cuda")
+
+    def run():
+        seen = []
+        caches = model.allocate_kv_cache(B, 32)
+        if where == "forward":
+            inner = type(module).forward
+            module.forward = lambda *a, **k: (seen.append(1), inner(module, *a, **k))[1]
+        elif where != "autocast":
+            handle = module.register_forward_hook(lambda *a: seen.append(1))
+        with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16, enabled=where == "autocast"):
+            model(ids[:, :5], kv_caches=caches, pos=0)
+            prompt = len(seen)
+            taken = model._step(ids[:, 5:], caches, 5)
+            out = model(ids[:, 5:], kv_caches=caches, pos=5).float()
+        if where == "forward":
+            del module.forward
+        elif where != "autocast":
+            handle.remove()
+        return prompt, len(seen) - prompt, taken, out
+
+    prompt, step, taken, out = run()
+    assert taken is None
+    model._native_blocks, model._step = lambda *a: None, lambda *a, **k: None
+    want = run()
+    assert (prompt, step) == want[:2] and torch.equal(out, want[3])
+    del model._native_blocks, model._step
+    assert model._step(ids[:, 5:], model.allocate_kv_cache(B, 32), 5) is not None

@@ -78,3 +78,18 @@ def test_modules_of_other_kinds():
         model = _model()
         change(model)
         assert not plain_modules(model)
+
+
+@pytest.mark.parametrize("pick", [lambda m: m.tok_emb, lambda m: m.trf_blocks[0].att, lambda m: m.trf_blocks[2].ff,
+                                  lambda m: m.trf_blocks[1].att.out_proj, lambda m: m.trf_blocks[1].ff.layers[2]])
+def test_calls_that_somebody_waits_for(pick):
+    model = _model()
+    watch = ModelWatch(model)
+    for register in (pick(model).register_forward_hook, pick(model).register_forward_pre_hook,
+                     nn.modules.module.register_module_forward_hook):
+        assert not watch.hooked()
+        handle = register(lambda *a: None)
+        assert watch.hooked() and watch.holds()
+        handle.remove()
+    pick(model).forward = lambda *a, **k: None           # of this module alone
+    assert not watch.holds() and not plain_modules(model)

@@ -329,7 +329,7 @@ class GPTModel(nn.Module):
     def _from_modules(self, name, make):
         """`make(self)`, kept for as long as the model consists of the modules, parameters and settings that it
         was made from (None, too: a model with an adapter in it goes through its modules until that is
-        taken out again)."""
+        taken out again).  None as well while there are hooks on modules that would not be called."""
         made = self.__dict__.setdefault("_made", {})
         kept = made.get(name)
         if kept is None or not kept[0].holds():
@@ -337,7 +337,7 @@ class GPTModel(nn.Module):
                 return None                     # making copies to the GPU: not while a graph is recorded
             watch = ModelWatch(self)            # first: what changes meanwhile is seen at the next call
             kept = made[name] = (watch, make(self))
-        return kept[1]
+        return None if kept[0].hooked() else kept[1]
 
     @property
     def _step_plan(self):
@@ -352,7 +352,7 @@ class GPTModel(nn.Module):
     def _step(self, in_idx, kv_caches, pos, **kw):
         """Logits of a single-token step through the one-launch kernel, or None when this model, batch
         or cache is not one for it."""
-        if self.training or kv_caches is None or not in_idx.is_cuda:
+        if self.training or kv_caches is None or not in_idx.is_cuda or torch.is_autocast_enabled():
             return None
         plan = self._step_plan
         return None if plan is None else plan.step(in_idx, kv_caches, pos, **kw)
@@ -384,10 +384,6 @@ class GPTModel(nn.Module):
         rows = self._block_rows
         if rows is None:
             return None
-        for blk in self.trf_blocks:
-            att, ff = blk.att, blk.ff
-            if att._forward_hooks or att._forward_pre_hooks or ff._forward_hooks or ff._forward_pre_hooks:
-                return None
         if kv_caches is not None:
             if not isinstance(kv_caches, list) or len(kv_caches) != len(rows):
                 return None

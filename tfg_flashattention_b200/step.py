@@ -49,15 +49,33 @@ class ModelWatch:
                     if child is not None:
                         todo.append(child)
             entries += [(d, name, d[name]) for name in ("impl_type", "num_heads", "d_out", "eps", "_qkv_w", "_qkv_b") if name in d]
+        called = called_modules(model)
+        entries += [(m.__dict__, "forward", m.__dict__.get("forward")) for m in called]
+        self.hooks = [d for m in called for d in (m._forward_hooks, m._forward_pre_hooks)]
+        self.hooks += [nn.modules.module._global_forward_hooks, nn.modules.module._global_forward_pre_hooks]
         self.dicts, self.keys, self.values = (list(part) for part in zip(*entries))
         self.tensors, self.addresses = tensors, [t.data_ptr() for t in tensors]
         self.blocks = model.trf_blocks._modules
         self.n_blocks = len(self.blocks)
 
+    def hooked(self):
+        """Whether somebody wants to hear of a call that those paths do not make."""
+        return any(self.hooks)
+
     def holds(self):
         return (all(map(operator.is_, map(dict.get, self.dicts, self.keys), self.values))
                 and len(self.blocks) == self.n_blocks
                 and list(map(torch.Tensor.data_ptr, self.tensors)) == self.addresses)
+
+
+def called_modules(model):
+    """The modules that the prepared model's own loops call (of the others they read the parameters)."""
+    called = [model.tok_emb, model.pos_emb, model.drop_emb]
+    for blk in model.trf_blocks:
+        att, ff = getattr(blk, "att", None), getattr(blk, "ff", None)
+        layers = getattr(ff, "layers", None)
+        called += [att, ff, getattr(att, "out_proj", None), layers[2] if isinstance(layers, nn.Sequential) and len(layers) > 2 else None]
+    return [m for m in called if isinstance(m, nn.Module)]
 
 
 def plain_modules(model):
@@ -81,7 +99,7 @@ def plain_modules(model):
             return False
         if blk.norm1.eps != model.final_norm.eps or blk.norm2.eps != model.final_norm.eps:
             return False
-    return True
+    return not any("forward" in m.__dict__ for m in called_modules(model))
 
 
 class StepPlan:
