@@ -223,3 +223,22 @@ def test_step_leaves_calls_to_the_modules(fa_lib, where, B):
     assert (prompt, step) == want[:2] and torch.equal(out, want[3])
     del model._native_blocks, model._step
     assert model._step(ids[:, 5:], model.allocate_kv_cache(B, 32), 5) is not None
+
+
+@pytest.mark.parametrize("new", [1, 4])
+def test_session_goes_on_behind_what_was_generated(fa_lib, new):
+    """generate() leaves the session's position behind its last step, greedy or sampled, so that the recorded
+    step can go on."""
+    model, _ = _model(256, 4, 2, 503, 64)
+    ids = torch.randint(0, 503, (2, 7), device="cuda")
+    for temperature in (0.0, 1.0):
+        session = gpt2.GenerationSession(model, 2, 64)
+        out = gpt2.generate(model, ids, new, 64, temperature=temperature, session=session)
+        assert session.position.index.item() == 7 + new - 1 and session.position.length.item() == 7 + new
+        got = session.step_fn(out[:, -1:]).clone()
+        caches = model.allocate_kv_cache(2, 64)
+        with torch.no_grad():
+            model(out[:, :7], kv_caches=caches, pos=0)
+            for t in range(7, 7 + new):
+                want = model(out[:, t:t + 1], kv_caches=caches, pos=t)
+        assert torch.equal(got, want)

@@ -657,6 +657,8 @@ def generate(model, idx, max_new_tokens, context_size, temperature=1.0, top_k=No
         idx = torch.cat((idx, idx_next), dim=1)
         if greedy is not None:
             greedy[:, :idx.shape[1]] = idx
+    if greedy is not None and position is not None:
+        position.set(pos)                      # where the recorded step would have left it
     return idx.contiguous()
 
 
