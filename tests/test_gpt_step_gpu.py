@@ -242,3 +242,24 @@ def test_session_goes_on_behind_what_was_generated(fa_lib, new):
             for t in range(7, 7 + new):
                 want = model(out[:, t:t + 1], kv_caches=caches, pos=t)
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("how", ["hook", "pre-hook", "forward", "subclass"])
+def test_generate_calls_the_model_where_somebody_waits_for_it(fa_lib, how):
+    model, _ = _model(256, 4, 2, 503, 64)
+    ids = torch.randint(0, 503, (2, 7), device="cuda")
+    want = gpt2.generate(model, ids, 5, 64, temperature=0.0)
+    seen = []
+    if how == "hook":
+        model.register_forward_hook(lambda *a: seen.append(1))
+    elif how == "pre-hook":
+        model.register_forward_pre_hook(lambda *a: seen.append(1))
+    elif how == "forward":
+        model.forward = lambda *a, **k: (seen.append(1), gpt2.GPTModel.forward(model, *a, **k))[1]
+    else:
+        class Model(gpt2.GPTModel):
+            def forward(self, *a, **k):
+                seen.append(1)
+                return super().forward(*a, **k)
+        model.__class__ = Model
+    assert torch.equal(gpt2.generate(model, ids, 5, 64, temperature=0.0), want) and len(seen) == 5

@@ -614,7 +614,9 @@ def generate(model, idx, max_new_tokens, context_size, temperature=1.0, top_k=No
             if cuda_graph:
                 step_fn, position = model.capture_decode_step(caches)
     greedy = None         # [B, prompt + new] ids that the one-launch step extends by itself
-    if use_cache and temperature <= 0.0 and max_new_tokens > 1 and isinstance(model, GPTModel) and model._step_plan is not None:
+    if (use_cache and temperature <= 0.0 and max_new_tokens > 1 and isinstance(model, GPTModel) and model._step_plan is not None
+            and type(model).forward is GPTModel.forward and "forward" not in model.__dict__
+            and not (model._forward_hooks or model._forward_pre_hooks)):       # nobody waits for the model's call
         greedy = torch.empty(idx.shape[0], idx.shape[1] + max_new_tokens, dtype=torch.long, device=idx.device)
     for step in range(max_new_tokens):
         if greedy is not None and step > 0:
