@@ -263,3 +263,15 @@ def test_generate_calls_the_model_where_somebody_waits_for_it(fa_lib, how):
                 return super().forward(*a, **k)
         model.__class__ = Model
     assert torch.equal(gpt2.generate(model, ids, 5, 64, temperature=0.0), want) and len(seen) == 5
+
+
+def test_positions_of_other_integer_types(fa_lib):
+    import numpy as np
+    model, _ = _model(256, 4, 2, 503, 64)
+    ids = torch.randint(0, 503, (2, 7), device="cuda")
+    caches = model.allocate_kv_cache(2, 32)
+    with torch.no_grad():
+        model(ids[:, :6], kv_caches=caches, pos=np.int64(0))
+        want = model(ids[:, 6:], kv_caches=caches, pos=6)
+        for kind in (np.int64, np.int32, np.uint8):
+            assert torch.equal(model(ids[:, 6:], kv_caches=caches, pos=kind(6)), want)

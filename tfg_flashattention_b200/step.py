@@ -215,9 +215,13 @@ class StepPlan:
         if found is None:
             return None
         table, rows, stride = found
-        on_device = not isinstance(pos, int)
-        if not on_device and not 0 <= pos < min(rows, self.positions):
-            return None
+        on_device = hasattr(pos, "index") and hasattr(pos, "length")
+        if not on_device:
+            if isinstance(pos, torch.Tensor) or not hasattr(pos, "__index__"):
+                return None
+            pos = operator.index(pos)            # (numpy's integers, too)
+            if not 0 <= pos < min(rows, self.positions):
+                return None
         if ids.dtype != torch.int64:
             ids = ids.long()
         stream = torch.cuda.current_stream(self.device).cuda_stream
