@@ -235,3 +235,24 @@ def test_decode_appends_the_new_row_itself(fa_lib):
     assert cfa.last_status() == 0
     with pytest.raises(RuntimeError):
         cfa.decode(q, k, v, 5, k_new=kn)
+
+
+def test_gradients_through_the_cache(golden_dir):
+    """A forward that fills the caches is differentiable like one without them: the caches are tensors of
+    their own, not views of one tensor."""
+    model, ids, _ = _load_tiny(golden_dir, "manual")
+    grads = []
+    for cached in (False, True):
+        model.zero_grad()
+        caches = model.allocate_kv_cache(ids.shape[0], 48) if cached else None
+        model(ids, kv_caches=caches).square().mean().backward()
+        grads.append([p.grad.clone() for p in model.parameters()])
+        if cached:
+            flat = [t for pair in caches for t in pair]
+            assert len({t.data_ptr() for t in flat}) == len(flat)
+    for a, b in zip(*grads):
+        torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-7)
+    with torch.inference_mode():
+        caches = model.allocate_kv_cache(ids.shape[0], 48)
+        first = model(ids[:, :25], kv_caches=caches, pos=0)
+        assert model(ids[:, 25:], kv_caches=caches, pos=25).shape[1] == ids.shape[1] - 25 and first.shape[1] == 25

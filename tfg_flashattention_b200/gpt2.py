@@ -367,7 +367,10 @@ class GPTModel(nn.Module):
         if dtype is None:
             dtype = torch.bfloat16 if self.cfg["impl_type"] == "cuda" else self.tok_emb.weight.dtype
         layers = self.cfg["n_layers"]       # one allocation and one fill instead of two per layer
-        kv = torch.zeros(2 * layers, batch, n_max, h, d, dtype=dtype, device=dev).unbind(0)
+        kv = torch.zeros(2 * layers, batch, n_max, h, d, dtype=dtype, device=dev)
+        # tensors of their own on that memory: to autograd, views of one tensor would be one tensor (writing
+        # into one of several views is an error, and counts as a change of them all)
+        kv = [t.data for t in kv.unbind(0)]
         return list(zip(kv[::2], kv[1::2]))
 
     def _native_blocks(self, x, kv_caches, pos):
