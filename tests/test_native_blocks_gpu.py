@@ -126,3 +126,38 @@ def test_replaced_modules_are_used(fa_lib, torch_binding, change):
             torch.zeros(2, 3, 256, **bf), None, 0) is None    # (gradients on)
     elif change != "impl_type":
         assert not torch.equal(got, old.float())
+
+
+@pytest.mark.parametrize("kind", ["one prompt for four", "head first", "every third column", "row of 66", "misaligned"])
+def test_caches_that_only_the_modules_write(fa_lib, torch_binding, kind):
+    """Caches that the copy of the Python loop takes and the cache kernel does not: the loop steps aside and the
+    result is the Python loop's."""
+    if torch_binding is None:
+        pytest.skip("the torch extension binding could not be built here")
+    model = _model()
+    B, n, H = (1 if kind == "one prompt for four" else 2), 20, 4
+    ids = torch.randint(0, 503, (B, n), device="cuda")
+
+    def cache():
+        zeros = lambda *s: torch.zeros(*s, dtype=torch.bfloat16, device="cuda")
+        if kind == "one prompt for four":
+            return zeros(4, 32, H, 64)
+        if kind == "head first":                         # (this one the kernel takes, too)
+            return zeros(B, H, 32, 64).transpose(1, 2)
+        if kind == "every third column":
+            return zeros(B, 32, H, 192)[..., ::3]
+        if kind == "row of 66":
+            return zeros(B, 32, H, 66)[..., :64]
+        return zeros(B * 32 * H * 64 + 4)[4:].view(B, 32, H, 64)
+
+    caches = [[(cache(), cache()) for _ in range(3)] for _ in range(2)]
+    x = torch.zeros(B, n, 256, dtype=torch.bfloat16, device="cuda")
+    with torch.no_grad():
+        assert (model._native_blocks(x, caches[0], 0) is not None) == (kind == "head first")
+        got = model(ids, kv_caches=caches[0], pos=0)
+        model._native_blocks = lambda *a: None
+        want = model(ids, kv_caches=caches[1], pos=0)
+    assert torch.equal(got, want)
+    for a, b in zip(*caches):
+        for t, r in zip(a, b):
+            assert torch.equal(t, r) and (t[:, :n].abs().sum((1, 2, 3)) > 0).all()

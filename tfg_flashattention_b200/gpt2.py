@@ -388,13 +388,22 @@ class GPTModel(nn.Module):
         if rows is None:
             return None
         if kv_caches is not None:
+            # what the cache kernel takes, the same in all layers; any other cache is written by the modules (one
+            # prompt into every sequence of a larger cache, other types, orders and devices)
             if not isinstance(kv_caches, list) or len(kv_caches) != len(rows):
                 return None
+            first, (batch, n) = kv_caches[0][0], x.shape[:2]
+            shape, stride = first.shape, first.stride()
+            if (first.dim() != 4 or shape[0] != batch or shape[1] < n or shape[2] != heads or shape[3] != 64 or stride[3] != 1
+                    or any(size > 1 and (s <= 0 or s % 8) for size, s in zip(shape[:3], stride))):
+                return None
             for pair in kv_caches:
-                k, v = pair
-                if (type(pair) is not tuple or k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16
-                        or k.shape != v.shape or k.stride() != v.stride() or not k.is_cuda):
+                if type(pair) is not tuple or len(pair) != 2:
                     return None
+                for t in pair:
+                    if (t.dtype != torch.bfloat16 or t.device != x.device or t.shape != shape or t.stride() != stride
+                            or t.data_ptr() % 16):
+                        return None
         return ext.blocks, rows
 
     def _list_block_rows(self):
