@@ -275,3 +275,23 @@ def test_positions_of_other_integer_types(fa_lib):
         want = model(ids[:, 6:], kv_caches=caches, pos=6)
         for kind in (np.int64, np.int32, np.uint8):
             assert torch.equal(model(ids[:, 6:], kv_caches=caches, pos=kind(6)), want)
+
+
+@pytest.mark.parametrize("generation", [65530, 65534, 0xfffffffb, 0xffffffff])
+def test_steps_across_the_wrap_of_the_generation(fa_lib, generation):
+    """The exchange words carry 16 bits of a counter that goes up by layers + 1 a step.  Steps from a counter
+    shortly before it wraps (in 16 bits, and in the 32 it is kept in) against a fresh workspace's, to the bit."""
+    model, _ = _model(768, 12, 2, 503, 64)
+    plan = model._step_plan
+    ids = torch.randint(0, 503, (4, 12), device="cuda")
+    runs = []
+    for start in (0, generation):
+        caches = model.allocate_kv_cache(4, 16)
+        workspace = plan.new_workspace(4)
+        outs = [model._step(ids[:, t:t + 1], caches, t, workspace=workspace) for t in range(3)]
+        if start:
+            workspace.view(torch.int32)[0] = start - (start >> 31 << 32)
+        outs += [model._step(ids[:, t:t + 1], caches, t, workspace=workspace) for t in range(3, 12)]
+        runs.append((torch.cat(outs), [torch.cat(pair) for pair in caches]))
+    assert torch.equal(runs[0][0], runs[1][0])
+    assert all(torch.equal(a, b) for a, b in zip(runs[0][1], runs[1][1]))

@@ -967,7 +967,8 @@ __global__ void __launch_bounds__(kStepThreads, 1) fa_gpt_step_kernel(const __gr
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int C = p.C, M = p.M;
   const long long pos64 = p.pos_ptr ? *p.pos_ptr : static_cast<long long>(p.pos);
-  const uint32_t generation = *p.generation;
+  // (reduced here: past 2^32 the remainders would repeat one, and a word of the layer before pass for new)
+  const uint32_t generation = *p.generation % 65535u;
   const int last = min(p.cache_rows, p.n_positions) - 1;
   const int pos = pos64 < 0 ? 0 : (pos64 > last ? last : static_cast<int>(pos64));
   const StepAttnCut cut(M * p.H, pos);
