@@ -295,3 +295,23 @@ def test_steps_across_the_wrap_of_the_generation(fa_lib, generation):
         runs.append((torch.cat(outs), [torch.cat(pair) for pair in caches]))
     assert torch.equal(runs[0][0], runs[1][0])
     assert all(torch.equal(a, b) for a, b in zip(runs[0][1], runs[1][1]))
+
+
+def test_head_strides_past_32_bits(fa_lib):
+    """Caches whose last head lies more than 2^31 elements behind the first (one allocation of 4.5 GB, K and V
+    interleaved in it): the new row goes where it belongs and nowhere else."""
+    model, _ = _model(1600, 25, 1, 503, 64)
+    stride = 2 ** 31 // 24 // 8 * 8 + 64
+    flat = torch.zeros(24 * stride + 4096, dtype=torch.bfloat16, device="cuda")
+    wide = [tuple(flat[at:].as_strided((1, 16, 25, 64), (64, 64, stride, 1)) for at in (0, 2048))]
+    assert wide[0][0].stride(2) * 24 > 2 ** 31
+    caches = model.allocate_kv_cache(1, 16)
+    ids = torch.randint(0, 503, (1, 6), device="cuda")
+    with torch.no_grad():
+        for t in range(6):
+            want = model._step(ids[:, t:t + 1], caches, t)
+            got = model._step(ids[:, t:t + 1], wide, t)
+            assert torch.equal(got, want)
+    for a, b in zip(caches[0], wide[0]):
+        assert torch.equal(a, b)
+    assert int((flat != 0).sum()) == sum(int((t != 0).sum()) for t in caches[0])

@@ -479,7 +479,7 @@ __device__ __forceinline__ StepCta step_linear(StepCta c, const StepParams& p, c
           if (n >= p.C) {                          // the caches get the row too, for the steps to come
             const bool is_k = n < 2 * p.C;
             const int nn = n - (is_k ? p.C : 2 * p.C);
-            (is_k ? p.k_cache[layer] : p.v_cache[layer])[tok * p.c_sb + static_cast<long long>(pos) * p.c_sn + (nn >> 6) * p.c_sh + (nn & 63)] =
+            (is_k ? p.k_cache[layer] : p.v_cache[layer])[tok * p.c_sb + static_cast<long long>(pos) * p.c_sn + static_cast<long long>(nn >> 6) * p.c_sh + (nn & 63)] =
                 __float2bfloat16_rn(val);
           }
         } else if (op == kStepFc) {
