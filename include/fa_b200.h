@@ -287,7 +287,8 @@ int fa_b200_linear_small(const fa_b200_linear_small_params* p);
  * B <= 8 sequences.  The reference's GPTModel.forward (src/py/model_inference.py:149-190) for a single
  * position with the earlier keys and values cached.
  *
- * Head dimension 64, so the width is C = 64 * H <= 1600; B * H <= 256; at most 64 layers.  All weights are bf16 in
+ * Head dimension 64, so the width is C = 64 * H <= 1600; B * H <= 256; at most 64 layers; fewer than 2^24
+ * words of vocabulary.  All weights are bf16 in
  * torch.nn.Linear's layout, dense and 16-byte aligned.  `layers` is DEVICE memory holding `n_layers`
  * records of device pointers (qkv_b may be NULL); the weights of the three projections are one
  * [3C, C] matrix.  k_cache / v_cache are host arrays of n_layers device pointers to caches of

@@ -181,3 +181,33 @@ def test_linear_small_rejects_before_any_cuda_call(fa_lib):
     assert call(params(resid=0x5000, sum_out=0x1000)) == -14
     assert call(params(ln_scale=0x5000, ln_shift=0x6000, eps=-1.0)) == -6
     assert b"overlap" in fa_lib.fa_b200_strerror(-14)
+
+
+def test_gpt_step_rejects_before_any_cuda_call(fa_lib):
+    caches = (ctypes.c_void_p * 2)(0x10000, 0x20000)
+
+    def params(**kw):
+        p = _lib.FaGptStepParams()
+        for i, name in enumerate(("layers", "tok_emb", "pos_emb", "lnf_scale", "lnf_shift", "head_w", "ids", "logits", "workspace")):
+            setattr(p, name, 0x1000 * (i + 1))
+        p.k_cache, p.v_cache = ctypes.addressof(caches), ctypes.addressof(caches) + 8
+        p.cache_strides = (ctypes.c_int64 * 3)(64 * 12 * 32, 64 * 12, 64)
+        p.n_layers, p.B, p.H, p.vocab, p.cache_rows, p.n_positions = 1, 2, 12, 50257, 32, 64
+        p.ids_stride, p.eps, p.device = 1, 1e-5, 0
+        p.workspace_bytes = 0
+        for k, v in kw.items():
+            setattr(p, k, v)
+        return p
+    call = lambda p: fa_lib.fa_b200_gpt_step(ctypes.byref(p))
+    assert fa_lib.fa_b200_gpt_step(None) == -1
+    assert call(params()) == -12                                       # everything else is in order
+    assert call(params(vocab=0)) == -3 and call(params(vocab=1 << 24)) == -3
+    assert call(params(vocab=(1 << 24) - 1)) == -12
+    assert call(params(B=9)) == -3 and call(params(H=26)) == -3 and call(params(n_layers=65)) == -3
+    assert call(params(pos=32)) == -3 and call(params(pos=-1)) == -3
+    assert call(params(cache_strides=(ctypes.c_int64 * 3)(64, 60, 64))) == -4
+    assert call(params(cache_strides=(ctypes.c_int64 * 3)(64, 64, 1 << 31))) == -4
+    assert call(params(head_w=0x1008)) == -5 and call(params(ids=0x1004)) == -5
+    assert call(params(eps=-1.0)) == -6
+    assert call(params(device=-1)) == -7
+    assert fa_lib.fa_b200_gpt_step_workspace_bytes(9, 12) == -3 and fa_lib.fa_b200_gpt_step_workspace_bytes(8, 12) > 0

@@ -816,6 +816,7 @@ int fa_b200_gpt_step(const fa_b200_gpt_step_params* p) {
       p->k_cache == nullptr || p->v_cache == nullptr || p->logits == nullptr)
     return FA_B200_ERR_NULL;
   if (!step_shape_ok(p->B, p->H) || p->n_layers < 1 || p->n_layers > fa::kStepMaxLayers || p->vocab < 1 ||
+      p->vocab >= fa::kStepMaxVocab ||
       p->cache_rows < 1 || p->n_positions < 1 || p->cache_rows > (1 << 22))
     return FA_B200_ERR_SHAPE;
   if (p->pos_device == nullptr && (p->pos < 0 || p->pos >= p->cache_rows || p->pos >= p->n_positions))

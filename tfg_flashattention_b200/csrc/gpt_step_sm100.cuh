@@ -83,6 +83,7 @@ static_assert(kStepCompute * kStepComputeRegs + 32 * kStepStreamWarps * kStepStr
 constexpr int kStepMaxRows = 8;                       // sequences (the 8-column side of the MMA)
 constexpr int kStepMaxLayers = 64;
 constexpr int kStepMaxPairs = 256;                    // (sequence, head) pairs
+constexpr int kStepMaxVocab = 1 << 24;                // step_cut multiplies row counts by block indices in 32 bits
 constexpr int kStepTile = 12;                         // rows of W per stage (of the MMA's 16)
 constexpr int kStepMmaRows = 16;
 constexpr int kStepGroup = 4;                         // tiles whose partial sums are added up together
@@ -163,7 +164,7 @@ struct __align__(16) StepCut {
   short tiles, tile;
   int lg_group;
 };
-__device__ __forceinline__ StepCut step_cut(int N, bool head) {          // N < 2^24, grid <= 160
+__device__ __forceinline__ StepCut step_cut(int N, bool head) {          // N < kStepMaxVocab, grid <= 160
   StepCut c;
   c.row0 = static_cast<int>(blockIdx.x * static_cast<uint32_t>(N) / gridDim.x);
   c.rows = static_cast<int>((blockIdx.x + 1) * static_cast<uint32_t>(N) / gridDim.x) - c.row0;

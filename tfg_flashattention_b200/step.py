@@ -20,6 +20,7 @@ MAX_BATCH = 8
 MAX_PAIRS = 256            # sequences x heads
 MAX_LAYERS = 64
 MAX_WIDTH = 1600
+MAX_VOCAB = 1 << 24        # fewer than that
 PLAIN_TENSORS = (torch.Tensor, nn.Parameter)     # a subclass may keep its numbers in another form
 MAX_WORKSPACES = 8         # streams that keep a workspace (about 1 MB each)
 
@@ -133,6 +134,8 @@ class StepPlan:
                              take(out, "weight", (width, 4 * width)), take(out, "bias", (width,))])
             plan.vocab = model.out_head.weight.shape[0]
             plan.positions = model.pos_emb.weight.shape[0]
+            if plan.vocab >= MAX_VOCAB:
+                return None
             plan.ends = [take(model.tok_emb, "weight", (plan.vocab, width)),
                          take(model.pos_emb, "weight", (plan.positions, width)),
                          take(model.final_norm, "scale", (width,)), take(model.final_norm, "shift", (width,)),
