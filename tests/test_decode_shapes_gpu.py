@@ -56,3 +56,20 @@ def test_more_heads_than_a_grid_dimension_of_65535(fa_lib):
     s = torch.einsum("bhd,bhnd->bhn", q.double(), k.double()) / 8.0
     want = torch.einsum("bhn,bhnd->bhd", torch.softmax(s, -1), v.double())
     assert _close(o, want)
+
+
+@pytest.mark.parametrize("B,H,kv", [(1, 3, 1), (1, 12, 95), (1, 25, 1025), (1, 12, 4100), (41, 25, 64)])
+def test_scores_far_below_zero(fa_lib, B, H, kv):
+    """Scores of about -1e33 (with LSE of that size), all equal but one in three: a softmax like any other.
+    The smallest is not as small as an empty lane group's maximum."""
+    from tfg_flashattention_b200 import custom_flash_attn as cfa
+    g = torch.Generator(device="cuda").manual_seed(kv)
+    q = torch.full((B, H, 64), 1e16, device="cuda").bfloat16()
+    k = torch.full((B, H, kv, 64), -1e16, device="cuda").bfloat16()
+    k[:, :, 1::3] *= 2
+    v = torch.randn(B, H, kv, 64, device="cuda", generator=g).bfloat16()
+    o, lse = cfa.decode(q, k, v, kv, return_lse=True)
+    s = torch.einsum("bhd,bhnd->bhn", q.double(), k.double()) / 8.0
+    want = torch.einsum("bhn,bhnd->bhd", torch.softmax(s, -1), v.double())
+    assert s.max().item() < -1e32 and _close(o, want)
+    assert ((lse.double() / torch.logsumexp(s, -1) - 1).abs() <= 1e-5).all()

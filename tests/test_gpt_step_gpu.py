@@ -315,3 +315,29 @@ def test_head_strides_past_32_bits(fa_lib):
     for a, b in zip(caches[0], wide[0]):
         assert torch.equal(a, b)
     assert int((flat != 0).sum()) == sum(int((t != 0).sum()) for t in caches[0])
+
+
+@pytest.mark.parametrize("B,pos", [(1, 0), (2, 5), (1, 200)])
+def test_scores_far_below_zero(fa_lib, B, pos):
+    """A layer whose scores are all about -1e33 against the same model layer by layer."""
+    model, _ = _model(256, 4, 1, 503, 256)
+    att = model.trf_blocks[0].att
+    with torch.no_grad():
+        att.W_query.weight.zero_()
+        att.W_key.weight.zero_()
+        att.W_query.bias.fill_(1e16)
+        att.W_key.bias.fill_(-1e16)
+    model.prepare_for_inference()
+    ids = torch.randint(0, 503, (B, pos + 1), generator=torch.Generator().manual_seed(1)).cuda()
+    runs = []
+    with torch.no_grad():
+        for stepped in (True, False):
+            caches = model.allocate_kv_cache(B, 256)
+            if pos:
+                model(ids[:, :pos], kv_caches=caches, pos=0)
+            if not stepped:
+                model._step = lambda *a, **k: None
+            runs.append(model(ids[:, pos:], kv_caches=caches, pos=pos).float())
+    got, want = runs
+    assert torch.isfinite(got).all()
+    assert ((got - want).norm() / want.norm()).item() <= 2 * 2.0 ** -8 * math.sqrt(8 + 4)

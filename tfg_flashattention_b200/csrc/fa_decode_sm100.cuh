@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) fa_decode_kernel(const D
     q2[2] = mul_f32x2(bf16x2_to_f32x2(raw.z), sc);
     q2[3] = mul_f32x2(bf16x2_to_f32x2(raw.w), sc);
   }
-  float m = -1e30f, l = 0.f;                       // finite: a group without rows weighs nothing
+  float m = kNoScore, l = 0.f;                       // finite: a group without rows weighs nothing
 #pragma unroll 1
   for (int left = r1 - r0; left > 0; left -= kGroups * kUnroll) {
     uint4 kraw[kUnroll], vraw[kUnroll];
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) fa_decode_kernel(const D
   }
   __syncthreads();
   if (kCluster) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-  float mm = -1e30f, ll = 0.f, oo = 0.f;
+  float mm = kNoScore, ll = 0.f, oo = 0.f;
   if (tid < 64) {
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) mm = fmaxf(mm, sm_w[w][0]);
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) fa_decode_kernel(const D
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (rank != 0) return;
     if (tid < 64) {
-      mm = -1e30f; ll = 0.f; oo = 0.f;
+      mm = kNoScore; ll = 0.f; oo = 0.f;
       for (int k = 0; k < ctas; ++k) mm = fmaxf(mm, sm_c[k][0]);
       for (int k = 0; k < ctas; ++k) {
         const float f = exp2f(sm_c[k][0] - mm);

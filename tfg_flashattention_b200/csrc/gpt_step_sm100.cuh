@@ -704,7 +704,7 @@ __device__ __forceinline__ StepCta step_attention(StepCta c, const StepParams& p
       q0 = make_uint4(step_pair(w[0].x, w[0].y), step_pair(w[0].z, w[0].w), step_pair(w[1].x, w[1].y), step_pair(w[1].z, w[1].w));
       q1 = make_uint4(step_pair(w[2].x, w[2].y), step_pair(w[2].z, w[2].w), step_pair(w[3].x, w[3].y), step_pair(w[3].z, w[3].w));
     }
-    float m = -1e30f, l = 0.f;
+    float m = kNoScore, l = 0.f;
     uint64_t acc[4] = {0ull, 0ull, 0ull, 0ull};
     // Stages of kStepBlocks blocks of 16 rows, one warp to a block: warps 0 to 3 take the even ring slots, 4
     // to 7 the odd ones (so a warp that waits for a slot has also waited for the slot's stage before).  A
@@ -795,7 +795,7 @@ __device__ __forceinline__ StepCta step_attention(StepCta c, const StepParams& p
       for (int o = 1; o <= 8; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       float* fresh = c.sm->seg[i][kStepWarps];
       const bool counts = un.slot == 0;
-      if (lane == 0) { fresh[0] = counts ? s * p.scale_log2 : -1e30f; fresh[1] = counts ? 1.f : 0.f; }
+      if (lane == 0) { fresh[0] = counts ? s * p.scale_log2 : kNoScore; fresh[1] = counts ? 1.f : 0.f; }
       if (lane < 16)
         *reinterpret_cast<float4*>(fresh + 4 + 4 * lane) = make_float4(val(w[2].x), val(w[2].y), val(w[2].z), val(w[2].w));
     }
@@ -805,11 +805,11 @@ __device__ __forceinline__ StepCta step_attention(StepCta c, const StepParams& p
   if (i < count) {
     const StepUnit un = c.sm->unit[i];
     const float(&seg)[kStepWarps + 1][68] = c.sm->seg[i];
-    float mm = -1e30f, ll = 0.f, oo = 0.f;
+    float mm = kNoScore, ll = 0.f, oo = 0.f;
 #pragma unroll
     for (int w = 0; w <= kStepWarps; ++w) mm = fmaxf(mm, seg[w][0]);
 #pragma unroll
-    for (int w = 0; w <= kStepWarps; ++w) {      // (a warp without rows: m = -1e30, l = o = 0)
+    for (int w = 0; w <= kStepWarps; ++w) {      // (a warp without rows: m = kNoScore, l = o = 0)
       const float f = ex2_approx(seg[w][0] - mm);
       ll = fmaf(seg[w][1], f, ll);
       oo = fmaf(seg[w][4 + e], f, oo);
@@ -828,7 +828,7 @@ __device__ __forceinline__ StepCta step_attention(StepCta c, const StepParams& p
       if (write) {                               // all partials are in: merge them
         __threadfence();
         if (e == 0) p.arrived[un.pair] = 0;
-        mm = -1e30f; ll = 0.f; oo = 0.f;
+        mm = kNoScore; ll = 0.f; oo = 0.f;
 #pragma unroll 1
         for (int k = 0; k < splits; ++k) {
           const float2 ml = __ldcg(pm + k);

@@ -266,6 +266,9 @@ __device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+// The running maximum of a softmax before its first score: finite (the difference of two of them is 0), and
+// no finite score is below it.
+constexpr float kNoScore = -3.402823466e38f;
 __device__ __forceinline__ uint64_t bf16x2_to_f32x2(uint32_t v) {
   return pack_f32x2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
 }
