@@ -73,3 +73,22 @@ def test_scores_far_below_zero(fa_lib, B, H, kv):
     want = torch.einsum("bhn,bhnd->bhd", torch.softmax(s, -1), v.double())
     assert s.max().item() < -1e32 and _close(o, want)
     assert ((lse.double() / torch.logsumexp(s, -1) - 1).abs() <= 1e-5).all()
+
+
+def test_length_written_by_the_kernel_in_front(fa_lib):
+    """A device length that is advanced between back-to-back launches, and a LayerNorm whose scale is."""
+    from tfg_flashattention_b200 import block_ops
+    from tfg_flashattention_b200 import custom_flash_attn as cfa
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v = (torch.randn(*s, device="cuda", generator=g).bfloat16() for s in ((1, 4, 64), (1, 4, 64, 64), (1, 4, 64, 64)))
+    x = torch.randn(8, 768, device="cuda", generator=g).bfloat16()
+    n, scale, shift = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.zeros(768, device="cuda").bfloat16(), torch.zeros(768, device="cuda").bfloat16()
+    outs, norms = [], []
+    for _ in range(64):
+        n.add_(1)
+        outs.append(cfa.decode(q, k, v, n))
+        scale.add_(1)
+        norms.append(block_ops.add_layernorm(x, None, scale, shift))
+    for i in range(64):
+        assert torch.equal(outs[i], cfa.decode(q, k, v, i + 1))
+        assert torch.equal(norms[i], block_ops.add_layernorm(x, None, torch.full_like(scale, i + 1), shift))

@@ -126,8 +126,8 @@ __global__ void __launch_bounds__(kLnWarpsPerCta * 32) fa_add_layernorm_kernel(c
     const int v = lane + 32 * i;
     if (v < nvec) {
       float g[8], b[8], y[8];
-      ln_unpack8(__ldg(sc + v), g);
-      ln_unpack8(__ldg(sh + v), b);
+      ln_unpack8(sc[v], g);
+      ln_unpack8(sh[v], b);
 #pragma unroll
       for (int e = 0; e < 8; ++e) y[e] = fmaf((x[i][e] - mean) * rstd, g[e], b[e]);
       out[v] = ln_pack8(y);

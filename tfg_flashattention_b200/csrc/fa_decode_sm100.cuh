@@ -72,7 +72,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) fa_decode_kernel(const D
   if (kCluster) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   pdl_trigger();
   pdl_wait();
-  const int kv_len = p.kv_len_ptr ? max(1, min(__ldg(p.kv_len_ptr), p.kv_len)) : p.kv_len;
+  // (an ordinary load: the kernel in front may still be writing it when this one has started)
+  const int kv_len = p.kv_len_ptr ? max(1, min(*static_cast<const volatile int*>(p.kv_len_ptr), p.kv_len)) : p.kv_len;
   const int r0 = kCluster ? static_cast<int>(static_cast<long long>(rank) * kv_len / ctas) : 0;
   const int r1 = kCluster ? static_cast<int>(static_cast<long long>(rank + 1) * kv_len / ctas) : kv_len;
   const __nv_bfloat16* kp = p.k + b * p.k_sb + h * p.k_sh + (r0 + g) * p.k_sn + 8 * c;    // row r0 + g

@@ -42,7 +42,8 @@ __device__ __forceinline__ void reg_dealloc() {
 
 // Programmatic dependent launch: a kernel launched with that attribute may start while the one in
 // front of it in the stream still runs; pdl_wait returns when that one has completed and its writes
-// are visible, and must come before the first access to global memory.  pdl_trigger lets the next
+// are visible, and must come before the first access to global memory.  (No access through the read-only
+// path at all: it is for memory that nobody writes while the kernel is there.)  pdl_trigger lets the next
 // kernel of the stream start (once every CTA of this one has said so); it then holds nothing but an
 // idle slot until this kernel is through.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
