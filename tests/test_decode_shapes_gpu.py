@@ -92,3 +92,23 @@ def test_length_written_by_the_kernel_in_front(fa_lib):
     for i in range(64):
         assert torch.equal(outs[i], cfa.decode(q, k, v, i + 1))
         assert torch.equal(norms[i], block_ops.add_layernorm(x, None, torch.full_like(scale, i + 1), shift))
+
+
+@pytest.mark.parametrize("binding", ["ext", "ctypes"])
+def test_rows_of_longer_tensors(fa_lib, torch_binding, binding):
+    """out, k_new and v_new of [B, H, n, 64] stand for their first rows, through both bindings."""
+    if binding == "ext" and torch_binding is None:
+        pytest.skip("the torch extension binding could not be built here")
+    from tfg_flashattention_b200 import custom_flash_attn as cfa
+    g = torch.Generator(device="cuda").manual_seed(9)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    q, k, v, kn, vn = rnd(2, 3, 1, 64), rnd(2, 3, 9, 64), rnd(2, 3, 9, 64), rnd(2, 3, 4, 64), rnd(2, 3, 4, 64)
+    want = cfa.decode(q, k.clone(), v.clone(), 7, k_new=kn[:, :, 0].contiguous(), v_new=vn[:, :, 0].contiguous())
+    cfa.set_binding(binding)
+    try:
+        out = torch.zeros(2, 3, 5, 64, dtype=torch.bfloat16, device="cuda")
+        got = cfa.decode(q, k, v, 7, out=out, k_new=kn, v_new=vn)
+    finally:
+        cfa.set_binding("auto")
+    assert got is out and torch.equal(out[:, :, :1], want) and (out[:, :, 1:] == 0).all()
+    assert torch.equal(k[:, :, 6], kn[:, :, 0]) and torch.equal(v[:, :, 6], vn[:, :, 0])

@@ -189,11 +189,11 @@ PyObject* forward(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* 
   });
 }
 
-// Whether t is [B, H, 64] or [B, H, 1, 64], dense in the last dimension.  (No view is made of it: three
-// of them cost more host time than the launch's arguments.)
+// Whether t is [B, H, 64] or [B, H, n, 64] (its first row is meant then), dense in the last dimension.  (No
+// view is made of it: three of them cost more host time than the launch's arguments.)
 bool is_row(const at::Tensor& t, int64_t B, int64_t H, int64_t d) {
   const int64_t n = t.dim();
-  return (n == 3 || (n == 4 && t.size(2) == 1)) && t.size(0) == B && t.size(1) == H && t.size(n - 1) == d && t.stride(n - 1) == 1;
+  return (n == 3 || (n == 4 && t.size(2) >= 1)) && t.size(0) == B && t.size(1) == H && t.size(n - 1) == d && t.stride(n - 1) == 1;
 }
 // {batch, head} strides of it; size-1 dimensions get a canonical stride
 void strides2(const at::Tensor& t, int64_t out[2]) {
