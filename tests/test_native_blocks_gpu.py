@@ -161,3 +161,41 @@ def test_caches_that_only_the_modules_write(fa_lib, torch_binding, kind):
     for a, b in zip(*caches):
         for t, r in zip(a, b):
             assert torch.equal(t, r) and (t[:, :n].abs().sum((1, 2, 3)) > 0).all()
+
+
+@pytest.mark.parametrize("width,B,n", [(320, 1, 73), (320, 3, 5), (64, 1, 1), (448, 1, 129), (256, 1, 73)])
+def test_native_loop_of_odd_heads_and_rows(fa_lib, torch_binding, width, B, n):
+    """An odd number of heads times an odd number of rows: parts of one buffer that are 128-byte aligned only
+    if nothing sees to it."""
+    if torch_binding is None:
+        pytest.skip("the torch extension binding could not be built here")
+    model = _model(width=width, layers=2)
+    ids = torch.randint(0, 503, (B, n), device="cuda")
+    with torch.no_grad():
+        assert model._native_blocks(torch.zeros(B, n, width, dtype=torch.bfloat16, device="cuda"), None, 0) is not None
+        got = model(ids)
+        model._native_blocks = lambda *a: None
+        want = model(ids)
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("offset", [8, 16, 64])
+def test_native_loop_of_weights_in_a_flat_buffer(fa_lib, torch_binding, offset):
+    """Parameters that are views into one buffer, 16, 32 and 128 bytes behind a 256-byte boundary.  The GEMMs'
+    algorithms depend on it and sum in their own orders: a rounding to bf16 (2^-9) on either side for each
+    of the eight per layer, taken as independent."""
+    if torch_binding is None:
+        pytest.skip("the torch extension binding could not be built here")
+    model = _model(layers=2)
+    for p in model.parameters():
+        flat = torch.zeros(p.numel() + offset, dtype=torch.bfloat16, device="cuda")
+        flat[offset:] = p.detach().flatten()
+        p.data = flat[offset:].view(p.shape)
+        assert p.data_ptr() % 256 == 2 * offset
+    ids = torch.randint(0, 503, (2, 37), device="cuda")
+    with torch.no_grad():
+        assert model._native_blocks(torch.zeros(2, 37, 256, dtype=torch.bfloat16, device="cuda"), None, 0) is not None
+        got = model(ids).float()
+        model._native_blocks = lambda *a: None
+        want = model(ids).float()
+    assert ((got - want).norm() / want.norm()).item() <= 2 * 2.0 ** -9 * (8 * 2 + 4) ** 0.5

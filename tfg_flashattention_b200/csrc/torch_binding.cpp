@@ -376,8 +376,17 @@ struct LtKey {
   int device;
   int64_t m, n, k;
   int epilogue;
-  bool operator==(const LtKey& o) const { return device == o.device && m == o.m && n == o.n && k == o.k && epilogue == o.epilogue; }
+  uint32_t align[3];      // of w, x and y: an algorithm may rely on them
+  bool operator==(const LtKey& o) const {
+    return device == o.device && m == o.m && n == o.n && k == o.k && epilogue == o.epilogue && align[0] == o.align[0] &&
+           align[1] == o.align[1] && align[2] == o.align[2];
+  }
 };
+// The largest power of two up to 256 (what the library assumes unless told) that the address is a multiple of.
+uint32_t alignment(const at::Tensor& t) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(t.data_ptr()) | 256u;
+  return static_cast<uint32_t>(a & (~a + 1));
+}
 struct LtPlan {
   LtKey key;
   bool usable = false;
@@ -397,15 +406,14 @@ bool lt_linear(const at::Tensor& x, const at::Tensor& w, const at::Tensor* bias,
                void* stream) {
   const LtApi& api = lt();
   if (!api.ok || !w.is_contiguous() || !x.is_contiguous() || (gelu && bias == nullptr)) return false;
-  if ((reinterpret_cast<uintptr_t>(w.data_ptr()) | reinterpret_cast<uintptr_t>(x.data_ptr()) |
-       (bias ? reinterpret_cast<uintptr_t>(bias->data_ptr()) : 0)) & 15u)
-    return false;
+  const uint32_t align[3] = {alignment(w), alignment(x), alignment(y)};
+  if (std::min({align[0], align[1], align[2], bias ? alignment(*bias) : 256u}) < 16) return false;
   constexpr int kPlans = 64;
   static thread_local LtPlan plans[kPlans];
   static thread_local int next = 0;
   const int64_t k = w.size(1), n = w.size(0), m = x.numel() / k;
   const int epilogue = gelu ? CUBLASLT_EPILOGUE_GELU_BIAS : (bias ? CUBLASLT_EPILOGUE_BIAS : CUBLASLT_EPILOGUE_DEFAULT);
-  const LtKey key{x.device().index(), m, n, k, epilogue};
+  const LtKey key{x.device().index(), m, n, k, epilogue, {align[0], align[1], align[2]}};
   LtPlan* plan = nullptr;
   for (LtPlan& p : plans)
     if (p.desc != nullptr && p.key == key) { plan = &p; break; }
@@ -434,6 +442,10 @@ bool lt_linear(const at::Tensor& x, const at::Tensor& w, const at::Tensor* bias,
                    ok(api.layout_create(&plan->w, type, k, n, k)) && ok(api.layout_create(&plan->x, type, k, m, k)) &&
                    ok(api.layout_create(&plan->y, type, n, m, n)) && ok(api.pref_create(&pref)) &&
                    ok(api.pref_set(pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &limit, sizeof(limit))) &&
+                   ok(api.pref_set(pref, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_A_BYTES, &align[0], sizeof(uint32_t))) &&
+                   ok(api.pref_set(pref, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_B_BYTES, &align[1], sizeof(uint32_t))) &&
+                   ok(api.pref_set(pref, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_C_BYTES, &align[2], sizeof(uint32_t))) &&
+                   ok(api.pref_set(pref, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_D_BYTES, &align[2], sizeof(uint32_t))) &&
                    ok(api.heuristic(handle, plan->desc, plan->w, plan->x, plan->y, plan->y, pref, 1, found, &count)) && count > 0;
     if (pref != nullptr) api.pref_destroy(pref);
     if (plan->usable) plan->algo = found[0].algo;
@@ -496,6 +508,11 @@ PyObject* blocks(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* k
       FA_CHECK(PyTuple_Check(t) && PyTuple_GET_SIZE(t) == 12, "a layer has twelve tensors");
       for (int i = 0; i < 12; ++i)
         if (PyTuple_GET_ITEM(t, i) != Py_None) layers[l].t[i] = tensor_arg(PyTuple_GET_ITEM(t, i), "a layer's parameter");
+      const at::Tensor &qkv_w = layers[l].t[2], &proj_w = layers[l].t[4], &fc_w = layers[l].t[8], &out_w = layers[l].t[10];
+      FA_CHECK(qkv_w.defined() && proj_w.defined() && fc_w.defined() && out_w.defined() && qkv_w.dim() == 2 && proj_w.dim() == 2 &&
+                   fc_w.dim() == 2 && out_w.dim() == 2 && qkv_w.size(0) == 3 * C && qkv_w.size(1) == C && proj_w.size(0) == C &&
+                   proj_w.size(1) == C && fc_w.size(1) == C && out_w.size(0) == C && out_w.size(1) == fc_w.size(0),
+               "a layer's weights are [3C, C], [C, C], [hidden, C] and [C, hidden]");
       if (cached) {
         PyObject* kv = PyList_GET_ITEM(a[2], l);
         FA_CHECK(PyTuple_Check(kv) && PyTuple_GET_SIZE(kv) == 2, "a cache is a pair");
@@ -518,11 +535,12 @@ PyObject* blocks(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* k
       // Buffers for all layers.  The hidden layer lies where the projection and the attention's output lay,
       // which are dead by then: 7 instead of 11 widths per row, so that more of a prompt stays in L2.
       const int64_t rows = B * n;
-      int64_t wide = 4 * C;
-      for (const Layer& L : layers) wide = std::max(wide, L.t[8].size(0));
-      const at::Tensor arena = empty_cuda({rows * wide}, torch::kBFloat16, x.device());
+      const int64_t ctx_at = (rows * 3 * C + 127) / 128 * 128;       // 256 bytes: any GEMM takes it
+      int64_t size = ctx_at + rows * C;
+      for (const Layer& L : layers) size = std::max(size, rows * L.t[8].size(0));
+      const at::Tensor arena = empty_cuda({size}, torch::kBFloat16, x.device());
       at::Tensor qkv = arena.narrow(0, 0, rows * 3 * C).view({B, n, 3 * C});
-      at::Tensor ctx = arena.narrow(0, rows * 3 * C, rows * C).view({B, n, C}), mid;
+      at::Tensor ctx = arena.narrow(0, ctx_at, rows * C).view({B, n, C}), mid;
       at::Tensor branch, added = empty_like_cuda(x), h = empty_like_cuda(x);
       const at::Tensor workspace = empty_cuda({static_cast<int64_t>(kLtWorkspace)}, torch::kUInt8, x.device());
       auto linear = [&](const at::Tensor& in, const at::Tensor& w, const at::Tensor& bias, at::Tensor& y) {
