@@ -35,7 +35,7 @@
 extern "C" {
 #endif
 
-#define FA_B200_ABI_VERSION 5
+#define FA_B200_ABI_VERSION 6
 
 /* argument errors (negative return values) */
 #define FA_B200_OK                 0
@@ -79,23 +79,20 @@ int fa_b200_fwd(const fa_b200_params* p);
 
 /* How fa_b200_fwd would schedule this problem on p->device, without launching anything.  The
  * reference launcher has one fixed shape, a CTA per 32-row tile (grid (ceil(N/32), H, B),
- * src/cpp/v1.cu:13-14, 25-34); this library picks one of four kernel schedules per call and this
+ * src/cpp/v1.cu:13-14, 25-34); this library picks one of three kernel schedules per call and this
  * query reports the pick, so that a test or a tuning run can tell which code ran:
- *   FA_B200_SCHEDULE_CTA_PER_TILE        one CTA per 128-row query tile, heaviest causal tile first
- *                                        (long causal sequences: a CTA that is through takes over one
- *                                        that has not started)
- *   FA_B200_SCHEDULE_PERSISTENT_PAIRED   causal, even tile count: the resident CTAs' slots work through
- *                                        the tiles, heavy ones next to light ones
- *   FA_B200_SCHEDULE_PERSISTENT_ROTATED  the same with an odd tile count
- *   FA_B200_SCHEDULE_PERSISTENT_FULL     the same, non-causal
- *   FA_B200_SCHEDULE_NONE                empty problem, nothing is launched
- * *grid receives the number of CTAs (persistent: of resident ones).  Either output pointer may be NULL.  Arguments are checked as
+ *   FA_B200_SCHEDULE_CTA_PER_TILE   one CTA per 128-row query tile, heaviest causal tile first
+ *   FA_B200_SCHEDULE_STATIC         as many CTAs as are resident at a time, each with every so-many-th tile
+ *   FA_B200_SCHEDULE_DYNAMIC        one CTA per tile is launched, and a CTA that is through takes over one that
+ *                                   has not started
+ *   FA_B200_SCHEDULE_NONE           empty problem, nothing is launched
+ * (1, 2 and 3 were schedules of earlier versions; ABI versions up to 5 went on reporting them.)
+ * *grid receives the number of CTAs launched.  Either output pointer may be NULL.  Arguments are checked as
  * by fa_b200_fwd; the first call on a device performs the same one-time device set-up. */
 #define FA_B200_SCHEDULE_NONE               -1
 #define FA_B200_SCHEDULE_CTA_PER_TILE        0
-#define FA_B200_SCHEDULE_PERSISTENT_PAIRED   1
-#define FA_B200_SCHEDULE_PERSISTENT_ROTATED  2
-#define FA_B200_SCHEDULE_PERSISTENT_FULL     3
+#define FA_B200_SCHEDULE_STATIC              4
+#define FA_B200_SCHEDULE_DYNAMIC             5
 int fa_b200_fwd_plan(const fa_b200_params* p, int32_t* schedule, int32_t* grid);
 
 /* Check arguments exactly as fa_b200_fwd does, without touching CUDA.  Returns 0 or a negative

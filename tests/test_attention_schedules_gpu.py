@@ -22,7 +22,7 @@ def _slots():
     (128, "slots"), (128, "slots+1"), (90, "3*slots"),              # one K/V tile: one item / static
     (300, "slots+3"), (500, "2*slots-4"), (512, "2*slots"),         # up to four: static, then dynamic
     (700, "4*slots//3-6"), (700, "4*slots//3+6"), (1024, "5*slots"),
-    (2048, "2*slots"), (2177, "2*slots"),                            # dynamic, reported as CTA per tile above 16 tiles
+    (2048, "2*slots"), (2177, "2*slots"),                            # dynamic
 ])
 @pytest.mark.parametrize("causal", [True, False])
 def test_schedule_borders(fa_lib, N, items, causal):

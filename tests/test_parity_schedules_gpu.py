@@ -81,13 +81,13 @@ def _tile_edge_rows(N, n_random, seed):
 
 @pytest.mark.parametrize("B,H,N", [(10, 20, 512), (10, 20, 1000), (5, 40, 384)])
 def test_persistent_noncausal_schedule(cfa, B, H, N):
-    """Non-causal, at least 592 work items of at most 8 K/V tiles: resident CTAs loop over items
-    (fa_fwd_kernel<true,false>); N = 1000 puts a ragged last K/V tile on that path.  Every row of
+    """Non-causal, at least 592 work items of at most 8 K/V tiles: CTAs take items over from CTAs that have
+    not started (fa_fwd_kernel<kDynamic, false>); N = 1000 puts a ragged last K/V tile on that path.  Every row of
     every head is compared with the oracle."""
     torch.manual_seed(7000 + N)
     q, k, v = (torch.randn(B, H, N, 64) for _ in range(3))
     qb, kb, vb = (t.to("cuda", torch.bfloat16) for t in (q, k, v))
-    assert cfa.plan(qb, kb, vb, causal=False)[0] == "persistent_full"
+    assert cfa.plan(qb, kb, vb, causal=False) == ("dynamic", B * H * -(-N // 128))
     o, lse = cfa.forward(qb, kb, vb, causal=False, return_lse=True)
     assert cfa.last_status() == 0
     assert torch.isfinite(o).all() and torch.isfinite(lse).all()
@@ -105,13 +105,14 @@ def test_persistent_noncausal_schedule(cfa, B, H, N):
 
 @pytest.mark.parametrize("B,H,N", [(8, 25, 384), (8, 25, 640), (8, 25, 600), (30, 20, 128)])
 def test_persistent_rotated_causal_schedule(cfa, B, H, N):
-    """Causal with an odd number of query tiles and at least 592 items: resident CTAs stride
-    through single tiles whose order inside a head is rotated by the head index.  Every row of
+    """Causal with an odd number of query tiles and at least 592 items: taken over from CTAs that have not
+    started, or, where a tile is all there is of a head, dealt to the resident CTAs.  Every row of
     every head is compared with the oracle; N = 600 adds a ragged last tile."""
     torch.manual_seed(8000 + N)
     q, k, v = (torch.randn(B, H, N, 64) for _ in range(3))
     qb, kb, vb = (t.to("cuda", torch.bfloat16) for t in (q, k, v))
-    assert cfa.plan(qb, kb, vb, causal=True)[0] == "persistent_rotated"
+    tiles, sms = -(-N // 128), torch.cuda.get_device_properties(0).multi_processor_count
+    assert cfa.plan(qb, kb, vb, causal=True) == (("static", 2 * sms) if tiles == 1 else ("dynamic", B * H * tiles))
     o, lse = cfa.forward(qb, kb, vb, causal=True, return_lse=True)
     assert cfa.last_status() == 0
     assert torch.isfinite(o).all() and torch.isfinite(lse).all()
@@ -127,8 +128,8 @@ def test_persistent_rotated_causal_schedule(cfa, B, H, N):
 
 @pytest.mark.parametrize("causal,N", [(True, 256), (False, 128), (True, 128)])
 def test_many_items_per_cta(cfa, causal, N):
-    """A persistent CTA decodes all its work items into a table of 256 entries when it starts.
-    Here every CTA gets about 250 of them (generated on the device: 1-2 GB of inputs); sampled
+    """A CTA of the static schedule decodes all its work items into a table of 256 entries when it starts.
+    Here every resident CTA gets about 250 of them, or takes them over one by one (generated on the device: 1-2 GB of inputs); sampled
     heads from the first to the last are compared with the oracle and with the same head computed
     alone.  One more batch entry per CTA than the table holds and the launcher takes one CTA per
     tile instead."""
@@ -139,8 +140,7 @@ def test_many_items_per_cta(cfa, causal, N):
     B, H = heads // 8, 8
     g = torch.Generator(device="cuda").manual_seed(9100 + N + int(causal))
     qb, kb, vb = (torch.randn(B, H, N, 64, device="cuda", generator=g).bfloat16() for _ in range(3))
-    want = {(True, 256): "persistent_paired", (True, 128): "persistent_rotated", (False, 128): "persistent_full"}
-    assert cfa.plan(qb, kb, vb, causal=causal) == (want[(causal, N)], 2 * sms)
+    assert cfa.plan(qb, kb, vb, causal=causal) == (("static", 2 * sms) if tiles == 1 else ("dynamic", heads // 8 * 8 * tiles))
     o, lse = cfa.forward(qb, kb, vb, causal=causal, return_lse=True)
     assert cfa.last_status() == 0
     assert torch.isfinite(o).all() and torch.isfinite(lse).all()
@@ -162,13 +162,16 @@ def test_plan_reports_each_schedule(cfa):
         t = torch.empty(B, H, N, 64, device="cuda", dtype=torch.bfloat16)
         return cfa.plan(t, t, t, causal=causal)
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    assert plan(32, 25, 1024, True) == ("persistent_paired", 2 * sms)
-    assert plan(4, 12, 1024, True)[0] == "persistent_paired"
-    assert plan(16, 16, 512, False) == ("persistent_full", 2 * sms)
+    assert sms == 148
+    assert plan(32, 25, 1024, True) == ("dynamic", 32 * 25 * 8)
+    assert plan(4, 12, 1024, True) == ("cta_per_tile", 4 * 12 * 8)
+    assert plan(16, 16, 512, False) == ("dynamic", 16 * 16 * 4)
+    assert plan(8, 16, 300, True) == ("static", 2 * sms)
+    assert plan(4, 25, 512, False) == ("static", 2 * sms)
     assert plan(16, 16, 4096, False) == ("cta_per_tile", 16 * 16 * 32)
-    assert plan(4, 25, 8192, True)[0] == "cta_per_tile"
+    assert plan(4, 25, 8192, True) == ("dynamic", 4 * 25 * 64)
     assert plan(2, 3, 300, True) == ("cta_per_tile", 18)
-    assert plan(8, 25, 384, True)[0] == "persistent_rotated"
+    assert plan(8, 25, 384, True) == ("dynamic", 8 * 25 * 3)
     assert plan(0, 4, 16, True) == ("none", 0)
 
 

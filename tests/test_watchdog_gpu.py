@@ -40,7 +40,7 @@ def test_wait_runs_out_is_reported_and_the_next_launch_is_correct(fa_lib):
     torch.manual_seed(3)
     # one CTA: B = H = 1, N = 256 is a single pair of causal tiles; its first item needs two K tiles
     q, k, v = (torch.randn(1, 1, 256, 64, device="cuda").bfloat16() for _ in range(3))
-    assert cfa.plan(q, k, v) == ("persistent_paired", 1)
+    assert cfa.plan(q, k, v) == ("static", 1)
     good = cfa.forward(q, k, v)
     assert cfa.last_status() == 0
 

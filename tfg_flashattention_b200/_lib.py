@@ -10,7 +10,7 @@ import os
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libfa_b200.so")
 
-ABI_VERSION = 5
+ABI_VERSION = 6
 
 
 class FaParams(ctypes.Structure):
@@ -93,8 +93,7 @@ EXPORTS = ("fa_b200_fwd", "fa_b200_fwd_plan", "fa_b200_validate", "fa_b200_strer
            "fa_b200_last_status", "fa_b200_abi_version", "fa_b200_decode", "fa_b200_decode_workspace_bytes", "fa_b200_decode_static", "fa_b200_decode_direct",
            "fa_b200_add_layernorm", "fa_b200_linear_small", "fa_b200_gpt_step", "fa_b200_gpt_step_workspace_bytes", "fa_b200_cache_write")
 
-SCHEDULES = {-1: "none", 0: "cta_per_tile", 1: "persistent_paired", 2: "persistent_rotated",
-             3: "persistent_full"}
+SCHEDULES = {-1: "none", 0: "cta_per_tile", 4: "static", 5: "dynamic"}
 
 _lib = None
 

@@ -369,16 +369,11 @@ int fa_b200_fwd_plan(const fa_b200_params* p, int32_t* schedule, int32_t* grid) 
   DeviceState* stp = nullptr;
   if ((rc = ready_device(p->device, &stp)) != 0) return rc;
   const FwdPlan pl = plan_fwd(p, *stp);
-  // reported by what a CTA slot does (see the header): several tiles in turn, or one
-  const long long slots = stp->resident_ctas;
-  const bool in_turn = pl.schedule == fa::kStatic || (pl.schedule == fa::kDynamic && (!p->causal || pl.kv_tiles <= 16)) ||
-                       (p->causal && pl.n_qtiles % 2 == 0 && pl.kv_tiles <= 16 && pl.items > slots && 3 * pl.items < 4 * slots);
   if (schedule != nullptr)
-    *schedule = !in_turn               ? FA_B200_SCHEDULE_CTA_PER_TILE
-                : !p->causal           ? FA_B200_SCHEDULE_PERSISTENT_FULL
-                : pl.n_qtiles % 2 == 0 ? FA_B200_SCHEDULE_PERSISTENT_PAIRED
-                                       : FA_B200_SCHEDULE_PERSISTENT_ROTATED;
-  if (grid != nullptr) *grid = static_cast<int32_t>(in_turn && pl.items > slots ? slots : pl.grid);
+    *schedule = pl.schedule == fa::kOneItem  ? FA_B200_SCHEDULE_CTA_PER_TILE
+                : pl.schedule == fa::kStatic ? FA_B200_SCHEDULE_STATIC
+                                             : FA_B200_SCHEDULE_DYNAMIC;
+  if (grid != nullptr) *grid = static_cast<int32_t>(pl.grid);
   return FA_B200_OK;
 }
 

@@ -169,8 +169,8 @@ def forward(Q, K, V, causal=True, return_lse=False, softmax_scale=None, out=None
 
 def plan(Q, K, V, causal=True):
     """Which kernel schedule `forward` would use for these tensors, without launching anything:
-    (name, grid) with name one of "cta_per_tile", "persistent_paired", "persistent_rotated",
-    "persistent_full", "none" (fa_b200_fwd_plan in include/fa_b200.h)."""
+    (name, CTAs launched) with name one of "cta_per_tile", "static", "dynamic", "none" (fa_b200_fwd_plan in
+    include/fa_b200.h)."""
     _check_qkv(Q, K, V)
     p = _fwd_params(Q, K, V, Q, None, causal, None)
     schedule, grid = ctypes.c_int32(-1), ctypes.c_int32(0)
