@@ -38,9 +38,14 @@ def test_wait_runs_out_is_reported_and_the_next_launch_is_correct(fa_lib):
     wt.fa_b200_strerror.restype = ctypes.c_char_p
 
     torch.manual_seed(3)
-    # one CTA: B = H = 1, N = 256 is a single pair of causal tiles; its first item needs two K tiles
+    # B = H = 1, N = 256: two causal tiles; the test build runs them as one CTA, whose first item needs two K tiles
     q, k, v = (torch.randn(1, 1, 256, 64, device="cuda").bfloat16() for _ in range(3))
-    assert cfa.plan(q, k, v) == ("static", 1)
+    assert cfa.plan(q, k, v) == ("cta_per_tile", 2)
+    schedule, grid = ctypes.c_int32(-1), ctypes.c_int32(0)
+    params = cfa._fwd_params(q, k, v, q, None, True, None)
+    wt.fa_b200_fwd_plan.argtypes = [ctypes.POINTER(_lib.FaParams), ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(ctypes.c_int32)]
+    assert wt.fa_b200_fwd_plan(ctypes.byref(params), ctypes.byref(schedule), ctypes.byref(grid)) == 0
+    assert (_lib.SCHEDULES[schedule.value], grid.value) == ("static", 1)
     good = cfa.forward(q, k, v)
     assert cfa.last_status() == 0
 
