@@ -341,3 +341,37 @@ def test_scores_far_below_zero(fa_lib, B, pos):
     got, want = runs
     assert torch.isfinite(got).all()
     assert ((got - want).norm() / want.norm()).item() <= 2 * 2.0 ** -8 * math.sqrt(8 + 4)
+
+
+@pytest.mark.parametrize("heads,B", [(25, 1), (25, 8), (12, 1), (12, 3), (1, 2)])
+@pytest.mark.parametrize("row", ["far from 0", "outlier in front", "outlier behind"])
+def test_layernorm_of_ill_conditioned_rows(fa_lib, heads, B, row):
+    """The first LayerNorm's output, taken from the K cache behind an identity projection, against fp64.  It is
+    rounded to bf16 twice (2^-9 each, as LayerNorm's output and as K, whose products with 1 and 0 are exact);
+    the variance may lose C * 2^-24 * 2 (see step_layernorm), half of that in the result."""
+    C = 64 * heads
+    model, _ = _model(C, heads, 1, 97, 64)
+    g = torch.Generator().manual_seed(heads)
+    flip = torch.randint(0, 2, (97, C), generator=g).float()
+    if row == "far from 0":
+        emb = 448 + 2 * flip                             # neighbours in bf16
+    else:
+        emb = (flip - 0.5) / 16
+        emb[:, 0 if row == "outlier in front" else C - 1] = 200.0
+    with torch.no_grad():
+        model.tok_emb.weight.copy_(emb)
+        model.pos_emb.weight.zero_()
+        blk = model.trf_blocks[0]
+        blk.att.W_key.weight.copy_(torch.eye(C))
+        blk.att.W_key.bias.zero_()
+        blk.norm1.scale.fill_(1)
+        blk.norm1.shift.zero_()
+    model.prepare_for_inference()
+    caches = model.allocate_kv_cache(B, 8)
+    ids = torch.randint(0, 97, (B, 1), generator=g).cuda()
+    with torch.no_grad():
+        assert model._step(ids, caches, 0) is not None
+    x = model.tok_emb.weight[ids[:, 0]].double()
+    want = (x - x.mean(-1, keepdim=True)) / torch.sqrt(x.var(-1, unbiased=False, keepdim=True) + 1e-5)
+    got = caches[0][0][:, 0].reshape(B, C).double()
+    assert ((got - want).abs() <= (2 * 2.0 ** -9 + C * 2.0 ** -24) * 1.01 * want.abs()).all()
