@@ -66,3 +66,56 @@ def test_wait_runs_out_is_reported_and_the_next_launch_is_correct(fa_lib):
     again = cfa.forward(q, k, v)
     assert cfa.last_status() == 0
     assert torch.equal(again, good)
+
+
+@pytest.mark.parametrize("B,pos", [(1, 5), (1, 900), (8, 70)])
+def test_step_gives_up_and_the_next_one_is_correct(fa_lib, monkeypatch, B, pos):
+    """The generation step: the test build's block 0 keeps back its words of the embedding, so that every block
+    waits for them until its wait runs out; the weight stream then waits for ring slots that nobody gives
+    back.  All of them give up, the launch returns, the workspace is made ready again."""
+    from types import SimpleNamespace
+
+    from tfg_flashattention_b200 import _lib, build, gpt2, step
+    from tfg_flashattention_b200 import custom_flash_attn as cfa
+    wt = ctypes.CDLL(build.build_wait_test_library())
+    for name in ("fa_b200_gpt_step", "fa_b200_last_status", "fa_b200_strerror"):
+        getattr(wt, name).argtypes, getattr(wt, name).restype = getattr(fa_lib, name).argtypes, getattr(fa_lib, name).restype
+
+    cfg = {"vocab_size": 503, "context_length": 1024, "emb_dim": 768, "n_heads": 12, "n_layers": 2, "drop_rate": 0.0,
+           "qkv_bias": True, "impl_type": "cuda"}
+    model = gpt2.init_random(gpt2.GPTModel(cfg, dtype=torch.bfloat16), seed=2).cuda().eval().prepare_for_inference()
+    ids = torch.randint(0, 503, (B, pos + 1), device="cuda")
+    caches = model.allocate_kv_cache(B, 1024)
+    with torch.no_grad():
+        model(ids[:, :pos], kv_caches=caches, pos=0)
+    plan = model._step_plan
+    workspace = plan.new_workspace(B)
+    good = model._step(ids[:, pos:], caches, pos, workspace=workspace)
+    assert good is not None and cfa.last_status() == 0
+
+    after = torch.full((B,), -1, dtype=torch.long, device="cuda")
+    scratch = [tuple(t.clone() for t in pair) for pair in caches]
+    t0 = time.perf_counter()
+    with monkeypatch.context() as m:
+        m.setattr(step, "_lib", SimpleNamespace(load=lambda: wt, FaGptStepParams=_lib.FaGptStepParams, strerror=_lib.strerror))
+        assert plan.step(ids[:, pos:], scratch, pos, workspace=workspace, next_ids=after) is not None      # launched
+    stream = torch.cuda.current_stream().cuda_stream
+    code = wt.fa_b200_last_status(0, stream)
+    elapsed = time.perf_counter() - t0
+    assert code & ~0xff == WATCHDOG_BASE and (code & 0xff) in (17, 18, 19), hex(code)
+    assert b"generation step" in wt.fa_b200_strerror(code)
+    assert elapsed < 2.0, f"the kernel took {elapsed:.2f} s to give up"
+    assert wt.fa_b200_last_status(0, stream) == 0
+    for new, old in zip(scratch, caches):              # no cached row but the step's own was written
+        for a, b in zip(new, old):
+            keep = torch.arange(1024, device="cuda") != pos
+            assert torch.equal(a[:, keep], b[:, keep])
+
+    # whoever asks for the status of the library that gave up gets its workspaces back in order
+    with monkeypatch.context() as m:
+        m.setattr(cfa, "_lib", SimpleNamespace(load=lambda: SimpleNamespace(fa_b200_last_status=lambda *a: code),
+                                               WATCHDOG_BASE=_lib.WATCHDOG_BASE))
+        workspace.fill_(1)
+        assert cfa.last_status() == code and (workspace == 0).all()
+    again = model._step(ids[:, pos:], caches, pos, workspace=workspace)
+    assert cfa.last_status() == 0 and torch.equal(again, good)

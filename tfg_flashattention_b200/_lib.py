@@ -11,6 +11,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libfa_b200.so")
 
 ABI_VERSION = 6
+WATCHDOG_BASE = 0x10000      # status words above it are codes of waits that ran out
 
 
 class FaParams(ctypes.Structure):

@@ -109,8 +109,16 @@ static_assert(kStepBlocks * 16 * 256 <= kStepStageBytes, "cached rows fit a stag
 // atomic per part: 1 x 900 rows, small / XL, us per step: unsplit 204 / 997, parts of 384 191 / 927, of
 // 192 191 / 956.
 constexpr int kStepSplitRows = 384;
-constexpr uint32_t kStepBarPolls = 1u << 24;          // bounds of the waits: about 65 clocks a poll of a barrier ...
-constexpr uint32_t kStepWordPolls = 1u << 21;         // ... and a trip to L2 a poll of exchange words: half a second
+// Bounds of the waits: of barriers by the clock (a poll of one may suspend the thread), of exchange words by
+// their number (a trip to L2 each, 0.3 to 1 us).  A wait behind one that has run out runs out as well.
+#ifdef FA_WAIT_TEST
+// Test build: short waits, and block 0 keeps back its words of the embedding, for which every block waits.
+constexpr uint32_t kStepWaitNs = 2u * 1000 * 1000, kStepWordPolls = 1u << 12;
+constexpr bool kStepKeepsBack = true;
+#else
+constexpr uint32_t kStepWaitNs = 500u * 1000 * 1000, kStepWordPolls = 1u << 21;
+constexpr bool kStepKeepsBack = false;
+#endif
 
 // Rows of a stage lie 64 bytes (mod 128) apart: the 8 lanes of a 128-bit load phase read two rows of
 // 64 bytes each, which then cover all banks (an even `units` is at most 24).
@@ -306,8 +314,17 @@ __device__ __forceinline__ void step_give_up(StepSmem& sm, uint32_t id) {
 // A bounded wait of a converged warp, small because it is inlined in the loops.
 __device__ __forceinline__ bool step_wait(uint32_t bar, uint32_t parity, StepSmem& sm, uint32_t id) {
   bool ok = false;
+  uint32_t since = 0;
 #pragma unroll 1
-  for (uint32_t polls = 0; polls < kStepBarPolls && !ok; ++polls) ok = mbar_try_wait(bar, parity);
+  for (uint32_t polls = 0; polls < (1u << 26); ++polls) {
+    ok = mbar_try_wait(bar, parity);
+    if (ok) break;
+    if ((polls & 63u) == 63u) {
+      const uint32_t now = globaltimer_lo_ns();
+      if (since == 0) since = now;
+      else if (now - since > kStepWaitNs) break;
+    }
+  }
   ok = __all_sync(0xffffffffu, ok);
   if (!ok) step_give_up(sm, id);
   return ok;
@@ -1056,7 +1073,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) fa_gpt_step_kernel(const __gr
         const float v = __bfloat162float(__float2bfloat16_rn(
             __bfloat162float(p.tok_emb[id * C + n]) + __bfloat162float(p.pos_emb[static_cast<long long>(pos) * C + n])));
         sm.own[threadIdx.x] = v;
-        step_put(p.x_mlp + tok * C + n, v, generation % 65535u + 1u);
+        if (!kStepKeepsBack || blockIdx.x > 0) step_put(p.x_mlp + tok * C + n, v, generation % 65535u + 1u);
       }
     }
     step_prefetch(sm, p, 0);

@@ -361,7 +361,12 @@ def forward_host(Q, K, V, out=None, causal=True, softmax_scale=None, device=None
 
 def last_status(device=None) -> int:
     """Synchronise the current stream of `device` and return (and clear) the kernel's watchdog
-    word: 0 when every kernel since the last call ran to completion."""
+    word: 0 when every kernel since the last call ran to completion.  After a code the device is
+    synchronised and the generation step's workspaces on it are made ready again."""
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     idx = dev.index if dev.index is not None else torch.cuda.current_device()
-    return _lib.load().fa_b200_last_status(idx, torch.cuda.current_stream(dev).cuda_stream)
+    code = _lib.load().fa_b200_last_status(idx, torch.cuda.current_stream(dev).cuda_stream)
+    if code > _lib.WATCHDOG_BASE:
+        from . import step
+        step.clear_workspaces(torch.device("cuda", idx))
+    return code

@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes
 import operator
+import weakref
 from collections import OrderedDict
 
 import torch
@@ -23,6 +24,19 @@ MAX_WIDTH = 1600
 MAX_VOCAB = 1 << 24        # fewer than that
 PLAIN_TENSORS = (torch.Tensor, nn.Parameter)     # a subclass may keep its numbers in another form
 MAX_WORKSPACES = 8         # streams that keep a workspace (about 1 MB each)
+
+
+_workspaces = weakref.WeakValueDictionary()     # every workspace that is still somebody's
+
+
+def clear_workspaces(device):
+    """Zero the workspaces on a device, after a kernel gave up a wait: it may have left counters in them that
+    the next launch would count on from."""
+    torch.cuda.synchronize(device)
+    for ws in list(_workspaces.values()):
+        if ws.device == device:
+            ws.zero_()
+    torch.cuda.synchronize(device)
 
 
 class ModelWatch:
@@ -188,7 +202,11 @@ class StepPlan:
     def new_workspace(self, batch):
         """A zeroed workspace, or None for a batch that the kernel does not take."""
         need = _lib.load().fa_b200_gpt_step_workspace_bytes(batch, self.heads)
-        return torch.zeros(need, dtype=torch.uint8, device=self.device) if need > 0 else None
+        if need <= 0:
+            return None
+        ws = torch.zeros(need, dtype=torch.uint8, device=self.device)
+        _workspaces[id(ws)] = ws
+        return ws
 
     def _workspace(self, batch, stream):
         """A zeroed workspace that only this stream uses (a launch leaves its counters at zero)."""
