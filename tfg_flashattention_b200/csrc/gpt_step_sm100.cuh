@@ -95,7 +95,6 @@ constexpr int kStepChunkUnits = 25;                   // columns per stage: at m
 constexpr int kStepStageBytes = kStepTile * kStepChunkUnits * 64;
 constexpr int kStepStages = 8;                        // one per warp: a group of tiles has at most as many
 static_assert(kStepStages >= kStepWarps, "a wait by parity is for the slot's next stage only while the one before is not given back");
-constexpr int kStepAhead = 1;                         // operations: weights sent for to L2 in advance
 constexpr uint32_t kStepAheadBytes = 192 * 1024, kStepAheadPiece = 2048;
 constexpr int kStepMaxWidth = 1600;                   // d_model: the fragments of 8 rows fill sm.x
 constexpr int kStepMaxUnits = kStepMaxWidth / kStepUnit;
@@ -1045,12 +1044,11 @@ __global__ void __launch_bounds__(kStepThreads, 1) fa_gpt_step_kernel(const __gr
     StepRing ring;
     uint32_t issued = 0;
     bool ok = true;
-    for (int i = 1; i < kStepAhead; ++i) step_ahead(sm, p, i, sw, lane);
 #pragma unroll 1
     for (int i = 0; i <= 4 * p.n_layers && ok; ++i) {
       int op;
       const __nv_bfloat16* w = step_weight(sm, p, i, op);
-      step_ahead(sm, p, i + kStepAhead, sw, lane);
+      step_ahead(sm, p, i + 1, sw, lane);
       ok = step_stream(sm, p, ring, issued, w, op, sw);
       if (ok && op == kStepQkv) ok = step_stream_rows(sm, p, ring, issued, i >> 2, sw, lane);
     }
