@@ -939,7 +939,7 @@ const char* fa_b200_strerror(int code) {
     case FA_B200_ERR_ARCH: return "fa_b200: device is not compute capability 10.x (B200); there is no fallback";
     case FA_B200_ERR_TENSORMAP: return "fa_b200: the driver rejected a TMA tensor map (check strides and sizes)";
     case FA_B200_ERR_DRIVER: return "fa_b200: cuTensorMapEncodeTiled is not available from this driver";
-    case FA_B200_ERR_STATIC_SCRATCH: return "fa_b200: this decode problem is past the size limit of fa_b200_decode_static (FA_B200_STATIC_SCRATCH_BYTES); use fa_b200_decode_direct";
+    case FA_B200_ERR_STATIC_SCRATCH: return "fa_b200: this decode problem is past the limit of fa_b200_decode_static, what its original form fitted into a built-in buffer (FA_B200_STATIC_SCRATCH_BYTES); use fa_b200_decode_direct";
     case FA_B200_ERR_ALIAS: return "fa_b200: an output buffer overlaps an input it must not overlap";
     case FA_B200_ERR_WORKSPACE: return "fa_b200: workspace is NULL, too small or (decode) not 16-byte aligned";
     case FA_B200_ERR_BUILD: return "fa_b200: the kernel image does not match this library's launch configuration; rebuild it";
