@@ -375,3 +375,21 @@ def test_layernorm_of_ill_conditioned_rows(fa_lib, heads, B, row):
     want = (x - x.mean(-1, keepdim=True)) / torch.sqrt(x.var(-1, unbiased=False, keepdim=True) + 1e-5)
     got = caches[0][0][:, 0].reshape(B, C).double()
     assert ((got - want).abs() <= (2 * 2.0 ** -9 + C * 2.0 ** -24) * 1.01 * want.abs()).all()
+
+
+@pytest.mark.parametrize("kind", ["rows", "row stride"])
+def test_caches_past_the_limits_go_layer_by_layer(fa_lib, kind):
+    """More rows, or rows further apart, than the one-launch step takes (0.5 and 4.3 GB a cache)."""
+    model, _ = _model(64, 1, 1, 97, 64)
+    shape, stride = ((1, (1 << 22) + 8, 1, 64), (64, 64, 64, 1)) if kind == "rows" else ((1, 2, 1, 64), (64, 1 << 31, 64, 1))
+    far = [tuple(torch.empty_strided(shape, stride, dtype=torch.bfloat16, device="cuda") for _ in range(2))]
+    near = model.allocate_kv_cache(1, 2)
+    ids = torch.randint(0, 97, (1, 2), device="cuda")
+    with torch.no_grad():
+        model._step(ids[:, :1], near, 0)
+        for a, b in zip(far[0], near[0]):
+            a[:, 0] = b[:, 0]
+        assert model._step(ids[:, 1:], far, 1) is None
+        got = model(ids[:, 1:], kv_caches=far, pos=1).float()
+        want = model(ids[:, 1:], kv_caches=near, pos=1).float()
+    assert ((got - want).norm() / want.norm()).item() <= 2 * 2.0 ** -8 * math.sqrt(8 + 4)

@@ -22,6 +22,8 @@ MAX_PAIRS = 256            # sequences x heads
 MAX_LAYERS = 64
 MAX_WIDTH = 1600
 MAX_VOCAB = 1 << 24        # fewer than that
+MAX_CACHE_ROWS = 1 << 22
+MAX_STRIDE = (1 << 31) - 1    # of a cache's rows and heads
 PLAIN_TENSORS = (torch.Tensor, nn.Parameter)     # a subclass may keep its numbers in another form
 MAX_WORKSPACES = 8         # streams that keep a workspace (about 1 MB each)
 
@@ -196,6 +198,8 @@ class StepPlan:
                     return None
                 table[j * self.layers + i] = t.data_ptr()
         if any(s % 8 for s in stride[:3]) or any(s <= 0 for s in stride[:3]):
+            return None
+        if shape[1] > MAX_CACHE_ROWS or max(stride[1], stride[2]) > MAX_STRIDE:
             return None
         return table, shape[1], stride
 
