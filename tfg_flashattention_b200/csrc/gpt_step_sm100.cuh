@@ -310,19 +310,16 @@ __device__ __forceinline__ void step_give_up(StepSmem& sm, uint32_t id) {
     *abort = kWatchdogBase | id;
   }
 }
-// A bounded wait of a converged warp, small because it is inlined in the loops.
+// A bounded wait of a converged warp, small because it is inlined in the loops.  (A step of GPT-2 small, 1
+// sequence / XL, 8 sequences at 900 rows, us: 148.4 / 1451 with the clock read at every poll but the first,
+// 148.8 / 1455 at every 256th, 152.5 / 1466 at every 64th in one loop; by a count of polls 147.9 / 1460.)
 __device__ __forceinline__ bool step_wait(uint32_t bar, uint32_t parity, StepSmem& sm, uint32_t id) {
-  bool ok = false;
-  uint32_t since = 0;
+  bool ok = mbar_try_wait(bar, parity);
+  if (!ok) {
+    const uint32_t since = globaltimer_lo_ns();
 #pragma unroll 1
-  for (uint32_t polls = 0; polls < (1u << 26); ++polls) {
-    ok = mbar_try_wait(bar, parity);
-    if (ok) break;
-    if ((polls & 63u) == 63u) {
-      const uint32_t now = globaltimer_lo_ns();
-      if (since == 0) since = now;
-      else if (now - since > kStepWaitNs) break;
-    }
+    do ok = mbar_try_wait(bar, parity);
+    while (!ok && globaltimer_lo_ns() - since < kStepWaitNs);
   }
   ok = __all_sync(0xffffffffu, ok);
   if (!ok) step_give_up(sm, id);
