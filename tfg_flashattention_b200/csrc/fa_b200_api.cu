@@ -231,6 +231,7 @@ struct FwdPlan {
   int n_qtiles, kv_tiles;
   long long items;     // B * H * n_qtiles
   unsigned grid;       // launched
+  bool early;          // let the next kernel of the stream start while this one runs
 };
 
 FwdPlan plan_fwd(const fa_b200_params* p, const DeviceState& st) {
@@ -258,6 +259,18 @@ FwdPlan plan_fwd(const fa_b200_params* p, const DeviceState& st) {
     pl.schedule = fa::kDynamic;
   }
   pl.grid = static_cast<unsigned>(pl.schedule == fa::kStatic ? slots : pl.items);
+  // The next kernel's CTAs are placed when this one says so, around the slots that it holds: where it leaves
+  // SMs free, some get two of them and others none, and two share an SM's pipes.  Back to back, early / at the
+  // end / a kernel without either (us): N = 8192 full, 64 items 84.3 / 67.2 / 69.8; N = 2048 causal, 256 items
+  // 25.7 / 21.6 / 24.7; N = 1300 causal, 385 items 19.1 / 17.7 / 27.0.  So early only
+  // - for single tiles, whose time is their start-up (N = 72, 290 items: 5.2 / 5.5 / 8.3), and for up to a quarter
+  //   of the SMs, where nobody has to share (N = 512 causal, 12 items 7.4 / 7.6 / 11.6; but N = 1300 full, 44 items
+  //   17.4 / 14.8 / 16.5);
+  // - where others wait for slots anyway: dynamic; full with more items than SMs (N = 512, 256 items: 9.6 /
+  //   10.6 / 12.4); causal with a second wave, as long as it is long enough for its tiles (N = 1024, 384 items
+  //   14.4 / 15.2 / 20.6, but 328 items 14.3 / 13.4; N = 640, 330 items 10.5 / 11.3 / 16.5).
+  pl.early = pl.kv_tiles == 1 || 4 * pl.items <= st.sm_count || pl.schedule == fa::kDynamic ||
+             (causal ? pl.kv_tiles <= 8 && pl.items >= slots + 16 * (pl.kv_tiles - 3) : pl.items > st.sm_count);
 #ifdef FA_WAIT_TEST    // the test's problem, one causal head of two tiles, as one CTA: what waits for what is then known
   if (causal && p->B * p->H == 1 && pl.n_qtiles == 2) {
     pl.schedule = fa::kStatic;
@@ -338,6 +351,7 @@ int fa_b200_fwd(const fa_b200_params* p) {
   kp.scale_log2 = scale * 1.4426950408889634f;
   kp.status = st.status;
   kp.n_items = static_cast<int>(pl.items);
+  kp.early = pl.early ? 1 : 0;
   const int first_wave = static_cast<int>(pl.items < st.resident_ctas ? pl.items : st.resident_ctas);
   kp.mirror_from = st.sm_count;
   kp.mirror_to = kp.causal ? first_wave : 0;

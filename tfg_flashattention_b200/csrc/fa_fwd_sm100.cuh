@@ -175,6 +175,7 @@ struct FwdParams {
   int group_items, last_group;   // ... their work items; heads of the last group
   FastDiv div_group_items, div_group, div_last_group;
   int causal;
+  int early;                  // the next kernel of the stream may start beside this one
   float scale_log2;           // softmax_scale * log2(e)
   unsigned int* status;       // [4] watchdog words in global memory
 };
@@ -338,7 +339,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     sm.items[threadIdx.x] = has ? make_int4(t.q_row, t.ns, t.h, t.b) : make_int4(0, 0, 0, 0);
   }
   // everything above touches no global memory and may run beside the previous kernel's last CTAs
-  pdl_trigger();
+  if (p.early) pdl_trigger();      // (otherwise: when the last CTA has ended)
   pdl_wait();
   tc_fence_before();
   __syncthreads();
