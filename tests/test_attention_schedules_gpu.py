@@ -81,3 +81,39 @@ def test_taking_over_while_the_first_wave_waits(fa_lib, B, N):
         torch.cuda.synchronize()
         assert cfa.last_status() == 0
         assert torch.equal(o, want) and torch.equal(lse, want_lse)
+
+
+def test_captured_launches_depend_early_only_on_the_librarys_own(fa_lib):
+    """In a graph, an edge of programmatic dependent launch between two of the library's kernels, a plain one
+    behind any other; two captures in a row; replays give what the calls give."""
+    import ctypes
+    from tfg_flashattention_b200 import block_ops
+    from tfg_flashattention_b200 import custom_flash_attn as cfa
+    g = torch.Generator(device="cuda").manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    x, scale, shift, q = rnd(8, 256), rnd(256), rnd(256), rnd(1, 4, 300, 64)
+
+    def work():
+        a = x + 1
+        b = block_ops.add_layernorm(a, None, scale, shift)                  # behind torch's
+        c = block_ops.add_layernorm(b, None, scale, shift)                  # behind ours
+        d = cfa.forward(q, q, q)                                            # ours
+        e = cfa.forward(d, d, d)                                            # ours
+        f = e + 1
+        return c, f, cfa.decode(f[:, :, 0].contiguous(), f, f, 300)         # behind torch's
+
+    want = work()
+    for _ in range(2):
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            got = work()
+        n = ctypes.c_size_t(64)
+        nodes, data = (ctypes.c_void_p * 64)(), (ctypes.c_uint8 * 8 * 64)()        # CUgraphEdgeData: ports, type, padding
+        assert ctypes.CDLL("libcuda.so.1").cuGraphGetEdges_v2(ctypes.c_void_p(graph.raw_cuda_graph()), nodes, (ctypes.c_void_p * 64)(),
+                                                              data, ctypes.byref(n)) == 0
+        assert sum(data[i][2] == 1 for i in range(n.value)) == 3 and n.value >= 6   # 1: CU_GRAPH_DEPENDENCY_TYPE_PROGRAMMATIC
+        graph.instantiate()
+        for t in got:
+            t.zero_()
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
