@@ -51,9 +51,9 @@ from tfg_flashattention_b200 import workloads  # noqa: E402
 METRIC = "causal_attention_fwd_tflops"
 UNIT = "TFLOP/s"
 # DRAM bytes per launch of fa_fwd_kernel on the headline workload (dram__bytes_read.sum +
-# dram__bytes_write.sum).  Captured with ncu at B=12 (118.03 + 18.10 MB per launch) and scaled by
+# dram__bytes_write.sum).  Captured with ncu at B=12 (118.03 + 19.01 MB per launch) and scaled by
 # 32/12 to the benchmark's B=32: every (batch, head) is independent, so traffic grows in proportion.
-NCU_TRAFFIC_BYTES_PER_LAUNCH = 136.13e6 * 32 / 12
+NCU_TRAFFIC_BYTES_PER_LAUNCH = 137.04e6 * 32 / 12
 NCU_TRAFFIC_NOTE = ("ncu capture at B=12 scaled by 32/12; reads equal Q+K+V exactly, writes are a lower bound "
                     "(part of O is still in L2 when the small capture's kernel ends)")
 E2E_CHUNKS = 8                # batch slices the host-buffer call pipelines through PCIe
@@ -805,8 +805,8 @@ def main():
 
     # ---------------------------------------------------------------- the reference's own benchmark
     # "time for 20 tokens" (model_inference.py:444-465): B=1, a ~70-token prompt, 20 new tokens,
-    # here with random-init weights and random token ids; with the K/V cache + decode kernel, and
-    # with the reference's recompute loop through the prefill kernel.
+    # here with random-init weights and random token ids; with the K/V cache and the one-launch step,
+    # and with the reference's recompute loop through the prefill kernel.
     gen = []
     if not args.no_sweep and rank == 0:
         from tfg_flashattention_b200 import gpt2
@@ -816,8 +816,8 @@ def main():
             model.prepare_for_inference()
             prompt = torch.randint(0, cfg["vocab_size"], (gb, gp), generator=torch.Generator().manual_seed(123)).cuda()
             row = {"model": name, "prompt_tokens": gp, "new_tokens": 20, "batch": gb, "dtype": "bf16",
-                   "note": "eager B=1 steps are launch-bound (Python + ~15 launches per layer and token); "
-                           "kv_cache_graph_ms replays one recorded CUDA graph per token (prefill eager)"}
+                   "note": "a step is one kernel launch (fa_b200_gpt_step), the prompt runs eagerly; "
+                           "kv_cache_graph_ms: with a GenerationSession kept across calls, kv_cache_ms: default arguments"}
             session = gpt2.GenerationSession(model, gb, 1024)      # caches + recorded decode step, reused
             for label, kw in (("kv_cache_graph_ms", {"session": session}), ("kv_cache_ms", {}),
                               ("recompute_ms", {"use_cache": False})):

@@ -86,10 +86,11 @@ def test_step_matches_fp32(fa_lib, width, heads, layers, vocab, B, pos, bias):
     _check(*_model(width, heads, layers, vocab, 256, bias), B, pos)
 
 
-@pytest.mark.parametrize("B,heads,pos", [(1, 1, 2047), (1, 1, 2048), (2, 2, 5000),
-                                         (1, 12, 272), (1, 12, 289),       # pair per CTA; one block more: parts of 8
-                                         (8, 25, 193), (8, 25, 901),       # three units in a CTA, owners and parts
-                                         (8, 12, 900), (5, 16, 480)])      # fewer pairs than CTAs, uneven shares
+@pytest.mark.parametrize("B,heads,pos", [(1, 1, 2047), (1, 1, 2048), (2, 2, 5000),     # pairs in parts, more than 8 of them
+                                         (1, 12, 767), (1, 12, 768),       # the border: one CTA a pair, two
+                                         (1, 12, 272), (1, 12, 289),       # a pair a CTA: whole blocks of 16 rows, one more
+                                         (8, 25, 193), (8, 25, 901),       # 200 pairs: two in some CTAs
+                                         (8, 12, 900), (5, 16, 480)])      # fewer pairs than CTAs, not enough to split
 def test_step_long_cache_is_split_over_ctas(fa_lib, B, heads, pos):
     _check(*_model(64 * heads, heads, 1, 211, pos + 8), B, pos)
 

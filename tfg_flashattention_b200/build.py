@@ -55,9 +55,10 @@ WAIT_TEST_LIB = os.path.join(HERE, "libfa_b200_waittest.so")
 
 
 def build_wait_test_library(force: bool = False) -> str:
-    """The library compiled with -DFA_WAIT_TEST, for tests/test_watchdog_gpu.py only: every bounded
-    wait in the attention kernel gives up after 2 ms and the TMA producer leaves out one K tile, so
-    a launch through it runs into the watchdog by construction, reports it and returns."""
+    """The library compiled with -DFA_WAIT_TEST, for tests/test_watchdog_gpu.py only: every bounded wait gives
+    up after about 2 ms, the attention kernel's TMA producer leaves out one K tile and the generation step's
+    first block keeps back some of its words, so a launch through it runs into the watchdog by
+    construction, reports it and returns."""
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))]
     if (not force and os.path.exists(WAIT_TEST_LIB)
             and all(os.path.getmtime(d) <= os.path.getmtime(WAIT_TEST_LIB) for d in deps)):

@@ -250,7 +250,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
   // side by side share a head's K/V in L2.  Causal: tile t costs t+1 K/V tiles, the heaviest come
   // first, through groups of heads whose K and V fit L2 together: all heads' last tiles, then all the
   // ones before, ...  (Head by head, a heavy tile of the last head starts when everybody else is
-  // nearly through: B = 4 H = 25 N = 16384 took 4.59 ms instead of 3.91.)
+  // nearly through: B = 4 H = 12 N = 1300 took 32.2 us instead of 24.2, B = 4 H = 25 N = 4096 331 instead of 302.)
   //   one item    a CTA per item, the hardware places them as others end;
   //   static      a CTA per resident slot, the list dealt back and forth over the grid;
   //   dynamic     a CTA per item is launched, but a running CTA takes over one that has not started
