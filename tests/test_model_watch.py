@@ -93,3 +93,29 @@ def test_calls_that_somebody_waits_for(pick):
         handle.remove()
     pick(model).forward = lambda *a, **k: None           # of this module alone
     assert not watch.holds() and not plain_modules(model)
+
+
+def test_copies_of_a_model_make_their_own():
+    """A copy must not take over what belongs to the original's addresses, nor a watch over dictionaries that are
+    no module's: whether it is pickled, copied, or a replica that shares all attributes but the modules."""
+    import io
+    model = _model()
+    model._fused_blocks = True                           # (of a model on a GPU)
+    seen = []
+    make = lambda m: (seen.append(m), object())[1]
+    mine = model._from_modules("x", make)
+    assert model._from_modules("x", make) is mine and seen == [model]
+    buffer = io.BytesIO()
+    torch.save(model, buffer)
+    buffer.seek(0)
+    replica = model._replicate_for_data_parallel()
+    replica._modules = dict(model._modules)
+    for other in (copy.deepcopy(model), torch.load(buffer, weights_only=False), replica):
+        assert other._from_modules("x", make) is not mine and seen[-1] is other
+    with torch.no_grad():
+        ids = torch.zeros(1, 4, dtype=torch.long)
+        for m in (model, copy.deepcopy(model)):
+            m._fused_blocks = False
+            for blk in m.trf_blocks:
+                blk.att.impl_type = "manual"
+        assert copy.deepcopy(model)(ids).shape == (1, 4, 97)

@@ -322,6 +322,9 @@ class GPTModel(nn.Module):
         self._made = {}
         return self
 
+    def __getstate__(self):                     # pickled or copied: addresses and identities stay behind
+        return {**self.__dict__, "_made": {}, "_recorded_tables": []}
+
     def _apply(self, fn, *args, **kwargs):      # .to(), .cuda(), .half(): the parameters move
         self._made = {}
         return super()._apply(fn, *args, **kwargs)
@@ -332,7 +335,7 @@ class GPTModel(nn.Module):
         taken out again).  None as well while there are hooks on modules that would not be called."""
         made = self.__dict__.setdefault("_made", {})
         kept = made.get(name)
-        if kept is None or not kept[0].holds():
+        if kept is None or kept[0].top is not self._modules or not kept[0].holds():
             if torch.cuda.is_available() and torch.cuda.is_current_stream_capturing():
                 return None                     # making copies to the GPU: not while a graph is recorded
             watch = ModelWatch(self)            # first: what changes meanwhile is seen at the next call

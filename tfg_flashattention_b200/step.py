@@ -72,6 +72,7 @@ class ModelWatch:
         self.hooks += [nn.modules.module._global_forward_hooks, nn.modules.module._global_forward_pre_hooks]
         self.dicts, self.keys, self.values = (list(part) for part in zip(*entries))
         self.tensors, self.addresses = tensors, [t.data_ptr() for t in tensors]
+        self.top = model._modules           # (a shallow copy of a model has its own)
         self.blocks = model.trf_blocks._modules
         self.n_blocks = len(self.blocks)
 
