@@ -199,3 +199,18 @@ def test_native_loop_of_weights_in_a_flat_buffer(fa_lib, torch_binding, offset):
         model._native_blocks = lambda *a: None
         want = model(ids).float()
     assert ((got - want).norm() / want.norm()).item() <= 2 * 2.0 ** -9 * (8 * 2 + 4) ** 0.5
+
+
+def test_no_blocks_and_another_device(fa_lib, torch_binding):
+    """A model without blocks (all cut away) still gives its logits, with caches or without; input that is not
+    where the weights are is left to the modules, which refuse it."""
+    model = _model()
+    ids = torch.randint(0, 503, (2, 9), device="cuda")
+    with torch.no_grad():
+        assert model._native_blocks(torch.zeros(2, 9, 256, dtype=torch.bfloat16), None, 0) is None
+        model.trf_blocks = model.trf_blocks[:0]
+        x = model.tok_emb(ids) + model.pos_emb(torch.arange(9, device="cuda"))
+        want = torch.nn.functional.linear(model.final_norm(x), model.out_head.weight).float()
+        for caches in (None, []):
+            got = model(ids, kv_caches=caches).float()
+            assert ((got - want).norm() / want.norm()).item() <= 2 * 2.0 ** -8

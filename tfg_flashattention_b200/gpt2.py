@@ -388,7 +388,7 @@ class GPTModel(nn.Module):
         if width != 64 * heads:
             return None
         rows = self._block_rows
-        if rows is None:
+        if not rows or rows[0][0].device != x.device:
             return None
         if kv_caches is not None:
             # what the cache kernel takes, the same in all layers; any other cache is written by the modules (one
