@@ -170,3 +170,27 @@ def test_linear_small_prologue_rejects(fa_lib):
         linear_small(x, w, ln_scale=one, ln_shift=one)            # K > 2048 with a prologue
     with pytest.raises(RuntimeError):
         linear_small(x[:, :64].contiguous(), w[:, :64].contiguous(), ln_scale=one[:64].contiguous())
+
+
+@pytest.mark.parametrize("cols", [768, 1280, 1288, 1600, 2048])
+def test_add_layernorm_is_the_same_for_any_number_of_rows(fa_lib, cols):
+    """From 1281 columns on the kernel fetches scale and shift ahead only up to two CTAs of 8 rows per SM: the same
+    rows above and below that border, to the bit, in the library's other binding too."""
+    from tfg_flashattention_b200 import custom_flash_attn
+    from tfg_flashattention_b200.block_ops import add_layernorm
+    border = 16 * torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    a, r = (torch.randn(border + 9, cols, device="cuda", generator=g).bfloat16() for _ in range(2))
+    w, b = (torch.randn(cols, device="cuda", generator=g).bfloat16() for _ in range(2))
+    whole = add_layernorm(a, r, w, b)
+    s = (a.float() + r.float()).bfloat16().float()
+    want = torch.nn.functional.layer_norm(s, (cols,), w.float(), b.float(), 1e-5)
+    assert torch.equal(whole[0].float(), s)
+    assert ((whole[1].float() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all()
+    for rows in (border, border + 1, 5):
+        custom_flash_attn.set_binding("ctypes" if rows == 5 else "auto")
+        try:
+            part = add_layernorm(a[-rows:].contiguous(), r[-rows:].contiguous(), w, b)
+        finally:
+            custom_flash_attn.set_binding("auto")
+        assert torch.equal(part[0], whole[0][-rows:]) and torch.equal(part[1], whole[1][-rows:])

@@ -622,10 +622,13 @@ extern "C++" {
 namespace {
 
 template <int kVec>
-cudaError_t launch_add_ln(const fa::AddLnParams& kp, cudaStream_t stream) {
+cudaError_t launch_add_ln(const fa::AddLnParams& kp, cudaStream_t stream, int sm_count) {
   const long long ctas = (kp.rows + fa::kLnWarpsPerCta - 1) / fa::kLnWarpsPerCta;
-  return launch_kernel(&fa::fa_add_layernorm_kernel<kVec>, dim3(static_cast<unsigned>(ctas)), fa::kLnWarpsPerCta * 32, 0,
-                       stream, 1, kp);
+  // (from 6 vectors a lane on only where no SM has a third CTA to lose; see the kernel)
+  auto kernel = &fa::fa_add_layernorm_kernel<kVec, true>;
+  if constexpr (kVec > 5)
+    if (ctas > 2 * sm_count) kernel = &fa::fa_add_layernorm_kernel<kVec, false>;
+  return launch_kernel(kernel, dim3(static_cast<unsigned>(ctas)), fa::kLnWarpsPerCta * 32, 0, stream, 1, kp);
 }
 
 }  // namespace
@@ -665,14 +668,14 @@ int fa_b200_add_layernorm(const fa_b200_add_layernorm_params* p) {
   const cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   cudaError_t e;
   switch ((p->cols + 255) / 256) {   // 16-byte vectors per lane
-    case 1: e = launch_add_ln<1>(kp, stream); break;
-    case 2: e = launch_add_ln<2>(kp, stream); break;
-    case 3: e = launch_add_ln<3>(kp, stream); break;
-    case 4: e = launch_add_ln<4>(kp, stream); break;
-    case 5: e = launch_add_ln<5>(kp, stream); break;
-    case 6: e = launch_add_ln<6>(kp, stream); break;
-    case 7: e = launch_add_ln<7>(kp, stream); break;
-    default: e = launch_add_ln<8>(kp, stream); break;
+    case 1: e = launch_add_ln<1>(kp, stream, st.sm_count); break;
+    case 2: e = launch_add_ln<2>(kp, stream, st.sm_count); break;
+    case 3: e = launch_add_ln<3>(kp, stream, st.sm_count); break;
+    case 4: e = launch_add_ln<4>(kp, stream, st.sm_count); break;
+    case 5: e = launch_add_ln<5>(kp, stream, st.sm_count); break;
+    case 6: e = launch_add_ln<6>(kp, stream, st.sm_count); break;
+    case 7: e = launch_add_ln<7>(kp, stream, st.sm_count); break;
+    default: e = launch_add_ln<8>(kp, stream, st.sm_count); break;
   }
   return static_cast<int>(e);
 }

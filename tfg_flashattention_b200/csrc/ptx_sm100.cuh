@@ -49,6 +49,25 @@ __device__ __forceinline__ void reg_dealloc() {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// 16 bytes of an input that this kernel writes nowhere, by an ordinary load that need not stay behind the stores
+// in front of it: `load_input` where the compiler likes (but not above the `ordered` that gave the address, which
+// stands behind a pdl_wait), `load_input_here` where it is written.
+__device__ __forceinline__ const uint4* ordered(const void* p) {
+  uint64_t a;
+  asm volatile("mov.u64 %0, %1;" : "=l"(a) : "l"(reinterpret_cast<uint64_t>(p)) : "memory");
+  return reinterpret_cast<const uint4*>(a);
+}
+__device__ __forceinline__ uint4 load_input(const uint4* p) {
+  uint4 r;
+  asm("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(reinterpret_cast<uint64_t>(p)));
+  return r;
+}
+__device__ __forceinline__ uint4 load_input_here(const uint4* p) {
+  uint4 r;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(reinterpret_cast<uint64_t>(p)));
+  return r;
+}
+
 // ----------------------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
