@@ -49,9 +49,9 @@ REPLACED = {
 def test_replacements_are_seen(what):
     model = _model()
     watch = ModelWatch(model)
-    assert watch.holds()
+    assert watch.holds(model)
     REPLACED[what](model)
-    assert not watch.holds()
+    assert not watch.holds(model)
     assert StepPlan.make(model) is None                  # (not on a GPU; and whatever was replaced, no error)
 
 
@@ -63,7 +63,7 @@ def test_what_is_no_replacement():
     model.to("cpu").requires_grad_(False)
     model.load_state_dict(model.state_dict())
     model.trf_blocks[0].att.W_query.bias = None          # (its part of the fused projection is what is used)
-    assert watch.holds()
+    assert watch.holds(model)
 
 
 def test_modules_of_other_kinds():
@@ -89,10 +89,10 @@ def test_calls_that_somebody_waits_for(pick):
                      nn.modules.module.register_module_forward_hook):
         assert not watch.hooked()
         handle = register(lambda *a: None)
-        assert watch.hooked() and watch.holds()
+        assert watch.hooked() and watch.holds(model)
         handle.remove()
     pick(model).forward = lambda *a, **k: None           # of this module alone
-    assert not watch.holds() and not plain_modules(model)
+    assert not watch.holds(model) and not plain_modules(model)
 
 
 def test_copies_of_a_model_make_their_own():

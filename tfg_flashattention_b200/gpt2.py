@@ -335,10 +335,11 @@ class GPTModel(nn.Module):
         taken out again).  None as well while there are hooks on modules that would not be called."""
         made = self.__dict__.setdefault("_made", {})
         kept = made.get(name)
-        if kept is None or kept[0].top is not self._modules or not kept[0].holds():
+        if kept is None or not kept[0].holds(self):
             if torch.cuda.is_available() and torch.cuda.is_current_stream_capturing():
                 return None                     # making copies to the GPU: not while a graph is recorded
-            watch = ModelWatch(self)            # first: what changes meanwhile is seen at the next call
+            # the watch first (of the other path where that still holds): what changes meanwhile is seen next time
+            watch = next((w for w, _ in list(made.values()) if w.holds(self)), None) or ModelWatch(self)
             kept = made[name] = (watch, make(self))
         return None if kept[0].hooked() else kept[1]
 

@@ -80,8 +80,8 @@ class ModelWatch:
         """Whether somebody wants to hear of a call that those paths do not make."""
         return any(self.hooks)
 
-    def holds(self):
-        return (all(map(operator.is_, map(dict.get, self.dicts, self.keys), self.values))
+    def holds(self, model):
+        return (self.top is model._modules and all(map(operator.is_, map(dict.get, self.dicts, self.keys), self.values))
                 and len(self.blocks) == self.n_blocks
                 and list(map(torch.Tensor.data_ptr, self.tensors)) == self.addresses)
 
