@@ -14,7 +14,6 @@
 #include "add_layernorm_sm100.cuh"
 #include "cache_write_sm100.cuh"
 #include "fa_decode_sm100.cuh"
-#include "fa_fwd_double_sm100.cuh"
 #include "fa_fwd_sm100.cuh"
 #include "gpt_step_sm100.cuh"
 #include "linear_small_sm100.cuh"
@@ -86,23 +85,6 @@ FwdKernel fwd_kernel(int schedule, bool causal, bool ragged, bool is_long = fals
          : schedule == fa::kStatic ? fwd_kernel_of<fa::kStatic>(causal, ragged) : fwd_kernel_of<fa::kDynamic>(causal, ragged);
 }
 
-FwdKernel fwd_double_kernel(bool causal, bool ragged) {
-  if (causal) return &fa::fa_fwd_double_kernel<true, false, 128>;
-  return ragged ? &fa::fa_fwd_double_kernel<false, true, 128> : &fa::fa_fwd_double_kernel<false, false, 128>;
-}
-
-// What every attention kernel needs before its first launch: see init_device.
-int ready_fwd(const void* fn, size_t smem) {
-  cudaFuncAttributes fattr;
-  cudaError_t e = cudaFuncGetAttributes(&fattr, fn);
-  if (e != cudaSuccess) return static_cast<int>(e);
-  if (fattr.numRegs != fa::kLaunchRegs) return FA_B200_ERR_BUILD;
-  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  if (e != cudaSuccess) return static_cast<int>(e);
-  // CTAs of 100 KB and more must fit: ask for the largest shared-memory carveout.
-  return static_cast<int>(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-}
-
 // Runs once per device, with that device current.
 void init_device(int dev) {
   DeviceState& st = g_dev[dev];
@@ -121,7 +103,16 @@ void init_device(int dev) {
     for (int schedule : {fa::kOneItem, fa::kDynamic}) variants[i++] = reinterpret_cast<const void*>(fwd_kernel(schedule, true, false, true));
   }
   for (const void* fn : variants) {
-    if ((st.init_error = ready_fwd(fn, fa::kSmemBytes)) != 0) return;
+    cudaFuncAttributes fattr;
+    e = cudaFuncGetAttributes(&fattr, fn);
+    if (e != cudaSuccess) { st.init_error = static_cast<int>(e); return; }
+    if (fattr.numRegs != fa::kLaunchRegs) { st.init_error = FA_B200_ERR_BUILD; return; }
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, fa::kSmemBytes);
+    if (e != cudaSuccess) { st.init_error = static_cast<int>(e); return; }
+    // Two CTAs of ~100 KB each must fit: ask for the largest shared-memory carveout.
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) { st.init_error = static_cast<int>(e); return; }
     // Two CTAs per SM each allocate half of tensor memory; a third resident CTA would block in
     // tcgen05.alloc until one of them exits.  Shared memory already limits residency to two; make
     // sure of it (a build with a much smaller footprint would break that assumption).
@@ -130,8 +121,6 @@ void init_device(int dev) {
     if (e != cudaSuccess) { st.init_error = static_cast<int>(e); return; }
     if (resident < 1 || resident > fa::kCtasPerSm) { st.init_error = FA_B200_ERR_BUILD; return; }
   }
-  for (int mask : {0, 1, 2})
-    if ((st.init_error = ready_fwd(reinterpret_cast<const void*>(fwd_double_kernel(mask == 2, mask == 1)), fa::kDoubleSmem<128>)) != 0) return;
   // The persistent grid is sized for kCtasPerSm per SM whatever the occupancy query answered: it
   // has been seen to answer 1 where the hardware co-schedules 2, and a CTA that has to wait for
   // a slot only starts later -- work items are partitioned by grid stride, no CTA waits on another.
@@ -285,7 +274,6 @@ struct FwdPlan {
   long long items;     // B * H * n_qtiles
   unsigned grid;       // launched
   bool early;          // let the next kernel of the stream start while this one runs
-  bool two_scores;     // one CTA per tile: as fa_fwd_double_kernel
 };
 
 FwdPlan plan_fwd(const fa_b200_params* p, const DeviceState& st) {
@@ -328,16 +316,10 @@ FwdPlan plan_fwd(const fa_b200_params* p, const DeviceState& st) {
   //   14.4 / 15.2 / 20.6, but 328 items 14.3 / 13.4; N = 640, 330 items 10.5 / 11.3 / 16.5).
   pl.early = pl.kv_tiles == 1 || 4 * pl.items <= st.sm_count || pl.schedule == fa::kDynamic ||
              (causal ? pl.kv_tiles <= 8 && pl.items >= slots + 16 * (pl.kv_tiles - 3) : pl.items > st.sm_count);
-  // A tile to an SM at most: the form that takes all of its tensor memory, from four K/V tiles on.  us, with two CTAs'
-  // worth / with all of it: N = 512 causal, 12 heads 7.4 / 7.3; 700 full, 24 heads 10.2 / 9.5; 1024 causal, 12 heads 11.9 /
-  // 11.1; 3000 full, 4 heads 29.0 / 26.0; 16384 causal, 1 head 132.9 / 123.1; but N = 300 causal, 12 heads 6.1 / 6.1, 200
-  // full, 48 heads 5.6 / 5.7.
-  pl.two_scores = pl.schedule == fa::kOneItem && pl.kv_tiles > 3 && pl.items <= st.sm_count;
 #ifdef FA_WAIT_TEST    // the test's problem, one causal head of two tiles, as one CTA: what waits for what is then known
   if (causal && p->B * p->H == 1 && pl.n_qtiles == 2) {
     pl.schedule = fa::kStatic;
     pl.grid = 1;
-    pl.two_scores = false;
   }
 #endif
   return pl;
@@ -431,9 +413,8 @@ int fa_b200_fwd(const fa_b200_params* p) {
   kp.div_last_group = fa::make_fast_div(static_cast<uint32_t>(kp.last_group));
   const cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   const bool ragged = (p->N % fa::kBlockN) != 0;   // non-causal only: the causal mask covers the columns past N
-  const FwdKernel kernel = pl.two_scores ? fwd_double_kernel(kp.causal != 0, ragged) : fwd_kernel(pl.schedule, kp.causal != 0, ragged, kp.causal != 0 && p->N >= kLongRows);
-  return static_cast<int>(launch_kernel(kernel, dim3(pl.grid), fa::kNumThreads, pl.two_scores ? fa::kDoubleSmem<128> : fa::kSmemBytes,
-                                        stream, 1, mq, mk, mv, mo, kp));
+  const FwdKernel kernel = fwd_kernel(pl.schedule, kp.causal != 0, ragged, kp.causal != 0 && p->N >= kLongRows);
+  return static_cast<int>(launch_kernel(kernel, dim3(pl.grid), fa::kNumThreads, fa::kSmemBytes, stream, 1, mq, mk, mv, mo, kp));
 }
 
 int fa_b200_fwd_plan(const fa_b200_params* p, int32_t* schedule, int32_t* grid) {
