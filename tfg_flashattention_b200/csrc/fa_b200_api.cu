@@ -288,8 +288,9 @@ FwdPlan plan_fwd(const fa_b200_params* p, const DeviceState& st) {
   // * Items of up to 4 K/V tiles that make less than two rounds, or of one: static.  (B=8 H=16 N=300,
   //   384 items: 8.5 us, dynamic 9.0, one item 10.3; B=4 H=25 N=512 non-causal: 14.1 against 16.0: who
   //   takes over an item does not know who else is on the SM.)
-  //   Two K/V tiles also between 2.1 and 2.7 rounds: static / dynamic at 2.2 rounds N=130 causal 10.0 / 11.9 us, N=200 10.4 /
-  //   12.2, full 13.1 / 15.1; at 2.6 10.8 / 12.5 and 15.2 / 15.3; but at 3.0 12.8 / 12.5 and 17.8 / 15.9.
+  //   Two K/V tiles up to 2.7 rounds: static / dynamic at 2.0 rounds N=130 causal 8.9 / 9.4 us, N=200 9.0 / 9.4, full 11.6-11.8 /
+  //   11.7-11.8; at 2.07 10.0 / 11.9, 10.3 / 11.9, 13.0 / 14.2-15.0; at 2.2 10.0 / 11.9, 10.4 / 12.2, 13.1 / 15.1; at 2.6 N=200 10.8 /
+  //   12.5 and 15.2 / 15.3; but at 3.0 12.8 / 12.5 and 17.8 / 15.9.
   // * Otherwise dynamic (B=32 H=25 N=777: 139 us, static 170, one item 191), except
   //   - non-causal sequences above 3072: one CTA per item, whose tile loop is the smallest code
   //     (B=4 H=25 N=8192: 1.94 ms, dynamic 2.12);
@@ -298,7 +299,7 @@ FwdPlan plan_fwd(const fa_b200_params* p, const DeviceState& st) {
   pl.schedule = fa::kOneItem;
   if (pl.items > slots * fa::kItemTable) {
   } else if (pl.kv_tiles == 1 || (pl.kv_tiles <= 4 && pl.items < 2 * slots) ||
-             (pl.kv_tiles == 2 && 10 * pl.items >= 21 * slots && 11 * pl.items <= 30 * slots)) {
+             (pl.kv_tiles == 2 && 11 * pl.items <= 30 * slots)) {
     if (pl.items > slots) pl.schedule = fa::kStatic;
   } else if (3 * pl.items >= 4 * slots && (causal || pl.kv_tiles <= 24)) {
     pl.schedule = fa::kDynamic;
