@@ -123,13 +123,18 @@ def test_two_tiles_above_two_rounds(fa_lib, items, causal):
 @pytest.mark.parametrize("N,heads", [(12287, 3), (12288, 3), (12300, 3), (12416, 6)])      # the border; one CTA per tile, taken over
 def test_long_causal_rows_are_those_of_a_shorter_sequence(fa_lib, N, heads):
     """Long causal sequences have the diagonal tile behind the tile loop: row for row the bits of the same rows in a
-    sequence that has it inside."""
+    sequence that has it inside.  Which of the two is launched: fa_fwd_kernel's template arguments (schedule, causal, ragged,
+    long)."""
     from tfg_flashattention_b200 import custom_flash_attn as cfa
     g = torch.Generator(device="cuda").manual_seed(N)
     q, k, v = (torch.randn(1, heads, N, 64, device="cuda", generator=g).bfloat16() for _ in range(3))
     k[:, :, ::701] *= 5
     o, lse = cfa.forward(q, k, v, return_lse=True, out=torch.full_like(q, float("nan")))
     assert cfa.last_status() == 0 and torch.isfinite(o).all() and torch.isfinite(lse).all()
+    one_item = cfa.plan(q, k, v)[0] == "cta_per_tile"
+    assert one_item == (heads == 3)
+    name, _ = _launched(lambda: cfa.forward(q, k, v, out=torch.empty_like(q)))
+    assert f"fa_fwd_kernelILi{0 if one_item else 2}ELb1ELb0ELb{int(N >= 12288)}EEEv" in name
     short, short_lse = cfa.forward(q[:, :, :12200], k[:, :, :12200], v[:, :, :12200], return_lse=True)
     assert torch.equal(o[:, :, :12200], short) and torch.equal(lse[:, :, :12200], short_lse)
 
