@@ -22,9 +22,17 @@ WATCHDOG_BASE = 0x10000
 # microsecond or two of each other, so which one runs out first -- and gets to write the word -- is
 # a matter of that microsecond; any of the three is the right report.
 EXPECTED_WAITS = {2: b"K/V tile load", 9: b"Q slot", 4: b"S = QK^T"}
+# The 96 CTAs of a long sequence, one tile each: the producer has more to load and stops at the slot of V 0 instead (3).
+EXPECTED_WAITS_LONG = {2: b"K/V tile load", 3: b"K/V slot", 4: b"S = QK^T"}
 
 
-def test_wait_runs_out_is_reported_and_the_next_launch_is_correct(fa_lib):
+@pytest.mark.parametrize("N,product,test_build,expected", [
+    # two causal tiles; the test build runs them as one CTA, whose first item needs two K tiles
+    (256, ("cta_per_tile", 2), ("static", 1), EXPECTED_WAITS),
+    # the form with the diagonal tile behind the tile loop; every CTA but the first tile's needs the missing K tile
+    (12288, ("cta_per_tile", 96), ("cta_per_tile", 96), EXPECTED_WAITS_LONG),
+])
+def test_wait_runs_out_is_reported_and_the_next_launch_is_correct(fa_lib, N, product, test_build, expected):
     if not torch.cuda.is_available():
         pytest.fail("GPU tests need a CUDA device")
     from tfg_flashattention_b200 import _lib, build
@@ -38,14 +46,13 @@ def test_wait_runs_out_is_reported_and_the_next_launch_is_correct(fa_lib):
     wt.fa_b200_strerror.restype = ctypes.c_char_p
 
     torch.manual_seed(3)
-    # B = H = 1, N = 256: two causal tiles; the test build runs them as one CTA, whose first item needs two K tiles
-    q, k, v = (torch.randn(1, 1, 256, 64, device="cuda").bfloat16() for _ in range(3))
-    assert cfa.plan(q, k, v) == ("cta_per_tile", 2)
+    q, k, v = (torch.randn(1, 1, N, 64, device="cuda").bfloat16() for _ in range(3))
+    assert cfa.plan(q, k, v) == product
     schedule, grid = ctypes.c_int32(-1), ctypes.c_int32(0)
     params = cfa._fwd_params(q, k, v, q, None, True, None)
     wt.fa_b200_fwd_plan.argtypes = [ctypes.POINTER(_lib.FaParams), ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(ctypes.c_int32)]
     assert wt.fa_b200_fwd_plan(ctypes.byref(params), ctypes.byref(schedule), ctypes.byref(grid)) == 0
-    assert (_lib.SCHEDULES[schedule.value], grid.value) == ("static", 1)
+    assert (_lib.SCHEDULES[schedule.value], grid.value) == test_build
     good = cfa.forward(q, k, v)
     assert cfa.last_status() == 0
 
@@ -56,9 +63,9 @@ def test_wait_runs_out_is_reported_and_the_next_launch_is_correct(fa_lib):
     assert wt.fa_b200_fwd(ctypes.byref(p)) == 0          # the launch itself succeeds
     code = wt.fa_b200_last_status(0, stream)             # synchronises: the kernel has returned
     elapsed = time.perf_counter() - t0
-    assert code & ~0xff == WATCHDOG_BASE and (code & 0xff) in EXPECTED_WAITS, hex(code)
+    assert code & ~0xff == WATCHDOG_BASE and (code & 0xff) in expected, hex(code)
     message = wt.fa_b200_strerror(code)
-    assert b"watchdog" in message and EXPECTED_WAITS[code & 0xff] in message
+    assert b"watchdog" in message and expected[code & 0xff] in message
     assert elapsed < 2.0, f"the kernel took {elapsed:.2f} s to give up"
     assert wt.fa_b200_last_status(0, stream) == 0        # reading the word cleared it
 
