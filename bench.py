@@ -922,7 +922,7 @@ def main():
                          "unit": "TFLOP/s", "frac": per_gpu / peaks["bf16_tflops"],
                          "traffic": NCU_TRAFFIC_BYTES_PER_LAUNCH, "traffic_note": NCU_TRAFFIC_NOTE,
                          "peak_source": f"of {peaks['source']}",
-                         "algorithmic_bytes": w.bytes(), "kernel": "fa::fa_fwd_kernel<2, true, false> (dynamic schedule, causal)",
+                         "algorithmic_bytes": w.bytes(), "kernel": "fa::fa_fwd_kernel<2, true, false, false> (dynamic schedule, causal)",
                          "burst": burst, "sustained": sustained},
             "e2e": dict({"value": e2e_value, "unit": UNIT, "ms_per_step": e2e_ms,
                          "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h}, **e2e_detail),

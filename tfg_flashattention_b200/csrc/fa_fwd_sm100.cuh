@@ -31,8 +31,12 @@
 //
 // Every mbarrier wait is bounded: a wait that exceeds kWaitLimitNs records a code in the status
 // word, raises the CTA's abort flag, and every role drains and leaves through the normal exit
-// (TMEM is freed).  Nothing traps and nothing spins without a limit.  The one hardware wait
-// without a limit, setmaxnreg.inc, is made safe by the static register budget below.
+// (TMEM is freed).  Nothing traps and nothing spins without a limit.  Two hardware waits have none:
+// setmaxnreg.inc, made safe by the static register budget below, and tcgen05.alloc.  Two CTAs of this file
+// have room for their columns on an SM and a third does not start there (its shared memory), so an
+// allocation waits only where another library's kernel holds more than half of the SM's columns, until that
+// CTA ends.  A kernel that is started early behind this one cannot be what it waits for: that start is let go
+// behind the allocation.
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>

@@ -778,7 +778,7 @@ __device__ __forceinline__ StepCta step_attention(StepCta c, const StepParams& p
     // A GPT-2 XL unit of 900 rows, clocks: 8900 with one maximum per warp and waits for all stages, 7500 so.
     // A stage goes back as soon as its rows are in registers: the stream of rows, not the arithmetic, is what the
     // longer caches wait for.  us per step, given back behind the arithmetic / so: GPT-2 small 8 x 900 rows 228 / 223,
-    // medium 8 x 600 447 / 440, XL 8 x 900 1471 / 1460, 4 x 500 960 / 952; two blocks at a time on top: 231, 449, 1499, 958.
+    // medium 8 x 600 446 / 439, XL 8 x 900 1467 / 1457, 4 x 500 944 / 940; two blocks at a time on top: 231, 449, 1499.
     {
       const int stages = (un.rows + kStepBlocks * 16 - 1) / (kStepBlocks * 16);
       const uint32_t own = (c.ring.stage & 1) == warp / kStepBlocks ? 0 : 1;
